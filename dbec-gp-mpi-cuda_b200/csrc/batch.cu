@@ -168,7 +168,7 @@ gpe_status build_tables(gpe_batch *b) {
          for (int a = 0; a < 3; a++) {
             A.mseg[a] = std::max(A.mseg[a], g.mseg[a]);
             A.stage[a] = std::max(A.stage[a], g.stage[a]);
-            A.blk[a] = std::max(A.blk[a], g.blk[a]);
+            A.xch[a] = std::max(A.xch[a], g.xch[a]);
             A.extra[a] = std::max(A.extra[a], g.extra[a]);
          }
          A.part = std::max(A.part, g.part);
@@ -178,12 +178,12 @@ gpe_status build_tables(gpe_batch *b) {
       // sweeps: 2-stage pipelines; as many CTAs per SM as shared memory and
       // the kernels' register budget allow
       for (int a = 0; a < 3; a++) {
-         size_t sm = 128 + 2 * (size_t) A.stage[a] + A.blk[a] + A.extra[a];
+         size_t sm = 128 + 2 * (size_t) A.stage[a] + A.xch[a] + A.extra[a];
          if (a == 2) sm += 2 * (size_t) A.part;
          if (sm > kSmemCap) return bfail(GPE_ERR_PARAM, "batch: sweep tiles exceed shared memory");
-         // the kernels' register budget holds kSweepCtas CTAs of 256 threads,
+         // the kernels' register budget holds cap0 CTAs of 256 threads,
          // so more of fewer threads
-         const int cap0 = a == 0 ? kSweepCtas[1] : kSweepCtas[0];
+         const int cap0 = sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32));
          const int cap = std::max(1, std::min(32, 256 * cap0 / std::max(32, (int) A.threads[kPXsweep + a])));
          const int ctas = std::max(1, std::min(cap, (int) (kSmemCap / sm)));
          G.sweep_smem[a] = sm;
@@ -284,20 +284,20 @@ template <class R, bool CPLX> struct BatchStep {
       BCKS(with_mseg(A.mseg[0], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
          return launch(kb_sweep_xy<R, CPLX, 0, true, M, 2>, (unsigned) G.sweep_grid[0], A.threads[kPXsweep],
-                       G.sweep_smem[0], st, tab, S(kPXsweep), (int) A.tiles[kPXsweep], A.stage[0], A.blk[0]);
+                       G.sweep_smem[0], st, tab, S(kPXsweep), (int) A.tiles[kPXsweep], A.stage[0], A.xch[0]);
       }));
       BCKS(mark(kPXsweep));
       BCKS(with_mseg(A.mseg[1], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
          return launch(kb_sweep_xy<R, CPLX, 1, false, M, 2>, (unsigned) G.sweep_grid[1], A.threads[kPYsweep],
-                       G.sweep_smem[1], st, tab, S(kPYsweep), (int) A.tiles[kPYsweep], A.stage[1], A.blk[1]);
+                       G.sweep_smem[1], st, tab, S(kPYsweep), (int) A.tiles[kPYsweep], A.stage[1], A.xch[1]);
       }));
       BCKS(mark(kPYsweep));
       BCKS(with_mseg(A.mseg[2], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
          constexpr int MOM = CPLX ? 0 : 1;
          return launch(kb_sweep_z<R, CPLX, MOM, M, 2>, (unsigned) G.sweep_grid[2], A.threads[kPZsweep],
-                       G.sweep_smem[2], st, tab, S(kPZsweep), (int) A.tiles[kPZsweep], A.stage[2], A.blk[2],
+                       G.sweep_smem[2], st, tab, S(kPZsweep), (int) A.tiles[kPZsweep], A.stage[2], A.xch[2],
                        A.part);
       }));
       BCKS(mark(kPZsweep));

@@ -71,7 +71,7 @@ struct BatchGeom {
    int zppt;                 // points per thread of the z passes
    int mseg[3];              // compile-time segment bound of each sweep
    uint32_t stage[3];        // sweeps: bytes of one pipeline stage
-   uint32_t blk[3];          // sweeps: bytes of the block maps
+   uint32_t xch[3];          // sweeps: bytes of the exchange buffer
    uint32_t extra[3];        // sweeps: FP64 tables (x: calcnu table; z: coefficient tables)
    uint32_t part;            // z sweep: bytes of one Simpson partial array
    int Ly, Lx;               // the instance's own FFT tile widths
@@ -192,19 +192,19 @@ __device__ __forceinline__ void copy_view(SweepView &dst, const SweepView &src) 
 }
 
 template <class R, bool CPLX, int AXIS, bool NU, int MSEG, int S>
-__global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) kb_sweep_xy(const BatchDesc *__restrict__ tab,
+__global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_xy(const BatchDesc *__restrict__ tab,
                                                                            const unsigned *__restrict__ work,
                                                                            int ntiles, uint32_t stage_bytes,
-                                                                           uint32_t blk_bytes) {
+                                                                           uint32_t xch_bytes) {
    using P = typename Tr<R, CPLX>::P;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t full[S];
    __shared__ __align__(16) SweepView sv;
    constexpr int E = CPLX ? 2 : 1;
-   // layout: S stages of (tile | phi tile) | block maps | FP64 calcnu table
+   // layout: S stages | exchange buffer | FP64 calcnu table
    unsigned char *base = (unsigned char *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
-   P *blk = (P *) (base + S * stage_bytes);
-   double *xtab = (double *) ((unsigned char *) blk + blk_bytes);
+   P *xch = (P *) (base + S * stage_bytes);
+   double *xtab = (double *) ((unsigned char *) xch + xch_bytes);
    // tile t of the work list: its instance and its place in that instance
    int acq = -1;  // thread 0: the instance whose tensor maps it last acquired
    auto copy_tile = [&](int t, int q, bool load) {
@@ -213,8 +213,9 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) kb_sweep_xy(const
       const SweepView &v = D.sv[AXIS];
       const int TW = v.TW, rows = v.boxn * v.nbox, nzb = (v.d.nz + TW - 1) / TW;
       const int other = r.local / nzb, z0 = (r.local - other * nzb) * TW;
-      P *tile = (P *) (base + q * stage_bytes);
-      R *ptile = (R *) (tile + rows * TW);
+      const XyStage lay = xy_stage<R, CPLX, NU>(rows, TW, v.tb.skip);
+      P *tile = (P *) (base + q * stage_bytes + lay.psi);
+      R *ptile = (R *) (base + q * stage_bytes + lay.phi);
       const CUtensorMap *tm_psi = &D.tm_psi[AXIS];
       if (r.inst != acq) {
          tmap_acquire(tm_psi);
@@ -265,8 +266,7 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) kb_sweep_xy(const
          copy_view(sv, D.sv[AXIS]);
          if constexpr (NU && AXIS == 0 && std::is_same<R, double>::value) {
             const SweepView &v = D.sv[AXIS];
-            const double *src = (const double *) v.lin.ex;
-            for (int e = threadIdx.x; e < (CPLX ? 2 : 1) * v.tb.n; e += blockDim.x) xtab[e] = src[e];
+            stage_xtab<CPLX>(xtab, v.lin.ex, v.tb.n, v.tb.skip);
          }
          cur = i;
       }
@@ -274,21 +274,17 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) kb_sweep_xy(const
       const int TW = sv.TW, rows = sv.boxn * sv.nbox, nzb = (sv.d.nz + TW - 1) / TW;
       const int lg = __ffs(TW) - 1;
       const int c = threadIdx.x & (TW - 1), p = threadIdx.x >> lg;
-      const int other = r.local / nzb, z0 = (r.local - other * nzb) * TW;
-      P *tile = (P *) (base + q * stage_bytes);
-      const double scale = NU ? sv.st->scale : 1.;
-      if constexpr (NU && std::is_same<R, double>::value) {
-         nu_pass_fp64<R, CPLX, AXIS>(tile, (const R *) (tile + rows * TW), sv.tb.n, lg, c, other, z0, sv.d, sv.trap,
-                                     sv.lin, xtab, sv.g, sv.gd, sv.dt, scale);
-         __syncthreads();
-      }
-      if constexpr (NU && std::is_same<R, float>::value) {
+      const XyStage lay = xy_stage<R, CPLX, NU>(rows, TW, sv.tb.skip);
+      P *col = (P *) (base + q * stage_bytes + lay.psi) + c;
+      if constexpr (NU) {
          static_assert(AXIS == 0, "calcnu is fused into the x sweep only");
-         const NuTrap32<CPLX> xf = nu_reads_fp32<CPLX>((const float *) (tile + rows * TW) + c, TW, other, z0, c, sv.d,
-                                                       sv.trap, sv.lin, sv.g, sv.gd, sv.dt, scale);
-         seg_sweep<R, CPLX, MSEG, 0>(tile, TW, 1, c, p, TW, sv.tb, blk, nullptr, nullptr, nullptr, nullptr, xf);
+         const int other = r.local / nzb, z0 = (r.local - other * nzb) * TW;
+         seg_sweep_any<R, CPLX, MSEG, false, false, 0>(
+             col, TW, p, sv.tb, xch + c, TW,
+             nu_xf<R, CPLX>((R *) (base + q * stage_bytes + lay.phi) + c, TW, other, z0, c, sv.d, sv.trap, sv.lin,
+                            xtab + E * sv.tb.skip, sv.g, sv.gd, sv.dt, sv.st->scale));
       } else {
-         seg_sweep<R, CPLX, MSEG, 0>(tile, TW, 1, c, p, TW, sv.tb, blk, nullptr, nullptr);
+         seg_sweep_any<R, CPLX, MSEG, false, false, 0>(col, TW, p, sv.tb, xch + c, TW, NoXf());
       }
       fence_proxy_async();
       __syncthreads();
@@ -298,23 +294,22 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) kb_sweep_xy(const
 }
 
 template <class R, bool CPLX, int MOM, int MSEG, int S>
-__global__ void __launch_bounds__(256, kSweepCtas[0]) kb_sweep_z(const BatchDesc *__restrict__ tab,
+__global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_z(const BatchDesc *__restrict__ tab,
                                                                  const unsigned *__restrict__ work, int ntiles,
-                                                                 uint32_t stage_bytes, uint32_t blk_bytes,
+                                                                 uint32_t stage_bytes, uint32_t xch_bytes,
                                                                  uint32_t part_bytes) {
    using P = typename Tr<R, CPLX>::P;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t full[S];
    __shared__ __align__(16) SweepView sv;
-   // layout: S stages of rows | block maps | Simpson partials (2 arrays) | FP64 tables
+   // layout: S stages of rows | exchange buffer | Simpson partials (2 arrays) | FP64 tables
    unsigned char *base = (unsigned char *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
-   P *blk = (P *) (base + S * stage_bytes);
-   double *part = (double *) ((unsigned char *) blk + blk_bytes);
+   P *xch = (P *) (base + S * stage_bytes);
+   double *part = (double *) ((unsigned char *) xch + xch_bytes);
    double *part2 = (double *) ((unsigned char *) part + part_bytes);
    double *tabs = (double *) ((unsigned char *) part2 + part_bytes);
    // FP64: the coefficient tables staged in shared memory, as k_sweep_z does
    constexpr bool STAB = std::is_same<R, double>::value;
-   constexpr int TE = CPLX ? 2 : 1;
    // one bulk copy per row, issued by the 32 lanes of warp 0 (the short rows
    // of small grids make many small copies); every lane commits and waits
    // for its own store groups
@@ -326,7 +321,7 @@ __global__ void __launch_bounds__(256, kSweepCtas[0]) kb_sweep_z(const BatchDesc
       const long long r0 = (long long) r.local * TR;
       const int nr = (int) ((v.d.nxy - r0) < TR ? (v.d.nxy - r0) : TR);
       const uint32_t row_bytes = (uint32_t) (nz * sizeof(P));
-      P *tile = (P *) (base + q * stage_bytes);
+      P *tile = (P *) (base + q * stage_bytes) + zrow_pad(v.tb.skip, (int) sizeof(P));
       if (load && lane == 0) mbar_arrive_expect_tx(&full[q], row_bytes * nr);
       __syncwarp();
       for (int rr = lane; rr < nr; rr += 32) {
@@ -344,6 +339,7 @@ __global__ void __launch_bounds__(256, kSweepCtas[0]) kb_sweep_z(const BatchDesc
    if (threadIdx.x < 32 && (int) blockIdx.x < ntiles) copy_tile(blockIdx.x, 0, true);
    int cur = -1;
    int it = 0;
+   SegTab tbs{};
    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, it++) {
       const int q = it % S;
       if (threadIdx.x < 32 && t + (int) gridDim.x < ntiles) {
@@ -357,29 +353,17 @@ __global__ void __launch_bounds__(256, kSweepCtas[0]) kb_sweep_z(const BatchDesc
          __syncthreads();
          const SweepView &v = tab[i].sv[2];
          copy_view(sv, v);
-         if constexpr (STAB) {
-            const void *src[4] = {v.tb.al, v.tb.ga, v.tb.M, v.tb.N};
-            for (int a = 0; a < 4; a++)
-               for (int e = threadIdx.x; e < v.tb.n * TE; e += blockDim.x)
-                  tabs[a * v.tb.n * TE + e] = ((const double *) src[a])[e];
-         }
+         tbs = v.tb;
+         if constexpr (STAB) tbs = stage_segtab<CPLX>(tabs, v.tb);
          cur = i;
       }
       if (__syncthreads_or(!mbar_wait(&full[q], (it / S) & 1, tab[i].err))) break;
-      SegTab tbs = sv.tb;
-      if constexpr (STAB) {
-         const int nn = sv.tb.n * TE;
-         tbs.al = tabs;
-         tbs.ga = tabs + nn;
-         tbs.M = tabs + 2 * nn;
-         tbs.N = tabs + 3 * nn;
-      }
       const int TR = sv.TW;
       const int c = threadIdx.x % TR, p = threadIdx.x / TR;
       const long long r0 = (long long) r.local * TR;
       const int nr = (int) ((sv.d.nxy - r0) < TR ? (sv.d.nxy - r0) : TR);
-      P *tile = (P *) (base + q * stage_bytes);
-      zsweep_tile<R, CPLX, MOM, MSEG, 0, STAB>(tile, nr, TR, sv.LS, c, p, tbs, blk, part, part2, sv.wz, sv.wz2, sv.hz3,
+      P *rows = (P *) (base + q * stage_bytes) + zrow_pad(sv.tb.skip, (int) sizeof(P));
+      zsweep_tile<R, CPLX, MOM, MSEG, STAB, true>(rows, nr, TR, sv.LS, c, p, tbs, xch, part, part2, sv.wz, sv.wz2, sv.hz3,
                                                sv.rowsum, sv.rowsum2, r0);
       if (threadIdx.x < 32) copy_tile(t, q, false);
    }

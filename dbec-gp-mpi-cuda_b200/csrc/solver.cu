@@ -101,10 +101,8 @@ struct gpe_solver {
       size_t smem = 0;
       CUtensorMap tm_psi{}, tm_phi{};
       SegTab tab{};
-      void *M = nullptr, *N = nullptr;
-      // mixed precision: alpha, gamma, M, N rounded once to FP32 (the values
-      // the FP32 sweeps would otherwise round from the FP64 tables at every use)
-      void *t32[4] = {nullptr, nullptr, nullptr, nullptr};
+      // coefficient tables (FP64, or rounded once to FP32 in mixed precision)
+      void *tabs[3] = {nullptr, nullptr, nullptr};
    } sw[3];
    double *wz = nullptr;      // Simpson weights along z (norm partials)
    double *wz2 = nullptr;     // wz[k] * z[k]^2 (rms partials)
@@ -119,6 +117,10 @@ struct gpe_solver {
 // rms samples gpe_run keeps on the device before copying them out (a run with
 // more samples copies every full batch of slots while it continues)
 constexpr long kRmsSlots = 256;
+
+// zero entries before index 0 of the tables the sweeps index from the rows
+// below a line (at least the longest segment)
+constexpr int kTabPad = 32;
 
 static void mark(gpe_solver *s) {
    if (s->prof_ev && s->prof_i < s->prof_cap) cudaEventRecord(s->prof_ev[s->prof_i++], s->st);
@@ -247,92 +249,92 @@ static gpe_status make_coef(gpe_solver *s, int ax, long n, double d2) {
    return GPE_OK;
 }
 
-// Segment tables of the parallel Thomas sweep of axis ax (line length n,
-// segment length m, P segments; the last segment ends at n-3):
-//   M[i] = prod_{j=i+1}^{H_p+1} gamma[j] A   for i in segment p < P-1
-//   N[k] = prod_{j=lo_p}^{k-1} alpha[j]       for k in (lo_p, hf_p + 1]
+// Segment tables of the parallel Thomas sweep of axis ax (line length n, P
+// segments of m points; segment p holds recurrence indices lo .. lo + m - 1,
+// lo = p m - skip, zero coefficients below index 0):
+//   M[i] = prod_{j=i+1}^{lo+m} gamma[j] A   in every segment but the top one
+//   N[k] = prod_{j=lo}^{k-1} alpha[j]        for k in (lo, lo + m], but the bottom one
 // computed in long double and rounded once.
-static gpe_status make_segtab(gpe_solver *s, int ax, long n, double d2, int m, int P) {
+static gpe_status make_segtab(gpe_solver *s, int ax, long n, int m, int P) {
    // the z sweep's Simpson partials take the weight of a point from its
    // parity within the segment, so segments start at even indices
-   if (m % 2) return fail(GPE_ERR_PARAM, "segment length must be even");
+   if (m % 2 || n % 2) return fail(GPE_ERR_PARAM, "segment and line lengths must be even");
    typedef std::complex<long double> Z;
-   const long double c = (long double) s->p.dt / (long double) d2 / (3.L - (long double) s->par);
-   Z A0, A;
-   if (!s->cplx) { A0 = 1.L + c; A = -0.5L * c; }
-   else { A0 = Z(1.L, c); A = Z(0.L, -0.5L * c); }
+   const int E = s->cplx ? 2 : 1;
    // coefficients as uploaded (double), promoted: the tables multiply exactly those
    std::vector<Z> al(n - 1), ga(n - 1);
    {
-      std::vector<double> ad((size_t) (s->cplx ? 2 : 1) * (n - 1)), gd((size_t) (s->cplx ? 2 : 1) * (n - 1));
+      std::vector<double> ad((size_t) E * (n - 1)), gd((size_t) E * (n - 1));
       CK(cudaMemcpy(ad.data(), s->alpha[ax], sizeof(double) * ad.size(), cudaMemcpyDeviceToHost));
       CK(cudaMemcpy(gd.data(), s->gamma[ax], sizeof(double) * gd.size(), cudaMemcpyDeviceToHost));
       for (long i = 0; i < n - 1; i++) {
          al[i] = s->cplx ? Z(ad[2 * i], ad[2 * i + 1]) : Z(ad[i], 0.L);
          ga[i] = s->cplx ? Z(gd[2 * i], gd[2 * i + 1]) : Z(gd[i], 0.L);
       }
-      const double2 Ad = s->A[ax];
-      A = Z(Ad.x, Ad.y);
    }
-   std::vector<Z> M(n, Z(0)), N(n, Z(0));
+   const Z A(s->A[ax].x, s->A[ax].y);
+   const long skip = (long) P * m - (n - 2), ne = (long) P * m;
+   std::vector<Z> tg(ne, Z(0)), tma(2 * ne, Z(0)), tn(ne, Z(0));
+   long double amax = 0, nmax = 0;  // largest decay of a segment's backward and forward map
    for (int p = 0; p < P; p++) {
-      const long lo = (long) p * m;
-      const bool top = p == P - 1;
-      const long hf = top ? n - 3 : lo + m - 1;
-      if (!top) {
-         Z r = 1;
-         for (long i = hf; i >= lo; i--) { r *= ga[i + 1] * A; M[i] = r; }
-      }
+      const long lo = (long) p * m - skip;
+      const long q0 = std::max(0L, -lo);
       Z r = 1;
-      for (long i = lo; i <= hf; i++) { r *= al[i]; N[i + 1] = r; }
-   }
-   if (!s->cplx) {
-      std::vector<double> a(n), b(n);
-      for (long i = 0; i < n; i++) { a[i] = (double) M[i].real(); b[i] = (double) N[i].real(); }
-      CKS(upload(&s->sw[ax].M, a.data(), n));
-      CKS(upload(&s->sw[ax].N, b.data(), n));
-   } else {
-      std::vector<double2> a(n), b(n);
-      for (long i = 0; i < n; i++) {
-         a[i] = make_double2((double) M[i].real(), (double) M[i].imag());
-         b[i] = make_double2((double) N[i].real(), (double) N[i].imag());
+      for (long q = m - 1; q >= q0; q--) {
+         const long e = (long) p * m + q, i = lo + q;
+         tg[e] = ga[i + 1];
+         r *= ga[i + 1] * A;
+         if (p < P - 1) tma[2 * e] = r;
+         tma[2 * e + 1] = al[i];
       }
-      CKS(upload(&s->sw[ax].M, a.data(), n));
-      CKS(upload(&s->sw[ax].N, b.data(), n));
-   }
-   SegTab &t = s->sw[ax].tab;
-   t.al = s->alpha[ax];
-   t.ga = s->gamma[ax];
-   t.M = s->sw[ax].M;
-   t.N = s->sw[ax].N;
-   if (s->fp32) {
-      // FP32 copies of the FP64 tables (alpha and gamma stay FP64 in HBM as
-      // computed; the FP32 kernels read these once-rounded copies).  In real
-      // time the gamma copy holds gamma + 1 (SegOps::back_step): gamma is -1
-      // plus a small number, which FP32 keeps to its own relative precision.
-      const void *src[4] = {s->alpha[ax], s->gamma[ax], s->sw[ax].M, s->sw[ax].N};
-      const size_t nd = (size_t) n * (s->cplx ? 2 : 1);
-      std::vector<double> h(nd);
-      std::vector<float> f(nd);
-      for (int q = 0; q < 4; q++) {
-         if (s->sw[ax].t32[q]) cudaFree(s->sw[ax].t32[q]);
-         s->sw[ax].t32[q] = nullptr;
-         CK(cudaMemcpy(h.data(), src[q], sizeof(double) * nd, cudaMemcpyDeviceToHost));
-         const bool shift = q == 1 && s->cplx;
-         for (size_t e = 0; e < nd; e++) f[e] = (float) (shift && e % 2 == 0 ? h[e] + 1. : h[e]);
-         CKS(upload(&s->sw[ax].t32[q], f.data(), nd));
+      if (p < P - 1) amax = std::max(amax, std::abs(r));
+      r = 1;
+      for (long q = q0; q < m; q++) {
+         r *= al[lo + q];
+         if (p > 0) tn[(long) p * m + q] = r;
       }
-      t.al = s->sw[ax].t32[0];
-      t.ga = s->sw[ax].t32[1];
-      t.M = s->sw[ax].t32[2];
-      t.N = s->sw[ax].t32[3];
+      if (p > 0) nmax = std::max(nmax, std::abs(r));
    }
+   // segments whose maps a thread composes: the carry from farther away is
+   // scaled by a product of D decays, dropped below 2^-64 (FP64) or 2^-40
+   // (FP32), under the rounding of the carry itself
+   const long double drop = s->fp32 ? ldexpl(1.L, -40) : ldexpl(1.L, -64), dec = std::max(amax, nmax);
+   int D = 1;
+   for (long double r = dec; D < P && r > drop; r *= dec) D++;
+   auto &w = s->sw[ax];
+   std::vector<Z> *src[3] = {&tg, &tma, &tn};
+   for (int q = 0; q < 3; q++) {
+      if (w.tabs[q]) cudaFree(w.tabs[q]);
+      w.tabs[q] = nullptr;
+      const std::vector<Z> &z = *src[q];
+      std::vector<double> h(z.size() * E);
+      for (size_t e = 0; e < z.size(); e++) {
+         h[E * e] = (double) z[e].real();
+         if (s->cplx) h[E * e + 1] = (double) z[e].imag();
+      }
+      if (s->fp32) {
+         // FP32 copies of the FP64 values (alpha and gamma stay FP64 in HBM
+         // as computed; the FP32 kernels read these once-rounded copies).  In
+         // real time the gamma copy holds gamma + 1 (SegOps::back_step):
+         // gamma is -1 plus a small number, which FP32 keeps to its own
+         // relative precision.
+         std::vector<float> f(h.size());
+         for (size_t e = 0; e < h.size(); e++) f[e] = (float) (q == 0 && s->cplx && e % 2 == 0 ? h[e] + 1. : h[e]);
+         CKS(upload(&w.tabs[q], f.data(), f.size()));
+      } else {
+         CKS(upload(&w.tabs[q], h.data(), h.size()));
+      }
+   }
+   SegTab &t = w.tab;
+   t.ga = w.tabs[0];
+   t.ma = w.tabs[1];
+   t.nn = w.tabs[2];
    t.A = s->A[ax];
-   t.A0r = s->A0r[ax];
-   t.mA = s->mA[ax];
    t.n = (int) n;
    t.m = m;
    t.P = P;
+   t.D = D;
+   t.skip = (int) skip;
    return GPE_OK;
 }
 
@@ -403,6 +405,15 @@ static int sweep_candidates(int n, int tw_base, int esz, int *TW, int *MSEG, int
    return k;
 }
 
+// Bytes of one pipeline stage of the x or y sweep.
+static size_t sweep_stage(const gpe_solver *s, int ax, int rows, int TW, int skip) {
+   if (s->fp32)
+      return s->cplx ? (ax == 0 ? xy_stage<float, true, true>(rows, TW, skip) : xy_stage<float, true, false>(rows, TW, skip)).bytes
+                     : (ax == 0 ? xy_stage<float, false, true>(rows, TW, skip) : xy_stage<float, false, false>(rows, TW, skip)).bytes;
+   return s->cplx ? (ax == 0 ? xy_stage<double, true, true>(rows, TW, skip) : xy_stage<double, true, false>(rows, TW, skip)).bytes
+                  : (ax == 0 ? xy_stage<double, false, true>(rows, TW, skip) : xy_stage<double, false, false>(rows, TW, skip)).bytes;
+}
+
 // Tile configuration of the sweeps and of the y / x FFT passes, and the FFT
 // plans: the heuristics below, or the values of s->tune where set.  May be
 // called again (gpe_set_tuning); it reuploads only the segment tables.
@@ -413,35 +424,33 @@ static gpe_status plan_tiles(gpe_solver *s) {
    const int E = s->cplx ? 2 : 1;
    const int tw_base = (int) (128 / esz);
    const long nn[3] = {d.nx, d.ny, d.nz};
-   const double h2[3] = {s->p.dx * s->p.dx, s->p.dy * s->p.dy, s->p.dz * s->p.dz};
    const size_t sm_cap = 227 * 1024;
    for (int ax = 0; ax < 3; ax++) {
       auto &w = s->sw[ax];
       // the widest tile for which as many CTAs as the kernels are compiled for
       // fit on an SM with a 2-stage pipeline (else the widest tile, fewer CTAs)
-      const int max_ctas = kSweepCtas[ax == 0 ? 1 : 0];
       int cTW[kSweepCand], cM[kSweepCand], cP[kSweepCand];
       bool prim[kSweepCand];
       const int nc = sweep_candidates((int) nn[ax], tw_base, (int) esz, cTW, cM, cP, prim);
-      auto sizes = [&](int TW, int P, size_t &stage, size_t &fixed) {
-         const int spw = 32 / TW;
-         const size_t blk = 2 * (size_t) ((P + spw - 1) / spw + 1) * TW * esz;
+      auto ctas_of = [&](int c) { return sweep_ctas(s->fp32, s->cplx, cM[c]); };
+      auto sizes = [&](int TW, int MS, int P, size_t &stage, size_t &fixed) {
+         const int skip = P * MS - (int) (nn[ax] - 2);
+         const size_t xch = (2 * (size_t) P * TW * esz + 15) & ~(size_t) 15;
          if (ax < 2) {
-            const long rows = (long) std::min<long>(nn[ax], 256) * ((nn[ax] + 255) / 256);
-            stage = (rows * TW * esz + (ax == 0 ? rows * TW * rsz : 0) + 127) & ~(size_t) 127;
+            const int rows = (int) (std::min<long>(nn[ax], 256) * ((nn[ax] + 255) / 256));
+            stage = sweep_stage(s, ax, rows, TW, skip);
             // FP64 x sweep: calcnu's per-x table staged in shared memory
-            fixed = 128 + blk + (ax == 0 && !s->fp32 ? (size_t) nn[0] * (s->cplx ? 16 : 8) : 0);
+            fixed = 128 + xch + (ax == 0 && !s->fp32 ? (size_t) (nn[0] + skip) * (s->cplx ? 16 : 8) : 0);
          } else {
-            stage = ((size_t) TW * (d.nz + 16 / esz) * esz + 127) & ~(size_t) 127;
-            // FP64: the four coefficient tables staged in shared memory
-            fixed = 128 + blk + 2 * (size_t) P * TW * sizeof(double) +
-                    (s->fp32 ? 0 : 4 * (size_t) nn[2] * (s->cplx ? 16 : 8));
+            stage = ((size_t) TW * zrow_stride(d.nz, skip, (int) esz) * esz + 127) & ~(size_t) 127;
+            // FP64: the coefficient tables staged in shared memory
+            fixed = 128 + xch + 2 * (size_t) P * TW * sizeof(double) + (s->fp32 ? 0 : 4 * (size_t) P * MS * esz);
          }
       };
       auto fits = [&](int c) {
          size_t st_, fx_;
-         sizes(cTW[c], cP[c], st_, fx_);
-         return (fx_ + 2 * st_) * max_ctas <= sm_cap;
+         sizes(cTW[c], cM[c], cP[c], st_, fx_);
+         return (fx_ + 2 * st_) * 2 <= sm_cap;
       };
       const int want_tw = s->tune.sweep_tw[ax], want_ms = s->tune.sweep_seg[ax];
       // a candidate matching the fields that are set (an unset segment
@@ -456,17 +465,22 @@ static gpe_status plan_tiles(gpe_solver *s) {
             if (match(c)) pick = c;
          if (pick < 0) return fail(GPE_ERR_PARAM, "tuning: sweep_tw / sweep_seg not available for this line length");
       } else {
-         // FP32 real z lines of 100 points or more: 32-point segments when
-         // that leaves at least four per line (128^3 z sweep 20.1 -> 16.6 us
-         // on B200; shorter lines, and the x and y sweeps, measured no faster
-         // or slower with them solo), on 16-row tiles where those fit (with
-         // a 3-stage pipeline, below: mixed 256^3 step 0.4117 -> 0.4088 ms,
-         // 512x512x256 1.676 -> 1.666 ms)
-         if (ax == 2 && esz == 4) {
+         // measured on B200 (us, choice against the widest tile with the
+         // shortest segments): FP64 real lines of 96 points or more: x and z 8
+         // lines of 16-point segments (256^3: x 93 -> 85, z 71 -> 62; 128^3: z
+         // 20.5 -> 18.5), y 16 of 16 (128^3: 14.4 -> 12.3); FP32 complex x 8
+         // of 8 (256^3: 121 -> 96; 160 points 27 -> 23); FP32 real z 16 of 32
+         // where that leaves 8 segments (512x512x256: 143 -> 138), else 16 of
+         // 16 (128^3: 16.1 -> 14.4)
+         auto want = [&](int tw, int m) {
             for (int c = 0; c < nc && pick < 0; c++)
-               if (cM[c] == 32 && cP[c] >= 4 && cTW[c] == 16 && fits(c)) pick = c;
-            for (int c = 0; c < nc && pick < 0; c++)
-               if (cM[c] == 32 && cP[c] >= 4 && fits(c)) pick = c;
+               if (cTW[c] == tw && cM[c] == m && fits(c)) pick = c;
+         };
+         if (!s->fp32 && !s->cplx && nn[ax] >= 96) want(ax == 1 ? 16 : 8, 16);
+         if (s->fp32 && s->cplx && ax == 0) want(8, 8);
+         if (s->fp32 && !s->cplx && ax == 2 && nn[ax] >= 96) {
+            if (nn[ax] - 2 > 7 * 32) want(16, 32);
+            want(16, 16);
          }
          for (int c = 0; c < nc && pick < 0; c++)
             if (prim[c] && fits(c)) pick = c;
@@ -475,12 +489,9 @@ static gpe_status plan_tiles(gpe_solver *s) {
       w.TW = cTW[pick];
       w.MSEG = cM[pick];
       const int P = cP[pick];
-      if (w.M) cudaFree(w.M);
-      if (w.N) cudaFree(w.N);
-      w.M = w.N = nullptr;
-      CKS(make_segtab(s, ax, nn[ax], h2[ax], w.MSEG, P));
+      CKS(make_segtab(s, ax, nn[ax], w.MSEG, P));
       size_t stage = 0, fixed = 0;
-      sizes(w.TW, P, stage, fixed);
+      sizes(w.TW, w.MSEG, P, stage, fixed);
       if (ax < 2) {
          w.boxn = (int) std::min<long>(nn[ax], 256);
          w.nbox = (int) ((nn[ax] + w.boxn - 1) / w.boxn);
@@ -488,7 +499,7 @@ static gpe_status plan_tiles(gpe_solver *s) {
          CKS(make_tmap(&w.tm_psi, s->psi, s->fp32 ? 4 : 8, E * d.nz, d.ny, d.nx, E * w.TW, by, bx));
          CKS(make_tmap(&w.tm_phi, s->phi, rsz, d.nz, d.ny, d.nx, w.TW, by, bx));
       } else {
-         w.LS = (int) (d.nz + 16 / esz);
+         w.LS = zrow_stride(d.nz, w.tab.skip, (int) esz);
       }
       // as many resident CTAs as allowed, then the deepest pipeline (2 or 3
       // stages) that keeps them
@@ -500,10 +511,10 @@ static gpe_status plan_tiles(gpe_solver *s) {
       const int s_hi = s->tune.sweep_stages[ax] > 0 ? s->tune.sweep_stages[ax] : ((ax == 2 && !z16) ? 2 : 3);
       const int s_lo = s->tune.sweep_stages[ax] > 0 ? s->tune.sweep_stages[ax] : 2;
       if (s_lo < 2 || s_hi > 3) return fail(GPE_ERR_PARAM, "tuning: sweep_stages must be 2 or 3");
-      // the register budget of max_ctas CTAs of 256 threads holds more CTAs
+      // the register budget of ctas_of() CTAs of 256 threads holds more CTAs
       // of fewer threads
       const int thr = (w.TW * P + 31) & ~31;
-      const int ct_max = std::min(32, 256 * max_ctas / thr);
+      const int ct_max = std::min(32, 256 * ctas_of(pick) / thr);
       w.ctas = 0;
       for (int ct = ct_max; ct >= 1 && !w.ctas; ct--)
          for (int S = s_hi; S >= s_lo && !w.ctas; S--)
@@ -568,15 +579,17 @@ static gpe_status setup_static(gpe_solver *s) {
    for (int k = 0; k < mm; k++) wz[k] = (k == 0 || k == mm - 1) ? 1. : ((k % 2) ? 4. : 2.);
    if (N % 2 == 0) { wz[N - 1] += 5. / 4.; wz[N - 2] += 8. / 4.; wz[N - 3] -= 1. / 4.; }
    void *t = nullptr;
+   // (kTabPad zero entries before index 0, for the sweeps' rows below the line)
+   wz.insert(wz.begin(), kTabPad, 0.);
    CKS(upload(&t, wz.data(), wz.size()));
-   s->wz = (double *) t;
-   std::vector<double> wz2(d.nz);
+   s->wz = (double *) t + kTabPad;
+   std::vector<double> wz2(kTabPad + d.nz, 0.);
    for (int k = 0; k < N; k++) {
       const double z = (k - d.nz / 2) * s->p.dz;  // the mesh of initpsi
-      wz2[k] = wz[k] * (z * z);
+      wz2[kTabPad + k] = wz[kTabPad + k] * (z * z);
    }
    CKS(upload(&t, wz2.data(), wz2.size()));
-   s->wz2 = (double *) t;
+   s->wz2 = (double *) t + kTabPad;
    CK(cudaMalloc(&s->err, sizeof(uint32_t)));
    CK(cudaMemset(s->err, 0, sizeof(uint32_t)));
    return GPE_OK;
@@ -612,22 +625,22 @@ static gpe_status make_udd(gpe_solver *s) {
 }
 
 static void free_all(gpe_solver *s) {
-   void *ptrs[] = {s->psi, s->spec, s->phi, s->twx, s->twy, s->twz, s->udd, s->x2, s->y2, s->z2, s->x2f, s->y2f, s->z2f,
+   void *ptrs[] = {s->psi, s->spec, s->phi, s->twx, s->twy, s->twz, s->udd, s->x2, s->y2, s->z2,
                    s->rowA, s->rowB, s->tmp, s->obs, s->state, s->rms_buf};
    for (void *q : ptrs)
       if (q) cudaFree(q);
    for (int a = 0; a < 3; a++) {
       if (s->alpha[a]) cudaFree(s->alpha[a]);
       if (s->gamma[a]) cudaFree(s->gamma[a]);
-      if (s->sw[a].M) cudaFree(s->sw[a].M);
-      if (s->sw[a].N) cudaFree(s->sw[a].N);
-      for (void *q : s->sw[a].t32)
+      for (void *q : s->sw[a].tabs)
          if (q) cudaFree(q);
    }
-   if (s->wz) cudaFree(s->wz);
+   if (s->wz) cudaFree(s->wz - kTabPad);
+   for (float *q : {s->x2f, s->y2f, s->z2f})
+      if (q) cudaFree(q - kTabPad);
    for (void *q : s->lin)
-      if (q) cudaFree(q);
-   if (s->wz2) cudaFree(s->wz2);
+      if (q) cudaFree(s->fp32 ? (void *) ((float *) q - kTabPad) : q);
+   if (s->wz2) cudaFree(s->wz2 - kTabPad);
    if (s->err) cudaFree(s->err);
    if (s->own_stream && s->st) cudaStreamDestroy(s->st);
 }
@@ -699,9 +712,10 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
       const std::vector<double> *sq[3] = {&s->hx2, &s->hy2, &s->hz2};
       float **dst[3] = {&s->x2f, &s->y2f, &s->z2f};
       for (int a = 0; a < 3; a++) {
-         std::vector<float> f(sq[a]->begin(), sq[a]->end());
+         std::vector<float> f(kTabPad, 0.f);
+         f.insert(f.end(), sq[a]->begin(), sq[a]->end());
          CKS(upload(&t, f.data(), f.size()));
-         *dst[a] = (float *) t;
+         *dst[a] = (float *) t + kTabPad;
       }
    }
    // trap factors per axis for calcnu: exp(-dt 0.5 par c x^2) in imaginary
@@ -732,8 +746,10 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
          std::vector<double> tab(n);
          for (size_t i = 0; i < n; i++) tab[i] = (double) expl(-dt * hp * cf[a] * (long double) (*sq[a])[i]);
          if (s->fp32) {
-            std::vector<float> f(tab.begin(), tab.end());
-            CKS(upload(&s->lin[a], f.data(), f.size()));
+            std::vector<float> f(kTabPad, 0.f);
+            f.insert(f.end(), tab.begin(), tab.end());
+            CKS(upload(&t, f.data(), f.size()));
+            s->lin[a] = (float *) t + kTabPad;
          } else {
             CKS(upload(&s->lin[a], tab.data(), tab.size()));
          }
@@ -1162,24 +1178,18 @@ template <class R, bool CPLX> struct Impl {
       const size_t esz = s->esz_psi;
       for (int ax = 0; ax < 3; ax++) {
          const auto &w = s->sw[ax];
-         const int TW = w.TW, P = w.tab.P, spw = 32 / TW;
+         const int TW = w.TW, P = w.tab.P;
          const int kp = kPXsweep + ax;
          g->mseg[ax] = w.MSEG;
          g->threads[kp] = (unsigned) ((TW * P + 31) & ~31);
          const int nzb = (d.nz + TW - 1) / TW;
          g->tiles[kp] = ax == 0 ? (long long) d.ny * nzb : (ax == 1 ? (long long) d.nx * nzb : (d.nxy + TW - 1) / TW);
-         size_t stage;
-         if (ax < 2) {
-            const size_t rows = (size_t) w.boxn * w.nbox;
-            stage = rows * TW * esz + (ax == 0 ? rows * TW * s->esz_r : 0);
-         } else {
-            stage = (size_t) TW * w.LS * esz;
-         }
+         const size_t stage = ax < 2 ? sweep_stage(s, ax, w.boxn * w.nbox, TW, w.tab.skip) : (size_t) TW * w.LS * esz;
          g->stage[ax] = (uint32_t) ((stage + 127) & ~(size_t) 127);
-         g->blk[ax] = (uint32_t) ((2 * (size_t) ((P + spw - 1) / spw + 1) * TW * esz + 15) & ~(size_t) 15);
+         g->xch[ax] = (uint32_t) ((2 * (size_t) P * TW * esz + 15) & ~(size_t) 15);
          if (!s->fp32) {
-            if (ax == 0) g->extra[ax] = (uint32_t) (d.nx * (s->cplx ? 16 : 8));
-            if (ax == 2) g->extra[ax] = (uint32_t) (4 * (size_t) d.nz * (s->cplx ? 16 : 8));
+            if (ax == 0) g->extra[ax] = (uint32_t) ((d.nx + w.tab.skip) * (s->cplx ? 16 : 8));
+            if (ax == 2) g->extra[ax] = (uint32_t) (4 * (size_t) P * w.MSEG * esz);
          }
          if (ax == 2) g->part = (uint32_t) (((size_t) P * TW * sizeof(double) + 15) & ~(size_t) 15);
       }

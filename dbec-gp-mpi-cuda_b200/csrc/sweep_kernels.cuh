@@ -5,10 +5,9 @@
 // A CTA owns TW lines.  The lines are brought in by one TMA tensor load (x
 // and y sweeps: box of TW z-columns by the whole line) or by one bulk copy
 // per row (z sweep), so every HBM access is a full 128-byte row segment and
-// no transpose is needed.  The per-axis coefficient tables are read through
-// the L1 cache, which the CTAs of an SM share.  Each line is split into P segments of m points,
-// one thread per (line, segment); the two first-order recurrences of the
-// Thomas algorithm
+// no transpose is needed.  Each line is cut into P segments of exactly m
+// points, one thread per (line, segment); the two first-order recurrences of
+// the Thomas algorithm
 //    beta[i-1] = gamma[i] (A beta[i] - c_i),      i = n-2 .. 1
 //    psi'[i+1] = alpha[i] psi'[i] + beta[i],      i = 0 .. n-3
 // run locally from a zero carry-in, and the true values follow from the
@@ -16,6 +15,25 @@
 // with the prefix products of (gamma_i A) and alpha_i precomputed per axis
 // (tables M and N).  The result equals the sequential recurrence up to
 // rounding.
+//
+// Segments are aligned at the top of the line: segment p owns the recurrence
+// indices lo .. lo + m - 1, lo = p m - skip with skip = P m - (n - 2), so the
+// top one ends at n - 3 and the bottom one starts skip rows below the line.
+// Those rows are zero and the tables hold zero coefficients there (so beta
+// and psi' are exactly zero below index 1): no index of the unrolled loops
+// needs a bound check.
+//
+// Carries: segment p maps the value entering at its top to beta[lo] by the
+// affine map x -> b_p + a_p x with a_p = M at its bottom.  |a_p| is the decay
+// of the recurrence over one segment (alpha^m, alpha about dt / (4 dx^2):
+// 1e-13 for dt = 0.1 dx^2 and m = 8), so a carry from D segments away is
+// scaled by a product of D such factors.  The host picks the smallest D for
+// which that product stays below 2^-64 (FP64) or 2^-40 (FP32), 2^-11 and
+// 2^-16 of the type's rounding unit (D = 1 or 2 for the usual time steps, up
+// to P for large ones), and a thread composes the maps of the D segments
+// beyond its own from a shared table of the b_p.  The scan over all segments
+// that this replaces (shuffles in the warp, then a chain over the warps) cost
+// about as many instructions as the recurrences.
 #pragma once
 
 #include <type_traits>
@@ -25,46 +43,45 @@
 
 namespace gpe {
 
-// Segment tables of one axis.
+// Segment tables of one axis, indexed by p m + q (recurrence index i = lo + q
+// of segment p): FP64 for the FP64 sweeps, once-rounded FP32 for the FP32 ones.
 struct SegTab {
-   const void *al, *ga;  // alpha, gamma padded to n entries (double or double2;
-                         // float or float2 for the FP32 sweeps)
-   const void *M, *N;    // prefix products, n entries each
-   double2 A, A0r, mA;
-   int n, m, P;
+   const void *ga;  // gamma[i + 1]
+   const void *ma;  // pairs (M[i], alpha[i])
+   const void *nn;  // N[i + 1]
+   double2 A;
+   int n, m, P, D, skip;
 };
+
+// Bytes of the zero rows below a tile of TW lines (kept a multiple of the 128
+// bytes a TMA destination is aligned to).
+__host__ __device__ __forceinline__ uint32_t sweep_pad(int skip, int TW, int esz) {
+   return (uint32_t) ((skip * TW * esz + 127) & ~127);
+}
 
 template <class R, bool CPLX> struct SegOps {
    using P = typename Tr<R, CPLX>::P;
-   // table entry i: FP64 tables for FP64 sweeps, their once-rounded FP32
-   // copies for FP32 sweeps
-   __device__ static P ld(const void *t, int i) {
-      if constexpr (std::is_same<R, float>::value) {
-         if constexpr (CPLX) return __ldg((const float2 *) t + i);
-         else return __ldg((const float *) t + i);
-      } else if constexpr (CPLX) {
-         const double2 v = __ldg((const double2 *) t + i);
-         return mk<R>((R) v.x, (R) v.y);
+   // coefficient entry: from global memory (read-only path) or staged in
+   // shared memory
+   template <bool STAB> __device__ __forceinline__ static P ld(const P *t) {
+      if constexpr (STAB) return *t;
+      else return __ldg(t);
+   }
+   // 16 bytes of a table: V entries
+   static constexpr int V = 16 / (int) sizeof(P);
+   template <bool STAB> __device__ __forceinline__ static void ldv(const P *t, P (&o)[V]) {
+      if constexpr (sizeof(P) == 4) {
+         const float4 v = STAB ? *(const float4 *) t : __ldg((const float4 *) t);
+         o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+      } else if constexpr (std::is_same<P, float2>::value) {
+         const float4 v = STAB ? *(const float4 *) t : __ldg((const float4 *) t);
+         o[0] = make_float2(v.x, v.y); o[1] = make_float2(v.z, v.w);
+      } else if constexpr (sizeof(P) == 8) {
+         const double2 v = STAB ? *(const double2 *) t : __ldg((const double2 *) t);
+         o[0] = v.x; o[1] = v.y;
       } else {
-         return (R) __ldg((const double *) t + i);
+         o[0] = ld<STAB>(t);
       }
-   }
-   // the same from a table staged in shared memory
-   __device__ static P lds(const void *t, int i) {
-      if constexpr (CPLX) {
-         const double2 v = ((const double2 *) t)[i];
-         return mk<R>((R) v.x, (R) v.y);
-      } else {
-         return (R) ((const double *) t)[i];
-      }
-   }
-   __device__ static P cv(double2 v) {
-      if constexpr (CPLX) return mk<R>((R) v.x, (R) v.y);
-      else return (R) v.x;
-   }
-   __device__ static P mul(P a, P b) {
-      if constexpr (CPLX) return cmul(a, b);
-      else return a * b;
    }
    // One backward Thomas step of the Crank-Nicolson system.  With the
    // coefficients of gencoef, minusA = -A and A0r = 1 + 2A in both modes
@@ -117,168 +134,218 @@ template <class R, bool CPLX> struct SegOps {
    }
 };
 
-// Segmented Thomas sweep of line c held in shared memory at
-// s[i * es + c * cs], i in [0, n).  Called by all threads of the CTA; thread
-// t = p * TW + c owns recurrence indices [p m, hf] of line c.  A warp holds
-// SPW = 32 / TW consecutive segments of each of its TW lines.  blk is a
-// shared scratch of 2 * (NW + 1) * TW elements (NW warps hold segments).
-// Writes the swept line back in place.  When simp_w and simp_w2 are
-// non-null, *simp receives this thread's share of sum_i simp_w[i] |psi'_i|^2
-// and *simp2 that of sum_i simp_w2[i] |psi'_i|^2.  When only simp_w is
-// non-null, *simp receives the share with the interior Simpson weights, 4 at
-// odd i and 2 at even i, applied by parity without reading the table (a
-// segment starts at an even index, m being even); the caller adds the end
-// correction of an even-length line (simp_w's other entries).  Every
-// value of the line the recurrence reads goes through xf(value, i) first
-// (the fused calcnu of the x sweep; identity otherwise); a thread reads its
-// own points and the two above its segment, so no transformed copy of the
-// line is stored.
-//
-// Carries: segment p maps the value entering at its top (index hf+1) to the
-// value at its bottom (index lo) by the affine map x -> b + a x with
-// a = M[lo], b = beta~[lo]; the value entering segment p is the composition
-// of the maps of all segments above it: a suffix scan, done with shuffles
-// inside a warp and a short chain over the warps above.  The forward
-// recurrence composes x -> psi'~[hf+1] + N[hf+1] x from the bottom (prefix).
+// Own points of a segment as they are (the y and z sweeps): w[q] = lp[q es].
 struct NoXf {
-   template <class P> __device__ __forceinline__ P operator()(P v, int) const { return v; }
+   static constexpr bool kNu = false;
 };
 
-template <class R, bool CPLX, int MSEG, int TWC = 0, class XF = NoXf, bool STAB = false>
-__device__ __forceinline__ void seg_sweep(typename Tr<R, CPLX>::P *s, int es, int cs, int c, int p, int tw_arg,
-                                          const SegTab &tb, typename Tr<R, CPLX>::P *blk, const double *simp_w,
-                                          double *simp, const double *simp_w2 = nullptr,
-                                          double *simp2 = nullptr, const XF &xf = XF()) {
+// Adjacent elements of a contiguous row (z sweep) move two at a time: every
+// segment starts at an even index and rows at 16-byte boundaries, and with a
+// row stride of an odd number of 16-byte units the 8 (16-byte accesses) rows
+// a phase of a warp touches fall on different banks.
+template <class P> struct Pair2 { using type = void; };
+template <> struct Pair2<float> { using type = float2; };
+template <> struct Pair2<double> { using type = double2; };
+template <> struct Pair2<float2> { using type = float4; };
+template <class P> __device__ __forceinline__ void ld2(const P *s, P &a, P &b) {
+   if constexpr (sizeof(P) == 16) {
+      a = s[0]; b = s[1];
+   } else {
+      const auto v = *(const typename Pair2<P>::type *) s;
+      if constexpr (std::is_same<P, float2>::value) { a = make_float2(v.x, v.y); b = make_float2(v.z, v.w); }
+      else { a = v.x; b = v.y; }
+   }
+}
+template <class P> __device__ __forceinline__ void st2(P *s, P a, P b) {
+   if constexpr (sizeof(P) == 16) {
+      s[0] = a; s[1] = b;
+   } else {
+      typename Pair2<P>::type v;
+      if constexpr (std::is_same<P, float2>::value) { v.x = a.x; v.y = a.y; v.z = b.x; v.w = b.y; }
+      else { v.x = a; v.y = b; }
+      *(typename Pair2<P>::type *) s = v;
+   }
+}
+
+// Segmented Thomas sweep of one line in shared memory (element i at
+// line[i es], rows -skip .. -1 present), by all threads of the CTA: thread p
+// of the line owns segment p of M points, threads with p >= tb.P only take
+// part in the barriers.  xch points at this line's column of an exchange
+// buffer of 2 P rows of xs elements.  The swept line is written back in
+// place.  ROW: es == 1 and 16-byte aligned rows, accessed in pairs.  STAB:
+// the tables are in shared memory.
+//
+// xf may transform the points first (the x sweep's calcnu): a thread
+// transforms its own M points into registers, publishes the two lowest (the
+// ones the segment below also reads) in the line, and the top thread
+// transforms the two points above the last segment itself.
+//
+// SIMP 1: *simp receives this thread's share of sum_i |psi'_i|^2 with the
+// interior Simpson weights, 4 at odd i and 2 at even i, by parity (lo is
+// even); the caller adds the end correction of an even-length line.  SIMP 2:
+// with the weights w1[i] into *simp and w2[i] into *simp2 (both arrays have
+// skip entries before index 0).
+template <class R, bool CPLX, int M, bool ROW, bool STAB, int SIMP, class XF>
+__device__ __forceinline__ void seg_sweep(typename Tr<R, CPLX>::P *line, int es_, int p, const SegTab &tb,
+                                          typename Tr<R, CPLX>::P *xch, int xs, const XF &xf,
+                                          const double *w1t = nullptr, const double *w2t = nullptr,
+                                          double *simp = nullptr, double *simp2 = nullptr) {
    using Op = SegOps<R, CPLX>;
    using P = typename Tr<R, CPLX>::P;
-   const int TW = TWC > 0 ? TWC : tw_arg;  // lines per CTA (compile time when TWC > 0)
-   const int n = tb.n, m = tb.m, NP = tb.P;
-   const int SPW = 32 / TW;              // segments of one line inside a warp
-   const int NW = (NP + SPW - 1) / SPW;  // warps that hold segments
-   const int lane = threadIdx.x & 31, j = lane / TW, w = threadIdx.x >> 5;
-   const bool act = p < NP;
-   const int lo = p * m;
-   const bool top = (p == NP - 1);
-   const int hf = top ? n - 3 : lo + m - 1;  // last owned recurrence index
-   const int K = hf - lo + 1;                // owned points, 1 <= K <= MSEG
+   constexpr int V = Op::V;
+   const int es = ROW ? 1 : es_;
+   const int NP = tb.P;
+   const bool act = p < NP, top = p == NP - 1;
+   const int lo = p * M - tb.skip;
    const R a = CPLX ? (R) tb.A.y : (R) tb.A.x;
-   P *line = s + c * cs;
-   auto L = [&](int i) -> P { return xf(line[i * es], i); };
-   // coefficient tables: global (read-only path) or staged in shared memory
-   auto T = [&](const void *t, int i) -> P { return STAB ? Op::lds(t, i) : Op::ld(t, i); };
-   P *ba = blk, *bb = blk + (NW + 1) * TW;  // per-warp block maps [NW][TW]
-   const unsigned fullmask = 0xffffffffu;
+   P *lp = line + lo * es;
+   const P *ga = (const P *) tb.ga + p * M, *ma = (const P *) tb.ma + 2 * p * M, *nn = (const P *) tb.nn + p * M;
+   P *xb = xch, *xv = xch + NP * xs;
+
+   P w[M];
+   P t2 = zero_of<P>(), t1 = zero_of<P>();  // the two points above the segment
+   if (act) {
+      if (p == 0) {  // zero rows below the line (only this thread reads them)
+         for (int q = 0; q < tb.skip; q++) lp[q * es] = zero_of<P>();
+         if constexpr (XF::kNu)
+            for (int q = 0; q < tb.skip; q++) xf.zero_row(q - tb.skip);
+      }
+      if constexpr (XF::kNu) {
+         xf.template own<M>(lp, lo, w);
+         if (top) {
+            P tt[2];
+            xf.template own<2>(lp + M * es, lo + M, tt);
+            t1 = tt[0];
+            t2 = tt[1];
+         }
+         lp[0] = w[0];
+         lp[es] = w[1];
+      } else if constexpr (ROW) {
+#pragma unroll
+         for (int q = 0; q < M; q += 2) ld2(lp + q, w[q], w[q + 1]);
+         ld2(lp + M, t1, t2);
+      } else {
+#pragma unroll
+         for (int q = 0; q < M; q++) w[q] = lp[q * es];
+         t1 = lp[M * es];
+         t2 = lp[(M + 1) * es];
+      }
+   }
+   if constexpr (XF::kNu) {
+      __syncthreads();
+      if (act && !top) {
+         t1 = lp[M * es];
+         t2 = lp[(M + 1) * es];
+      }
+   }
 
    // ---- backward local recurrence: bt[q] = beta~[lo + q]
-   P bt[MSEG];
+   P bt[M];
    if (act) {
-      P b = top ? L(n - 1) : zero_of<P>();  // beta[n-2] = psi[n-1] is exact
-      // the step producing beta[lo+q] uses i = lo+q+1: psi[i+1], psi[i], psi[i-1]
-      P w2 = L(lo + K + 1);
-      P w1 = L(lo + K);
+      P b = top ? t2 : zero_of<P>();  // beta[n-2] = psi[n-1] is exact
 #pragma unroll
-      for (int q = MSEG - 1; q >= 0; q--) {
-         if (q < K) {
-            const P w0 = L(lo + q);
-            b = Op::back_step(b, w2, w1, w0, T(tb.ga, lo + q + 1), a);
+      for (int q0 = M - V; q0 >= 0; q0 -= V) {
+         P g[V];
+         Op::template ldv<STAB>(ga + q0, g);
+#pragma unroll
+         for (int j = V - 1; j >= 0; j--) {
+            const int q = q0 + j;
+            b = Op::back_step(b, q + 2 < M ? w[q + 2 < M ? q + 2 : 0] : (q + 1 < M ? t1 : t2),
+                              q + 1 < M ? w[q + 1 < M ? q + 1 : 0] : t1, w[q], g[j], a);
             bt[q] = b;
-            w2 = w1;
-            w1 = w0;
          }
       }
-   }
-   // ---- suffix scan of the backward maps: in-warp, then over the warps above
-   P sa = zero_of<P>(), sb = zero_of<P>();
-   if (act) {
-      sa = top ? zero_of<P>() : T(tb.M, lo);
-      sb = bt[0];
-   }
-   for (int dd = 1; dd < SPW; dd <<= 1) {
-      const P a2 = shfl_down_any(fullmask, sa, dd * TW), b2 = shfl_down_any(fullmask, sb, dd * TW);
-      if (j + dd < SPW && p + dd < NP) {
-         sb = Op::fma_(sa, b2, sb);
-         sa = Op::mul(sa, a2);
-      }
-   }
-   if (j == 0 && w < NW) {
-      ba[w * TW + c] = sa;
-      bb[w * TW + c] = sb;
+      xb[p * xs] = b;
    }
    __syncthreads();  // also: every read of the line is complete before it is rewritten
-   P bin = zero_of<P>();
-   {
-      // value entering the top segment of this warp from the warps above
-      P x = zero_of<P>();
-      for (int ww = NW - 1; ww > w; ww--) x = Op::fma_(ba[ww * TW + c], x, bb[ww * TW + c]);
-      const P here = Op::fma_(sa, x, sb);  // beta at the bottom of this segment
-      const P nxt = shfl_down_any(fullmask, here, TW);
-      bin = (j + 1 < SPW) ? nxt : x;
-      if (!act || top) bin = zero_of<P>();
-   }
-   __syncthreads();  // the block maps are reused below
-
-   // ---- forward local recurrence: bt[q] becomes psi'~[lo + q + 1]
    P v = zero_of<P>();
-   sa = zero_of<P>();
    if (act) {
+      // ---- beta entering at the top of this segment
+      P bin = zero_of<P>();
+      int s = min(p + tb.D, NP - 1);
+      if (s > p) bin = xb[s * xs];
+      for (s--; s > p; s--) bin = Op::fma_(Op::template ld<STAB>((const P *) tb.ma + 2 * s * M), bin, xb[s * xs]);
+      // ---- forward local recurrence: bt[q] becomes psi'~[lo + q + 1]
 #pragma unroll
-      for (int q = 0; q < MSEG; q++) {
-         if (q < K) {
-            const int i = lo + q;
-            const P beta = Op::fma_(T(tb.M, i), bin, bt[q]);
-            v = Op::fma_(T(tb.al, i), v, beta);
-            bt[q] = v;
+      for (int q0 = 0; q0 < M; q0 += (V > 1 ? V / 2 : 1)) {
+         constexpr int G = V > 1 ? V / 2 : 1;  // (M, alpha) pairs per 16 bytes
+         P c[2 * G];
+         if constexpr (V > 1) {
+            P cc[V];
+            Op::template ldv<STAB>(ma + 2 * q0, cc);
+#pragma unroll
+            for (int j = 0; j < V; j++) c[j] = cc[j];
+         } else {
+            c[0] = Op::template ld<STAB>(ma + 2 * q0);
+            c[1] = Op::template ld<STAB>(ma + 2 * q0 + 1);
+         }
+#pragma unroll
+         for (int j = 0; j < G; j++) {
+            const P beta = Op::fma_(c[2 * j], bin, bt[q0 + j]);
+            v = Op::fma_(c[2 * j + 1], v, beta);
+            bt[q0 + j] = v;
          }
       }
-      sa = T(tb.N, hf + 1);
-   }
-   // ---- prefix scan of the forward maps
-   sb = v;
-   for (int dd = 1; dd < SPW; dd <<= 1) {
-      const P a2 = shfl_up_any(fullmask, sa, dd * TW), b2 = shfl_up_any(fullmask, sb, dd * TW);
-      if (j >= dd) {
-         sb = Op::fma_(sa, b2, sb);
-         sa = Op::mul(sa, a2);
-      }
-   }
-   if (j == SPW - 1 && w < NW) {
-      ba[w * TW + c] = sa;
-      bb[w * TW + c] = sb;
+      xv[p * xs] = v;
    }
    __syncthreads();
    double acc = 0., acc2 = 0., acc_o = 0., acc_e = 0.;
-   {
-      P x = zero_of<P>();  // psi' entering the first segment of this warp
-      for (int ww = 0; ww < w; ww++) x = Op::fma_(ba[ww * TW + c], x, bb[ww * TW + c]);
-      const P upto = Op::fma_(sa, x, sb);  // psi'[hf + 1] of this segment
-      const P prv = shfl_up_any(fullmask, upto, TW);
-      const P fin = (j >= 1) ? prv : x;  // psi'[lo]
-      if (act) {
+   if (act) {
+      // ---- psi' entering at the bottom of this segment (zero for p = 0)
+      P fin = zero_of<P>();
+      int s = max(p - tb.D, 0);
+      if (s < p) fin = xv[s * xs];
+      for (s++; s < p; s++) fin = Op::fma_(Op::template ld<STAB>((const P *) tb.nn + s * M + M - 1), fin, xv[s * xs]);
 #pragma unroll
-         for (int q = 0; q < MSEG; q++) {
-            if (q < K) {
-               const int k = lo + q + 1;
-               const P val = Op::fma_(T(tb.N, k), fin, bt[q]);
-               line[k * es] = val;
-               if (simp_w) {
-                  const double f = (double) dens2(val);
-                  if (simp_w2) {
-                     acc += simp_w[k] * f;
-                     acc2 += simp_w2[k] * f;
-                  } else if (q & 1) {  // k = lo + q + 1 even
-                     acc_e += f;
-                  } else {
-                     acc_o += f;
-                  }
-               }
+      for (int q0 = 0; q0 < M; q0 += V) {
+         P g[V];
+         Op::template ldv<STAB>(nn + q0, g);
+#pragma unroll
+         for (int j = 0; j < V; j++) {
+            const int q = q0 + j;
+            bt[q] = Op::fma_(g[j], fin, bt[q]);
+            if constexpr (SIMP == 1) {
+               const double f = (double) dens2(bt[q]);
+               if (q & 1) acc_e += f;  // index lo + q + 1 even
+               else acc_o += f;
+            } else if constexpr (SIMP == 2) {
+               const double f = (double) dens2(bt[q]);
+               acc += w1t[lo + q + 1] * f;
+               acc2 += w2t[lo + q + 1] * f;
             }
          }
-         if (p == 0) line[0] = zero_of<P>();
-         if (top) line[(n - 1) * es] = zero_of<P>();
       }
+      if constexpr (ROW) {
+         lp[1] = bt[0];
+#pragma unroll
+         for (int q = 1; q + 1 < M; q += 2) st2(lp + q + 1, bt[q], bt[q + 1]);
+         lp[M] = bt[M - 1];
+      } else {
+#pragma unroll
+         for (int q = 0; q < M; q++) lp[(q + 1) * es] = bt[q];
+      }
+      if (p == 0) line[0] = zero_of<P>();
+      if (top) line[(tb.n - 1) * es] = zero_of<P>();
    }
-   if (simp) *simp = simp_w2 ? acc : fma(4., acc_o, 2. * acc_e);
-   if (simp2) *simp2 = acc2;
+   if constexpr (SIMP == 1) *simp = fma(4., acc_o, 2. * acc_e);
+   if constexpr (SIMP == 2) {
+      *simp = acc;
+      *simp2 = acc2;
+   }
+}
+
+// The same for the run-time segment length of the table (8, 16 or, up to
+// MMAX, 32 points).
+template <class R, bool CPLX, int MMAX, bool ROW, bool STAB, int SIMP, class XF>
+__device__ __forceinline__ void seg_sweep_any(typename Tr<R, CPLX>::P *line, int es, int p, const SegTab &tb,
+                                              typename Tr<R, CPLX>::P *xch, int xs, const XF &xf,
+                                              const double *w1t = nullptr, const double *w2t = nullptr,
+                                              double *simp = nullptr, double *simp2 = nullptr) {
+   if constexpr (MMAX >= 32)
+      if (tb.m == 32) return seg_sweep<R, CPLX, 32, ROW, STAB, SIMP>(line, es, p, tb, xch, xs, xf, w1t, w2t, simp, simp2);
+   if constexpr (MMAX >= 16)
+      if (tb.m == 16) return seg_sweep<R, CPLX, 16, ROW, STAB, SIMP>(line, es, p, tb, xch, xs, xf, w1t, w2t, simp, simp2);
+   seg_sweep<R, CPLX, 8, ROW, STAB, SIMP>(line, es, p, tb, xch, xs, xf, w1t, w2t, simp, simp2);
 }
 
 // exp(-i t) = (cos t, -sin t) for the nonlinear part of the real-time phase,
@@ -320,116 +387,182 @@ __device__ __forceinline__ double2 expi_small(double t) {
    return make_double2(cs, -sn);
 }
 
-// FP64 calcnu over a staged tile before its sweep (the x sweep's fused
-// calcnu_kernel, imag3d-mpicuda.cu:1759, real3d-mpicuda.cu:1856), one z
-// column per thread, with the pending 1/norm applied first.  Tile t of the
-// sweep covers z columns [z0, z0 + TW) of plane `other` (y for the x sweep,
-// x for the y sweep); xtab is calcnu's per-x table staged in shared memory
-// (imaginary time: exp(-dt V_x); real time: the phase exp(-i dt V_x)).  The
-// trap part of the exponent is a product of per-axis factors (V is a sum
-// over the axes), so only the nonlinear part is evaluated per point, by a
-// series.  The caller synchronises the CTA afterwards.
-template <class R, bool CPLX, int AXIS>
-__device__ __forceinline__ void nu_pass_fp64(typename Tr<R, CPLX>::P *tile, const R *ptile, int n, int lg, int c,
-                                             int other, int z0, const Dims &d, const Trap &trap, const LinPhase &lin,
-                                             const double *xtab, double g, double gd, double dt, double scale) {
-   const R invN = (R) (1.0 / (double) d.npts);
-   const int k = z0 + c;
-   if (k >= d.nz) return;
-   const int step = blockDim.x >> lg;
-   if constexpr (!CPLX && AXIS == 0) {
-      // imaginary time: trap factor exp(-dt V) from the axis tables, series
-      // for the nonlinear part (measured faster than exp of the sum; in real
-      // time CUDA's sincos of the sum measured faster than the split, so real
-      // time keeps nu_op)
-      const double eyz = __ldg((const double *) lin.ey + other) * __ldg((const double *) lin.ez + k);
-      for (int ii = threadIdx.x >> lg; ii < n; ii += step) {
-         const int e = (ii << lg) + c;
-         const double lx = xtab[ii] * eyz;
-         tile[e] = nu_split(scl(tile[e], scale), (double) ptile[e], lx, g, gd, dt, (double) invN);
-      }
-   } else if constexpr (CPLX && AXIS == 0) {
-      // real time: psi exp(-i dt V_x) exp(-i dt (V_y + V_z)) exp(-i dt (g |psi|^2 + gd phi / N))
-      const double2 ey = __ldg((const double2 *) lin.ey + other), ez = __ldg((const double2 *) lin.ez + k);
-      const double2 eyz = cmul(ey, ez);
-      const double2 *ex = (const double2 *) xtab;
-      for (int ii = threadIdx.x >> lg; ii < n; ii += step) {
-         const int e = (ii << lg) + c;
-         const double2 p = scl(tile[e], scale);
-         const double thn = dt * fma(fma(p.x, p.x, p.y * p.y), g, ((double) ptile[e] * invN) * gd);
-         tile[e] = cmul(p, cmul(cmul(ex[ii], eyz), expi_small(thn)));
-      }
-   } else {
-      // Trap::v with the terms of the two fixed coordinates hoisted
-      const double tz = mrn(trap.vl2, trap.z2[k]);
-      const double to = AXIS == 0 ? mrn(trap.vn2, trap.y2[other]) : mrn(trap.vg2, trap.x2[other]);
-      const double *va = AXIS == 0 ? xtab : trap.y2;
-      const double ca = AXIS == 0 ? trap.vg2 : trap.vn2;
-#pragma unroll 2
-      for (int ii = threadIdx.x >> lg; ii < n; ii += step) {
-         const int e = (ii << lg) + c;
-         const double sv = AXIS == 0 ? arn(arn(mrn(ca, va[ii]), to), tz) : arn(arn(to, mrn(ca, va[ii])), tz);
-         const R V = (R) mrn(trap.hp, sv);
-         tile[e] = nu_op<R>(scl(tile[e], scale), ptile[e], V, (R) g, (R) gd, (R) dt, invN);
-      }
-   }
+// calcnu of the x sweep (calcnu_kernel, imag3d-mpicuda.cu:1759,
+// real3d-mpicuda.cu:1856) on the points of one line column: the pending 1/norm
+// first, then the trap and nonlinear factors.  V is a sum over the axes, so
+// its factor is a product of per-axis ones: `fix` holds the part of the two
+// coordinates the column fixes, xt the table along the line.
+//
+// own<M>() transforms a thread's segment straight into registers with the
+// short series that holds for small nonlinear exponents (the usual case), all
+// points unrolled; a thread that met a larger exponent redoes its points one
+// by one in place (one(), which picks the series or the library function per
+// point) and reloads them.  Transforming the tile in a pass of its own took
+// 82 instructions per FP64 point in imaginary time, mostly indexing and the
+// second trip through shared memory.
+
+// Maclaurin series of exp on |t| <= 1/8 through t^10 (first omitted term
+// below 3e-18).
+__device__ __forceinline__ double exp_series10(double t) {
+   constexpr double f2 = 1. / 2, f3 = f2 / 3, f4 = f3 / 4, f5 = f4 / 5, f6 = f5 / 6, f7 = f6 / 7, f8 = f7 / 8,
+                    f9 = f8 / 9, f10 = f9 / 10;
+   double e = f10;
+   e = fma(e, t, f9);
+   e = fma(e, t, f8);
+   e = fma(e, t, f7);
+   e = fma(e, t, f6);
+   e = fma(e, t, f5);
+   e = fma(e, t, f4);
+   e = fma(e, t, f3);
+   e = fma(e, t, f2);
+   e = fma(e, t, 1.);
+   return fma(e, t, 1.);
 }
 
-// calcnu of the mixed-precision x sweep, applied as the sweep's recurrence
-// reads each point (measured faster than a separate pass over the tile in
-// FP32; slower in FP64, where a thread's extra evaluations for the two points
-// above its segment cost more), entirely in FP32 like the step's other
-// exponentials: real time recomputes V from the FP32 trap tables (the order
-// of Trap::v) and takes sincosf of the exponent; imaginary time multiplies the
-// FP32 trap factors exp(-dt V_x) exp(-dt V_y) exp(-dt V_z) and takes expf of
-// the nonlinear part only.  The pending 1/norm is applied first.
-template <bool CPLX> struct NuTrap32 {
-   const float *ptile;  // phi tile, row stride tw
-   int tw;
-   const float *va;     // along the line: x^2 (real time) or exp(-dt V_x) (imaginary time)
-   float ca, to, tz, hp;  // real time: V = hp ((ca va + to) + tz)
-   float lfix;            // imaginary time: exp(-dt V_y) exp(-dt V_z) of this column
-   float scale, g, gd, dt, invN;
-   template <class P> __device__ __forceinline__ P operator()(P v, int i) const {
-      const float phi = ptile[i * tw];
-      if constexpr (CPLX) {
-         const float2 p = make_float2(v.x * scale, v.y * scale);
-         const float sv = __fadd_rn(__fadd_rn(__fmul_rn(ca, va[i]), to), tz);
-         return nu_op<float>(p, phi, __fmul_rn(hp, sv), g, gd, dt, invN);
-      } else {
+// (cos t, -sin t) on |t| <= 1/32: sin through t^7, cos through t^6 (omitted
+// terms below 3e-18 relative to sin and 3e-17 to cos).
+__device__ __forceinline__ double2 expi_series7(double t) {
+   constexpr double s3 = 1. / 6, s5 = s3 / 20, s7 = s5 / 42, c2 = 1. / 2, c4 = c2 / 12, c6 = c4 / 30;
+   const double t2 = t * t;
+   double sq = fma(-s7, t2, s5);
+   sq = fma(sq, t2, -s3);
+   double cq = fma(-c6, t2, c4);
+   cq = fma(cq, t2, -c2);
+   return make_double2(fma(cq, t2, 1.), -fma(sq * t2, t, t));
+}
+
+// (cos t, -sin t) in FP32 on |t| <= 256: t is reduced by the nearest multiple
+// of pi / 2 in two steps (Cody and Waite), then Maclaurin series on |r| <= pi/4
+// (sine through r^9, cosine through r^10; omitted terms below 3e-9).
+__device__ __forceinline__ float2 expi_f32(float t) {
+   constexpr double pio2 = 1.57079632679489661923;
+   constexpr float hi = (float) pio2, lo = (float) (pio2 - (double) hi), inv = (float) (1. / pio2);
+   constexpr float s3 = (float) (1. / 6), s5 = (float) (1. / 120), s7 = (float) (1. / 5040), s9 = (float) (1. / 362880),
+                   c2 = 0.5f, c4 = (float) (1. / 24), c6 = (float) (1. / 720), c8 = (float) (1. / 40320),
+                   c10 = (float) (1. / 3628800);
+   const float km = fmaf(t, inv, 12582912.f);  // 1.5 2^23: the sum's low bits are the rounded multiple
+   const int q = __float_as_int(km);
+   const float k = km - 12582912.f;
+   const float r = fmaf(k, -lo, fmaf(k, -hi, t)), r2 = r * r;
+   float sq = fmaf(s9, r2, -s7);
+   sq = fmaf(sq, r2, s5);
+   sq = fmaf(sq, r2, -s3);
+   const float sn = fmaf(sq * r2, r, r);
+   float cq = fmaf(-c10, r2, c8);
+   cq = fmaf(cq, r2, -c6);
+   cq = fmaf(cq, r2, c4);
+   cq = fmaf(cq, r2, -c2);
+   const float cs = fmaf(cq, r2, 1.f);
+   const float c = q & 1 ? sn : cs, s = q & 1 ? cs : sn;  // up to sign
+   return make_float2((q + 1) & 2 ? -c : c, q & 2 ? s : -s);
+}
+
+template <class R, bool CPLX> struct NuXf {
+   using P = typename Tr<R, CPLX>::P;
+   using T = typename std::conditional<CPLX && std::is_same<R, double>::value, double2, R>::type;
+   static constexpr bool kNu = true;
+   R *ph;        // phi of this column, row i at ph[i es]
+   int es;
+   // along the line: exp(-dt V_x) in imaginary time, the phase exp(-i dt V_x)
+   // in FP64 real time, x^2 in FP32 real time
+   const T *xt;
+   T fix;        // the other two factors; FP32 real time: unused
+   R scale, dtg, dtgd;      // 1/norm, dt g, dt gd / N
+   R ca, to, tz, hp, dt;    // FP32 real time: V = hp ((ca x^2 + to) + tz)
+
+   __device__ __forceinline__ void zero_row(int i) const { ph[i * es] = (R) 0; }
+
+   __device__ __forceinline__ R expo(P p, R f) const {  // nonlinear exponent
+      return fma(dens2(p), dtg, f * dtgd);
+   }
+   // FP32 real time: the whole exponent.  It stays one phase: FP32 factors
+   // per axis would each round cos and sin near 1, the same error at every
+   // step.
+   __device__ __forceinline__ float expo32(float2 p, float f, float x2) const {
+      const float sv = __fadd_rn(__fadd_rn(__fmul_rn(ca, x2), to), tz);
+      return fmaf(dt, __fmul_rn(hp, sv), fmaf(dens2(p), dtg, f * dtgd));
+   }
+
+   __device__ __forceinline__ P one(P v, int i) const {
+      if constexpr (std::is_same<R, double>::value && !CPLX) {
+         const double p = v * scale;
+         return p * ((xt[i] * fix) * exp_small(-expo(p, ph[i * es])));
+      } else if constexpr (std::is_same<R, double>::value) {
+         return cmul(v, cmul(cmul(xt[i], fix), expi_small(expo(v, ph[i * es]))));
+      } else if constexpr (!CPLX) {
          const float p = v * scale;
-         const float thn = dt * fmaf(p * p, g, (phi * invN) * gd);
-         return p * ((va[i] * lfix) * expf(-thn));
+         return p * ((xt[i] * fix) * expf(-expo(p, ph[i * es])));
+      } else {
+         float sn, cs;
+         sincosf(-expo32(v, ph[i * es], xt[i]), &sn, &cs);
+         return cmul(v, make_float2(cs, sn));
+      }
+   }
+
+   template <int M> __device__ __forceinline__ void own(P *lp, int lo, P (&w)[M]) const {
+      const R *f = ph + lo * es;
+      const T *x = xt + lo;
+      bool big = false;
+#pragma unroll
+      for (int q = 0; q < M; q++) {
+         if constexpr (std::is_same<R, double>::value && !CPLX) {
+            const double p = lp[q * es] * scale, t = expo(p, f[q * es]);
+            big |= !(fabs(t) <= 0.125);
+            w[q] = p * ((x[q] * fix) * exp_series10(-t));
+         } else if constexpr (std::is_same<R, double>::value) {
+            const double2 p = lp[q * es];
+            const double t = expo(p, f[q * es]);
+            big |= !(fabs(t) <= 0.03125);
+            w[q] = cmul(p, cmul(cmul(x[q], fix), expi_series7(t)));
+         } else if constexpr (!CPLX) {
+            const float p = lp[q * es] * scale;
+            w[q] = p * ((__ldg(x + q) * fix) * expf(-expo(p, f[q * es])));
+         } else {
+            const float2 p = lp[q * es];
+            const float t = expo32(p, f[q * es], __ldg(x + q));
+            big |= !(fabsf(t) <= 256.f);
+            w[q] = cmul(p, expi_f32(t));
+         }
+      }
+      if (big) {
+#pragma unroll 1
+         for (int q = 0; q < M; q++) lp[q * es] = one(lp[q * es], lo + q);
+#pragma unroll
+         for (int q = 0; q < M; q++) w[q] = lp[q * es];
       }
    }
 };
 
-// The calcnu functor of tile column c of an x sweep tile covering z columns
-// [z0, z0 + TW) of plane y = other (mixed precision).
-template <bool CPLX>
-__device__ __forceinline__ NuTrap32<CPLX> nu_reads_fp32(const float *ptile_c, int TW, int other, int z0, int c,
-                                                        const Dims &d, const Trap &trap, const LinPhase &lin, double g,
-                                                        double gd, double dt, double scale) {
+// The functor of tile column c of an x sweep tile covering z columns
+// [z0, z0 + TW) of plane y = other; pcol is phi's column in the tile, xtab the
+// staged table (FP64; the FP32 sweeps read theirs through L1).
+template <class R, bool CPLX>
+__device__ __forceinline__ NuXf<R, CPLX> nu_xf(R *pcol, int TW, int other, int z0, int c, const Dims &d,
+                                               const Trap &trap, const LinPhase &lin, const double *xtab, double g,
+                                               double gd, double dt, double scale) {
    const int k = min(z0 + c, d.nz - 1);  // columns past nz are zero fill, never stored
-   NuTrap32<CPLX> f;
-   f.ptile = ptile_c;
-   f.tw = TW;
-   f.scale = (float) scale;
-   f.g = (float) g;
-   f.gd = (float) gd;
-   f.dt = (float) dt;
-   f.invN = (float) (1.0 / (double) d.npts);
-   if constexpr (CPLX) {
-      f.va = trap.x2f;
+   NuXf<R, CPLX> f;
+   using T = typename NuXf<R, CPLX>::T;
+   f.ph = pcol;
+   f.es = TW;
+   f.scale = (R) scale;
+   f.dtg = (R) (dt * g);
+   f.dtgd = (R) (dt * gd / (double) d.npts);
+   if constexpr (std::is_same<R, float>::value && CPLX) {
+      f.xt = trap.x2f;
+      f.fix = 0.f;
       f.ca = (float) trap.vg2;
       f.to = __fmul_rn((float) trap.vn2, trap.y2f[other]);
       f.tz = __fmul_rn((float) trap.vl2, trap.z2f[k]);
       f.hp = (float) trap.hp;
-      f.lfix = 0.f;
+      f.dt = (float) dt;
    } else {
-      f.va = (const float *) lin.ex;
-      f.lfix = __ldg((const float *) lin.ey + other) * __ldg((const float *) lin.ez + k);
-      f.ca = f.to = f.tz = f.hp = 0.f;
+      const T ey = __ldg((const T *) lin.ey + other), ez = __ldg((const T *) lin.ez + k);
+      if constexpr (CPLX) f.fix = cmul(ey, ez);
+      else f.fix = ey * ez;
+      if constexpr (std::is_same<R, double>::value) f.xt = (const T *) xtab;
+      else f.xt = (const T *) lin.ex;
+      f.ca = f.to = f.tz = f.hp = f.dt = (R) 0;
    }
    return f;
 }
@@ -442,19 +575,45 @@ __device__ __forceinline__ NuTrap32<CPLX> nu_reads_fp32(const float *ptile_c, in
 // refilling a stage it waits until the bulk store that last read the stage
 // has finished reading (all but the newest S-2 store groups: wait_stage_free).
 //
-// Resident CTAs per SM the sweep kernels are compiled for (register
-// budget): [0] plain sweeps, [1] the x sweep fused with calcnu, whose tile
-// also stages phi.  The host never launches more per SM.  Three CTAs (80
-// registers) spill the 16-point segments and measured slower on B200.
-constexpr int kSweepCtas[2] = {2, 2};
+// Resident CTAs of 256 threads per SM the sweep kernels are compiled for
+// (register budget); the host never launches more per SM.
+__host__ __device__ constexpr int sweep_ctas(bool fp32, bool cplx, int m) {
+   if (fp32) return m == 32 ? 2 : (cplx && m == 16 ? 3 : 4);
+   return !cplx && m == 8 ? 3 : 2;
+}
 
+// Shared-memory layout of one pipeline stage of an x or y sweep tile: zero
+// rows below the tile, the tile, and with calcnu the same for phi.
+struct XyStage {
+   uint32_t psi, phi, bytes;  // offsets of row 0 of psi and phi, size of the stage
+};
+template <class R, bool CPLX, bool NU>
+__host__ __device__ __forceinline__ XyStage xy_stage(int rows, int TW, int skip) {
+   constexpr int esz = (int) sizeof(R) * (CPLX ? 2 : 1);
+   XyStage g;
+   g.psi = sweep_pad(skip, TW, esz);
+   g.phi = g.bytes = g.psi + (uint32_t) ((rows * TW * esz + 127) & ~127);
+   if (NU) {
+      g.phi += sweep_pad(skip, TW, (int) sizeof(R));
+      g.bytes = g.phi + (uint32_t) ((rows * TW * (int) sizeof(R) + 127) & ~127);
+   }
+   return g;
+}
+
+// calcnu's per-x table staged in shared memory (FP64: the tiles leave little
+// L1 for it), with `skip` zero entries before index 0.
+template <bool CPLX> __device__ __forceinline__ void stage_xtab(double *xtab, const void *ex, int n, int skip) {
+   constexpr int E = CPLX ? 2 : 1;
+   const double *src = (const double *) ex;
+   for (int e = threadIdx.x; e < E * (n + skip); e += blockDim.x) xtab[e] = e < E * skip ? 0. : src[e - E * skip];
+}
 
 // x or y sweep.  Tile: TW consecutive z columns of one y (x sweep) or one x
 // (y sweep) plane, the whole line along the swept axis, brought in by TMA.
 // With NU the x sweep first applies the pending 1/norm and calcnu to the tile
 // (needs phi).
 template <class R, bool CPLX, int AXIS, bool NU, int MSEG, int S, int TWC>
-__global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) k_sweep_xy(const __grid_constant__ CUtensorMap tm_psi,
+__global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k_sweep_xy(const __grid_constant__ CUtensorMap tm_psi,
                                                      const __grid_constant__ CUtensorMap tm_phi, Dims d, SegTab tb,
                                                      Trap trap, LinPhase lin, double g, double gd, double dt,
                                                      const State *__restrict__ st, int tw_arg, int boxn, int nbox,
@@ -468,19 +627,19 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) k_sweep_xy(const 
    const int n = tb.n;
    const int rows = boxn * nbox;  // rows staged (>= n)
    constexpr int E = CPLX ? 2 : 1;
-   const uint32_t psi_bytes = (uint32_t) (rows * TW * sizeof(P));
-   const uint32_t phi_bytes = NU ? (uint32_t) (rows * TW * sizeof(R)) : 0u;
-   const uint32_t stage_bytes = (psi_bytes + phi_bytes + 127u) & ~127u;
-   // layout: S stages of (tile | phi tile) | block maps  (TMA targets 128-byte aligned)
+   const XyStage lay = xy_stage<R, CPLX, NU>(rows, TW, tb.skip);
+   const uint32_t tx = (uint32_t) (rows * TW * sizeof(P)) + (NU ? (uint32_t) (rows * TW * sizeof(R)) : 0u);
+   // layout: S stages | exchange buffer | calcnu table  (TMA targets 128-byte aligned)
    unsigned char *base = (unsigned char *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
-   P *blk = (P *) (base + S * stage_bytes);
+   P *xch = (P *) (base + S * lay.bytes);
+   double *xtab = (double *) (xch + 2 * tb.P * TW);
    const int nzb = (d.nz + TW - 1) / TW;
    const int ntiles = (AXIS == 0 ? d.ny : d.nx) * nzb;
    auto copy_tile = [&](int t, int q, bool load) {
       const int other = t / nzb, z0 = (t - other * nzb) * TW;
-      P *tile = (P *) (base + q * stage_bytes);
-      R *ptile = (R *) (tile + rows * TW);
-      if (load) mbar_arrive_expect_tx(&full[q], psi_bytes + phi_bytes);
+      P *tile = (P *) (base + q * lay.bytes + lay.psi);
+      R *ptile = (R *) (base + q * lay.bytes + lay.phi);
+      if (load) mbar_arrive_expect_tx(&full[q], tx);
       for (int b = 0; b < nbox; b++) {
          const int a0 = b * boxn;
          if (load) {
@@ -497,17 +656,7 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) k_sweep_xy(const 
       }
       if (!load) bulk_commit();
    };
-   // FP64: calcnu's per-x factor (the phase exp(-i dt V_x) in real time,
-   // exp(-dt V_x) in imaginary time) staged once per CTA after the block
-   // maps, the shared tiles leaving little L1 for the tables (real-time x
-   // sweep 223 -> 219 us at 256^3 when it held x^2; the FP32 sweep reads its
-   // tables from global)
-   double *xtab = (double *) (blk + 2 * (((tb.P + 32 / TW - 1) / (32 / TW)) + 1) * TW);
-   if constexpr (NU && AXIS == 0 && std::is_same<R, double>::value) {
-      // imaginary time: exp(-dt V_x); real time: (cos, sin) of -dt V_x
-      const double *src = (const double *) lin.ex;
-      for (int e = threadIdx.x; e < (CPLX ? 2 : 1) * n; e += blockDim.x) xtab[e] = src[e];
-   }
+   if constexpr (NU && std::is_same<R, double>::value) stage_xtab<CPLX>(xtab, lin.ex, n, tb.skip);
    if (threadIdx.x == 0) {
       for (int q = 0; q < S; q++) mbar_init(&full[q], 1);
       fence_mbar_init();
@@ -526,20 +675,16 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) k_sweep_xy(const 
       }
       // a timed-out copy makes the whole CTA leave together
       if (__syncthreads_or(!mbar_wait(&full[q], (i / S) & 1, err))) break;
-      P *tile = (P *) (base + q * stage_bytes);
-      const int other = t / nzb, z0 = (t - other * nzb) * TW;
-      if constexpr (NU && std::is_same<R, double>::value) {
-         nu_pass_fp64<R, CPLX, AXIS>(tile, (const R *) (tile + rows * TW), n, lg, c, other, z0, d, trap, lin, xtab, g,
-                                     gd, dt, scale);
-         __syncthreads();
-      }
-      if constexpr (NU && std::is_same<R, float>::value) {
+      P *col = (P *) (base + q * lay.bytes + lay.psi) + c;
+      if constexpr (NU) {
          static_assert(AXIS == 0, "calcnu is fused into the x sweep only");
-         const NuTrap32<CPLX> xf = nu_reads_fp32<CPLX>((const float *) (tile + rows * TW) + c, TW, other, z0, c, d,
-                                                       trap, lin, g, gd, dt, scale);
-         seg_sweep<R, CPLX, MSEG, TWC>(tile, TW, 1, c, p, TW, tb, blk, nullptr, nullptr, nullptr, nullptr, xf);
+         const int other = t / nzb, z0 = (t - other * nzb) * TW;
+         seg_sweep<R, CPLX, MSEG, false, false, 0>(
+             col, TW, p, tb, xch + c, TW,
+             nu_xf<R, CPLX>((R *) (base + q * lay.bytes + lay.phi) + c, TW, other, z0, c, d, trap, lin,
+                            xtab + E * tb.skip, g, gd, dt, scale));
       } else {
-         seg_sweep<R, CPLX, MSEG, TWC>(tile, TW, 1, c, p, TW, tb, blk, nullptr, nullptr);
+         seg_sweep<R, CPLX, MSEG, false, false, 0>(col, TW, p, tb, xch + c, TW, NoXf());
       }
       fence_proxy_async();
       __syncthreads();
@@ -548,59 +693,100 @@ __global__ void __launch_bounds__(256, kSweepCtas[NU ? 1 : 0]) k_sweep_xy(const 
    if (threadIdx.x == 0) bulk_wait_all();
 }
 
-// The z sweep of one staged tile of TR rows (nr of them inside the grid)
-// starting at grid row row0, with the Simpson row partials of MOM >= 1; ends
-// with the tile written back in shared memory and a CTA barrier (the caller
-// then stores it).
-template <class R, bool CPLX, int MOM, int MSEG, int TWC, bool STAB>
-__device__ __forceinline__ void zsweep_tile(typename Tr<R, CPLX>::P *tile, int nr, int TR, int LS, int c, int p,
-                                            const SegTab &tbs, typename Tr<R, CPLX>::P *blk, double *part,
+// Entries before element 0 of a staged z row (room for the zero entries,
+// rounded so that element 0 stays 16-byte aligned) and the row stride: an odd
+// number of 16-byte units, so that the rows of a warp fall on different banks.
+__host__ __device__ __forceinline__ int zrow_pad(int skip, int esz) {
+   const int u = 16 / esz;
+   return (skip + u - 1) / u * u;
+}
+__host__ __device__ __forceinline__ int zrow_stride(int nz, int skip, int esz) {
+   const int u = 16 / esz;
+   const int units = (nz + zrow_pad(skip, esz) + u - 1) / u;
+   return (units | 1) * u;
+}
+
+// The z sweep of one staged tile of TR rows (nr of them inside the grid;
+// `rows` is element 0 of the first, LS the row stride) starting at grid row
+// row0, with the Simpson row partials of MOM >= 1; ends with the tile written
+// back in shared memory and a CTA barrier (the caller then stores it).
+template <class R, bool CPLX, int MOM, int MSEG, bool STAB, bool ANY>
+__device__ __forceinline__ void zsweep_tile(typename Tr<R, CPLX>::P *rows, int nr, int TR, int LS, int c, int p,
+                                            const SegTab &tbs, typename Tr<R, CPLX>::P *xch, double *part,
                                             double *part2, const double *__restrict__ wz,
                                             const double *__restrict__ wz2, double hz3, double *__restrict__ rowsum,
                                             double *__restrict__ rowsum2, long long row0) {
    using P = typename Tr<R, CPLX>::P;
    constexpr bool SIMP = MOM >= 1;
    if (nr < TR) {  // rows beyond the grid are zero so their sweep stays finite
-      for (int e = threadIdx.x; e < (TR - nr) * LS; e += blockDim.x) tile[nr * LS + e] = zero_of<P>();
+      for (int e = threadIdx.x; e < (TR - nr) * tbs.n; e += blockDim.x)
+         rows[(nr + e / tbs.n) * LS + e % tbs.n] = zero_of<P>();
       __syncthreads();
    }
    double my = 0., my2 = 0.;
-   seg_sweep<R, CPLX, MSEG, TWC, NoXf, STAB>(tile, 1, LS, c, p, TR, tbs, blk, SIMP ? wz : nullptr, SIMP ? &my : nullptr,
-                                             MOM == 2 ? wz2 : nullptr, MOM == 2 ? &my2 : nullptr);
+   if constexpr (ANY)
+      seg_sweep_any<R, CPLX, MSEG, true, STAB, MOM>(rows + c * LS, 1, p, tbs, xch + c, TR, NoXf(), wz, wz2, &my, &my2);
+   else
+      seg_sweep<R, CPLX, MSEG, true, STAB, MOM>(rows + c * LS, 1, p, tbs, xch + c, TR, NoXf(), wz, wz2, &my, &my2);
    if (SIMP && p < tbs.P) part[p * TR + c] = my;
    if (MOM == 2 && p < tbs.P) part2[p * TR + c] = my2;
    fence_proxy_async();
    __syncthreads();
-   // row rr's sums on the last warp, so that warp 0 (whose thread 0 issues
-   // the tile's store and the next load) goes on at once (TR <= 32)
-   const int rr = (int) threadIdx.x - ((int) blockDim.x - 32);
-   if (SIMP && rr >= 0 && rr < nr) {
-      double sum = 0.;
-      for (int pp = 0; pp < tbs.P; pp++) sum += part[pp * TR + rr];
-      if (MOM == 1 && !(tbs.n & 1)) {
-         // the end correction of an even nz: the weights of points nz-2 and
-         // nz-3 are 3 and 3.75 where the interior weights give 2 and 4
-         const int n = tbs.n;
-         const typename Tr<R, CPLX>::P *row = tile + rr * LS;
-         sum += (double) dens2(row[n - 2]) - 0.25 * (double) dens2(row[n - 3]);
+   // the rows' sums on the last warp, so that warp 0 (whose lanes issue the
+   // tile's store and the next load) goes on at once: 32 / TR lanes per row
+   const int ln = (int) threadIdx.x - ((int) blockDim.x - 32);
+   if (SIMP && ln >= 0) {
+      const int rr = ln % TR;
+      double sum = 0., sum2 = 0.;
+      if (rr < nr)
+         for (int pp = ln / TR; pp < tbs.P; pp += 32 / TR) {
+            sum += part[pp * TR + rr];
+            if (MOM == 2) sum2 += part2[pp * TR + rr];
+         }
+      for (int q = TR; q < 32; q <<= 1) {
+         sum += __shfl_xor_sync(0xffffffffu, sum, q);
+         if (MOM == 2) sum2 += __shfl_xor_sync(0xffffffffu, sum2, q);
       }
-      rowsum[row0 + rr] = sum * hz3;
-      if (MOM == 2) {
-         double sum2 = 0.;
-         for (int pp = 0; pp < tbs.P; pp++) sum2 += part2[pp * TR + rr];
-         rowsum2[row0 + rr] = sum2 * hz3;
+      if (ln < nr) {
+         if (MOM == 1 && !(tbs.n & 1)) {
+            // the end correction of an even nz: the weights of points nz-2
+            // and nz-3 are 3 and 3.75 where the interior weights give 2 and 4
+            const int n = tbs.n;
+            const P *row = rows + rr * LS;
+            sum += (double) dens2(row[n - 2]) - 0.25 * (double) dens2(row[n - 3]);
+         }
+         rowsum[row0 + rr] = sum * hz3;
+         if (MOM == 2) rowsum2[row0 + rr] = sum2 * hz3;
       }
    }
 }
 
+// FP64: the coefficient tables staged in shared memory once per CTA, the
+// shared rows leaving little L1 for them (z sweep 129 -> 128 us real, 94 -> 93
+// us imaginary time at 256^3; FP32 measured slower with it).  4 P m entries.
+template <bool CPLX> __device__ __forceinline__ SegTab stage_segtab(double *tabs, const SegTab &tb) {
+   const int ne = tb.P * tb.m * (CPLX ? 2 : 1);
+   SegTab o = tb;
+   for (int e = threadIdx.x; e < ne; e += blockDim.x) {
+      tabs[e] = ((const double *) tb.ga)[e];
+      tabs[ne + e] = ((const double *) tb.ma)[e];
+      tabs[2 * ne + e] = ((const double *) tb.ma)[ne + e];
+      tabs[3 * ne + e] = ((const double *) tb.nn)[e];
+   }
+   o.ga = tabs;
+   o.ma = tabs + ne;
+   o.nn = tabs + 3 * ne;
+   return o;
+}
+
 // z sweep.  Tile: TR consecutive (x, y) rows, each copied by one bulk copy to
-// a padded shared row (stride LS elements).  With MOM >= 1 every row also
-// yields its Simpson integral of |psi'|^2 over z (simpint, diffint.cu:106),
-// for the norm of the step (rowsum); with MOM = 2 also that of z^2 |psi'|^2
-// (rowsum2), the row partials of calcrms, so an rms sample after the step
-// needs no extra pass over psi.
+// a padded shared row (zrow_pad, stride LS elements).  With MOM >= 1 every row
+// also yields its Simpson integral of |psi'|^2 over z (simpint,
+// diffint.cu:106), for the norm of the step (rowsum); with MOM = 2 also that
+// of z^2 |psi'|^2 (rowsum2), the row partials of calcrms, so an rms sample
+// after the step needs no extra pass over psi.
 template <class R, bool CPLX, int MOM, int MSEG, int S, int TWC>
-__global__ void __launch_bounds__(256, kSweepCtas[0]) k_sweep_z(typename Tr<R, CPLX>::P *__restrict__ psi, Dims d, SegTab tb,
+__global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k_sweep_z(typename Tr<R, CPLX>::P *__restrict__ psi, Dims d, SegTab tb,
                                                     int tr_arg, int LS, const double *__restrict__ wz,
                                                     const double *__restrict__ wz2, double hz3,
                                                     double *__restrict__ rowsum, double *__restrict__ rowsum2,
@@ -614,38 +800,31 @@ __global__ void __launch_bounds__(256, kSweepCtas[0]) k_sweep_z(typename Tr<R, C
    const int nz = d.nz;
    const uint32_t row_bytes = (uint32_t) (nz * sizeof(P));
    const uint32_t stage_bytes = ((uint32_t) (TR * LS * sizeof(P)) + 127u) & ~127u;
-   // layout: S stages of rows | block maps | Simpson partials
+   const int pad = zrow_pad(tb.skip, (int) sizeof(P));
+   // layout: S stages of rows | exchange buffer | Simpson partials | FP64 tables
    unsigned char *base = (unsigned char *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
-   const int NW = (tb.P + 32 / TR - 1) / (32 / TR);
-   P *blk = (P *) (base + S * stage_bytes);
-   double *part = (double *) (blk + 2 * (NW + 1) * TR);
+   P *xch = (P *) (base + S * stage_bytes);
+   double *part = (double *) ((unsigned char *) xch + ((2 * tb.P * TR * sizeof(P) + 15) & ~(size_t) 15));
    double *part2 = part + tb.P * TR;
-   // FP64: the coefficient tables (alpha, gamma, M, N) staged once per CTA,
-   // the shared rows leaving little L1 for them (z sweep 129 -> 128 us real,
-   // 94 -> 93 us imaginary time at 256^3; FP32 measured slower with it)
    constexpr bool STAB = std::is_same<R, double>::value;
-   constexpr int TE = CPLX ? 2 : 1;  // doubles per entry
    double *tabs = part2 + tb.P * TR;
    SegTab tbs = tb;
-   if constexpr (STAB) {
-      const void *src[4] = {tb.al, tb.ga, tb.M, tb.N};
-      for (int a = 0; a < 4; a++)
-         for (int e = threadIdx.x; e < tb.n * TE; e += blockDim.x) tabs[a * tb.n * TE + e] = ((const double *) src[a])[e];
-      tbs.al = tabs;
-      tbs.ga = tabs + tb.n * TE;
-      tbs.M = tabs + 2 * tb.n * TE;
-      tbs.N = tabs + 3 * tb.n * TE;
-   }
+   if constexpr (STAB) tbs = stage_segtab<CPLX>(tabs, tb);
    const int ntiles = (int) ((d.nxy + TR - 1) / TR);
    auto nrows = [&](int t) -> int {
       const long long r0 = (long long) t * TR;
       return (int) ((d.nxy - r0) < TR ? (d.nxy - r0) : TR);
    };
+   // one bulk copy per row, issued by the lanes of warp 0 (one thread issuing
+   // them kept the CTA waiting); every lane commits and waits for its own
+   // store groups
+   const int lane = threadIdx.x & 31;
    auto copy_tile = [&](int t, int q, bool load) {
-      P *tile = (P *) (base + q * stage_bytes);
+      P *tile = (P *) (base + q * stage_bytes) + pad;
       const int nr = nrows(t);
-      if (load) mbar_arrive_expect_tx(&full[q], row_bytes * nr);
-      for (int r = 0; r < nr; r++) {
+      if (load && lane == 0) mbar_arrive_expect_tx(&full[q], row_bytes * nr);
+      __syncwarp();
+      for (int r = lane; r < nr; r += 32) {
          P *g = psi + ((long long) t * TR + r) * nz;
          if (load) bulk_load(tile + r * LS, g, row_bytes, &full[q]);
          else bulk_store(g, tile + r * LS, row_bytes);
@@ -657,22 +836,22 @@ __global__ void __launch_bounds__(256, kSweepCtas[0]) k_sweep_z(typename Tr<R, C
       fence_mbar_init();
    }
    __syncthreads();
-   if (threadIdx.x == 0 && (int) blockIdx.x < ntiles) copy_tile(blockIdx.x, 0, true);
+   if (threadIdx.x < 32 && (int) blockIdx.x < ntiles) copy_tile(blockIdx.x, 0, true);
    const int c = threadIdx.x % TR, p = threadIdx.x / TR;
    int i = 0;
    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, i++) {
       const int q = i % S;
-      if (threadIdx.x == 0 && t + (int) gridDim.x < ntiles) {
+      if (threadIdx.x < 32 && t + (int) gridDim.x < ntiles) {
          wait_stage_free<S>();
          copy_tile(t + gridDim.x, (i + 1) % S, true);
       }
       if (__syncthreads_or(!mbar_wait(&full[q], (i / S) & 1, err))) break;
-      P *tile = (P *) (base + q * stage_bytes);
-      zsweep_tile<R, CPLX, MOM, MSEG, TWC, STAB>(tile, nrows(t), TR, LS, c, p, tbs, blk, part, part2, wz, wz2, hz3,
-                                                rowsum, rowsum2, (long long) t * TR);
-      if (threadIdx.x == 0) copy_tile(t, q, false);
+      P *rows = (P *) (base + q * stage_bytes) + pad;
+      zsweep_tile<R, CPLX, MOM, MSEG, STAB, false>(rows, nrows(t), TR, LS, c, p, tbs, xch, part, part2, wz, wz2, hz3, rowsum,
+                                            rowsum2, (long long) t * TR);
+      if (threadIdx.x < 32) copy_tile(t, q, false);
    }
-   if (threadIdx.x == 0) bulk_wait_all();
+   if (threadIdx.x < 32) bulk_wait_all();
 }
 
 }  // namespace gpe

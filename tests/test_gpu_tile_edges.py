@@ -1,0 +1,85 @@
+"""The sweeps, FFT passes and observables at the sizes where their tiles and
+segments can go wrong (GPU), against the oracle.
+
+Tolerances: FP64 <= 1e-12 of the largest value, the bar of the operator tests.
+Mixed precision: an operator's FP32 arithmetic is a few roundings per point
+along a contracting recurrence or of log2 n stages, each 2^-24 = 6e-8; 2e-6
+leaves a factor of thirty.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = {0: 1e-12, 1: 2e-6}
+
+
+def rel(a, b):
+    return float(np.max(np.abs(a - b)) / np.max(np.abs(b)))
+
+
+def pair(gpe, oracle_mod, mode, prec, n, dtf=0.1, seed=0):
+    """A handle and the oracle with the same random psi (exact in FP32)."""
+    dx = 0.25
+    args = (*n, dx, 1.1 * dx, 0.9 * dx, dtf * dx * dx, 0.5, 1.0, 1.5, 0.5 * min(n) * dx)
+    s, o = gpe.Solver(gpe.make_params(mode, *args, precision=prec)), oracle_mod.Oracle(mode, 1, *args)
+    r = np.random.default_rng(seed)
+    psi = r.standard_normal(n).astype(np.float32).astype(np.float64)
+    if mode:
+        psi = psi + 1j * r.standard_normal(n).astype(np.float32)
+    s.set_psi(psi)
+    o.set_psi(psi)
+    return s, o, psi
+
+
+# line lengths: one segment, a full last segment, every remainder class, the
+# longest; time steps whose carries reach one, several and all segments
+@pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("n,dtf", [((8, 10, 8), .1), ((18, 36, 20), 1.), ((60, 50, 36), 3.), ((1024, 8, 8), .1),
+                                   ((8, 1024, 8), .3), ((8, 8, 1024), 1.), ((150, 96, 100), 3.)])
+def test_sweeps_at_segment_edges(gpe_lib, oracle_mod, mode, prec, n, dtf):
+    s, o, psi = pair(gpe_lib, oracle_mod, mode, prec, n, dtf)
+    for name in ("calclux", "calcluy", "calcluz"):
+        s.set_psi(psi)
+        o.set_psi(psi)
+        getattr(s, name)()
+        getattr(o, name)()
+        assert rel(s.get_psi(), o.get_psi()) <= TOL[prec], name
+    s.close()
+    o.close()
+
+
+@pytest.mark.parametrize("prec,tw,n", [(0, 4, (18, 10, 48)), (1, 4, (18, 10, 48)), (0, 2, (10, 18, 12)),
+                                       (1, 8, (20, 12, 20))])
+def test_narrow_tiles_keep_copies_aligned(gpe_lib, oracle_mod, prec, tw, n):
+    """Tiles whose bytes are no multiple of 128: the phi tile behind the psi
+    tile starts on a 128-byte boundary all the same."""
+    s, o, psi = pair(gpe_lib, oracle_mod, 0, prec, n)
+    t = gpe_lib.Tuning()
+    t.sweep_tw[0] = t.sweep_tw[1] = t.sweep_tw[2] = tw
+    s.set_tuning(t)
+    s.calcnorm(True)
+    o.calcnorm(True)
+    s.run(2, 20., 5.)
+    o.run(2, 20., 5.)
+    assert rel(s.get_psi(), o.get_psi()) <= TOL[prec]
+    s.close()
+    o.close()
+
+
+# exponents beyond each series' range: the per-point fallback of calcnu
+@pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("g", [1., 60., 2000.])
+def test_calcnu_exponent_ranges(gpe_lib, oracle_mod, mode, prec, g):
+    s, o, _ = pair(gpe_lib, oracle_mod, mode, prec, (30, 24, 20), 0.3)
+    s.run(1, g, 0.)
+    o.run(1, g, 0.)
+    a, b = s.get_psi(), o.get_psi()
+    # mixed precision in real time: the FP32 phase itself is rounded, to 2^-24
+    # of its largest value, dt (V + g |psi|^2) <= 0.3 dx^2 (60 + 40 g)
+    tol = max(TOL[prec], 2 ** -23 * 0.02 * (60. + 40. * g)) if prec and mode else TOL[prec]
+    if prec and not mode:
+        tol = max(tol, 2 ** -22 * 0.02 * 40. * g)
+    assert rel(a, b) <= tol
+    s.close()
+    o.close()
