@@ -1367,22 +1367,48 @@ gpe_status Impl<R, CPLX>::density(gpe_solver *s, int kind, long sx, long sy, lon
    if (!(s)) return fail(GPE_ERR_PARAM, "null solver handle")
 
 // ------------------------------------------------------------------ psi I/O
-// FP64 psi is copied as is (the host layout equals the device layout); the
-// mixed-precision handle converts through a host float buffer.
+// FP64 arrays are copied as they are (the host layout equals the device
+// layout).  A mixed-precision handle converts on the device, through the
+// spectrum buffer in pieces (its contents live only inside one convolution):
+// converting on the host, through a buffer allocated for the call, took 220
+// ms for 512x512x256 points, whose copy takes 10 ms.
+static gpe_status fetch(gpe_solver *s, double *host, const void *dev, size_t nd) {
+   if (!s->fp32) {
+      CK(cudaMemcpyAsync(host, dev, sizeof(double) * nd, cudaMemcpyDeviceToHost, s->st));
+   } else {
+      const size_t cap = s->esz_c * (size_t) s->d.nzp * (size_t) s->d.nxy / sizeof(double);
+      for (size_t at = 0; at < nd; at += cap) {
+         const size_t m = std::min(cap, nd - at);
+         k_convert<<<(unsigned) std::min<size_t>(592, (m + 255) / 256), 256, 0, s->st>>>(
+             (double *) s->spec, (const float *) dev + at, (long long) m);
+         CKL();
+         CK(cudaMemcpyAsync(host + at, s->spec, sizeof(double) * m, cudaMemcpyDeviceToHost, s->st));
+         s->launches++;
+      }
+   }
+   CK(cudaStreamSynchronize(s->st));
+   return GPE_OK;
+}
+
 extern "C" gpe_status gpe_set_psi(gpe_solver *s, const double *psi) {
    CHECK_HANDLE(s);
    if (!psi) return fail(GPE_ERR_PARAM, "null psi");
    CK(cudaSetDevice(s->dev));
    const size_t nd = (size_t) s->d.npts * (s->cplx ? 2 : 1);
    if (s->fp32) {
-      std::vector<float> b(nd);
-      for (size_t q = 0; q < nd; q++) b[q] = (float) psi[q];
-      CK(cudaMemcpyAsync(s->psi, b.data(), sizeof(float) * nd, cudaMemcpyHostToDevice, s->st));
-      CK(cudaStreamSynchronize(s->st));
+      const size_t cap = s->esz_c * (size_t) s->d.nzp * (size_t) s->d.nxy / sizeof(double);
+      for (size_t at = 0; at < nd; at += cap) {
+         const size_t m = std::min(cap, nd - at);
+         CK(cudaMemcpyAsync(s->spec, psi + at, sizeof(double) * m, cudaMemcpyHostToDevice, s->st));
+         k_convert<<<(unsigned) std::min<size_t>(592, (m + 255) / 256), 256, 0, s->st>>>(
+             (float *) s->psi + at, (const double *) s->spec, (long long) m);
+         CKL();
+         s->launches++;
+      }
    } else {
       CK(cudaMemcpyAsync(s->psi, psi, sizeof(double) * nd, cudaMemcpyHostToDevice, s->st));
-      CK(cudaStreamSynchronize(s->st));
    }
+   CK(cudaStreamSynchronize(s->st));
    k_state_set<<<1, 1, 0, s->st>>>(s->state, 1.);
    CKL();
    return GPE_OK;
@@ -1392,17 +1418,7 @@ extern "C" gpe_status gpe_get_psi(gpe_solver *s, double *psi) {
    CHECK_HANDLE(s);
    if (!psi) return fail(GPE_ERR_PARAM, "null psi");
    CK(cudaSetDevice(s->dev));
-   const size_t nd = (size_t) s->d.npts * (s->cplx ? 2 : 1);
-   if (s->fp32) {
-      std::vector<float> b(nd);
-      CK(cudaMemcpyAsync(b.data(), s->psi, sizeof(float) * nd, cudaMemcpyDeviceToHost, s->st));
-      CK(cudaStreamSynchronize(s->st));
-      for (size_t q = 0; q < nd; q++) psi[q] = b[q];
-   } else {
-      CK(cudaMemcpyAsync(psi, s->psi, sizeof(double) * nd, cudaMemcpyDeviceToHost, s->st));
-      CK(cudaStreamSynchronize(s->st));
-   }
-   return GPE_OK;
+   return fetch(s, psi, s->psi, (size_t) s->d.npts * (s->cplx ? 2 : 1));
 }
 
 // initpsi Gaussian (imag3d-mpicuda.cu:835-867), evaluated on the host like
@@ -1590,17 +1606,7 @@ extern "C" gpe_status gpe_get_phi(gpe_solver *s, double *phi) {
    CHECK_HANDLE(s);
    if (!phi) return fail(GPE_ERR_PARAM, "null phi");
    CK(cudaSetDevice(s->dev));
-   const long long n = s->d.npts;
-   if (s->fp32) {
-      std::vector<float> b((size_t) n);
-      CK(cudaMemcpyAsync(b.data(), s->phi, sizeof(float) * n, cudaMemcpyDeviceToHost, s->st));
-      CK(cudaStreamSynchronize(s->st));
-      for (long long q = 0; q < n; q++) phi[q] = b[(size_t) q];
-   } else {
-      CK(cudaMemcpyAsync(phi, s->phi, sizeof(double) * n, cudaMemcpyDeviceToHost, s->st));
-      CK(cudaStreamSynchronize(s->st));
-   }
-   return GPE_OK;
+   return fetch(s, phi, s->phi, (size_t) s->d.npts);
 }
 
 extern "C" gpe_status gpe_calcnu(gpe_solver *s, double g, double gd) {

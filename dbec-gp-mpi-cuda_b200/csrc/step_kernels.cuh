@@ -653,6 +653,13 @@ __global__ void k_gather_dens(const typename Tr<R, CPLX>::P *__restrict__ psi, D
    }
 }
 
+// n elements of one type to the other (psi and phi of mixed-precision handles
+// on their way to and from the caller's FP64 arrays).
+template <class D, class S> __global__ void k_convert(D *__restrict__ dst, const S *__restrict__ src, long long n) {
+   for (long long q = blockIdx.x * (long long) blockDim.x + threadIdx.x; q < n; q += (long long) gridDim.x * blockDim.x)
+      dst[q] = (D) src[q];
+}
+
 template <class R, bool CPLX>
 __global__ void k_init_density(typename Tr<R, CPLX>::P *__restrict__ psi, const double *__restrict__ rho, long long n) {
    using P = typename Tr<R, CPLX>::P;

@@ -83,3 +83,16 @@ def test_calcnu_exponent_ranges(gpe_lib, oracle_mod, mode, prec, g):
     assert rel(a, b) <= tol
     s.close()
     o.close()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [(8, 8, 8), (10, 12, 20), (64, 40, 48)])
+def test_mixed_psi_round_trip_is_exact(gpe_lib, mode, n):
+    """psi of a mixed-precision handle is the caller's FP64 psi rounded once to
+    FP32, in pieces of the spectrum buffer."""
+    s = gpe_lib.Solver(gpe_lib.make_params(mode, *n, .25, .25, .25, .006, 1., 1., 1., 1., precision=1))
+    r = np.random.default_rng(3)
+    psi = r.standard_normal(n) + (1j * r.standard_normal(n) if mode else 0.)
+    s.set_psi(psi)
+    assert np.array_equal(s.get_psi(), psi.astype(np.complex64 if mode else np.float32))
+    s.close()
