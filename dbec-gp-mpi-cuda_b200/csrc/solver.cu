@@ -1069,10 +1069,21 @@ template <class R, bool CPLX> struct Impl {
       return GPE_OK;
    }
 
-   static gpe_status calcnorm(gpe_solver *s, bool renorm) {
+   static void rows_dens(gpe_solver *s, double *a, double *b) {
+      k_rows_dens<R, CPLX><<<blocks_for(s->d.nxy, kRowWarps), 32 * kRowWarps, 0, s->st>>>(
+          (const P *) s->psi, s->d, s->p.dz / 3., s->wz, s->wz2, a, b);
+   }
+
+   // line integrals of |psi|^2 along `axis` into rowA (z: a warp per row)
+   static void lineint(gpe_solver *s, int axis, double h) {
       const Dims &d = s->d;
-      k_rows_dens<R, CPLX><<<blocks_for(d.nxy, 128), 128, 0, s->st>>>((const P *) s->psi, d, s->p.dz, s->rowA, nullptr,
-                                                                     s->z2);
+      if (axis == 2) return rows_dens(s, s->rowA, nullptr);
+      const long long nl = (long long) (axis == 0 ? d.ny : d.nx) * d.nz;
+      k_lineint_psi<R, CPLX><<<blocks_for(nl, 128), 128, 0, s->st>>>((const P *) s->psi, d, axis, h, s->rowA);
+   }
+
+   static gpe_status calcnorm(gpe_solver *s, bool renorm) {
+      rows_dens(s, s->rowA, nullptr);
       CKL();
       CKS(norm_final(s, s->obs));
       s->launches++;
@@ -1086,9 +1097,7 @@ template <class R, bool CPLX> struct Impl {
    }
 
    static gpe_status rms(gpe_solver *s, double *dev_out) {
-      const Dims &d = s->d;
-      k_rows_dens<R, CPLX><<<blocks_for(d.nxy, 128), 128, 0, s->st>>>((const P *) s->psi, d, s->p.dz, s->rowA, s->rowB,
-                                                                     s->z2);
+      rows_dens(s, s->rowA, s->rowB);
       CKL();
       s->launches++;
       return rms_final(s, dev_out);
@@ -1108,15 +1117,20 @@ template <class R, bool CPLX> struct Impl {
    static gpe_status muen(gpe_solver *s, double g, double gd, double *dev_out) {
       const Dims &d = s->d;
       CKS(psidd2(s));
-      k_muen_rows<R, CPLX><<<blocks_for(d.nxy, 128), 128, 0, s->st>>>((const P *) s->psi, (const R *) s->phi, d,
-                                                                     trap_of(s), g, gd, s->p.dx, s->p.dy, s->p.dz,
-                                                                     s->par, s->rowA, s->rowB);
+      // chunks of x planes so that about four CTAs per SM run, at least 16
+      // planes each (a chunk reads four more), with room for the partials
+      const unsigned bz = blocks_for(d.nz, kMuZ), by = blocks_for(d.ny, kMuY);
+      const long long want = std::max<long long>(1, 4LL * s->nsm / ((long long) bz * by));
+      const long long most = std::max<long long>(1, s->row_cap / (2LL * bz * by));
+      const int chunk = (int) std::max<long long>(std::min<long long>(16, d.nx), (d.nx + std::min(want, most) - 1) / std::min(want, most));
+      const unsigned bx = blocks_for(d.nx, chunk);
+      k_muen<R, CPLX><<<dim3(bz, by, bx), kMuY * kMuZ, 0, s->st>>>((const P *) s->psi, (const R *) s->phi, d, trap_of(s),
+                                                                  g, gd, s->p.dx, s->p.dy, s->p.dz, s->par, chunk,
+                                                                  s->rowA);
       CKL();
-      k_xy_final<<<1, 256, sizeof(double) * d.nx, s->st>>>(s->rowA, d, s->p.dx, s->p.dy, dev_out);
+      k_sum2<<<1, 256, 0, s->st>>>(s->rowA, (int) (bx * by * bz), s->p.dx * s->p.dy * s->p.dz / 27., dev_out);
       CKL();
-      k_xy_final<<<1, 256, sizeof(double) * d.nx, s->st>>>(s->rowB, d, s->p.dx, s->p.dy, dev_out + 1);
-      CKL();
-      s->launches += 3;
+      s->launches += 2;
       return GPE_OK;
    }
 
@@ -1281,8 +1295,7 @@ gpe_status Impl<R, CPLX>::density(gpe_solver *s, int kind, long sx, long sy, lon
       const int second = (keep == 0) ? 1 : 0;  // y for x profile, x otherwise
       const int o1 = first == 0 ? 1 : 0, o2 = first == 2 ? 1 : 2;  // axes of the 2D result
       if ((long long) n[o1] * n[o2] > s->row_cap) return fail(GPE_ERR_STATE, "row buffer too small");
-      k_lineint_psi<R, CPLX><<<blocks_for((long long) n[o1] * n[o2], 128), 128, 0, s->st>>>(psi, d, first, hh[first],
-                                                                                          s->rowA);
+      lineint(s, first, hh[first]);
       CKL();
       const int ax = (second == o1) ? 0 : 1;  // integrate rows (0) or columns (1)
       const int m = n[keep];
@@ -1301,8 +1314,7 @@ gpe_status Impl<R, CPLX>::density(gpe_solver *s, int kind, long sx, long sy, lon
       const int integ = 2 - (kind - GPE_DEN_2D_XY);  // xy -> z, xz -> y, yz -> x
       const int a1 = integ == 0 ? 1 : 0, a2 = integ == 2 ? 1 : 2;
       if ((long long) n[a1] * n[a2] > s->row_cap) return fail(GPE_ERR_STATE, "row buffer too small");
-      k_lineint_psi<R, CPLX><<<blocks_for((long long) n[a1] * n[a2], 128), 128, 0, s->st>>>(psi, d, integ, hh[integ],
-                                                                                          s->rowA);
+      lineint(s, integ, hh[integ]);
       CKL();
       s->launches++;
       buf.resize((size_t) n[a1] * n[a2]);

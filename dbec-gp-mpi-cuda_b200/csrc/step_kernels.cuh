@@ -391,23 +391,36 @@ __global__ void k_calcnu(typename Tr<R, CPLX>::P *__restrict__ psi, const R *__r
 // Reductions.
 // ===========================================================================
 
-// Per-row Simpson of |psi|^2 along z (no sweep).
+// Per-row Simpson integrals along z of |psi|^2 (rowA) and, with rowB, of z^2
+// |psi|^2, by a warp per row with the weights wz, wz2 (in units of h / 3): the
+// loads of a warp are consecutive and four rounds of them are in flight.  One
+// thread per row left the loads of a warp a row apart (96 us at 256^3 FP64,
+// whose 134 MB take 20 us).
+constexpr int kRowWarps = 8;
 template <class R, bool CPLX>
-__global__ void k_rows_dens(const typename Tr<R, CPLX>::P *__restrict__ psi, Dims d, double hz,
-                            double *__restrict__ rowA, double *__restrict__ rowB, const double *__restrict__ z2) {
-   const long long row = (long long) blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * kRowWarps) k_rows_dens(const typename Tr<R, CPLX>::P *__restrict__ psi, Dims d,
+                                                              double hz3, const double *__restrict__ wz,
+                                                              const double *__restrict__ wz2,
+                                                              double *__restrict__ rowA, double *__restrict__ rowB) {
+   const long long row = (long long) blockIdx.x * kRowWarps + threadIdx.x / 32;
    if (row >= d.nxy) return;
+   const int lane = threadIdx.x % 32;
    const auto *ps = psi + row * d.nz;
-   Simpson a, b;
-   a.init(d.nz);
-   b.init(d.nz);
-   for (int k = 0; k < d.nz; k++) {
+   double a = 0., b = 0.;
+#pragma unroll 4
+   for (int k = lane; k < d.nz; k += 32) {
       const double f = (double) dens2(ps[k]);
-      a.add(k, f);
-      if (rowB) b.add(k, z2[k] * f);
+      a = fma(wz[k], f, a);
+      if (rowB) b = fma(wz2[k], f, b);
    }
-   rowA[row] = a.finish(hz);
-   if (rowB) rowB[row] = b.finish(hz);
+   for (int o = 16; o; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (rowB) b += __shfl_xor_sync(0xffffffffu, b, o);
+   }
+   if (lane == 0) {
+      rowA[row] = a * hz3;
+      if (rowB) rowB[row] = b * hz3;
+   }
 }
 
 // norm = sqrt(S_x S_y rowsum) (calcnorm, imag3d-mpicuda.cu:1194-1218), stores
@@ -554,60 +567,115 @@ static __global__ void __launch_bounds__(32 * kNormRowsPerCta) k_rms_final(const
    }
 }
 
-// Generic S_x S_y of a per-row array (mu, E, norm).
-static __global__ void k_xy_final(const double *__restrict__ rowA, Dims d, double hx, double hy, double *__restrict__ out) {
-   extern __shared__ double tx[];
-   for (int i = threadIdx.x; i < d.nx; i += blockDim.x) tx[i] = simpint_arr(hy, rowA + (long long) i * d.ny, d.ny);
-   __syncthreads();
-   if (threadIdx.x == 0) *out = simpint_arr(hx, tx, d.nx);
-}
-
 // 4th-order first derivative with the reference's edge rules
-// (calcmuen_kernel1x/1y/1z, imag3d-mpicuda.cu:1293-1422).
-template <class F>
-__device__ __forceinline__ double fd4(F f, int i, int n, double h) {
+// (calcmuen_kernel1x/1y/1z, imag3d-mpicuda.cu:1293-1422) at index i of n from
+// the five values around it (those beyond the line are not used).
+__device__ __forceinline__ double fd4(double m2, double m1, double p1, double p2, int i, int n, double r2h,
+                                      double r12h) {
    if (i == 0 || i == n - 1) return 0.;
-   if (i == 1) return (f(2) - f(0)) / (2. * h);
-   if (i == n - 2) return (f(n - 1) - f(n - 3)) / (2. * h);
-   return (f(i - 2) - 8. * f(i - 1) + 8. * f(i + 1) - f(i + 2)) / (12. * h);
+   if (i == 1 || i == n - 2) return (p1 - m1) * r2h;
+   return (m2 - p2 + 8. * (p1 - m1)) * r12h;
 }
 
-// Per-row Simpson of the mu and E integrands (calcmuen_kernel2,
-// imag3d-mpicuda.cu:1424-1450); real time differentiates |psi| (real:1401).
+// mu and E (calcmuen_kernel2, imag3d-mpicuda.cu:1424-1450; real time
+// differentiates |psi|, real3d-mpicuda.cu:1401): a CTA owns kMuY rows of y by
+// kMuZ points of z and walks along x over a ring of kMuRing planes of |psi|
+// with their two-point halo, so each amplitude is loaded, and its square root
+// taken, once per tile and plane.  The integrands are summed with the product
+// of the Simpson weights of the three axes (the nested rule of simpint is
+// that product); part[2 CTA] receives the CTA's sums, k_sum2 adds them.  One
+// thread per (x, y) row walking z (32 rows apart in a warp's loads, 13 square
+// roots a point) took 2.5 ms at 256^3 complex FP64.
+constexpr int kMuY = 8, kMuZ = 32, kMuRing = 6;
 template <class R, bool CPLX>
-__global__ void k_muen_rows(const typename Tr<R, CPLX>::P *__restrict__ psi, const R *__restrict__ phi, Dims d,
-                            Trap trap, double g, double gd, double dx, double dy, double dz, double par,
-                            double *__restrict__ rowMu, double *__restrict__ rowEn) {
-   const long long row = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-   if (row >= d.nxy) return;
-   const int i = (int) (row / d.ny), j = (int) (row - (long long) i * d.ny);
-   const long long sx = (long long) d.ny * d.nz, sy = d.nz;
-   const auto *base = psi + row * d.nz;
-   const double invN = 1.0 / (double) d.npts;
-   auto amp = [&](const typename Tr<R, CPLX>::P &v) -> double {
-      if (CPLX) return sqrt((double) dens2(v));
-      return (double) *(const R *) &v;
+__global__ void __launch_bounds__(kMuY *kMuZ) k_muen(const typename Tr<R, CPLX>::P *__restrict__ psi,
+                                                     const R *__restrict__ phi, Dims d, Trap trap, double g, double gd,
+                                                     double dx, double dy, double dz, double par, int xchunk,
+                                                     double *__restrict__ part) {
+   constexpr int PY = kMuY + 4, PZ = kMuZ + 4, NT = kMuY * kMuZ;
+   __shared__ double ring[kMuRing][PY * PZ];
+   __shared__ double red[2 * NT / 32];
+   const int z0 = blockIdx.x * kMuZ, y0 = blockIdx.y * kMuY, x0 = blockIdx.z * xchunk;
+   const int x1 = min(x0 + xchunk, d.nx);
+   const int tz = threadIdx.x % kMuZ, ty = threadIdx.x / kMuZ;
+   const int j = y0 + ty, k = z0 + tz;
+   const bool in = j < d.ny && k < d.nz;
+   auto plane = [&](int x) {  // |psi| of plane x with the halo, zero outside the grid
+      double *r = ring[(x + kMuRing) % kMuRing];
+      for (int e = threadIdx.x; e < PY * PZ; e += NT) {
+         const int jj = y0 - 2 + e / PZ, kk = z0 - 2 + e % PZ;
+         double v = 0.;
+         if (x >= 0 && x < d.nx && jj >= 0 && jj < d.ny && kk >= 0 && kk < d.nz) {
+            const auto p = psi[((long long) x * d.ny + jj) * d.nz + kk];
+            if constexpr (CPLX) v = sqrt((double) dens2(p));
+            else v = (double) p;
+         }
+         r[e] = v;
+      }
    };
-   Simpson smu, sen;
-   smu.init(d.nz);
-   sen.init(d.nz);
-   for (int k = 0; k < d.nz; k++) {
-      const auto *pk = base + k;
-      const double ddx = fd4([&](int q) { return amp(pk[(long long) (q - i) * sx]); }, i, d.nx, dx);
-      const double ddy = fd4([&](int q) { return amp(pk[(long long) (q - j) * sy]); }, j, d.ny, dy);
-      const double ddz = fd4([&](int q) { return amp(base[q]); }, k, d.nz, dz);
-      double dpsi = (ddx * ddx) / (3. - par);
-      dpsi += (ddy * ddy) / (3. - par);
-      dpsi += (ddz * ddz) / (3. - par);
-      const double psi2 = (double) dens2(*pk);
-      const double psi2lin = psi2 * g;
-      const double psidd2lin = ((double) phi[row * d.nz + k] * invN) * gd;
-      const double tmppot = trap.v(i, j, k);
-      smu.add(k, (tmppot + psi2lin + psidd2lin) * psi2 + dpsi);
-      sen.add(k, (tmppot + 0.5 * psi2lin + 0.5 * psidd2lin) * psi2 + dpsi);
+   const double invN = 1.0 / (double) d.npts, ipar = 1. / (3. - par);
+   const double hx2 = 1. / (2. * dx), hx12 = 1. / (12. * dx), hy2 = 1. / (2. * dy), hy12 = 1. / (12. * dy),
+                hz2 = 1. / (2. * dz), hz12 = 1. / (12. * dz);
+   const double wyz = in ? simp_w(j, d.ny) * simp_w(k, d.nz) : 0.;
+   double mu = 0., en = 0.;
+   const int c = (ty + 2) * PZ + tz + 2;
+   for (int x = x0 - 2; x < x0 + 2; x++) plane(x);
+   for (int x = x0; x < x1; x++) {
+      plane(x + 2);
+      __syncthreads();  // the slot this fills was last read two iterations ago (six planes, five in use)
+      if (in) {
+         const double *r = ring[x % kMuRing];
+         auto rx = [&](int q) { return ring[(x + q + kMuRing) % kMuRing][c]; };
+         const double ddx = fd4(rx(-2), rx(-1), rx(1), rx(2), x, d.nx, hx2, hx12);
+         const double ddy = fd4(r[c - 2 * PZ], r[c - PZ], r[c + PZ], r[c + 2 * PZ], j, d.ny, hy2, hy12);
+         const double ddz = fd4(r[c - 2], r[c - 1], r[c + 1], r[c + 2], k, d.nz, hz2, hz12);
+         const double dpsi = (ddx * ddx + ddy * ddy + ddz * ddz) * ipar;
+         const long long q = ((long long) x * d.ny + j) * d.nz + k;
+         const double psi2 = (double) dens2(psi[q]);
+         const double lin = psi2 * g + ((double) phi[q] * invN) * gd;
+         const double v = trap.v(x, j, k), w = simp_w(x, d.nx) * wyz;
+         mu = fma(w, fma(v + lin, psi2, dpsi), mu);
+         en = fma(w, fma(v + 0.5 * lin, psi2, dpsi), en);
+      }
    }
-   rowMu[row] = smu.finish(dz);
-   rowEn[row] = sen.finish(dz);
+   for (int o = 16; o; o >>= 1) {
+      mu += __shfl_xor_sync(0xffffffffu, mu, o);
+      en += __shfl_xor_sync(0xffffffffu, en, o);
+   }
+   if (threadIdx.x % 32 == 0) {
+      red[threadIdx.x / 32] = mu;
+      red[NT / 32 + threadIdx.x / 32] = en;
+   }
+   __syncthreads();
+   if (threadIdx.x < 2) {
+      double s = 0.;
+      for (int w = 0; w < NT / 32; w++) s += red[threadIdx.x * (NT / 32) + w];
+      const long long cta = ((long long) blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+      part[2 * cta + threadIdx.x] = s;
+   }
+}
+
+// out[0] and out[1]: scaled sums of n pairs, in a fixed order (one CTA).
+static __global__ void __launch_bounds__(256) k_sum2(const double *__restrict__ part, int n, double scale,
+                                                    double *__restrict__ out) {
+   __shared__ double red[2][256];
+   double a = 0., b = 0.;
+   for (int e = threadIdx.x; e < n; e += 256) {
+      const double2 v = ((const double2 *) part)[e];
+      a += v.x;
+      b += v.y;
+   }
+   red[0][threadIdx.x] = a;
+   red[1][threadIdx.x] = b;
+   __syncthreads();
+   for (int h = 128; h; h >>= 1) {
+      if (threadIdx.x < h) {
+         red[0][threadIdx.x] += red[0][threadIdx.x + h];
+         red[1][threadIdx.x] += red[1][threadIdx.x + h];
+      }
+      __syncthreads();
+   }
+   if (threadIdx.x < 2) out[threadIdx.x] = red[threadIdx.x][0] * scale;
 }
 
 // ---- density outputs -------------------------------------------------------

@@ -85,6 +85,19 @@ def test_calcnu_exponent_ranges(gpe_lib, oracle_mod, mode, prec, g):
     o.close()
 
 
+@pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("n", [(8, 8, 8), (20, 18, 36), (10, 36, 100), (48, 50, 32)])
+def test_observables_at_tile_edges(gpe_lib, oracle_mod, mode, prec, n):
+    s, o, _ = pair(gpe_lib, oracle_mod, mode, prec, n)
+    assert s.calcnorm(False) == pytest.approx(o.calcnorm(False), rel=TOL[prec])
+    assert s.calcmuen(30., 8.) == pytest.approx(o.calcmuen(30., 8.), rel=TOL[prec])
+    assert np.allclose(s.calcrms(), o.calcrms(), rtol=TOL[prec], atol=0)
+    for k in ("1d_z", "2d_xy"):
+        assert rel(s.density(k), o.density(k)) <= TOL[prec], k
+    s.close()
+    o.close()
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("n", [(8, 8, 8), (10, 12, 20), (64, 40, 48)])
 def test_mixed_psi_round_trip_is_exact(gpe_lib, mode, n):
