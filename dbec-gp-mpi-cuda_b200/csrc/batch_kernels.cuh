@@ -33,9 +33,8 @@ struct SweepView {
    const State *st;
    uint32_t *err;
    void *psi;               // z sweep: psi rows
-   const double *wz, *wz2;  // z sweep: Simpson weights (norm, rms partials)
-   double *rowsum, *rowsum2;
-   double g, gd, dt, hz3;
+   ZOut zo;                 // z sweep: norm and rms partials
+   double g, gd, dt;
    int TW, boxn, nbox, LS;
 };
 
@@ -56,7 +55,7 @@ struct alignas(64) BatchDesc {
    const double *udd;
    State *state;
    uint32_t *err;
-   double *rowA, *xs;
+   double *rowA;
    double hx, hy;
    int LSr, LSo, boxy, nboxy, boxx, nboxx, Ly, Lx;
 };
@@ -166,13 +165,14 @@ __global__ void kb_phifix(const BatchDesc *__restrict__ tab, const unsigned *__r
    phifix_body<R>((R *) D.phi, d, r.local);
 }
 
-static __global__ void __launch_bounds__(32 * kNormRowsPerCta) kb_norm_final(const BatchDesc *__restrict__ tab,
-                                                                             const unsigned *__restrict__ work) {
+// The norm of one instance per CTA, from its z sweep's tile partials.
+static __global__ void __launch_bounds__(256) kb_norm_final(const BatchDesc *__restrict__ tab,
+                                                            const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
-   const Dims d = D.d;
-   norm_final_body(D.rowA, d, D.hx, D.hy, D.state, D.xs, nullptr, r.local,
-                   (d.nx + kNormRowsPerCta - 1) / kNormRowsPerCta);
+   __shared__ double red[256];
+   const double sum = sum_tiles(D.rowA, (int) ((D.d.nxy + D.sv[2].TW - 1) / D.sv[2].TW), red);
+   if (threadIdx.x == 0) set_norm(D.state, sum, D.hx, D.hy, nullptr);
 }
 
 // ------------------------------------------------------------------- sweeps
@@ -363,8 +363,8 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
       const long long r0 = (long long) r.local * TR;
       const int nr = (int) ((sv.d.nxy - r0) < TR ? (sv.d.nxy - r0) : TR);
       P *rows = (P *) (base + q * stage_bytes) + zrow_pad(sv.tb.skip, (int) sizeof(P));
-      zsweep_tile<R, CPLX, MOM, MSEG, STAB, true>(rows, nr, TR, sv.LS, c, p, tbs, xch, part, part2, sv.wz, sv.wz2, sv.hz3,
-                                               sv.rowsum, sv.rowsum2, r0);
+      zsweep_tile<R, CPLX, MOM, MSEG, STAB, true>(rows, nr, TR, sv.LS, c, p, tbs, xch, part, part2, sv.d,
+                                                        sv.zo, r0, r.local);
       if (threadIdx.x < 32) copy_tile(t, q, false);
    }
    if (threadIdx.x < 32) bulk_wait_all();

@@ -138,6 +138,34 @@ template <> __device__ __forceinline__ float zero_of<float>() { return 0.f; }
 template <> __device__ __forceinline__ double2 zero_of<double2>() { return make_double2(0., 0.); }
 template <> __device__ __forceinline__ float2 zero_of<float2>() { return make_float2(0.f, 0.f); }
 
+// Two adjacent elements of a shared-memory row in one access (s at an even
+// index of a 16-byte aligned row).  With a row stride of an odd number of
+// 16-byte units the rows that a phase of a warp touches fall on different
+// banks.
+template <class P> struct Pair2 { using type = void; };
+template <> struct Pair2<float> { using type = float2; };
+template <> struct Pair2<double> { using type = double2; };
+template <> struct Pair2<float2> { using type = float4; };
+template <class P> __device__ __forceinline__ void ld2(const P *s, P &a, P &b) {
+   if constexpr (sizeof(P) == 16) {
+      a = s[0]; b = s[1];
+   } else {
+      const auto v = *(const typename Pair2<P>::type *) s;
+      if constexpr (std::is_same<P, float2>::value) { a = make_float2(v.x, v.y); b = make_float2(v.z, v.w); }
+      else { a = v.x; b = v.y; }
+   }
+}
+template <class P> __device__ __forceinline__ void st2(P *s, P a, P b) {
+   if constexpr (sizeof(P) == 16) {
+      s[0] = a; s[1] = b;
+   } else {
+      typename Pair2<P>::type v;
+      if constexpr (std::is_same<P, float2>::value) { v.x = a.x; v.y = a.y; v.z = b.x; v.w = b.y; }
+      else { v.x = a; v.y = b; }
+      *(typename Pair2<P>::type *) s = v;
+   }
+}
+
 // Composite Simpson rule accumulated while walking a line in index order,
 // with the reference's three partial sums and end correction
 // (src/utils/diffint.cu:37-66): odd samples (sumi), the even sample before

@@ -1013,7 +1013,7 @@ template <class R, bool CPLX> struct Impl {
 
    static gpe_status ysweep(gpe_solver *s) { return sweep_xy<1, false>(s, 0., 0.); }
 
-   template <int MOM, int MSEG, int S, int TWC> static gpe_status sweep_z_launch_t(gpe_solver *s) {
+   template <int MOM, int MSEG, int S, int TWC> static gpe_status sweep_z_launch_t(gpe_solver *s, double *dev_norm) {
       auto &w = s->sw[2];
       const Dims &d = s->d;
       const void *f = (const void *) k_sweep_z<R, CPLX, MOM, MSEG, S, TWC>;
@@ -1021,41 +1021,42 @@ template <class R, bool CPLX> struct Impl {
       const long long ntiles = (d.nxy + w.TW - 1) / w.TW;
       const unsigned grid = (unsigned) std::min<long long>(ntiles, (long long) w.ctas * s->nsm);
       CKS(launch_pdl(k_sweep_z<R, CPLX, MOM, MSEG, S, TWC>, grid, ((w.TW * w.tab.P + 31) & ~31), w.smem, s,
-          (P *) s->psi, d, w.tab, w.TW, w.LS, s->wz, s->wz2, s->p.dz / 3., s->rowA, s->rowB, s->err));
+          (P *) s->psi, d, w.tab, w.TW, w.LS, zout(s), s->p.dx, s->p.dy, s->state, dev_norm, s->err));
       CKL();
       mark(s);
       s->launches++;
       return GPE_OK;
    }
 
-   template <int MOM, int MSEG, int S> static gpe_status sweep_z_launch(gpe_solver *s) {
+   template <int MOM, int MSEG, int S> static gpe_status sweep_z_launch(gpe_solver *s, double *nrm) {
       if constexpr (std::is_same<R, double>::value) {
-         if (s->sw[2].TW == 8) return sweep_z_launch_t<MOM, MSEG, S, 8>(s);
-         if (s->sw[2].TW == 16) return sweep_z_launch_t<MOM, MSEG, S, 16>(s);
+         if (s->sw[2].TW == 8) return sweep_z_launch_t<MOM, MSEG, S, 8>(s, nrm);
+         if (s->sw[2].TW == 16) return sweep_z_launch_t<MOM, MSEG, S, 16>(s, nrm);
       }
-      return sweep_z_launch_t<MOM, MSEG, S, 0>(s);
+      return sweep_z_launch_t<MOM, MSEG, S, 0>(s, nrm);
    }
 
-   template <int MOM> static gpe_status zsweep_m(gpe_solver *s) {
+   template <int MOM> static gpe_status zsweep_m(gpe_solver *s, double *nrm) {
       const auto &w = s->sw[2];
       if constexpr (kSeg32)
-         if (w.MSEG == 32) return w.S == 3 ? sweep_z_launch<MOM, 32, 3>(s) : sweep_z_launch<MOM, 32, 2>(s);
-      if (w.MSEG == 8) return w.S == 3 ? sweep_z_launch<MOM, 8, 3>(s) : sweep_z_launch<MOM, 8, 2>(s);
-      return w.S == 3 ? sweep_z_launch<MOM, 16, 3>(s) : sweep_z_launch<MOM, 16, 2>(s);
+         if (w.MSEG == 32) return w.S == 3 ? sweep_z_launch<MOM, 32, 3>(s, nrm) : sweep_z_launch<MOM, 32, 2>(s, nrm);
+      if (w.MSEG == 8) return w.S == 3 ? sweep_z_launch<MOM, 8, 3>(s, nrm) : sweep_z_launch<MOM, 8, 2>(s, nrm);
+      return w.S == 3 ? sweep_z_launch<MOM, 16, 3>(s, nrm) : sweep_z_launch<MOM, 16, 2>(s, nrm);
    }
 
-   // z sweep; mom 1: each row also yields its Simpson integral of |psi|^2
-   // (norm); mom 2: and of z^2 |psi|^2 (rms row partials)
-   static gpe_status zsweep(gpe_solver *s, int mom) {
-      if (mom == 2) return zsweep_m<2>(s);
-      return mom == 1 ? zsweep_m<1>(s) : zsweep_m<0>(s);
+   // z sweep; mom 1: also the norm of the step (dev_norm may be null) and the
+   // pending renormalisation; mom 2: the rms row partials
+   static gpe_status zsweep(gpe_solver *s, int mom, double *dev_norm = nullptr) {
+      if (mom == 2) return zsweep_m<2>(s, nullptr);
+      return mom == 1 ? zsweep_m<1>(s, dev_norm) : zsweep_m<0>(s, nullptr);
    }
+
+   static ZOut zout(const gpe_solver *s) { return ZOut{s->wz, s->wz2, s->p.dz / 3., s->rowA, s->rowA, s->rowB}; }
 
    static gpe_status norm_final(gpe_solver *s, double *dev_out) {
       CKS(launch_pdl(k_norm_final, blocks_for(s->d.nx, kNormRowsPerCta), 32 * kNormRowsPerCta, 0, s,
           s->rowA, s->d, s->p.dx, s->p.dy, s->state, s->tmp, dev_out));
       CKL();
-      mark(s);
       s->launches++;
       return GPE_OK;
    }
@@ -1143,8 +1144,8 @@ template <class R, bool CPLX> struct Impl {
       CKS(xsweep(s, true, g, gd));
       CKS(ysweep(s));
       const bool imag = !CPLX;
-      CKS(zsweep(s, imag ? 1 : (rms_rows ? 2 : 0)));
-      if (imag) CKS(norm_final(s, dev_norm));
+      CKS(zsweep(s, imag ? 1 : (rms_rows ? 2 : 0), dev_norm));
+      if (imag) mark(s);  // (norm: the z sweep's last CTA)
       return GPE_OK;
    }
 
@@ -1208,8 +1209,8 @@ template <class R, bool CPLX> struct Impl {
          if (ax == 2) g->part = (uint32_t) (((size_t) P * TW * sizeof(double) + 15) & ~(size_t) 15);
       }
       // norm (imaginary time)
-      g->tiles[kPNorm] = s->cplx ? 0 : (d.nx + kNormRowsPerCta - 1) / kNormRowsPerCta;
-      g->threads[kPNorm] = 32 * kNormRowsPerCta;
+      g->tiles[kPNorm] = s->cplx ? 0 : 1;
+      g->threads[kPNorm] = 256;
       return GPE_OK;
    }
 
@@ -1231,14 +1232,10 @@ template <class R, bool CPLX> struct Impl {
          v.st = s->state;
          v.err = s->err;
          v.psi = s->psi;
-         v.wz = s->wz;
-         v.wz2 = s->wz2;
-         v.rowsum = s->rowA;
-         v.rowsum2 = s->rowB;
+         v.zo = zout(s);
          v.g = g;
          v.gd = gd;
          v.dt = s->p.dt;
-         v.hz3 = s->p.dz / 3.;
          v.TW = w.TW;
          v.boxn = w.boxn;
          v.nbox = w.nbox;
@@ -1258,7 +1255,6 @@ template <class R, bool CPLX> struct Impl {
       D->state = s->state;
       D->err = s->err;
       D->rowA = s->rowA;
-      D->xs = s->tmp;
       D->hx = s->p.dx;
       D->hy = s->p.dy;
       D->LSr = s->LSr;
@@ -1736,8 +1732,8 @@ extern "C" double gpe_step_kernel_bytes(gpe_solver *s, int i) {
    case 5: return planes;
    case 6: return npts * (2. * sp + r);
    case 7: return 2. * npts * sp;
-   case 8: return 2. * npts * sp + (s->cplx ? 0. : 8. * (double) d.nxy);
-   case 9: return s->cplx ? 0. : 8. * (double) d.nxy;
+   case 8: return 2. * npts * sp;
+   case 9: return 0.;  // folded into case 8
    default: return 0.;
    }
 }
@@ -1954,7 +1950,7 @@ gpe_status params_of(gpe_solver *s, gpe_params *p) {
    return GPE_OK;
 }
 int device_of(gpe_solver *s) { return s->dev; }
-long long kernels_per_step(gpe_solver *s) { return s->cplx ? 9 : 10; }
+long long kernels_per_step(gpe_solver *) { return 9; }
 unsigned long long plan_generation(gpe_solver *s) { return s->plan_gen; }
 gpe_status tuning_as_set(gpe_solver *s, gpe_tuning *t) {
    CHECK_HANDLE(s);

@@ -423,6 +423,40 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_dens(const typename Tr<
    }
 }
 
+// Sum of n tile partials in an order that depends on n only: 256 strided
+// partial sums, then a tree over them.  Every thread of the CTA calls it; the
+// result is valid in thread 0.  red: 256 doubles.
+__device__ __forceinline__ double sum_tiles(const double *__restrict__ part, int n, double *red) {
+   constexpr int U = 8;  // loads in flight per lane
+   for (int v = threadIdx.x; v < 256; v += blockDim.x) {
+      double acc = 0.;
+      for (int k0 = v; k0 < n; k0 += 256 * U) {
+         double x[U];
+#pragma unroll
+         for (int u = 0; u < U; u++) x[u] = k0 + 256 * u < n ? __ldcg(part + k0 + 256 * u) : 0.;
+#pragma unroll
+         for (int u = 0; u < U; u++) acc += x[u];
+      }
+      red[v] = acc;
+   }
+   __syncthreads();
+   for (int h = 128; h; h >>= 1) {
+      for (int v = threadIdx.x; v < h; v += blockDim.x) red[v] += red[v + h];
+      __syncthreads();
+   }
+   return red[0];
+}
+
+// The step's norm from S = sum w_x w_y S_z |psi|^2 into the state.
+__device__ __forceinline__ void set_norm(State *st, double sum, double hx, double hy, double *out_norm) {
+   const double nrm = sqrt(sum * (hx / 3.) * (hy / 3.));
+   const double t = 1. / nrm;
+   st->norm = nrm;
+   st->scale = t;
+   st->scale2 = t * t;
+   if (out_norm) *out_norm = nrm;
+}
+
 // norm = sqrt(S_x S_y rowsum) (calcnorm, imag3d-mpicuda.cu:1194-1218), stores
 // norm, scale = 1/norm and scale^2 in the state.  Each warp forms the
 // weighted Simpson sum over y of one x row (shuffle reduction) into xs[i];

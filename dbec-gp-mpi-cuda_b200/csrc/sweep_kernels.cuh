@@ -39,6 +39,7 @@
 #include <type_traits>
 
 #include "kernels.cuh"
+#include "step_kernels.cuh"
 #include "tma.cuh"
 
 namespace gpe {
@@ -138,34 +139,6 @@ template <class R, bool CPLX> struct SegOps {
 struct NoXf {
    static constexpr bool kNu = false;
 };
-
-// Adjacent elements of a contiguous row (z sweep) move two at a time: every
-// segment starts at an even index and rows at 16-byte boundaries, and with a
-// row stride of an odd number of 16-byte units the 8 (16-byte accesses) rows
-// a phase of a warp touches fall on different banks.
-template <class P> struct Pair2 { using type = void; };
-template <> struct Pair2<float> { using type = float2; };
-template <> struct Pair2<double> { using type = double2; };
-template <> struct Pair2<float2> { using type = float4; };
-template <class P> __device__ __forceinline__ void ld2(const P *s, P &a, P &b) {
-   if constexpr (sizeof(P) == 16) {
-      a = s[0]; b = s[1];
-   } else {
-      const auto v = *(const typename Pair2<P>::type *) s;
-      if constexpr (std::is_same<P, float2>::value) { a = make_float2(v.x, v.y); b = make_float2(v.z, v.w); }
-      else { a = v.x; b = v.y; }
-   }
-}
-template <class P> __device__ __forceinline__ void st2(P *s, P a, P b) {
-   if constexpr (sizeof(P) == 16) {
-      s[0] = a; s[1] = b;
-   } else {
-      typename Pair2<P>::type v;
-      if constexpr (std::is_same<P, float2>::value) { v.x = a.x; v.y = a.y; v.z = b.x; v.w = b.y; }
-      else { v.x = a; v.y = b; }
-      *(typename Pair2<P>::type *) s = v;
-   }
-}
 
 // Segmented Thomas sweep of one line in shared memory (element i at
 // line[i es], rows -skip .. -1 present), by all threads of the CTA: thread p
@@ -706,16 +679,23 @@ __host__ __device__ __forceinline__ int zrow_stride(int nz, int skip, int esz) {
    return (units | 1) * u;
 }
 
+// What the z sweep leaves besides psi.  MOM 1 (imaginary time): per tile the
+// sum over its rows of w_x w_y S_z |psi'|^2 (tile, the norm's partials).  MOM
+// 2: per row S_z |psi'|^2 and S_z z^2 |psi'|^2 (row partials of calcrms).
+struct ZOut {
+   const double *wz, *wz2;  // Simpson weights along z (MOM 2)
+   double hz3;
+   double *tile, *rowA, *rowB;
+};
+
 // The z sweep of one staged tile of TR rows (nr of them inside the grid;
 // `rows` is element 0 of the first, LS the row stride) starting at grid row
-// row0, with the Simpson row partials of MOM >= 1; ends with the tile written
-// back in shared memory and a CTA barrier (the caller then stores it).
+// row0; ends with the tile written back in shared memory and a CTA barrier
+// (the caller then stores it).
 template <class R, bool CPLX, int MOM, int MSEG, bool STAB, bool ANY>
 __device__ __forceinline__ void zsweep_tile(typename Tr<R, CPLX>::P *rows, int nr, int TR, int LS, int c, int p,
                                             const SegTab &tbs, typename Tr<R, CPLX>::P *xch, double *part,
-                                            double *part2, const double *__restrict__ wz,
-                                            const double *__restrict__ wz2, double hz3, double *__restrict__ rowsum,
-                                            double *__restrict__ rowsum2, long long row0) {
+                                            double *part2, const Dims &d, const ZOut &o, long long row0, int tile) {
    using P = typename Tr<R, CPLX>::P;
    constexpr bool SIMP = MOM >= 1;
    if (nr < TR) {  // rows beyond the grid are zero so their sweep stays finite
@@ -725,9 +705,9 @@ __device__ __forceinline__ void zsweep_tile(typename Tr<R, CPLX>::P *rows, int n
    }
    double my = 0., my2 = 0.;
    if constexpr (ANY)
-      seg_sweep_any<R, CPLX, MSEG, true, STAB, MOM>(rows + c * LS, 1, p, tbs, xch + c, TR, NoXf(), wz, wz2, &my, &my2);
+      seg_sweep_any<R, CPLX, MSEG, true, STAB, MOM>(rows + c * LS, 1, p, tbs, xch + c, TR, NoXf(), o.wz, o.wz2, &my, &my2);
    else
-      seg_sweep<R, CPLX, MSEG, true, STAB, MOM>(rows + c * LS, 1, p, tbs, xch + c, TR, NoXf(), wz, wz2, &my, &my2);
+      seg_sweep<R, CPLX, MSEG, true, STAB, MOM>(rows + c * LS, 1, p, tbs, xch + c, TR, NoXf(), o.wz, o.wz2, &my, &my2);
    if (SIMP && p < tbs.P) part[p * TR + c] = my;
    if (MOM == 2 && p < tbs.P) part2[p * TR + c] = my2;
    fence_proxy_async();
@@ -747,16 +727,27 @@ __device__ __forceinline__ void zsweep_tile(typename Tr<R, CPLX>::P *rows, int n
          sum += __shfl_xor_sync(0xffffffffu, sum, q);
          if (MOM == 2) sum2 += __shfl_xor_sync(0xffffffffu, sum2, q);
       }
-      if (ln < nr) {
-         if (MOM == 1 && !(tbs.n & 1)) {
-            // the end correction of an even nz: the weights of points nz-2
-            // and nz-3 are 3 and 3.75 where the interior weights give 2 and 4
-            const int n = tbs.n;
-            const P *row = rows + rr * LS;
-            sum += (double) dens2(row[n - 2]) - 0.25 * (double) dens2(row[n - 3]);
+      if (MOM == 2 && ln < nr) {
+         o.rowA[row0 + rr] = sum * o.hz3;
+         o.rowB[row0 + rr] = sum2 * o.hz3;
+      }
+      if (MOM == 1) {
+         if (ln < nr) {
+            if (!(tbs.n & 1)) {
+               // the end correction of an even nz: the weights of points nz-2
+               // and nz-3 are 3 and 3.75 where the interior weights give 2
+               // and 4
+               const int n = tbs.n;
+               const P *row = rows + rr * LS;
+               sum += (double) dens2(row[n - 2]) - 0.25 * (double) dens2(row[n - 3]);
+            }
+            const int i = (int) ((row0 + rr) / d.ny), j = (int) (row0 + rr) - i * d.ny;
+            sum *= o.hz3 * simp_w(i, d.nx) * simp_w(j, d.ny);
+         } else {
+            sum = 0.;
          }
-         rowsum[row0 + rr] = sum * hz3;
-         if (MOM == 2) rowsum2[row0 + rr] = sum2 * hz3;
+         for (int q = 16; q; q >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, q);
+         if (ln == 0) o.tile[tile] = sum;
       }
    }
 }
@@ -780,17 +771,15 @@ template <bool CPLX> __device__ __forceinline__ SegTab stage_segtab(double *tabs
 }
 
 // z sweep.  Tile: TR consecutive (x, y) rows, each copied by one bulk copy to
-// a padded shared row (zrow_pad, stride LS elements).  With MOM >= 1 every row
-// also yields its Simpson integral of |psi'|^2 over z (simpint,
-// diffint.cu:106), for the norm of the step (rowsum); with MOM = 2 also that
-// of z^2 |psi'|^2 (rowsum2), the row partials of calcrms, so an rms sample
-// after the step needs no extra pass over psi.
+// a padded shared row (zrow_pad, stride LS elements).  MOM 1 also yields the
+// norm of the step (simpint, diffint.cu:106): the last CTA to finish adds the
+// tile partials and sets the state (hx, hy; out_norm may be null), which was a
+// launch of its own.  MOM 2 yields the row partials of calcrms, so an rms
+// sample after the step needs no extra pass over psi.
 template <class R, bool CPLX, int MOM, int MSEG, int S, int TWC>
 __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k_sweep_z(typename Tr<R, CPLX>::P *__restrict__ psi, Dims d, SegTab tb,
-                                                    int tr_arg, int LS, const double *__restrict__ wz,
-                                                    const double *__restrict__ wz2, double hz3,
-                                                    double *__restrict__ rowsum, double *__restrict__ rowsum2,
-                                                    uint32_t *err) {
+                                                    int tr_arg, int LS, ZOut out, double hx, double hy,
+                                                    State *st, double *out_norm, uint32_t *err) {
    pdl_trigger();
    pdl_wait();
    const int TR = TWC > 0 ? TWC : tr_arg;
@@ -847,11 +836,28 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
       }
       if (__syncthreads_or(!mbar_wait(&full[q], (i / S) & 1, err))) break;
       P *rows = (P *) (base + q * stage_bytes) + pad;
-      zsweep_tile<R, CPLX, MOM, MSEG, STAB, false>(rows, nrows(t), TR, LS, c, p, tbs, xch, part, part2, wz, wz2, hz3, rowsum,
-                                            rowsum2, (long long) t * TR);
+      zsweep_tile<R, CPLX, MOM, MSEG, STAB, false>(rows, nrows(t), TR, LS, c, p, tbs, xch, part, part2, d, out,
+                                                   (long long) t * TR, t);
       if (threadIdx.x < 32) copy_tile(t, q, false);
    }
    if (threadIdx.x < 32) bulk_wait_all();
+   if constexpr (MOM == 1) {
+      __shared__ bool last;
+      __shared__ double red[256];
+      // the tile partials were written by this warp's lane 0
+      if (threadIdx.x == blockDim.x - 32) {
+         __threadfence();
+         last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
+      }
+      __syncthreads();
+      if (!last) return;
+      __threadfence();
+      const double sum = sum_tiles(out.tile, ntiles, red);
+      if (threadIdx.x == 0) {
+         st->ticket = 0u;
+         set_norm(st, sum, hx, hy, out_norm);
+      }
+   }
 }
 
 }  // namespace gpe
