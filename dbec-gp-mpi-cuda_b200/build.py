@@ -28,9 +28,12 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
                   "-Xcompiler", "-fPIC", "-I" + INCLUDE, "-I" + CSRC]
 
-LIB_SOURCES = ["solver.cu", "noalloc.cu", "batch.cu", "server.cpp"]
-LIB_DEPS = LIB_SOURCES + ["common.cuh", "fft.cuh", "kernels.cuh", "step_kernels.cuh", "sweep_kernels.cuh", "tma.cuh",
-                          "batch_kernels.cuh", "internal.h"]
+LIB_SOURCES = ["conv_f64.cu", "conv_f32.cu", "impl_f64i.cu", "impl_f64r.cu", "impl_f32i.cu", "impl_f32r.cu",
+               "batch_f64i.cu", "batch_f64r.cu", "batch_f32i.cu", "batch_f32r.cu", "solver.cu", "noalloc.cu", "batch.cu",
+               "server.cpp"]
+LIB_DEPS = LIB_SOURCES + ["common.cuh", "fft.cuh", "fftn.cuh", "kernels.cuh", "step_kernels.cuh", "sweep_kernels.cuh", "tma.cuh",
+                          "batch_kernels.cuh", "batch_group.h", "batch_step.cuh", "impl.cuh", "solver.cuh",
+                          "internal.h"]
 OBJ_DIR = os.path.join(PKG, "_build")
 HOST_COMMON = ["cfg.cpp", "cli.cpp"]
 PROGRAMS = {"imag3d-mpicuda": "imag3d_main.cpp", "real3d-mpicuda": "real3d_main.cpp"}

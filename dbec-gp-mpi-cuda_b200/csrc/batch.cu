@@ -20,29 +20,9 @@
 #include <tuple>
 #include <vector>
 
-#include "batch_kernels.cuh"
-#include "gpe.h"
-#include "internal.h"
+#include "batch_group.h"
 
 using namespace gpe;
-
-namespace {
-
-// One group: instances of one (mode, precision), with the aggregated launch
-// geometry of its passes.
-struct Group {
-   bool cplx = false, fp32 = false;
-   std::vector<int> members;  // instance indices
-   int Ly = 0, Lx = 0;        // FFT tile widths (the narrowest of the members)
-   BatchGeom geo{};           // maxima over the members (tiles: sums)
-   long long off[kNPass + 1] = {};  // start of each pass's work list in dwork
-   BatchDesc *dtab = nullptr;        // device descriptor table
-   unsigned *dwork = nullptr;        // device work lists (TileRef packed per tile)
-   int sweep_grid[3] = {0, 0, 0};
-   size_t sweep_smem[3] = {0, 0, 0};
-};
-
-}  // namespace
 
 struct gpe_batch {
    std::vector<gpe_solver *> inst;
@@ -64,22 +44,6 @@ struct gpe_batch {
 };
 
 namespace {
-
-gpe_status bfail(gpe_status st, const std::string &m) {
-   gpe::set_last_error(m);
-   return st;
-}
-
-#define BCK(x)                                                                        \
-   do {                                                                               \
-      cudaError_t e_ = (x);                                                           \
-      if (e_ != cudaSuccess) return bfail(GPE_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
-   } while (0)
-#define BCKS(...)                     \
-   do {                               \
-      gpe_status s_ = (__VA_ARGS__);  \
-      if (s_ != GPE_OK) return s_;    \
-   } while (0)
 
 void drop_graph(gpe_batch *b) {
    if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -183,7 +147,7 @@ gpe_status build_tables(gpe_batch *b) {
          if (sm > kSmemCap) return bfail(GPE_ERR_PARAM, "batch: sweep tiles exceed shared memory");
          // the kernels' register budget holds cap0 CTAs of 256 threads,
          // so more of fewer threads
-         const int cap0 = sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32));
+         const int cap0 = kb_sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32));
          const int cap = std::max(1, std::min(32, 256 * cap0 / std::max(32, (int) A.threads[kPXsweep + a])));
          const int ctas = std::max(1, std::min(cap, (int) (kSmemCap / sm)));
          G.sweep_smem[a] = sm;
@@ -212,111 +176,15 @@ gpe_status build_tables(gpe_batch *b) {
    return GPE_OK;
 }
 
-template <class K, class... A>
-gpe_status launch(K kern, unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
-   if (grid == 0) return GPE_OK;
-   if (smem > 48 * 1024)
-      BCK(cudaFuncSetAttribute((const void *) kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-   kern<<<grid, block, smem, st>>>(args...);
-   BCK(cudaGetLastError());
-   return GPE_OK;
-}
-
-// The passes of one batch step of group G, on stream st.
-template <class R, bool CPLX> struct BatchStep {
-   using C = cpx<R>;
-   template <class F> static gpe_status with_ppt(int ppt, F f) {
-      if (ppt <= 8) return f(std::integral_constant<int, 8>());
-      if (ppt <= 16) return f(std::integral_constant<int, 16>());
-      return f(std::integral_constant<int, 32>());
-   }
-   template <class F> static gpe_status with_L(int L, F f) {
-      if (L >= 16) return f(std::integral_constant<int, 16>());
-      if (L == 8) return f(std::integral_constant<int, 8>());
-      if (L == 4) return f(std::integral_constant<int, 4>());
-      return f(std::integral_constant<int, 2>());
-   }
-   template <class F> static gpe_status with_mseg(int m, F f) {
-      if constexpr (std::is_same<R, float>::value && !CPLX)
-         if (m > 16) return f(std::integral_constant<int, 32>());
-      if (m > 8) return f(std::integral_constant<int, 16>());
-      return f(std::integral_constant<int, 8>());
-   }
-
-   // ev (may be null): an event recorded after every pass, index = pass
-   static gpe_status run(const Group &G, cudaStream_t st, long long *kernels, cudaEvent_t *ev = nullptr) {
-      const BatchGeom &A = G.geo;
-      const BatchDesc *tab = G.dtab;
-      auto S = [&](int q) { return (const unsigned *) (G.dwork + G.off[q]); };
-      auto T = [&](int q) { return (unsigned) A.tiles[q]; };
-      constexpr int ZL = 8;
-      auto mark = [&](int q) -> gpe_status {
-         if (ev) BCK(cudaEventRecord(ev[q], st));
-         return GPE_OK;
-      };
-      BCKS(with_ppt(A.zppt, [&](auto pc) {
-         constexpr int PPT = decltype(pc)::value;
-         return launch(kb_zfwd<R, CPLX, PPT, ZL>, T(kPZfwd), A.threads[kPZfwd], A.smem[kPZfwd], st, tab, S(kPZfwd));
-      }));
-      BCKS(mark(kPZfwd));
-      BCKS(with_L(G.Ly, [&](auto lc) {
-         constexpr int L = decltype(lc)::value;
-         return launch(kb_yfft<R, false, L>, T(kPYfft), A.threads[kPYfft], A.smem[kPYfft], st, tab, S(kPYfft));
-      }));
-      BCKS(mark(kPYfft));
-      BCKS(with_L(G.Lx, [&](auto lc) {
-         constexpr int L = decltype(lc)::value;
-         return launch(kb_xconv<R, L>, T(kPXconv), A.threads[kPXconv], A.smem[kPXconv], st, tab, S(kPXconv));
-      }));
-      BCKS(mark(kPXconv));
-      BCKS(with_L(G.Ly, [&](auto lc) {
-         constexpr int L = decltype(lc)::value;
-         return launch(kb_yfft<R, true, L>, T(kPYinv), A.threads[kPYinv], A.smem[kPYinv], st, tab, S(kPYinv));
-      }));
-      BCKS(mark(kPYinv));
-      BCKS(with_ppt(A.zppt, [&](auto pc) {
-         constexpr int PPT = decltype(pc)::value;
-         return launch(kb_zinv<R, PPT, ZL>, T(kPZinv), A.threads[kPZinv], A.smem[kPZinv], st, tab, S(kPZinv));
-      }));
-      BCKS(mark(kPZinv));
-      BCKS(launch(kb_phifix<R>, T(kPPhifix), A.threads[kPPhifix], 0, st, tab, S(kPPhifix)));
-      BCKS(mark(kPPhifix));
-      BCKS(with_mseg(A.mseg[0], [&](auto mc) {
-         constexpr int M = decltype(mc)::value;
-         return launch(kb_sweep_xy<R, CPLX, 0, true, M, 2>, (unsigned) G.sweep_grid[0], A.threads[kPXsweep],
-                       G.sweep_smem[0], st, tab, S(kPXsweep), (int) A.tiles[kPXsweep], A.stage[0], A.xch[0]);
-      }));
-      BCKS(mark(kPXsweep));
-      BCKS(with_mseg(A.mseg[1], [&](auto mc) {
-         constexpr int M = decltype(mc)::value;
-         return launch(kb_sweep_xy<R, CPLX, 1, false, M, 2>, (unsigned) G.sweep_grid[1], A.threads[kPYsweep],
-                       G.sweep_smem[1], st, tab, S(kPYsweep), (int) A.tiles[kPYsweep], A.stage[1], A.xch[1]);
-      }));
-      BCKS(mark(kPYsweep));
-      BCKS(with_mseg(A.mseg[2], [&](auto mc) {
-         constexpr int M = decltype(mc)::value;
-         constexpr int MOM = CPLX ? 0 : 1;
-         return launch(kb_sweep_z<R, CPLX, MOM, M, 2>, (unsigned) G.sweep_grid[2], A.threads[kPZsweep],
-                       G.sweep_smem[2], st, tab, S(kPZsweep), (int) A.tiles[kPZsweep], A.stage[2], A.xch[2],
-                       A.part);
-      }));
-      BCKS(mark(kPZsweep));
-      if (!CPLX) BCKS(launch(kb_norm_final, T(kPNorm), A.threads[kPNorm], 0, st, tab, S(kPNorm)));
-      BCKS(mark(kPNorm));
-      *kernels += CPLX ? 9 : 10;
-      return GPE_OK;
-   }
-};
-
 // ev (may be null): per group, kNPass events recorded after its passes
 gpe_status queue_step(gpe_batch *b, cudaStream_t st, long long *kernels, cudaEvent_t *ev = nullptr) {
    for (size_t gi = 0; gi < b->groups.size(); gi++) {
       const Group &G = b->groups[gi];
       cudaEvent_t *e = ev ? ev + gi * kNPass : nullptr;
       if (G.fp32)
-         BCKS(G.cplx ? BatchStep<float, true>::run(G, st, kernels, e) : BatchStep<float, false>::run(G, st, kernels, e));
+         BCKS(G.cplx ? batch_step<float, true>(G, st, kernels, e) : batch_step<float, false>(G, st, kernels, e));
       else
-         BCKS(G.cplx ? BatchStep<double, true>::run(G, st, kernels, e) : BatchStep<double, false>::run(G, st, kernels, e));
+         BCKS(G.cplx ? batch_step<double, true>(G, st, kernels, e) : batch_step<double, false>(G, st, kernels, e));
    }
    return GPE_OK;
 }

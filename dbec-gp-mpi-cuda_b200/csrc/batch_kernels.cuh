@@ -5,7 +5,8 @@
 // their own grids, parameters and couplings together.  Every pass of the step
 // (z forward FFT, y FFT, x convolution, inverse y FFT, z inverse FFT, phi
 // boundary planes, x sweep with calcnu, y sweep, z sweep, norm) is ONE launch
-// over the tiles of all instances of a group (same mode and precision): a
+// over the tiles of all instances of a group (same mode and precision; mixed
+// precision folds the boundary planes into the z inverse pass): a
 // per-instance descriptor table in device memory holds each instance's
 // dimensions, pointers, FFT plans, coefficient tables, couplings and TMA
 // tensor maps, and a work list per pass maps a tile to its instance and its
@@ -48,10 +49,11 @@ struct alignas(64) BatchDesc {
    CUtensorMap tm_phi;     // x sweep tiles of phi
    CUtensorMap tm_spec_y, tm_spec_x;
    SweepView sv[3];
-   FftPlan px, py, ph;
+   FftPlan px, pxi, py, ph;
    Dims d;
    void *psi, *spec, *phi;
-   const void *twx, *twy, *twz;
+   const void *twx, *twy, *twz;  // roots of unity (ztab_roots in step_kernels.cuh)
+   int fastx, fasty, fastz;      // compile-time passes
    const double *udd;
    State *state;
    uint32_t *err;
@@ -102,59 +104,99 @@ __device__ __forceinline__ void stage_plan(FftPlan &dst, const FftPlan &src) {
    __syncthreads();
 }
 
+// Resident CTAs of 256 threads per SM (register budgets): 128 registers for
+// the FP64 FFT passes, whose compile-time transforms hold 16 points per
+// thread, 64 for FP32; the sweeps as sweep_ctas, with 80 for the FP32 ones of
+// up to 16-point segments, which hold the code of two segment lengths.
+template <class R> constexpr int kb_fft_ctas() { return sizeof(R) == 8 ? 2 : 4; }
+__host__ __device__ constexpr int kb_sweep_ctas(bool fp32, bool cplx, int m) {
+   return fp32 && m == 16 ? 3 : sweep_ctas(fp32, cplx, m);
+}
+
 // ---------------------------------------------------------------- FFT passes
 // One CTA per tile; tile numbering of each instance as its single-solve grid.
 
 template <class R, bool CPLX, int PPT, int L>
-__global__ void __launch_bounds__(256, L >= 16 ? 3 : 4) kb_zfwd(const BatchDesc *__restrict__ tab,
+__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_zfwd(const BatchDesc *__restrict__ tab,
                                                                 const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
+   using P = typename Tr<R, CPLX>::P;
    __shared__ FftPlan pl;
-   stage_plan(pl, D.ph);
    const Dims d = D.d;
-   zfwd_body<R, CPLX, PPT, L>((const typename Tr<R, CPLX>::P *) D.psi, (cpx<R> *) D.spec, d, pl,
-                              (const cpx<R> *) D.twz, D.LSr, D.err, (long long) r.local * L);
+   const long long r0 = (long long) r.local * L;
+   with_len(D.fastz ? d.nz / 2 : 0, [&](auto nc) {
+      constexpr int H = decltype(nc)::value;
+      if constexpr (H > 0 && H <= kLenMaxH && L == kLenRows) {
+         zfwd_body_n<R, CPLX, L, H>((const P *) D.psi, (cpx<R> *) D.spec, d, (const cpx<R> *) D.twz, D.err, r0);
+      } else if constexpr (H == 0) {
+         stage_plan(pl, D.ph);
+         zfwd_body<R, CPLX, PPT, L>((const P *) D.psi, (cpx<R> *) D.spec, d, pl, (const cpx<R> *) D.twz, D.LSr, D.err, r0);
+      }
+   });
 }
 
 template <class R, bool INV, int L>
-__global__ void __launch_bounds__(256, 4) kb_yfft(const BatchDesc *__restrict__ tab,
+__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_yfft(const BatchDesc *__restrict__ tab,
                                                   const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
    __shared__ FftPlan pl;
    if (threadIdx.x == 0) tmap_acquire(&D.tm_spec_y);
-   stage_plan(pl, D.py);
    const Dims d = D.d;
-   const int nkb = (d.nzh + L - 1) / L;
-   const int x = r.local / nkb, k0 = (r.local - x * nkb) * L;
-   yfft_body<R, INV, L>(&D.tm_spec_y, d, pl, (const cpx<R> *) D.twy, D.boxy, D.nboxy, D.err, x, k0);
+   with_len(D.fasty ? d.ny : 0, [&](auto nc) {
+      constexpr int N = decltype(nc)::value, LT = N > 0 ? LenCols<R>::L : L;
+      const int nkb = (d.nzh + LT - 1) / LT;
+      const int x = r.local / nkb, k0 = (r.local - x * nkb) * LT;
+      if constexpr (N > 0) {
+         yfft_body_n<R, INV, LT, N>(&D.tm_spec_y, (const cpx<R> *) D.twy, D.err, x, k0);
+      } else {
+         stage_plan(pl, D.py);
+         yfft_body<R, INV, L>(&D.tm_spec_y, d, pl, (const cpx<R> *) D.twy, D.boxy, D.nboxy, D.err, x, k0);
+      }
+   });
 }
 
 template <class R, int L>
-__global__ void __launch_bounds__(256, 4) kb_xconv(const BatchDesc *__restrict__ tab,
+__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_xconv(const BatchDesc *__restrict__ tab,
                                                    const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
-   __shared__ FftPlan pl;
+   __shared__ FftPlan pl, pli;
    if (threadIdx.x == 0) tmap_acquire(&D.tm_spec_x);
-   stage_plan(pl, D.px);
    const Dims d = D.d;
-   const int nkb = (d.nzh + L - 1) / L;
-   const int y = r.local / nkb, k0 = (r.local - y * nkb) * L;
-   xconv_body<R, L>(&D.tm_spec_x, d, pl, (const cpx<R> *) D.twx, D.udd, D.state, D.boxx, D.nboxx, D.err, y, k0);
+   with_len(D.fastx ? d.nx : 0, [&](auto nc) {
+      constexpr int N = decltype(nc)::value, LT = N > 0 ? LenCols<R>::L : L;
+      const int nkb = (d.nzh + LT - 1) / LT;
+      const int y = r.local / nkb, k0 = (r.local - y * nkb) * LT;
+      if constexpr (N > 0) {
+         xconv_body_n<R, LT, N>(&D.tm_spec_x, nullptr, D.udd, d, (const cpx<R> *) D.twx, D.state, D.err, y, k0);
+      } else {
+         stage_plan(pl, D.px);
+         stage_plan(pli, D.pxi);
+         xconv_body<R, L>(&D.tm_spec_x, nullptr, D.udd, d, pl, pli, (const cpx<R> *) D.twx, D.state, D.boxx,
+                          D.nboxx, D.err, y, k0);
+      }
+   });
 }
 
-template <class R, int PPT, int L>
-__global__ void __launch_bounds__(256, L >= 16 ? 3 : 4) kb_zinv(const BatchDesc *__restrict__ tab,
+template <class R, int PPT, int L, bool FOLD>
+__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_zinv(const BatchDesc *__restrict__ tab,
                                                                 const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
    __shared__ FftPlan pl;
-   stage_plan(pl, D.ph);
    const Dims d = D.d;
-   zinv_body<R, PPT, L>((const cpx<R> *) D.spec, (R *) D.phi, d, pl, (const cpx<R> *) D.twz, D.LSo, D.err,
-                        (long long) r.local * L);
+   const long long r0 = (long long) r.local * L;
+   with_len(D.fastz ? d.nz / 2 : 0, [&](auto nc) {
+      constexpr int H = decltype(nc)::value;
+      if constexpr (H > 0 && H <= kLenMaxH && L == kLenRows) {
+         zinv_body_n<R, L, H, FOLD>((const cpx<R> *) D.spec, (R *) D.phi, d, (const cpx<R> *) D.twz, D.err, r0);
+      } else if constexpr (H == 0) {
+         stage_plan(pl, D.ph);
+         zinv_body<R, PPT, L, FOLD>((const cpx<R> *) D.spec, (R *) D.phi, d, pl, (const cpx<R> *) D.twz, D.LSo, D.err, r0);
+      }
+   });
 }
 
 template <class R>
@@ -170,7 +212,7 @@ static __global__ void __launch_bounds__(256) kb_norm_final(const BatchDesc *__r
                                                             const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
-   __shared__ double red[256];
+   __shared__ double red[8];
    const double sum = sum_tiles(D.rowA, (int) ((D.d.nxy + D.sv[2].TW - 1) / D.sv[2].TW), red);
    if (threadIdx.x == 0) set_norm(D.state, sum, D.hx, D.hy, nullptr);
 }
@@ -192,7 +234,7 @@ __device__ __forceinline__ void copy_view(SweepView &dst, const SweepView &src) 
 }
 
 template <class R, bool CPLX, int AXIS, bool NU, int MSEG, int S>
-__global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_xy(const BatchDesc *__restrict__ tab,
+__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_xy(const BatchDesc *__restrict__ tab,
                                                                            const unsigned *__restrict__ work,
                                                                            int ntiles, uint32_t stage_bytes,
                                                                            uint32_t xch_bytes) {
@@ -294,7 +336,7 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
 }
 
 template <class R, bool CPLX, int MOM, int MSEG, int S>
-__global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_z(const BatchDesc *__restrict__ tab,
+__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_z(const BatchDesc *__restrict__ tab,
                                                                  const unsigned *__restrict__ work, int ntiles,
                                                                  uint32_t stage_bytes, uint32_t xch_bytes,
                                                                  uint32_t part_bytes) {

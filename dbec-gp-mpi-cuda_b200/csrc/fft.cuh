@@ -15,12 +15,14 @@
 //   j in [0, n/r), k = j mod Ns,  v[t] = src[j + t n/r] * W^(t k n/(Ns r))
 //   v = DFT_r(v),  dst[(j / Ns) Ns r + k + t Ns] = v[t],  Ns *= r
 // leaving the result in natural order; src and dst are the same buffer, the
-// reads of a stage finishing (barrier) before its writes start.  W = exp(-2 pi i / n) comes from a
-// table of the n-th roots computed on the host in long double (twmul > 1
-// reads a table of a longer transform with stride twmul).  Inverse
+// reads of a stage finishing (barrier) before its writes start.  W = exp(-2 pi i / n): the
+// factors of a stage lie in a table in the order the stage reads them,
+// computed on the host in long double.  Inverse
 // transforms use conjugated twiddles and are unnormalised, like cuFFT's
 // CUFFT_INVERSE.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -35,6 +37,33 @@ struct FftPlan {
    int ns[kMaxStages];             // Ns before the stage
    unsigned magic[kMaxStages];     // ceil(2^32 / Ns): j / Ns == umulhi(j, magic) for j < 2^16
 };
+
+// Radices of an n-point transform with powers of two up to 2^log2max, in the
+// order the stages run: the power of two split over as few stages as that
+// allows, as evenly as possible, larger radices first (64 points: 8 x 8) but,
+// of three stages with radices up to 8, the odd one in the middle (256: 8 x 4
+// x 8), so that a transform and the inverse that runs its stages backwards
+// share one table of roots; then the threes and fives.  Returns their number (0 when n has
+// another factor).
+inline int make_radices(int n, int log2max, int *rad) {
+   int a = 0, k = 0;
+   while (n % 2 == 0) { n /= 2; a++; }
+   const int st2 = (a + log2max - 1) / log2max;
+   int e[32];
+   for (int q = 0, r = a; q < st2; q++) {
+      e[q] = (r + st2 - q - 1) / (st2 - q);
+      r -= e[q];
+   }
+   if (log2max == 3 && st2 == 3 && e[0] != e[2]) {
+      const int odd = e[0] == e[1] ? e[2] : e[0], two = e[1];
+      e[0] = e[2] = two;
+      e[1] = odd;
+   }
+   for (int q = 0; q < st2; q++) rad[k++] = 1 << e[q];
+   while (n % 3 == 0 && k < kMaxStages) { rad[k++] = 3; n /= 3; }
+   while (n % 5 == 0 && k < kMaxStages) { rad[k++] = 5; n /= 5; }
+   return n == 1 ? k : 0;
+}
 
 // ---- small DFT kernels (constants are exact values of cos/sin) -------------
 template <class C, bool INV> __device__ __forceinline__ void dft2(C *v) {
@@ -152,33 +181,41 @@ template <int R, class C, bool INV> __device__ __forceinline__ void dftr(C *v) {
 // butterflies of the stage (at most PPT values of the L n points per
 // thread, PPT * blockDim.x >= n L), the CTA synchronises, then every thread
 // writes its results.  Half the shared memory of a ping-pong pair of
-// buffers, for one more barrier per stage.
+// buffers, for one more barrier per stage.  tw: this stage's roots in the
+// order they are read, [t - 1][k].  Butterfly b is point b of the interleaved
+// buffer; its inputs and roots follow at fixed strides, its outputs start
+// (j / Ns) Ns (RAD - 1) rows further on, so each access costs one addition.
 template <int RAD, int L, class C, bool INV, int PPT>
-__device__ __forceinline__ void fft_stage_ip(C *buf, int n, int Ns, unsigned magic, const C *__restrict__ tw,
-                                             int twmul) {
+__device__ __forceinline__ void fft_stage_ip(C *buf, int n, int Ns, unsigned magic, const C *tw) {
    constexpr int MAXU = (PPT + RAD - 1) / RAD;  // butterflies per thread
-   const int nr = n / RAD;
-   const int nb = nr * L;
-   const int twstep = (n / (Ns * RAD)) * twmul;
+   const int nb = n / RAD * L;
    C v[MAXU][RAD];
+   int off[MAXU];
 #pragma unroll
    for (int u = 0; u < MAXU; u++) {
       const int b = threadIdx.x + u * blockDim.x;
+      off[u] = -1;
       if (b < nb) {
-         const int l = b % L;
          const int j = b / L;
-         const int g = Ns == 1 ? j : (int) __umulhi((unsigned) j, magic);
-         const int k = j - g * Ns;
-         const C *src = buf + j * L + l;
+         const C *src = buf + b;
 #pragma unroll
-         for (int t = 0; t < RAD; t++) v[u][t] = src[t * nr * L];
+         for (int t = 0; t < RAD; t++) {
+            v[u][t] = *src;
+            src += nb;
+         }
          if (Ns > 1) {
+            const int g = (int) __umulhi((unsigned) j, magic);
+            const C *w = tw + (j - g * Ns);
+            off[u] = b + g * (Ns * (RAD - 1) * L);
 #pragma unroll
             for (int t = 1; t < RAD; t++) {
-               C w = tw[t * k * twstep];
-               if (INV) w.y = -w.y;
-               v[u][t] = cmul(v[u][t], w);
+               C x = *w;
+               w += Ns;
+               if (INV) x.y = -x.y;
+               v[u][t] = cmul(v[u][t], x);
             }
+         } else {
+            off[u] = b + j * ((RAD - 1) * L);
          }
          dftr<RAD, C, INV>(v[u]);
       }
@@ -186,36 +223,71 @@ __device__ __forceinline__ void fft_stage_ip(C *buf, int n, int Ns, unsigned mag
    __syncthreads();
 #pragma unroll
    for (int u = 0; u < MAXU; u++) {
-      const int b = threadIdx.x + u * blockDim.x;
-      if (b < nb) {
-         const int l = b % L;
-         const int j = b / L;
-         const int g = Ns == 1 ? j : (int) __umulhi((unsigned) j, magic);
-         const int k = j - g * Ns;
-         C *dst = buf + (g * Ns * RAD + k) * L + l;
+      if (off[u] >= 0) {
+         C *dst = buf + off[u];
 #pragma unroll
-         for (int t = 0; t < RAD; t++) dst[t * Ns * L] = v[u][t];
+         for (int t = 0; t < RAD; t++) {
+            *dst = v[u][t];
+            dst += Ns * L;
+         }
       }
    }
    __syncthreads();
 }
 
-// Full in-place transform of L interleaved lines in buf (PPT as above).
-template <int L, class C, bool INV, int PPT>
-__device__ __forceinline__ void fft_lines_ip(C *buf, const FftPlan &pl, const C *tw, int twmul) {
-   // make_plan orders the stages by radix (16, 8, 4, 2, 3, 5): one loop per
-   // radix (a switch over the radix inside one loop made ptxas spill the
-   // values held across the barriers).  Radix 16 only where a thread holds
-   // 16 points (PPT >= 16, the FP32 passes).
+// Full in-place transform of L interleaved lines in buf (PPT as above) with the
+// stage-ordered roots tw (each stage after the first).  REV: the plan lists its stages in the reverse order (the inverse transform of a
+// convolution, which starts with the radix the forward one ended on).
+template <int L, class C, bool INV, int PPT, bool REV = false>
+__device__ __forceinline__ void fft_lines_ip(C *buf, const FftPlan &pl, const C *tw) {
+   // make_radices lists the powers of two as runs of 16, 8, 4, 8, 4, 2, then
+   // 3 and 5: one loop per run (a switch over the radix inside one loop made
+   // ptxas spill the values held across the barriers).  Radix 16 only where a
+   // thread holds 16 points (PPT >= 16, the FP32 passes).
    int st = 0;
-   if constexpr (PPT >= 16)
-      for (; st < pl.nst && pl.rad[st] == 16; st++)
-         fft_stage_ip<16, L, C, INV, PPT>(buf, pl.n, pl.ns[st], pl.magic[st], tw, twmul);
-   for (; st < pl.nst && pl.rad[st] == 8; st++) fft_stage_ip<8, L, C, INV, PPT>(buf, pl.n, pl.ns[st], pl.magic[st], tw, twmul);
-   for (; st < pl.nst && pl.rad[st] == 4; st++) fft_stage_ip<4, L, C, INV, PPT>(buf, pl.n, pl.ns[st], pl.magic[st], tw, twmul);
-   for (; st < pl.nst && pl.rad[st] == 2; st++) fft_stage_ip<2, L, C, INV, PPT>(buf, pl.n, pl.ns[st], pl.magic[st], tw, twmul);
-   for (; st < pl.nst && pl.rad[st] == 3; st++) fft_stage_ip<3, L, C, INV, PPT>(buf, pl.n, pl.ns[st], pl.magic[st], tw, twmul);
-   for (; st < pl.nst && pl.rad[st] == 5; st++) fft_stage_ip<5, L, C, INV, PPT>(buf, pl.n, pl.ns[st], pl.magic[st], tw, twmul);
+   auto run = [&](auto rc) {
+      constexpr int RAD = decltype(rc)::value;
+      const int Ns = pl.ns[st];
+      fft_stage_ip<RAD, L, C, INV, PPT>(buf, pl.n, Ns, pl.magic[st], tw);
+      if (Ns > 1) tw += (RAD - 1) * Ns;
+   };
+   if constexpr (REV) {
+      for (; st < pl.nst && pl.rad[st] == 5; st++)
+         run(std::integral_constant<int, 5>());
+      for (; st < pl.nst && pl.rad[st] == 3; st++)
+         run(std::integral_constant<int, 3>());
+      for (; st < pl.nst && pl.rad[st] == 2; st++)
+         run(std::integral_constant<int, 2>());
+      for (; st < pl.nst && pl.rad[st] == 4; st++)
+         run(std::integral_constant<int, 4>());
+      for (; st < pl.nst && pl.rad[st] == 8; st++)
+         run(std::integral_constant<int, 8>());
+      for (; st < pl.nst && pl.rad[st] == 4; st++)
+         run(std::integral_constant<int, 4>());
+      for (; st < pl.nst && pl.rad[st] == 8; st++)
+         run(std::integral_constant<int, 8>());
+      if constexpr (PPT >= 16)
+         for (; st < pl.nst && pl.rad[st] == 16; st++)
+            run(std::integral_constant<int, 16>());
+   } else {
+      if constexpr (PPT >= 16)
+         for (; st < pl.nst && pl.rad[st] == 16; st++)
+            run(std::integral_constant<int, 16>());
+      for (; st < pl.nst && pl.rad[st] == 8; st++)
+         run(std::integral_constant<int, 8>());
+      for (; st < pl.nst && pl.rad[st] == 4; st++)
+         run(std::integral_constant<int, 4>());
+      for (; st < pl.nst && pl.rad[st] == 8; st++)
+         run(std::integral_constant<int, 8>());
+      for (; st < pl.nst && pl.rad[st] == 4; st++)
+         run(std::integral_constant<int, 4>());
+      for (; st < pl.nst && pl.rad[st] == 2; st++)
+         run(std::integral_constant<int, 2>());
+      for (; st < pl.nst && pl.rad[st] == 3; st++)
+         run(std::integral_constant<int, 3>());
+      for (; st < pl.nst && pl.rad[st] == 5; st++)
+         run(std::integral_constant<int, 5>());
+   }
 }
 
 }  // namespace gpe

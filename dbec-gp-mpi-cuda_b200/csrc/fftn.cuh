@@ -1,0 +1,182 @@
+// fftn.cuh -- FFTs of compile-time length on lines in shared memory, for the
+// lengths most grids have; fft.cuh transforms any other length.
+//
+// The transform is the one of fft.cuh (Stockham stages in the order of the
+// same radix plan, the same roots of unity, L lines interleaved [j][L]), so
+// both give the same values.  With the length, the line count and the CTA
+// size known to the compiler every index is a constant offset from one base
+// per butterfly: the run-time stages spent 100 warp instructions per point of
+// a 256-point FP64 line of which 24 were FP64 arithmetic, the rest mostly
+// integer indexing.  Three more things follow from the known plan:
+//  - the roots of stage s lie in a table in the order the stage reads them
+//    (stage_roots in solver.cu), one base address per butterfly;
+//  - the first stage takes its points from a functor and the last one hands
+//    them to a functor, so packing |psi|^2, the real-FFT merge and the final
+//    row layout need no pass over shared memory of their own;
+//  - a convolution keeps the points of the last forward stage in registers,
+//    multiplies them and starts the inverse transform with the same radix on
+//    them (conv_lines: the inverse runs the radices in reverse order).
+#pragma once
+
+#include <type_traits>
+
+#include "fft.cuh"
+
+namespace gpe {
+
+template <int... RS> struct Rads {};
+
+// Radix plan of a compile-time length: RadixPlan<N, LOG> with radices up to
+// 2^LOG, as make_radices (fft.cuh) lists them, and its reverse.
+template <int N, int LOG> struct RadixPlan;
+#define GPE_RADIX_PLAN(N, LOG, FWD, REV)          \
+   template <> struct RadixPlan<N, LOG> {         \
+      using fwd = Rads<GPE_UNPAREN FWD>;          \
+      using rev = Rads<GPE_UNPAREN REV>;          \
+   };
+#define GPE_UNPAREN(...) __VA_ARGS__
+GPE_RADIX_PLAN(24, 4, (8, 3), (3, 8))
+GPE_RADIX_PLAN(32, 4, (8, 4), (4, 8))
+GPE_RADIX_PLAN(48, 4, (16, 3), (3, 16))
+GPE_RADIX_PLAN(64, 4, (8, 8), (8, 8))
+GPE_RADIX_PLAN(96, 4, (8, 4, 3), (3, 4, 8))
+GPE_RADIX_PLAN(128, 4, (16, 8), (8, 16))
+GPE_RADIX_PLAN(256, 4, (16, 16), (16, 16))
+GPE_RADIX_PLAN(512, 4, (8, 8, 8), (8, 8, 8))
+
+// Points per thread, in both precisions, and log2 of the largest radix.  FP64
+// threads hold 16 points in 64 of their 128 registers; half as many threads
+// with 8 points, three stages of radix 8 and 4 for two of radix 16, measured
+// slower at 256^3 (us: x 92 -> 78, z inverse 55.5 -> 50.6, z forward 60 -> 57).
+constexpr int kLenPpt = 16, kLenLog = 4;
+
+// whether a convolution's inverse reads the same table of roots as its forward
+template <int N> __host__ __device__ constexpr bool palin_plan() {
+   using PL = RadixPlan<N, kLenLog>;
+   return std::is_same<typename PL::fwd, typename PL::rev>::value;
+}
+
+template <int RAD, int NB, int NT> struct StageRegs {
+   static constexpr int U = (NB + NT - 1) / NT;  // butterflies per thread
+};
+
+// Reads and transforms this thread's butterflies of one stage (Ns = NS): v[u]
+// holds butterfly b = tid + u NT of line b % L.  tw: this stage's roots,
+// [t - 1][k].
+template <int N, int L, int NT, int RAD, int NS, class C, bool INV, class LD, int U>
+__device__ __forceinline__ void stage_read(C (&v)[U][RAD], const C *tw, const LD &ld) {
+   constexpr int nr = N / RAD, nb = nr * L;
+#pragma unroll
+   for (int u = 0; u < U; u++) {
+      const int b = threadIdx.x + u * NT;
+      if ((int) threadIdx.x < NT && (nb % NT == 0 || b < nb)) {
+         const int l = b % L, j = b / L;
+#pragma unroll
+         for (int t = 0; t < RAD; t++) v[u][t] = ld(l, j + t * nr);
+         if constexpr (NS > 1) {
+            const C *w0 = tw + j % NS;
+#pragma unroll
+            for (int t = 1; t < RAD; t++) {
+               C w = w0[(t - 1) * NS];
+               if (INV) w.y = -w.y;
+               v[u][t] = cmul(v[u][t], w);
+            }
+         }
+         dftr<RAD, C, INV>(v[u]);
+      }
+   }
+}
+
+// Hands the outputs of a stage to st(line, index, value).
+template <int N, int L, int NT, int RAD, int NS, class C, class ST, int U>
+__device__ __forceinline__ void stage_write(const C (&v)[U][RAD], const ST &st) {
+   constexpr int nr = N / RAD, nb = nr * L;
+#pragma unroll
+   for (int u = 0; u < U; u++) {
+      const int b = threadIdx.x + u * NT;
+      if ((int) threadIdx.x < NT && (nb % NT == 0 || b < nb)) {
+         const int l = b % L, j = b / L;
+         const int o = (j / NS) * (NS * RAD) + j % NS;
+#pragma unroll
+         for (int t = 0; t < RAD; t++) st(l, o + t * NS, v[u][t]);
+      }
+   }
+}
+
+// The stages R0, RS... from Ns = NS on, in place on buf between the first
+// stage's reads (ld) and the last one's writes (st).  tw: the roots of the
+// first of them (the stage with Ns = 1 has none).  Every thread of the CTA
+// calls it (NT of them work); ends without a barrier after the last writes.
+template <int N, int L, int NT, class C, bool INV, int NS, int R0, int... RS, class LD, class ST>
+__device__ __forceinline__ void stages(Rads<R0, RS...>, C *buf, const C *tw, const LD &ld, const ST &st) {
+   constexpr int U = StageRegs<R0, N / R0 * L, NT>::U;
+   {
+      C v[U][R0];
+      stage_read<N, L, NT, R0, NS, C, INV>(v, tw, ld);
+      __syncthreads();
+      if constexpr (sizeof...(RS) == 0) stage_write<N, L, NT, R0, NS, C>(v, st);
+      else stage_write<N, L, NT, R0, NS, C>(v, [&](int l, int i, C x) { buf[i * L + l] = x; });
+   }
+   if constexpr (sizeof...(RS) > 0) {
+      __syncthreads();
+      stages<N, L, NT, C, INV, NS * R0>(Rads<RS...>(), buf, NS == 1 ? tw : tw + (R0 - 1) * NS,
+                                        [&](int l, int i) { return buf[i * L + l]; }, st);
+   }
+}
+
+// Transform of L lines of N points: point i of line l comes from ld(l, i) and
+// goes to st(l, i, value).
+template <int N, int L, int NT, class C, bool INV, class LD, class ST>
+__device__ __forceinline__ void fft_lines(C *buf, const C *tw, const LD &ld, const ST &st) {
+   using PL = RadixPlan<N, kLenLog>;
+   stages<N, L, NT, C, INV, 1>(typename PL::fwd(), buf, tw, ld, st);
+}
+
+// Forward transform, multiplication of point i of line l by mul(l, i), and
+// inverse transform, in place on buf.  The last forward stage's outputs stay
+// in registers: butterfly j ends on the points j + t N / RAD, exactly those
+// the inverse's first stage (the same radix) starts from.
+template <int N, int L, int NT, class C, int NS, int R0, int... RS, int I0, int... IS, class MUL>
+__device__ __forceinline__ void conv_stages(Rads<R0, RS...>, Rads<I0, IS...> inv, C *buf, const C *tw, const C *twi,
+                                            const MUL &mul) {
+   constexpr int U = StageRegs<R0, N / R0 * L, NT>::U;
+   auto ld = [&](int l, int i) { return buf[i * L + l]; };
+   auto st = [&](int l, int i, C x) { buf[i * L + l] = x; };
+   if constexpr (sizeof...(RS) > 0) {
+      {
+         C v[U][R0];
+         stage_read<N, L, NT, R0, NS, C, false>(v, tw, ld);
+         __syncthreads();
+         stage_write<N, L, NT, R0, NS, C>(v, st);
+      }
+      __syncthreads();
+      conv_stages<N, L, NT, C, NS * R0>(Rads<RS...>(), inv, buf, NS == 1 ? tw : tw + (R0 - 1) * NS, twi, mul);
+   } else {
+      static_assert(R0 == I0 && sizeof...(IS) > 0, "the inverse plan starts with the forward plan's last radix");
+      {
+         C v[U][R0];
+         stage_read<N, L, NT, R0, NS, C, false>(v, tw, ld);
+#pragma unroll
+         for (int u = 0; u < U; u++) {
+            const int b = threadIdx.x + u * NT;
+            if ((int) threadIdx.x < NT && ((N / R0 * L) % NT == 0 || b < N / R0 * L)) {
+               const int l = b % L, j = b / L;
+#pragma unroll
+               for (int t = 0; t < R0; t++) v[u][t] = cscale(v[u][t], mul(l, j + t * (N / R0)));
+               dftr<R0, C, true>(v[u]);
+            }
+         }
+         __syncthreads();
+         stage_write<N, L, NT, R0, 1, C>(v, st);
+      }
+      __syncthreads();
+      stages<N, L, NT, C, true, R0>(Rads<IS...>(), buf, twi, ld, st);
+   }
+}
+template <int N, int L, int NT, class C, class MUL>
+__device__ __forceinline__ void conv_lines(C *buf, const C *tw, const C *twi, const MUL &mul) {
+   using PL = RadixPlan<N, kLenLog>;
+   conv_stages<N, L, NT, C, 1>(typename PL::fwd(), typename PL::rev(), buf, tw, twi, mul);
+}
+
+}  // namespace gpe

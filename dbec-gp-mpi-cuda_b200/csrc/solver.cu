@@ -17,9 +17,7 @@
 
 #include "gpe.h"
 #include "internal.h"
-#include "step_kernels.cuh"
-#include "sweep_kernels.cuh"
-#include "batch_kernels.cuh"
+#include "solver.cuh"
 
 using namespace gpe;
 
@@ -32,113 +30,13 @@ namespace gpe {
 void set_last_error(const std::string &msg) { g_err = msg; }
 }  // namespace gpe
 
-static gpe_status fail(gpe_status st, const std::string &msg) {
+gpe_status fail(gpe_status st, const std::string &msg) {
    g_err = msg;
    return st;
 }
 
-// On failure the runtime's last-error slot is cleared so that a non-sticky
-// error is reported once, by the call that caused it.
-#define CK(call)                                                                                   \
-   do {                                                                                           \
-      cudaError_t e_ = (call);                                                                    \
-      if (e_ != cudaSuccess) {                                                                    \
-         (void) cudaGetLastError();                                                               \
-         return fail(e_ == cudaErrorMemoryAllocation ? GPE_ERR_OOM : GPE_ERR_CUDA,                \
-                     std::string(#call) + ": " + cudaGetErrorString(e_));                          \
-      }                                                                                           \
-   } while (0)
-
-#define CKL()                                                                                      \
-   do {                                                                                           \
-      cudaError_t e_ = cudaGetLastError();                                                        \
-      if (e_ != cudaSuccess) return fail(GPE_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e_)); \
-   } while (0)
-
-#define CKS(expr)                                                                                  \
-   do {                                                                                           \
-      gpe_status s_ = (expr);                                                                     \
-      if (s_ != GPE_OK) return s_;                                                                \
-   } while (0)
-
-struct gpe_solver {
-   gpe_params p;
-   int dev = 0;
-   cudaStream_t st = nullptr;
-   bool own_stream = false;
-   bool cplx = false, fp32 = false;
-   Dims d{};
-   double par = 1.;
-   FftPlan px{}, py{}, ph{};  // x, y lines and half-length z lines
-   int LSr = 0, LSo = 0;                  // shared row strides of the z passes
-   CUtensorMap tm_spec_y{}, tm_spec_x{};  // spectrum tiles of the y and x passes
-   int boxy = 0, nboxy = 1, boxx = 0, nboxx = 1;
-   int Ly = 8, Lx = 8;  // kz columns per tile of the y and x passes
-   gpe_tuning tune{};   // requested tile configuration (0 = default heuristic)
-   // bumped whenever the tiles are planned again (their tables reallocated):
-   // batches built over this handle rebuild their descriptors when it moves
-   unsigned long long plan_gen = 0;
-   size_t esz_psi = 8, esz_c = 16, esz_r = 8;
-   void *psi = nullptr, *spec = nullptr, *phi = nullptr;
-   void *twx = nullptr, *twy = nullptr, *twz = nullptr;
-   double *udd = nullptr;
-   void *alpha[3] = {nullptr, nullptr, nullptr}, *gamma[3] = {nullptr, nullptr, nullptr};
-   double2 A[3], A0r[3], mA[3];
-   double *x2 = nullptr, *y2 = nullptr, *z2 = nullptr;
-   float *x2f = nullptr, *y2f = nullptr, *z2f = nullptr;  // FP32 copies (mixed precision)
-   void *lin[3] = {nullptr, nullptr, nullptr};  // per-axis trap factors of calcnu, imag (LinPhase)
-   double *rowA = nullptr, *rowB = nullptr, *tmp = nullptr, *obs = nullptr;
-   double *rms_buf = nullptr;  // rms samples of gpe_run, kRmsSlots x 4 doubles
-
-   long long row_cap = 0;  // doubles in rowA / rowB: the largest of nx*ny, nx*nz, ny*nz
-   State *state = nullptr;
-   std::vector<double> hx, hy, hz, hx2, hy2, hz2;
-   long long launches = 0;
-   size_t obs_cap = 0;
-   // sweep configuration per axis (x, y: TMA tensor tiles; z: bulk rows)
-   struct Sweep {
-      int TW = 8, MSEG = 8, boxn = 0, nbox = 1, LS = 0, S = 2, ctas = 1;
-      size_t smem = 0;
-      CUtensorMap tm_psi{}, tm_phi{};
-      SegTab tab{};
-      // coefficient tables (FP64, or rounded once to FP32 in mixed precision)
-      void *tabs[3] = {nullptr, nullptr, nullptr};
-   } sw[3];
-   double *wz = nullptr;      // Simpson weights along z (norm partials)
-   double *wz2 = nullptr;     // wz[k] * z[k]^2 (rms partials)
-   int nsm = 148;             // streaming multiprocessors of the device
-   uint32_t *err = nullptr;   // device status word (bounded waits)
-   // per-kernel profiling: when prof_ev is set, mark() records an event
-   // after every kernel of a step
-   cudaEvent_t *prof_ev = nullptr;
-   int prof_i = 0, prof_cap = 0;
-};
-
-// rms samples gpe_run keeps on the device before copying them out (a run with
-// more samples copies every full batch of slots while it continues)
-constexpr long kRmsSlots = 256;
-
-// zero entries before index 0 of the tables the sweeps index from the rows
-// below a line (at least the longest segment)
-constexpr int kTabPad = 32;
-
-static void mark(gpe_solver *s) {
-   if (s->prof_ev && s->prof_i < s->prof_cap) cudaEventRecord(s->prof_ev[s->prof_i++], s->st);
-}
-
 // ---------------------------------------------------------------- planning
-// Radices in the order the stages are grouped (fft_lines_ip loops over them
-// in this order); max_radix 8, 4 or 2 drops the larger powers of two.  Radix
-// 16 is for the FP32 passes only, whose threads hold 16 points.
-static bool make_plan(int n, FftPlan &pl, int max_radix = 8) {
-   pl.n = n;
-   pl.nst = 0;
-   int m = n;
-   static const int pref[] = {16, 8, 4, 2, 3, 5};
-   for (int r : pref) {
-      if ((r == 16 || r == 8 || r == 4) && r > max_radix) continue;
-      while (m % r == 0 && pl.nst < kMaxStages) { pl.rad[pl.nst++] = r; m /= r; }
-   }
+static void set_stages(FftPlan &pl) {
    int ns = 1;
    for (int st = 0; st < pl.nst; st++) {
       pl.ns[st] = ns;
@@ -146,7 +44,24 @@ static bool make_plan(int n, FftPlan &pl, int max_radix = 8) {
       pl.magic[st] = ns == 1 ? 0u : (unsigned) ((0x100000000ULL + (unsigned long long) ns - 1) / (unsigned long long) ns);
       ns *= pl.rad[st];
    }
-   return m == 1;
+}
+
+// Stages of an n-point transform (make_radices); max_radix 8, 4 or 2 drops
+// the larger powers of two.  Radix 16 is for the FP32 passes only, whose
+// threads hold 16 points.
+static bool make_plan(int n, FftPlan &pl, int max_radix = 8) {
+   pl.n = n;
+   pl.nst = make_radices(n, max_radix == 16 ? 4 : (max_radix == 8 ? 3 : (max_radix == 4 ? 2 : 1)), pl.rad);
+   set_stages(pl);
+   return pl.nst > 0;
+}
+
+// The same stages in the reverse order.
+static FftPlan reverse_plan(const FftPlan &pl) {
+   FftPlan r = pl;
+   for (int st = 0; st < pl.nst; st++) r.rad[st] = pl.rad[pl.nst - 1 - st];
+   set_stages(r);
+   return r;
 }
 
 static gpe_status validate(const gpe_params *p) {
@@ -196,18 +111,49 @@ template <class T> static gpe_status upload(void **dst, const T *src, size_t n) 
    return GPE_OK;
 }
 
-static gpe_status make_twiddles(gpe_solver *s, int n, void **dst) {
-   std::vector<double2> t(n);
-   for (int m = 0; m < n; m++) {
-      const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double) m / (long double) n;
-      t[m] = make_double2((double) cosl(a), (double) sinl(a));
+// Roots of unity of the stages of pl in the order fft_lines / conv_lines read
+// them: per stage after the first, exp(-2 pi i t k / (Ns r)) at [t - 1][k].
+static void stage_roots(const FftPlan &pl, std::vector<double2> &out) {
+   const size_t at = out.size();
+   for (int st = 1; st < pl.nst; st++)
+      for (int t = 1; t < pl.rad[st]; t++)
+         for (int k = 0; k < pl.ns[st]; k++) {
+            // the root of the n-point table the run-time stages read
+            const long m = (long) t * k * (pl.n / (pl.ns[st] * pl.rad[st]));
+            const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double) m / (long double) pl.n;
+            out.push_back(make_double2((double) cosl(a), (double) sinl(a)));
+         }
+   out.resize(at + pl.n, make_double2(0., 0.));
+}
+
+// The tables of roots (ztab_roots in step_kernels.cuh) for the plans in use.
+static gpe_status make_roots(gpe_solver *s) {
+   const Dims &d = s->d;
+   auto put = [&](const std::vector<double2> &t, void **dst) -> gpe_status {
+      if (*dst) cudaFree(*dst);
+      *dst = nullptr;
+      if (!s->fp32) return upload(dst, t.data(), t.size());
+      std::vector<float2> f(t.size());
+      for (size_t e = 0; e < t.size(); e++) f[e] = make_float2((float) t[e].x, (float) t[e].y);
+      return upload(dst, f.data(), f.size());
+   };
+   std::vector<double2> t;
+   stage_roots(s->px, t);
+   stage_roots(s->pxi, t);
+   CKS(put(t, &s->twx));
+   t.clear();
+   stage_roots(s->py, t);
+   CKS(put(t, &s->twy));
+   t.clear();
+   const int h = d.nz / 2;
+   stage_roots(s->ph, t);
+   t.resize(ztab_roots(h), make_double2(0., 0.));
+   for (int k = 0; k <= h; k++) {
+      const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double) k / (long double) d.nz;
+      t.push_back(make_double2((double) cosl(a), (double) sinl(a)));
    }
-   if (s->fp32) {
-      std::vector<float2> f(n);
-      for (int m = 0; m < n; m++) f[m] = make_float2((float) t[m].x, (float) t[m].y);
-      return upload(dst, f.data(), n);
-   }
-   return upload(dst, t.data(), n);
+   t.resize(ztab_len(h), make_double2(0., 0.));
+   return put(t, &s->twz);
 }
 
 // gencoef (imag3d-mpicuda.cu:894-931, real3d-mpicuda.cu:991-1035).
@@ -355,11 +301,8 @@ static gpe_status encoder(EncodeTiledFn *fn) {
    return GPE_OK;
 }
 
-// 3D tensor map over a [nx][ny][w * nz] array of `esz`-byte scalars with box
-// {bw, by, bx} (innermost first).
-// Rows are `pitch` elements apart (pitch = w_nz when 0).
-static gpe_status make_tmap(CUtensorMap *m, void *base, size_t esz, long w_nz, long ny, long nx, int bw, int by, int bx,
-                            long pitch = 0) {
+gpe_status make_tmap(CUtensorMap *m, void *base, size_t esz, long w_nz, long ny, long nx, int bw, int by, int bx,
+                     long pitch) {
    EncodeTiledFn enc;
    CKS(encoder(&enc));
    if (pitch == 0) pitch = w_nz;
@@ -403,15 +346,6 @@ static int sweep_candidates(int n, int tw_base, int esz, int *TW, int *MSEG, int
       k = 1;
    }
    return k;
-}
-
-// Bytes of one pipeline stage of the x or y sweep.
-static size_t sweep_stage(const gpe_solver *s, int ax, int rows, int TW, int skip) {
-   if (s->fp32)
-      return s->cplx ? (ax == 0 ? xy_stage<float, true, true>(rows, TW, skip) : xy_stage<float, true, false>(rows, TW, skip)).bytes
-                     : (ax == 0 ? xy_stage<float, false, true>(rows, TW, skip) : xy_stage<float, false, false>(rows, TW, skip)).bytes;
-   return s->cplx ? (ax == 0 ? xy_stage<double, true, true>(rows, TW, skip) : xy_stage<double, true, false>(rows, TW, skip)).bytes
-                  : (ax == 0 ? xy_stage<double, false, true>(rows, TW, skip) : xy_stage<double, false, false>(rows, TW, skip)).bytes;
 }
 
 // Tile configuration of the sweeps and of the y / x FFT passes, and the FFT
@@ -561,11 +495,23 @@ static gpe_status plan_tiles(gpe_solver *s) {
       if (mr != 16 && mr != 8 && mr != 4 && mr != 2)
          return fail(GPE_ERR_PARAM, "tuning: fft_max_radix must be 16, 8, 4 or 2");
       if (mr == 16 && !s->fp32) return fail(GPE_ERR_PARAM, "tuning: radix 16 is for mixed precision only");
-      make_plan(d.nx, s->px, mr);
-      make_plan(d.ny, s->py, mr);
-      make_plan(d.nz / 2, s->ph, mr);
+      // lengths with a compile-time pass: radices up to 16 in both precisions
+      // (their threads hold 16 points)
+      const bool plain = s->tune.fft_max_radix <= 0 || s->tune.fft_max_radix == (s->fp32 ? 16 : 8);
+      const int rx = plain && has_len(d.nx) && s->Lx == len_cols(s->fp32) ? 16 : mr;
+      const int ry = plain && has_len(d.ny) && s->Ly == len_cols(s->fp32) ? 16 : mr;
+      const int rz = plain && has_len(d.nz / 2) && d.nz / 2 <= kLenMaxH ? 16 : mr;
+      s->fastx = rx == 16 && has_len(d.nx) && s->Lx == len_cols(s->fp32);
+      s->fasty = ry == 16 && has_len(d.ny) && s->Ly == len_cols(s->fp32);
+      s->fastz = rz == 16 && has_len(d.nz / 2) && d.nz / 2 <= kLenMaxH;
+      make_plan(d.nx, s->px, rx);
+      s->pxi = reverse_plan(s->px);
+      make_plan(d.ny, s->py, ry);
+      make_plan(d.nz / 2, s->ph, rz);
+      CKS(make_roots(s));
       CKS(make_tmap(&s->tm_spec_y, s->spec, rsz, 2 * d.nzh, d.ny, d.nx, 2 * s->Ly, s->boxy, 1, 2 * d.nzp));
       CKS(make_tmap(&s->tm_spec_x, s->spec, rsz, 2 * d.nzh, d.ny, d.nx, 2 * s->Lx, 1, s->boxx, 2 * d.nzp));
+      CKS(make_udd_tmap(s, &s->tm_udd, s->Lx));
    }
    return GPE_OK;
 }
@@ -596,7 +542,7 @@ static gpe_status setup_static(gpe_solver *s) {
 }
 
 // initpotdd (imag3d-mpicuda.cu:945-980) on the octant |kx| <= nx/2,
-// |ky| <= ny/2, kz <= nz/2, stored [|kx|][|ky|][kz]: Udd depends on kx^2,
+// |ky| <= ny/2, kz <= nz/2, stored [|kx|][|ky|][kz] (udd_pitch): Udd depends on kx^2,
 // ky^2, kz^2 only, and the squares of the reference's negative k values equal
 // those of the octant.
 static gpe_status make_udd(gpe_solver *s) {
@@ -608,14 +554,15 @@ static gpe_status make_udd(gpe_solver *s) {
    for (long i = 0; i < nxh; i++) { double k = i * dkx; kx2[i] = k * k; }
    for (long i = 0; i < nyh; i++) { double k = i * dky; ky2[i] = k * k; }
    for (long i = 0; i < nzh; i++) { double k = i * dkz; kz2[i] = k * k; }
-   std::vector<double> u((size_t) (nzh * nxh * nyh));
+   const long nzu = udd_pitch((int) nzh);
+   std::vector<double> u((size_t) (nzu * nxh * nyh), 0.);
    for (long i = 0; i < nxh; i++)
       for (long j = 0; j < nyh; j++)
          for (long k = 0; k < nzh; k++) {
             const double xk = std::sqrt(kz2[k] + kx2[i] + ky2[j]);
             const double tmp = 1. + 3. * std::cos(xk * cutoff) / (xk * xk * cutoff * cutoff) -
                                3. * std::sin(xk * cutoff) / (xk * xk * xk * cutoff * cutoff * cutoff);
-            u[(size_t) ((i * nyh + j) * nzh + k)] = (4. * pi * (3. * kz2[k] / (kx2[i] + ky2[j] + kz2[k]) - 1.) / 3.) * tmp;
+            u[(size_t) ((i * nyh + j) * nzu + k)] = (4. * pi * (3. * kz2[k] / (kx2[i] + ky2[j] + kz2[k]) - 1.) / 3.) * tmp;
          }
    u[0] = 0.;  // imag3d-mpicuda.cu:975-977
    void *dp = nullptr;
@@ -687,9 +634,6 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    st0.norm = 1.; st0.scale = 1.; st0.scale2 = 1.;
    CK(cudaMemcpy(s->state, &st0, sizeof(State), cudaMemcpyHostToDevice));
 
-   CKS(make_twiddles(s, d.nx, &s->twx));
-   CKS(make_twiddles(s, d.ny, &s->twy));
-   CKS(make_twiddles(s, d.nz, &s->twz));
    CKS(make_coef(s, 0, d.nx, p->dx * p->dx));
    CKS(make_coef(s, 1, d.ny, p->dy * p->dy));
    CKS(make_coef(s, 2, d.nz, p->dz * p->dz));
@@ -785,591 +729,9 @@ extern "C" void gpe_destroy(gpe_solver *s) {
 
 extern "C" const char *gpe_last_error(void) { return g_err.c_str(); }
 
-// ------------------------------------------------------------------ launches
-static Trap trap_of(const gpe_solver *s) {
-   Trap t;
-   t.x2 = s->x2; t.y2 = s->y2; t.z2 = s->z2;
-   t.x2f = s->x2f; t.y2f = s->y2f; t.z2f = s->z2f;
-   t.hp = 0.5 * s->par;
-   t.vg2 = s->p.gamma * s->p.gamma;
-   t.vn2 = s->p.nu * s->p.nu;
-   t.vl2 = s->p.lambda * s->p.lambda;
-   return t;
-}
-
-static unsigned blocks_for(long long n, int bs) { return (unsigned) ((n + bs - 1) / bs); }
-
-// Launch on the handle's stream with programmatic dependent launch: the
-// kernel may be scheduled while its predecessor finishes its last wave (its
-// CTAs call pdl_trigger / pdl_wait before touching memory), which hides the
-// gap between the kernels of a step (FP64 0.880 -> 0.872 ms real, 0.722 ->
-// 0.712 ms imaginary time; mixed precision 0.429 -> 0.415 ms at 256^3 and
-// 0.107 -> 0.103 ms at 128^3, 512x512x256 unchanged at 1.69 ms, on B200).
-template <class... KP, class... A>
-static gpe_status launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, const gpe_solver *s, A... args) {
-   cudaLaunchAttribute at[1];
-   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-   at[0].val.programmaticStreamSerializationAllowed = 1;
-   cudaLaunchConfig_t cfg{};
-   cfg.gridDim = grid;
-   cfg.blockDim = block;
-   cfg.dynamicSmemBytes = smem;
-   cfg.stream = s->st;
-   cfg.attrs = at;
-   cfg.numAttrs = 1;
-   CK(cudaLaunchKernelEx(&cfg, k, ((KP) args)...));
-   return GPE_OK;
-}
-
-template <class R, bool CPLX> struct Impl {
-   using P = typename Tr<R, CPLX>::P;
-   using C = cpx<R>;
-
-   static gpe_status smem_attr(const void *f, size_t bytes) {
-      if (bytes > 48 * 1024) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes));
-      return GPE_OK;
-   }
-
-   // runs f(std::integral_constant<int, v>) for v in {2, 4, 8, 16} (tile
-   // widths) or {8, 16, 32} (points per thread)
-   template <class F> static gpe_status with_L(int L, F f) {
-      if (L == 16) return f(std::integral_constant<int, 16>());
-      if (L == 8) return f(std::integral_constant<int, 8>());
-      if (L == 4) return f(std::integral_constant<int, 4>());
-      return f(std::integral_constant<int, 2>());
-   }
-   template <class F> static gpe_status with_ppt(int ppt, F f) {
-      if (ppt <= 8) return f(std::integral_constant<int, 8>());
-      if (ppt <= 16) return f(std::integral_constant<int, 16>());
-      return f(std::integral_constant<int, 32>());
-   }
-   // points per thread of the z passes: (nz/2) L over 256 threads, at least
-   // 16 in FP32 (the radix-16 stages need them)
-   static int zppt(const gpe_solver *s, int L) {
-      const int p = (int) (((s->d.nz / 2) * L + 255) / 256);
-      return s->fp32 ? std::max(p, 16) : p;
-   }
-   // threads of a z inverse pass CTA, and of a forward pass CTA over real
-   // rows: PPT points each of the L half-length lines (the forward passes
-   // over complex rows keep 256: sized CTAs measured slower there, 101 -> 105
-   // us at 256^3 complex FP64)
-   static unsigned z_threads(const gpe_solver *s, int L, int ppt) {
-      const long t = ((long) (s->d.nz / 2) * L + ppt - 1) / ppt;
-      return (unsigned) std::min<long>(256, std::max<long>(32, (t + 31) / 32 * 32));
-   }
-
-   // threads of a y / x pass CTA: PPT points each over a tile of rows x L
-   // (at most 256: the kernels' register budget)
-   static unsigned fft_threads(long rows, int L) {
-      const long t = (rows * L + FftL<R>::PPT - 1) / FftL<R>::PPT;
-      return (unsigned) std::min<long>(256, std::max<long>(32, (t + 31) / 32 * 32));
-   }
-
-   template <bool INV, int L> static gpe_status yfft(gpe_solver *s) {
-      const Dims &d = s->d;
-      const int nkb = (d.nzh + L - 1) / L;
-      const size_t smy = 128 + (size_t) s->boxy * s->nboxy * L * sizeof(C) + d.ny * sizeof(C);
-      CKS(smem_attr((const void *) k_yfft<R, INV, L>, smy));
-      CKS(launch_pdl(k_yfft<R, INV, L>, (unsigned) (d.nx * nkb), fft_threads(s->boxy * s->nboxy, L), smy, s, s->tm_spec_y, d, s->py,
-                     (const C *) s->twy, s->boxy, s->nboxy, s->err));
-      CKL();
-      mark(s);
-      return GPE_OK;
-   }
-
-   template <int L> static gpe_status xconv(gpe_solver *s) {
-      const Dims &d = s->d;
-      const int nkb = (d.nzh + L - 1) / L;
-      const size_t sm = 128 + (size_t) s->boxx * s->nboxx * L * sizeof(C) + d.nx * sizeof(C) +
-                        (size_t) (d.nx / 2 + 1) * L * sizeof(double);
-      CKS(smem_attr((const void *) k_xconv<R, L>, sm));
-      CKS(launch_pdl(k_xconv<R, L>, (unsigned) (d.ny * nkb), fft_threads(s->boxx * s->nboxx, L), sm, s, s->tm_spec_x, d, s->px, (const C *) s->twx, s->udd,
-                                                                 s->state, s->boxx, s->nboxx, s->err));
-      CKL();
-      mark(s);
-      return GPE_OK;
-   }
-
-   // z pass kernels for a tile of L rows
-   template <int L> static gpe_status zfwd_L(gpe_solver *s, size_t sm, bool sized) {
-      const Dims &d = s->d;
-      return with_ppt(zppt(s, L), [&](auto pc) {
-         constexpr int PPT = decltype(pc)::value;
-         CKS(smem_attr((const void *) k_zfwd<R, CPLX, PPT, L>, sm));
-         const unsigned nt = sized ? z_threads(s, L, PPT) : 256u;
-         CKS(launch_pdl(k_zfwd<R, CPLX, PPT, L>, blocks_for(d.nxy, L), nt, sm, s, (const P *) s->psi, (C *) s->spec, d,
-                        s->ph, (const C *) s->twz, s->LSr, s->err));
-         CKL();
-         mark(s);
-         return GPE_OK;
-      });
-   }
-
-   template <int L> static gpe_status zinv_L(gpe_solver *s, size_t sm) {
-      const Dims &d = s->d;
-      return with_ppt(zppt(s, L), [&](auto pc) {
-         constexpr int PPT = decltype(pc)::value;
-         CKS(smem_attr((const void *) k_zinv<R, PPT, L>, sm));
-         CKS(launch_pdl(k_zinv<R, PPT, L>, blocks_for(d.nxy, L), z_threads(s, L, PPT), sm, s, (const C *) s->spec, (R *) s->phi, d, s->ph,
-                        (const C *) s->twz, s->LSo, s->err));
-         CKL();
-         mark(s);
-         return GPE_OK;
-      });
-   }
-
-   // shared memory of the z passes for L rows; the rows per CTA start at the
-   // preferred value and halve (down to 4) until the tile fits
-   static size_t zfwd_smem(const gpe_solver *s, int L) {
-      const Dims &d = s->d;
-      return 128 + (size_t) L * s->LSr * sizeof(P) + (size_t) (d.nz / 2) * L * sizeof(C) + d.nz * sizeof(C);
-   }
-   static size_t zinv_smem(const gpe_solver *s, int L) {
-      const Dims &d = s->d;
-      const size_t in_el = std::max((size_t) L * d.nzp, ((size_t) L * s->LSo * sizeof(R) + sizeof(C) - 1) / sizeof(C));
-      return 128 + ((in_el + 7) & ~(size_t) 7) * sizeof(C) + (size_t) (d.nz / 2) * L * sizeof(C) + d.nz * sizeof(C);
-   }
-   template <class SM> static int zrows(const gpe_solver *s, int pref, SM smem) {
-      int L = pref;
-      while (L > 4 && smem(s, L) > 227 * 1024) L /= 2;
-      return L;
-   }
-   template <class F> static gpe_status with_zrows(int L, F f) {
-      if (L == 16) return f(std::integral_constant<int, 16>());
-      if (L == 8) return f(std::integral_constant<int, 8>());
-      return f(std::integral_constant<int, 4>());
-   }
-
-   static gpe_status psidd2(gpe_solver *s) {
-      const Dims &d = s->d;
-      {
-         // real rows: 8-row tiles on CTAs sized to them, except FP64 rows
-         // shorter than 128 points, which keep 16 rows on 256 threads (sized
-         // CTAs of 32 threads measured slower at 64^3: 8.8 -> 10.8 us)
-         const bool sized = !CPLX && (sizeof(R) == 4 || d.nz >= 128);
-         const int L = zrows(s, (!CPLX && !sized) ? 16 : ZRows<R, CPLX>::fwd, zfwd_smem);
-         const size_t sm = zfwd_smem(s, L);
-         CKS(with_zrows(L, [&](auto lc) { return zfwd_L<decltype(lc)::value>(s, sm, sized); }));
-      }
-      CKS(with_L(s->Ly, [&](auto Lc) { return yfft<false, decltype(Lc)::value>(s); }));
-      CKS(with_L(s->Lx, [&](auto Lc) { return xconv<decltype(Lc)::value>(s); }));
-      CKS(with_L(s->Ly, [&](auto Lc) { return yfft<true, decltype(Lc)::value>(s); }));
-      {
-         const int L = zrows(s, ZRows<R, CPLX>::inv, zinv_smem);
-         const size_t sm = zinv_smem(s, L);
-         CKS(with_zrows(L, [&](auto lc) { return zinv_L<decltype(lc)::value>(s, sm); }));
-      }
-      CKS(launch_pdl(k_phifix<R>, (unsigned) std::max<long>(1, (d.ny - 1) + (d.nx - 1)),
-                     (unsigned) std::min<long>(256, std::max<long>(32, (d.nz - 1 + 31) / 32 * 32)), 0, s, (R *) s->phi, d));
-      CKL();
-      mark(s);
-      s->launches += 6;
-      return GPE_OK;
-   }
-
-   template <int AXIS, bool NU, int MSEG, int S, int TWC> static gpe_status sweep_xy_launch_t(gpe_solver *s, double g, double gd) {
-      auto &w = s->sw[AXIS];
-      const Dims &d = s->d;
-      const void *f = (const void *) k_sweep_xy<R, CPLX, AXIS, NU, MSEG, S, TWC>;
-      CKS(smem_attr(f, w.smem));
-      const int nzb = (d.nz + w.TW - 1) / w.TW;
-      const int ntiles = (AXIS == 0 ? d.ny : d.nx) * nzb;
-      const unsigned grid = (unsigned) std::min(ntiles, w.ctas * s->nsm);
-      CKS(launch_pdl(k_sweep_xy<R, CPLX, AXIS, NU, MSEG, S, TWC>, grid, ((w.TW * w.tab.P + 31) & ~31), w.smem, s,
-          w.tm_psi, w.tm_phi, d, w.tab, trap_of(s), LinPhase{s->lin[0], s->lin[1], s->lin[2]}, g, gd, s->p.dt,
-          s->state, w.TW, w.boxn, w.nbox, s->err));
-      CKL();
-      mark(s);
-      s->launches++;
-      return GPE_OK;
-   }
-
-   // FP64 tiles of 8 or 16 lines use kernels compiled for that width
-   template <int AXIS, bool NU, int MSEG, int S> static gpe_status sweep_xy_launch(gpe_solver *s, double g, double gd) {
-      if constexpr (std::is_same<R, double>::value) {
-         if (s->sw[AXIS].TW == 8) return sweep_xy_launch_t<AXIS, NU, MSEG, S, 8>(s, g, gd);
-         if (s->sw[AXIS].TW == 16) return sweep_xy_launch_t<AXIS, NU, MSEG, S, 16>(s, g, gd);
-      }
-      return sweep_xy_launch_t<AXIS, NU, MSEG, S, 0>(s, g, gd);
-   }
-
-   // 32-point segments exist for FP32 real lines only (register budget)
-   static constexpr bool kSeg32 = std::is_same<R, float>::value && !CPLX;
-
-   template <int AXIS, bool NU> static gpe_status sweep_xy(gpe_solver *s, double g, double gd) {
-      const auto &w = s->sw[AXIS];
-      if constexpr (kSeg32)
-         if (w.MSEG == 32)
-            return w.S == 3 ? sweep_xy_launch<AXIS, NU, 32, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 32, 2>(s, g, gd);
-      if (w.MSEG == 8) return w.S == 3 ? sweep_xy_launch<AXIS, NU, 8, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 8, 2>(s, g, gd);
-      return w.S == 3 ? sweep_xy_launch<AXIS, NU, 16, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 16, 2>(s, g, gd);
-   }
-
-   // x sweep; with nu the pending 1/norm and calcnu are applied on load
-   // (calcnu_kernel imag3d-mpicuda.cu:1759 fused with calclux_kernel :1802).
-   static gpe_status xsweep(gpe_solver *s, bool nu, double g, double gd) {
-      return nu ? sweep_xy<0, true>(s, g, gd) : sweep_xy<0, false>(s, g, gd);
-   }
-
-   static gpe_status ysweep(gpe_solver *s) { return sweep_xy<1, false>(s, 0., 0.); }
-
-   template <int MOM, int MSEG, int S, int TWC> static gpe_status sweep_z_launch_t(gpe_solver *s, double *dev_norm) {
-      auto &w = s->sw[2];
-      const Dims &d = s->d;
-      const void *f = (const void *) k_sweep_z<R, CPLX, MOM, MSEG, S, TWC>;
-      CKS(smem_attr(f, w.smem));
-      const long long ntiles = (d.nxy + w.TW - 1) / w.TW;
-      const unsigned grid = (unsigned) std::min<long long>(ntiles, (long long) w.ctas * s->nsm);
-      CKS(launch_pdl(k_sweep_z<R, CPLX, MOM, MSEG, S, TWC>, grid, ((w.TW * w.tab.P + 31) & ~31), w.smem, s,
-          (P *) s->psi, d, w.tab, w.TW, w.LS, zout(s), s->p.dx, s->p.dy, s->state, dev_norm, s->err));
-      CKL();
-      mark(s);
-      s->launches++;
-      return GPE_OK;
-   }
-
-   template <int MOM, int MSEG, int S> static gpe_status sweep_z_launch(gpe_solver *s, double *nrm) {
-      if constexpr (std::is_same<R, double>::value) {
-         if (s->sw[2].TW == 8) return sweep_z_launch_t<MOM, MSEG, S, 8>(s, nrm);
-         if (s->sw[2].TW == 16) return sweep_z_launch_t<MOM, MSEG, S, 16>(s, nrm);
-      }
-      return sweep_z_launch_t<MOM, MSEG, S, 0>(s, nrm);
-   }
-
-   template <int MOM> static gpe_status zsweep_m(gpe_solver *s, double *nrm) {
-      const auto &w = s->sw[2];
-      if constexpr (kSeg32)
-         if (w.MSEG == 32) return w.S == 3 ? sweep_z_launch<MOM, 32, 3>(s, nrm) : sweep_z_launch<MOM, 32, 2>(s, nrm);
-      if (w.MSEG == 8) return w.S == 3 ? sweep_z_launch<MOM, 8, 3>(s, nrm) : sweep_z_launch<MOM, 8, 2>(s, nrm);
-      return w.S == 3 ? sweep_z_launch<MOM, 16, 3>(s, nrm) : sweep_z_launch<MOM, 16, 2>(s, nrm);
-   }
-
-   // z sweep; mom 1: also the norm of the step (dev_norm may be null) and the
-   // pending renormalisation; mom 2: the rms row partials
-   static gpe_status zsweep(gpe_solver *s, int mom, double *dev_norm = nullptr) {
-      if (mom == 2) return zsweep_m<2>(s, nullptr);
-      return mom == 1 ? zsweep_m<1>(s, dev_norm) : zsweep_m<0>(s, nullptr);
-   }
-
-   static ZOut zout(const gpe_solver *s) { return ZOut{s->wz, s->wz2, s->p.dz / 3., s->rowA, s->rowA, s->rowB}; }
-
-   static gpe_status norm_final(gpe_solver *s, double *dev_out) {
-      CKS(launch_pdl(k_norm_final, blocks_for(s->d.nx, kNormRowsPerCta), 32 * kNormRowsPerCta, 0, s,
-          s->rowA, s->d, s->p.dx, s->p.dy, s->state, s->tmp, dev_out));
-      CKL();
-      s->launches++;
-      return GPE_OK;
-   }
-
-   static gpe_status apply_scale(gpe_solver *s) {
-      k_apply_scale<R, CPLX><<<592, 256, 0, s->st>>>((P *) s->psi, s->d.npts, s->state);
-      CKL();
-      k_state_set<<<1, 1, 0, s->st>>>(s->state, 1.);
-      CKL();
-      s->launches += 2;
-      return GPE_OK;
-   }
-
-   static void rows_dens(gpe_solver *s, double *a, double *b) {
-      k_rows_dens<R, CPLX><<<blocks_for(s->d.nxy, kRowWarps), 32 * kRowWarps, 0, s->st>>>(
-          (const P *) s->psi, s->d, s->p.dz / 3., s->wz, s->wz2, a, b);
-   }
-
-   // line integrals of |psi|^2 along `axis` into rowA (z: a warp per row)
-   static void lineint(gpe_solver *s, int axis, double h) {
-      const Dims &d = s->d;
-      if (axis == 2) return rows_dens(s, s->rowA, nullptr);
-      const long long nl = (long long) (axis == 0 ? d.ny : d.nx) * d.nz;
-      k_lineint_psi<R, CPLX><<<blocks_for(nl, 128), 128, 0, s->st>>>((const P *) s->psi, d, axis, h, s->rowA);
-   }
-
-   static gpe_status calcnorm(gpe_solver *s, bool renorm) {
-      rows_dens(s, s->rowA, nullptr);
-      CKL();
-      CKS(norm_final(s, s->obs));
-      s->launches++;
-      if (renorm) {
-         CKS(apply_scale(s));
-      } else {
-         k_state_set<<<1, 1, 0, s->st>>>(s->state, 1.);
-         CKL();
-      }
-      return GPE_OK;
-   }
-
-   static gpe_status rms(gpe_solver *s, double *dev_out) {
-      rows_dens(s, s->rowA, s->rowB);
-      CKL();
-      s->launches++;
-      return rms_final(s, dev_out);
-   }
-
-   // rms from the row partials in rowA / rowB (k_rows_dens, or the z sweep
-   // of the step with mom = 2)
-   static gpe_status rms_final(gpe_solver *s, double *dev_out) {
-      const Dims &d = s->d;
-      CKS(launch_pdl(k_rms_final, blocks_for(d.nx, kNormRowsPerCta), 32 * kNormRowsPerCta, 0, s,
-          s->rowA, s->rowB, d, s->p.dx, s->p.dy, s->x2, s->y2, s->state, s->tmp, dev_out));
-      CKL();
-      s->launches++;
-      return GPE_OK;
-   }
-
-   static gpe_status muen(gpe_solver *s, double g, double gd, double *dev_out) {
-      const Dims &d = s->d;
-      CKS(psidd2(s));
-      // chunks of x planes so that about four CTAs per SM run, at least 16
-      // planes each (a chunk reads four more), with room for the partials
-      const unsigned bz = blocks_for(d.nz, kMuZ), by = blocks_for(d.ny, kMuY);
-      const long long want = std::max<long long>(1, 4LL * s->nsm / ((long long) bz * by));
-      const long long most = std::max<long long>(1, s->row_cap / (2LL * bz * by));
-      const int chunk = (int) std::max<long long>(std::min<long long>(16, d.nx), (d.nx + std::min(want, most) - 1) / std::min(want, most));
-      const unsigned bx = blocks_for(d.nx, chunk);
-      k_muen<R, CPLX><<<dim3(bz, by, bx), kMuY * kMuZ, 0, s->st>>>((const P *) s->psi, (const R *) s->phi, d, trap_of(s),
-                                                                  g, gd, s->p.dx, s->p.dy, s->p.dz, s->par, chunk,
-                                                                  s->rowA);
-      CKL();
-      k_sum2<<<1, 256, 0, s->st>>>(s->rowA, (int) (bx * by * bz), s->p.dx * s->p.dy * s->p.dz / 27., dev_out);
-      CKL();
-      s->launches += 2;
-      return GPE_OK;
-   }
-
-   // One split step (imag3d-mpicuda.cu:319-324): calcpsidd2, calcnu (fused
-   // into the x sweep), x, y, z sweeps, and in imaginary time the norm.
-   // rms_rows: (real time) the z sweep also leaves the rms row partials of
-   // the new psi in rowA / rowB for rms_final.
-   static gpe_status step(gpe_solver *s, double g, double gd, double *dev_norm, bool rms_rows = false) {
-      CKS(psidd2(s));
-      CKS(xsweep(s, true, g, gd));
-      CKS(ysweep(s));
-      const bool imag = !CPLX;
-      CKS(zsweep(s, imag ? 1 : (rms_rows ? 2 : 0), dev_norm));
-      if (imag) mark(s);  // (norm: the z sweep's last CTA)
-      return GPE_OK;
-   }
-
-   static gpe_status calcnu(gpe_solver *s, double g, double gd) {
-      k_calcnu<R, CPLX><<<592, 256, 0, s->st>>>((P *) s->psi, (const R *) s->phi, s->d, trap_of(s), g, gd, s->p.dt);
-      CKL();
-      s->launches++;
-      return GPE_OK;
-   }
-
-   static gpe_status density(gpe_solver *s, int kind, long sx, long sy, long sz, double *out, long cap, long *count);
-
-   // ---- batched launches: geometry and descriptor of this instance
-   static gpe_status geom(gpe_solver *s, int Ly, int Lx, BatchGeom *g) {
-      const Dims &d = s->d;
-      *g = BatchGeom{};
-      g->Ly = s->Ly;
-      g->Lx = s->Lx;
-      if (Ly <= 0 || Lx <= 0) return GPE_OK;
-      // z passes: 8-row tiles on CTAs sized to them
-      constexpr int L = 8;
-      const int zp = zppt(s, L);
-      const int ppt = zp <= 8 ? 8 : (zp <= 16 ? 16 : 32);
-      g->zppt = ppt;
-      g->tiles[kPZfwd] = g->tiles[kPZinv] = (d.nxy + L - 1) / L;
-      g->threads[kPZfwd] = g->threads[kPZinv] = z_threads(s, L, ppt);
-      g->smem[kPZfwd] = zfwd_smem(s, L);
-      g->smem[kPZinv] = zinv_smem(s, L);
-      if (g->smem[kPZfwd] > 227 * 1024 || g->smem[kPZinv] > 227 * 1024)
-         return fail(GPE_ERR_PARAM, "batch: z rows too long for 8-row tiles");
-      // y / x passes
-      const long ry = (long) s->boxy * s->nboxy, rx = (long) s->boxx * s->nboxx;
-      if (ry * Ly > 256L * FftL<R>::PPT || rx * Lx > 256L * FftL<R>::PPT)
-         return fail(GPE_ERR_PARAM, "batch: FFT tile too wide for this grid");
-      g->tiles[kPYfft] = g->tiles[kPYinv] = (long long) d.nx * ((d.nzh + Ly - 1) / Ly);
-      g->tiles[kPXconv] = (long long) d.ny * ((d.nzh + Lx - 1) / Lx);
-      g->threads[kPYfft] = g->threads[kPYinv] = fft_threads(ry, Ly);
-      g->threads[kPXconv] = fft_threads(rx, Lx);
-      g->smem[kPYfft] = g->smem[kPYinv] = 128 + (size_t) ry * Ly * sizeof(C) + d.ny * sizeof(C);
-      g->smem[kPXconv] = 128 + (size_t) rx * Lx * sizeof(C) + d.nx * sizeof(C) + (size_t) (d.nx / 2 + 1) * Lx * sizeof(double);
-      // boundary planes of phi
-      g->tiles[kPPhifix] = std::max<long>(1, (d.ny - 1) + (d.nx - 1));
-      g->threads[kPPhifix] = (unsigned) std::min<long>(256, std::max<long>(32, (d.nz - 1 + 31) / 32 * 32));
-      // sweeps
-      const size_t esz = s->esz_psi;
-      for (int ax = 0; ax < 3; ax++) {
-         const auto &w = s->sw[ax];
-         const int TW = w.TW, P = w.tab.P;
-         const int kp = kPXsweep + ax;
-         g->mseg[ax] = w.MSEG;
-         g->threads[kp] = (unsigned) ((TW * P + 31) & ~31);
-         const int nzb = (d.nz + TW - 1) / TW;
-         g->tiles[kp] = ax == 0 ? (long long) d.ny * nzb : (ax == 1 ? (long long) d.nx * nzb : (d.nxy + TW - 1) / TW);
-         const size_t stage = ax < 2 ? sweep_stage(s, ax, w.boxn * w.nbox, TW, w.tab.skip) : (size_t) TW * w.LS * esz;
-         g->stage[ax] = (uint32_t) ((stage + 127) & ~(size_t) 127);
-         g->xch[ax] = (uint32_t) ((2 * (size_t) P * TW * esz + 15) & ~(size_t) 15);
-         if (!s->fp32) {
-            if (ax == 0) g->extra[ax] = (uint32_t) ((d.nx + w.tab.skip) * (s->cplx ? 16 : 8));
-            if (ax == 2) g->extra[ax] = (uint32_t) (4 * (size_t) P * w.MSEG * esz);
-         }
-         if (ax == 2) g->part = (uint32_t) (((size_t) P * TW * sizeof(double) + 15) & ~(size_t) 15);
-      }
-      // norm (imaginary time)
-      g->tiles[kPNorm] = s->cplx ? 0 : 1;
-      g->threads[kPNorm] = 256;
-      return GPE_OK;
-   }
-
-   static gpe_status desc(gpe_solver *s, int Ly, int Lx, double g, double gd, BatchDesc *D) {
-      const Dims &d = s->d;
-      std::memset((void *) D, 0, sizeof(BatchDesc));
-      D->tm_psi[0] = s->sw[0].tm_psi;
-      D->tm_psi[1] = s->sw[1].tm_psi;
-      D->tm_phi = s->sw[0].tm_phi;
-      CKS(make_tmap(&D->tm_spec_y, s->spec, s->esz_r, 2 * d.nzh, d.ny, d.nx, 2 * Ly, s->boxy, 1, 2 * d.nzp));
-      CKS(make_tmap(&D->tm_spec_x, s->spec, s->esz_r, 2 * d.nzh, d.ny, d.nx, 2 * Lx, 1, s->boxx, 2 * d.nzp));
-      for (int ax = 0; ax < 3; ax++) {
-         const auto &w = s->sw[ax];
-         SweepView &v = D->sv[ax];
-         v.tb = w.tab;
-         v.trap = trap_of(s);
-         v.lin = LinPhase{s->lin[0], s->lin[1], s->lin[2]};
-         v.d = d;
-         v.st = s->state;
-         v.err = s->err;
-         v.psi = s->psi;
-         v.zo = zout(s);
-         v.g = g;
-         v.gd = gd;
-         v.dt = s->p.dt;
-         v.TW = w.TW;
-         v.boxn = w.boxn;
-         v.nbox = w.nbox;
-         v.LS = w.LS;
-      }
-      D->px = s->px;
-      D->py = s->py;
-      D->ph = s->ph;
-      D->d = d;
-      D->psi = s->psi;
-      D->spec = s->spec;
-      D->phi = s->phi;
-      D->twx = s->twx;
-      D->twy = s->twy;
-      D->twz = s->twz;
-      D->udd = s->udd;
-      D->state = s->state;
-      D->err = s->err;
-      D->rowA = s->rowA;
-      D->hx = s->p.dx;
-      D->hy = s->p.dy;
-      D->LSr = s->LSr;
-      D->LSo = s->LSo;
-      D->boxy = s->boxy;
-      D->nboxy = s->nboxy;
-      D->boxx = s->boxx;
-      D->nboxx = s->nboxx;
-      D->Ly = Ly;
-      D->Lx = Lx;
-      return GPE_OK;
-   }
-};
-
-template <class R, bool CPLX>
-gpe_status Impl<R, CPLX>::density(gpe_solver *s, int kind, long sx, long sy, long sz, double *out, long cap,
-                                  long *count) {
-   const Dims &d = s->d;
-   const P *psi = (const P *) s->psi;
-   const double hh[3] = {s->p.dx, s->p.dy, s->p.dz};
-   const int n[3] = {d.nx, d.ny, d.nz};
-   const std::vector<double> *crd[3] = {&s->hx, &s->hy, &s->hz};
-   const long stp[3] = {sx, sy, sz};
-   std::vector<double> buf;
-   long o = 0;
-   auto need = [&](long m) -> gpe_status {
-      if (m > cap) return fail(GPE_ERR_PARAM, "density output buffer too small");
-      return GPE_OK;
-   };
-   if (kind >= GPE_DEN_1D_X && kind <= GPE_DEN_1D_Z) {
-      // axis integrated first, then the second one (reference nesting)
-      const int keep = kind - GPE_DEN_1D_X;
-      const int first = (keep == 2) ? 1 : 2;   // z (or y for the z profile)
-      const int second = (keep == 0) ? 1 : 0;  // y for x profile, x otherwise
-      const int o1 = first == 0 ? 1 : 0, o2 = first == 2 ? 1 : 2;  // axes of the 2D result
-      if ((long long) n[o1] * n[o2] > s->row_cap) return fail(GPE_ERR_STATE, "row buffer too small");
-      lineint(s, first, hh[first]);
-      CKL();
-      const int ax = (second == o1) ? 0 : 1;  // integrate rows (0) or columns (1)
-      const int m = n[keep];
-      k_lineint_arr<<<blocks_for(m, 128), 128, 0, s->st>>>(s->rowA, n[o1], n[o2], ax == 0 ? 0 : 1, hh[second], s->tmp);
-      CKL();
-      s->launches += 2;
-      buf.resize(m);
-      CK(cudaMemcpyAsync(buf.data(), s->tmp, sizeof(double) * m, cudaMemcpyDeviceToHost, s->st));
-      CK(cudaStreamSynchronize(s->st));
-      for (long c = 0; c < m; c += stp[keep]) {
-         CKS(need(o + 2));
-         out[o++] = (*crd[keep])[c];
-         out[o++] = buf[c];
-      }
-   } else if (kind >= GPE_DEN_2D_XY && kind <= GPE_DEN_2D_YZ) {
-      const int integ = 2 - (kind - GPE_DEN_2D_XY);  // xy -> z, xz -> y, yz -> x
-      const int a1 = integ == 0 ? 1 : 0, a2 = integ == 2 ? 1 : 2;
-      if ((long long) n[a1] * n[a2] > s->row_cap) return fail(GPE_ERR_STATE, "row buffer too small");
-      lineint(s, integ, hh[integ]);
-      CKL();
-      s->launches++;
-      buf.resize((size_t) n[a1] * n[a2]);
-      CK(cudaMemcpyAsync(buf.data(), s->rowA, sizeof(double) * buf.size(), cudaMemcpyDeviceToHost, s->st));
-      CK(cudaStreamSynchronize(s->st));
-      for (long u = 0; u < n[a1]; u += stp[a1])
-         for (long v = 0; v < n[a2]; v += stp[a2]) {
-            CKS(need(o + 3));
-            out[o++] = (*crd[a1])[u];
-            out[o++] = (*crd[a2])[v];
-            out[o++] = buf[(size_t) u * n[a2] + v];
-         }
-   } else if (kind >= GPE_DEN_3D_XY0 && kind <= GPE_DEN_3D_0YZ) {
-      const int fixed = 2 - (kind - GPE_DEN_3D_XY0);  // xy0 -> z fixed, x0z -> y, 0yz -> x
-      const int a1 = fixed == 0 ? 1 : 0, a2 = fixed == 2 ? 1 : 2;
-      int lo[3] = {0, 0, 0}, hi[3] = {d.nx, d.ny, d.nz}, sp[3] = {(int) sx, (int) sy, (int) sz};
-      lo[fixed] = n[fixed] / 2; hi[fixed] = lo[fixed] + 1; sp[fixed] = 1;
-      const long na = (n[a1] + stp[a1] - 1) / stp[a1], nb = (n[a2] + stp[a2] - 1) / stp[a2];
-      double *dv = nullptr;
-      CK(cudaMalloc(&dv, sizeof(double) * na * nb));
-      k_gather_dens<R, CPLX><<<blocks_for(na * nb, 256), 256, 0, s->st>>>(psi, d, lo[0], hi[0], sp[0], lo[1], hi[1], sp[1],
-                                                                         lo[2], hi[2], sp[2], dv);
-      s->launches++;
-      buf.resize(na * nb);
-      cudaError_t e1 = cudaGetLastError();
-      cudaError_t e2 = cudaMemcpyAsync(buf.data(), dv, sizeof(double) * buf.size(), cudaMemcpyDeviceToHost, s->st);
-      cudaError_t e3 = cudaStreamSynchronize(s->st);
-      cudaFree(dv);
-      if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) return fail(GPE_ERR_CUDA, "density cut failed");
-      for (long u = 0; u < na; u++)
-         for (long v = 0; v < nb; v++) {
-            CKS(need(o + 3));
-            out[o++] = (*crd[a1])[u * stp[a1]];
-            out[o++] = (*crd[a2])[v * stp[a2]];
-            out[o++] = buf[(size_t) u * nb + v];
-         }
-   } else if (kind == GPE_DEN_3D) {
-      const long na = (d.nx + sx - 1) / sx, nb = (d.ny + sy - 1) / sy, nc = (d.nz + sz - 1) / sz;
-      CKS(need(na * nb * nc));
-      double *dv = nullptr;
-      CK(cudaMalloc(&dv, sizeof(double) * na * nb * nc));
-      k_gather_dens<R, CPLX><<<592, 256, 0, s->st>>>(psi, d, 0, d.nx, (int) sx, 0, d.ny, (int) sy, 0, d.nz, (int) sz, dv);
-      s->launches++;
-      cudaError_t e1 = cudaGetLastError();
-      cudaError_t e2 = cudaMemcpyAsync(out, dv, sizeof(double) * na * nb * nc, cudaMemcpyDeviceToHost, s->st);
-      cudaError_t e3 = cudaStreamSynchronize(s->st);
-      cudaFree(dv);
-      if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) return fail(GPE_ERR_CUDA, "density copy failed");
-      o = na * nb * nc;
-   } else {
-      return fail(GPE_ERR_PARAM, "unknown density kind");
-   }
-   if (count) *count = o;
-   return GPE_OK;
-}
-
 #define DISPATCH(s, CALL)                                                                 \
-   (((s)->fp32) ? (((s)->cplx) ? Impl<float, true>::CALL : Impl<float, false>::CALL)     \
-                : (((s)->cplx) ? Impl<double, true>::CALL : Impl<double, false>::CALL))
+   (((s)->fp32) ? (((s)->cplx) ? Ops<float, true>::CALL : Ops<float, false>::CALL)     \
+                : (((s)->cplx) ? Ops<double, true>::CALL : Ops<double, false>::CALL))
 
 #define CHECK_HANDLE(s) \
    if (!(s)) return fail(GPE_ERR_PARAM, "null solver handle")
@@ -1384,7 +746,7 @@ static gpe_status fetch(gpe_solver *s, double *host, const void *dev, size_t nd)
    if (!s->fp32) {
       CK(cudaMemcpyAsync(host, dev, sizeof(double) * nd, cudaMemcpyDeviceToHost, s->st));
    } else {
-      const size_t cap = s->esz_c * (size_t) s->d.nzp * (size_t) s->d.nxy / sizeof(double);
+      const size_t cap = spec_doubles(s);
       for (size_t at = 0; at < nd; at += cap) {
          const size_t m = std::min(cap, nd - at);
          k_convert<<<(unsigned) std::min<size_t>(592, (m + 255) / 256), 256, 0, s->st>>>(
@@ -1404,7 +766,7 @@ extern "C" gpe_status gpe_set_psi(gpe_solver *s, const double *psi) {
    CK(cudaSetDevice(s->dev));
    const size_t nd = (size_t) s->d.npts * (s->cplx ? 2 : 1);
    if (s->fp32) {
-      const size_t cap = s->esz_c * (size_t) s->d.nzp * (size_t) s->d.nxy / sizeof(double);
+      const size_t cap = spec_doubles(s);
       for (size_t at = 0; at < nd; at += cap) {
          const size_t m = std::min(cap, nd - at);
          CK(cudaMemcpyAsync(s->spec, psi + at, sizeof(double) * m, cudaMemcpyHostToDevice, s->st));
@@ -1723,13 +1085,12 @@ extern "C" double gpe_step_kernel_bytes(gpe_solver *s, int i) {
    const double sp = (double) s->esz_psi, sc = (double) s->esz_c, r = (double) s->esz_r;
    const double npts = (double) d.npts, half = (double) d.nzh * (double) d.nxy;
    const double oct = (double) d.nzh * (d.nx / 2 + 1) * (d.ny / 2 + 1) * 8.;
-   const double planes = ((double) (d.ny - 1) * (d.nz - 1) + (double) (d.nx - 1) * (d.nz - 1)) * 2. * r;
    switch (i) {
    case 0: return npts * sp + half * sc;
    case 1: case 3: return 2. * half * sc;
    case 2: return 2. * half * sc + oct;
-   case 4: return half * sc + npts * r;
-   case 5: return planes;
+   case 4: return half * sc + npts * r;  // with the boundary planes (a rewrite of rows it stores anyway)
+   case 5: return 0.;                    // folded into case 4
    case 6: return npts * (2. * sp + r);
    case 7: return 2. * npts * sp;
    case 8: return 2. * npts * sp;
@@ -1950,7 +1311,7 @@ gpe_status params_of(gpe_solver *s, gpe_params *p) {
    return GPE_OK;
 }
 int device_of(gpe_solver *s) { return s->dev; }
-long long kernels_per_step(gpe_solver *) { return 9; }
+long long kernels_per_step(gpe_solver *) { return 8; }
 unsigned long long plan_generation(gpe_solver *s) { return s->plan_gen; }
 gpe_status tuning_as_set(gpe_solver *s, gpe_tuning *t) {
    CHECK_HANDLE(s);

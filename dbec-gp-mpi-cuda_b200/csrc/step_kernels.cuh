@@ -2,6 +2,7 @@
 // fused calcnu + sweeps, norm) and of the observables.
 #pragma once
 
+#include "fftn.cuh"
 #include "kernels.cuh"
 #include "tma.cuh"
 
@@ -44,6 +45,35 @@ template <class R, bool CPLX> struct ZRows {
    static constexpr int inv = 8;
 };
 
+// Tables of roots: a y line has n stage roots (padded to n entries), an x line
+// n forward and n inverse ones (one set where the plan reads the same both
+// ways), a z line of half length h its stage roots, padded to even, and then
+// W^k, k <= h, padded to even.
+__host__ __device__ constexpr int ztab_roots(int h) { return (h + 1) & ~1; }
+__host__ __device__ constexpr int ztab_len(int h) { return ztab_roots(h) + ((h + 2) & ~1); }
+__host__ __device__ __forceinline__ int conv_roots(const FftPlan &px) {
+   for (int q = 0; q < px.nst / 2; q++)
+      if (px.rad[q] != px.rad[px.nst - 1 - q]) return 2 * px.n;
+   return px.n;
+}
+
+// Udd's columns of an x tile: nb boxes of rows |kx| rows (at most the 256 a TMA
+// box may have) by L columns, FP64; of several boxes each is a multiple of 8
+// rows, so that the next one lands on a 128-byte boundary.
+struct UddBox {
+   int nb, rows;
+   uint32_t bytes;  // shared memory of one tile's columns, a multiple of 128
+};
+__host__ __device__ __forceinline__ constexpr UddBox udd_box(int nx, int L) {
+   const int nxh = nx / 2 + 1, nb = (nxh + 255) / 256;
+   const int rows = nb == 1 ? nxh : ((nxh + nb - 1) / nb + 7) & ~7;
+   return UddBox{nb, rows, (uint32_t) ((nb * rows * L * 8 + 127) & ~127)};
+}
+// Bytes of a tile of `rows` by L columns of complex R, a multiple of 128.
+template <class R> __host__ __device__ __forceinline__ constexpr uint32_t fft_tile_bytes(int rows, int L) {
+   return (uint32_t) ((rows * L * 2 * (int) sizeof(R) + 127) & ~127);
+}
+
 // |psi|^2 of L rows (row stride LS elements) packed as complex lines of
 // length h = nz/2 in the interleaved layout: buf[m L + l] = (rho[2m], rho[2m+1]).
 template <class R, bool CPLX, int L>
@@ -55,26 +85,109 @@ __device__ __forceinline__ void zfwd_pack(const typename Tr<R, CPLX>::P *rows, i
    }
 }
 
-// Real-FFT split of the transformed lines Z into half-spectrum rows
-// out[l pitch + k], k < nzh, zero padding for nzh <= k < nzp, rows l < nr.
+// Real-FFT split of the transformed lines Z (interleaved) into half-spectrum
+// rows out[l pitch + k], k <= h, and zero padding up to nzp.  X[k] and X[h-k]
+// come from the same pair of inputs: X[k] = E + W^k O, X[h-k] = conj(E - W^k O).
 template <class R, int L>
-__device__ __forceinline__ void zfwd_split(const cpx<R> *Z, const cpx<R> *tw, int h, int nzh, int nzp,
-                                           cpx<R> *out, long long pitch, int nr) {
+__device__ __forceinline__ void zfwd_split(const cpx<R> *Z, const cpx<R> *W, int h, int nzp, cpx<R> *out,
+                                           int nt) {
    using C = cpx<R>;
-   for (int e = threadIdx.x; e < nzp * L; e += blockDim.x) {
+   for (int e = threadIdx.x; e < (h / 2 + 1) * L; e += nt) {
       const int l = e % L, k = e / L;
-      if (l >= nr) continue;
-      if (k >= nzh) {  // row padding
-         out[l * pitch + k] = mk<R>(0, 0);
-         continue;
-      }
-      const C a = Z[(k == h ? 0 : k) * L + l];
+      const C a = Z[k * L + l];
       const C b = cconj(Z[(k == 0 ? 0 : h - k) * L + l]);
       const C E = cscale(cadd(a, b), (R) 0.5);
       const C t = csub(a, b);
-      const C O = mk<R>(t.y * (R) 0.5, -t.x * (R) 0.5);
-      out[l * pitch + k] = cadd(E, cmul(tw[k], O));
+      const C O = cmul(W[k], mk<R>(t.y * (R) 0.5, -t.x * (R) 0.5));
+      C *o = out + l * nzp;
+      o[k] = cadd(E, O);
+      if (2 * k != h) o[h - k] = cconj(csub(E, O));
    }
+   if (nzp > h + 1)
+      for (int l = threadIdx.x; l < L; l += nt) out[l * nzp + h + 1] = mk<R>(0, 0);
+}
+
+// The same for a compile-time length, in place: every thread takes its pairs
+// into registers before any output row (which overlaps the lines) is written.
+template <class R, int L, int H, int NT>
+__device__ __forceinline__ void zfwd_split_n(const cpx<R> *Z, const cpx<R> *W, int nzp, cpx<R> *out) {
+   using C = cpx<R>;
+   constexpr int NE = (H / 2 + 1) * L, U = (NE + NT - 1) / NT;
+   C lo[U], hi[U];
+#pragma unroll
+   for (int u = 0; u < U; u++) {
+      const int e = threadIdx.x + u * NT;
+      if ((int) threadIdx.x < NT && e < NE) {
+         const int l = e % L, k = e / L;
+         const C a = Z[k * L + l];
+         const C b = cconj(Z[(k == 0 ? 0 : H - k) * L + l]);
+         const C E = cscale(cadd(a, b), (R) 0.5);
+         const C t = csub(a, b);
+         const C O = cmul(W[k], mk<R>(t.y * (R) 0.5, -t.x * (R) 0.5));
+         lo[u] = cadd(E, O);
+         hi[u] = cconj(csub(E, O));
+      }
+   }
+   __syncthreads();
+#pragma unroll
+   for (int u = 0; u < U; u++) {
+      const int e = threadIdx.x + u * NT;
+      if ((int) threadIdx.x < NT && e < NE) {
+         const int l = e % L, k = e / L;
+         C *o = out + l * nzp;
+         o[k] = lo[u];
+         if (2 * k != H) o[H - k] = hi[u];
+      }
+   }
+   if (nzp > H + 1)
+      for (int l = threadIdx.x; l < L; l += NT) out[l * nzp + H + 1] = mk<R>(0, 0);
+}
+
+// Real-FFT merge: Z_k of the inverse transform from X_k and X_{h-k} (row of
+// nzp half-spectrum points); the DC and Nyquist bins are real.
+template <class R>
+__device__ __forceinline__ cpx<R> zinv_merge(const cpx<R> *row, const cpx<R> *W, int h, int k) {
+   using C = cpx<R>;
+   C a = row[k], b = row[h - k];
+   if (k == 0) { a.y = 0; b.y = 0; }
+   b = cconj(b);
+   const C E = cadd(a, b);
+   const C O = cmul(csub(a, b), cconj(W[k]));
+   return mk<R>(E.x - O.y, E.y + O.x);
+}
+
+// Lengths with compile-time transforms (RadixPlan in fftn.cuh): runs
+// f(std::integral_constant<int, n>), with 0 for any other length.
+template <class F> __host__ __device__ __forceinline__ auto with_len(int n, F f) {
+   switch (n) {
+   case 24: return f(std::integral_constant<int, 24>());
+   case 32: return f(std::integral_constant<int, 32>());
+   case 48: return f(std::integral_constant<int, 48>());
+   case 64: return f(std::integral_constant<int, 64>());
+   case 96: return f(std::integral_constant<int, 96>());
+   case 128: return f(std::integral_constant<int, 128>());
+   case 256: return f(std::integral_constant<int, 256>());
+   case 512: return f(std::integral_constant<int, 512>());
+   default: return f(std::integral_constant<int, 0>());
+   }
+}
+// kz columns of the y and x tiles these are compiled for, rows of the z tiles
+// and the longest half-length z line.
+__host__ __device__ constexpr int len_cols(bool fp32) { return fp32 ? 8 : 4; }
+template <class R> struct LenCols { static constexpr int L = len_cols(sizeof(R) == 4); };
+constexpr int kLenRows = 8, kLenMaxH = 256;
+__host__ __device__ __forceinline__ bool has_len(int n) {
+   return n == 24 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 256 || n == 512;
+}
+// Threads of a CTA that transforms L lines of N points, and the resident CTAs
+// its kernels are compiled for: 64 registers per FP32 thread, 128 per FP64 one.
+template <class R> __host__ __device__ constexpr int len_threads(int N, int L) {
+   const int t = (N * L / kLenPpt + 31) / 32 * 32;
+   return t < 32 ? 32 : t;
+}
+template <class R> __host__ __device__ constexpr int len_ctas(int N, int L) {
+   const int c = (sizeof(R) == 8 ? 512 : 1024) / len_threads<R>(N, L);
+   return c < 1 ? 1 : c;
 }
 
 // Pass 1: |psi|^2 rows -> half spectrum rows (L rows per CTA).
@@ -91,30 +204,33 @@ __device__ __forceinline__ void zfwd_body(const typename Tr<R, CPLX>::P *__restr
 
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
-   const int nz = d.nz, h = nz / 2, nzh = d.nzh, nzp = d.nzp;
+   const int nz = d.nz, h = nz / 2, nzp = d.nzp;
    // layout: rows [L][LSr] (later the output rows [L][nzp]) | FFT buffer | twiddles
    P *rows = (P *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
    C *buf = (C *) (rows + L * LSr);
    C *tw = buf + h * L;
    const int nr = (int) ((d.nxy - r0) < L ? (d.nxy - r0) : L);
    const uint32_t row_bytes = (uint32_t) (nz * sizeof(P));
+   // the roots do not depend on the previous kernel: their copies start
+   // before it has finished
    if (threadIdx.x == 0) {
       mbar_init(&bar, 1);
       fence_mbar_init();
+      mbar_arrive_expect_tx(&bar, row_bytes * nr + (uint32_t) (ztab_len(h) * sizeof(C)));
+      bulk_load(tw, twz, (uint32_t) (ztab_len(h) * sizeof(C)), &bar);
    }
-   __syncthreads();
+   pdl_wait();
    if (threadIdx.x == 0) {
-      mbar_arrive_expect_tx(&bar, row_bytes * nr + (uint32_t) (nz * sizeof(C)));
-      bulk_load(tw, twz, (uint32_t) (nz * sizeof(C)), &bar);
       for (int r = 0; r < nr; r++) bulk_load(rows + r * LSr, psi + (r0 + r) * nz, row_bytes, &bar);
    }
+   __syncthreads();
    for (int e = threadIdx.x; e < (L - nr) * LSr; e += blockDim.x) rows[nr * LSr + e] = zero_of<P>();
    if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
    zfwd_pack<R, CPLX, L>(rows, LSr, buf, h);
    __syncthreads();
-   fft_lines_ip<L, C, false, PPT>(buf, ph, tw, 2);
+   fft_lines_ip<L, C, false, PPT>(buf, ph, tw);
    C *out = (C *) rows;  // [L][nzp]; the rows are no longer read
-   zfwd_split<R, L>(buf, tw, h, nzh, nzp, out, nzp, L);
+   zfwd_split<R, L>(buf, tw + ztab_roots(h), h, nzp, out, blockDim.x);
    fence_proxy_async();
    __syncthreads();
    if (threadIdx.x == 0) {
@@ -129,7 +245,6 @@ __global__ void __launch_bounds__(256, L >= 16 ? 3 : 4) k_zfwd(const typename Tr
                                               cpx<R> *__restrict__ spec, Dims d, FftPlan ph,
                                               const cpx<R> *__restrict__ twz, int LSr, uint32_t *err) {
    pdl_trigger();
-   pdl_wait();
    zfwd_body<R, CPLX, PPT, L>(psi, spec, d, ph, twz, LSr, err, (long long) blockIdx.x * L);
 }
 
@@ -148,18 +263,21 @@ __device__ __forceinline__ void yfft_body(const CUtensorMap *tm, const Dims &d, 
    const int ny = d.ny, rows = boxn * nbox;
    C *buf = (C *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
    C *tw = buf + rows * L;
+   // the roots do not depend on the previous kernel: their copies start
+   // before it has finished
    if (threadIdx.x == 0) {
       mbar_init(&bar, 1);
       fence_mbar_init();
-   }
-   __syncthreads();
-   if (threadIdx.x == 0) {
       mbar_arrive_expect_tx(&bar, (uint32_t) (rows * L * sizeof(C) + ny * sizeof(C)));
       bulk_load(tw, twy, (uint32_t) (ny * sizeof(C)), &bar);
+   }
+   pdl_wait();
+   if (threadIdx.x == 0) {
       for (int b = 0; b < nbox; b++) tma_load_3d(buf + b * boxn * L, tm, 2 * k0, b * boxn, x, &bar);
    }
+   __syncthreads();
    if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
-   fft_lines_ip<L, C, INV, PPT>(buf, py, tw, 1);
+   fft_lines_ip<L, C, INV, PPT>(buf, py, tw);
    fence_proxy_async();
    __syncthreads();
    if (threadIdx.x == 0) {
@@ -173,18 +291,29 @@ template <class R, bool INV, int L>
 __global__ void __launch_bounds__(256, 4) k_yfft(const __grid_constant__ CUtensorMap tm, Dims d, FftPlan py,
                                                  const cpx<R> *__restrict__ twy, int boxn, int nbox, uint32_t *err) {
    pdl_trigger();
-   pdl_wait();
    const int nkb = (d.nzh + L - 1) / L;
    const int x = blockIdx.x / nkb, k0 = (blockIdx.x - x * nkb) * L;
    yfft_body<R, INV, L>(&tm, d, py, twy, boxn, nbox, err, x, k0);
+}
+
+// Udd's columns of an x tile by asynchronous 8-byte copies of every thread
+// (batched passes: a second tensor map in global memory costs each CTA an
+// acquire, x pass of 64 grids 167 us this way and 203 us by TMA; one solve, its
+// map a kernel parameter, gained by TMA, 78 -> 68 us at 256^3 FP64).
+__device__ __forceinline__ void udd_copy(double *ud, const double *udd, const Dims &d, int nx, int L, int ay, int k0) {
+   const int nyh = d.ny / 2 + 1, nzu = (d.nzh + 1) & ~1;
+   for (int e = threadIdx.x; e < (nx / 2 + 1) * L; e += blockDim.x) {
+      const int ax = e / L, k = k0 + e % L;
+      cp_async8(ud + e, udd + ((long long) ax * nyh + ay) * nzu + (k < d.nzh ? k : d.nzh - 1));
+   }
 }
 
 // Pass 3: FFT along x, multiply by Udd(k) * scale^2, inverse FFT along x, for
 // L kz columns of one y plane.  Udd octant layout [|kx|][|ky|][kz].  CTA size
 // as for the y passes.
 template <class R, int L>
-__device__ __forceinline__ void xconv_body(const CUtensorMap *tm, const Dims &d, const FftPlan &px,
-                                           const cpx<R> *__restrict__ twx, const double *__restrict__ udd,
+__device__ __forceinline__ void xconv_body(const CUtensorMap *tm, const CUtensorMap *tm_udd, const double *udd, const Dims &d,
+                                           const FftPlan &px, const FftPlan &pxi, const cpx<R> *__restrict__ twx,
                                            const State *__restrict__ st, int boxn, int nbox, uint32_t *err, int y,
                                            int k0) {
    using C = cpx<R>;
@@ -192,35 +321,31 @@ __device__ __forceinline__ void xconv_body(const CUtensorMap *tm, const Dims &d,
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
    const int nx = d.nx, ny = d.ny, rows = boxn * nbox;
+   const UddBox ub = udd_box(nx, L);
    C *buf = (C *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
-   C *tw = buf + rows * L;
-   double *ud = (double *) (tw + nx);  // Udd of this y plane and these columns, [|kx|][L]
-   const int nxh = nx / 2 + 1, nyh = ny / 2 + 1, nzh = d.nzh;
+   double *ud = (double *) ((unsigned char *) buf + fft_tile_bytes<R>(rows, L));  // [|kx|][L]
+   C *tw = (C *) ((unsigned char *) ud + ub.bytes);
+   const int ntw = conv_roots(px);  // stage roots, forward then inverse
    const int ay = (y <= ny / 2) ? y : ny - y;
+   // the roots and Udd do not depend on the previous kernel: their copies start
+   // before it has finished
    if (threadIdx.x == 0) {
       mbar_init(&bar, 1);
       fence_mbar_init();
+      mbar_arrive_expect_tx(&bar, (uint32_t) ((rows * L + ntw) * sizeof(C)) + (tm_udd ? (uint32_t) (ub.nb * ub.rows * L * 8) : 0u));
+      bulk_load(tw, twx, (uint32_t) (ntw * sizeof(C)), &bar);
+      if (tm_udd)
+         for (int b = 0; b < ub.nb; b++) tma_load_3d(ud + b * ub.rows * L, tm_udd, k0, ay, b * ub.rows, &bar);
    }
-   __syncthreads();
+   if (!tm_udd) udd_copy(ud, udd, d, nx, L, ay, k0);
+   pdl_wait();
    if (threadIdx.x == 0) {
-      mbar_arrive_expect_tx(&bar, (uint32_t) (rows * L * sizeof(C) + nx * sizeof(C)));
-      bulk_load(tw, twx, (uint32_t) (nx * sizeof(C)), &bar);
       for (int b = 0; b < nbox; b++) tma_load_3d(buf + b * boxn * L, tm, 2 * k0, y, b * boxn, &bar);
    }
-   // the Udd factors of the tile travel while the tile and the forward FFT do
-   // (loaded after the FFT, their latency measured exposed)
-   for (int e = threadIdx.x; e < nxh * L; e += blockDim.x) {
-      const int ax = e / L, c = e - ax * L;
-      const int k = k0 + c < nzh ? k0 + c : nzh - 1;
-      cp_async8(ud + e, udd + ((long long) ax * nyh + ay) * nzh + k);
-   }
-   if (__syncthreads_or(!mbar_wait(&bar, 0, err))) {
-      cp_async_wait_all();
-      return;
-   }
-   fft_lines_ip<L, C, false, PPT>(buf, px, tw, 1);
-   cp_async_wait_all();
    __syncthreads();
+   if (!tm_udd) cp_async_wait_all();
+   if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
+   fft_lines_ip<L, C, false, PPT>(buf, px, tw);
    C *res = buf;
    const double s2 = st->scale2;
    for (int e = threadIdx.x; e < nx * L; e += blockDim.x) {
@@ -230,7 +355,7 @@ __device__ __forceinline__ void xconv_body(const CUtensorMap *tm, const Dims &d,
       res[e] = cscale(res[e], u);
    }
    __syncthreads();
-   fft_lines_ip<L, C, true, PPT>(buf, px, tw, 1);
+   fft_lines_ip<L, C, true, PPT, true>(buf, pxi, ntw > nx ? tw + nx : tw);
    fence_proxy_async();
    __syncthreads();
    if (threadIdx.x == 0) {
@@ -241,18 +366,63 @@ __device__ __forceinline__ void xconv_body(const CUtensorMap *tm, const Dims &d,
 }
 
 template <class R, int L>
-__global__ void __launch_bounds__(256, 4) k_xconv(const __grid_constant__ CUtensorMap tm, Dims d, FftPlan px,
-                                                  const cpx<R> *__restrict__ twx, const double *__restrict__ udd,
+__global__ void __launch_bounds__(256, 4) k_xconv(const __grid_constant__ CUtensorMap tm,
+                                                  const __grid_constant__ CUtensorMap tm_udd, Dims d, FftPlan px, FftPlan pxi,
+                                                  const cpx<R> *__restrict__ twx,
                                                   const State *__restrict__ st, int boxn, int nbox, uint32_t *err) {
    pdl_trigger();
-   pdl_wait();
    const int nkb = (d.nzh + L - 1) / L;
    const int y = blockIdx.x / nkb, k0 = (blockIdx.x - y * nkb) * L;
-   xconv_body<R, L>(&tm, d, px, twx, udd, st, boxn, nbox, err, y, k0);
+   xconv_body<R, L>(&tm, &tm_udd, nullptr, d, px, pxi, twx, st, boxn, nbox, err, y, k0);
+}
+
+// Ends the inverse z pass: stores the phi rows out[l LSo + k], l < nr, with
+// the boundary planes (calcpsidd2_kernel2a/2b with last = 1,
+// imag3d-mpicuda.cu:1591-1625): z = nz-1 <- z = 0, x = nx-1 <- x = 0 and
+// y = ny-1 <- y = 0, each excluding the other two last indices.  z is fixed
+// inside the row.  With FOLD the first nz-1 points of a row (0, y) or (x, 0)
+// go to the matching boundary row too and that row's own CTA stores only its
+// last point; without, a pass of its own copies the planes (k_phifix).  One
+// thread per row; a copied row's points beyond the last 16-byte multiple of
+// nz-1 are stored one by one.  Folding the planes saves a launch of 6 us per
+// step.
+template <class R, bool FOLD>
+__device__ __forceinline__ void zinv_finish(R *__restrict__ phi, R *out, int LSo, const Dims &d, long long r0, int nr) {
+   const int nz = d.nz;
+   long long x = 0, y = 0;
+   if (threadIdx.x < nr) {
+      const long long row = r0 + threadIdx.x;
+      x = row / d.ny, y = row - x * d.ny;
+      if (x < d.nx - 1 && y < d.ny - 1) out[threadIdx.x * LSo + nz - 1] = out[threadIdx.x * LSo];
+   }
+   fence_proxy_async();
+   __syncthreads();
+   if (threadIdx.x < nr) {
+      const R *o = out + threadIdx.x * LSo;
+      R *own = phi + (r0 + threadIdx.x) * nz;
+      const bool bx = x == d.nx - 1 && y < d.ny - 1, by = y == d.ny - 1 && x < d.nx - 1;
+      if (FOLD && (bx || by)) {
+         own[nz - 1] = o[nz - 1];
+      } else {
+         bulk_store(own, o, (uint32_t) (nz * sizeof(R)));
+      }
+      if (FOLD) {
+         constexpr int V = 16 / (int) sizeof(R);
+         const int nb = (nz - 1) / V * V;  // nz is a multiple of V
+         for (int q = 0; q < 2; q++) {
+            if (q == 0 ? !(x == 0 && y < d.ny - 1) : !(y == 0 && x < d.nx - 1)) continue;
+            R *to = phi + (q == 0 ? (long long) (d.nx - 1) * d.ny + y : x * d.ny + d.ny - 1) * nz;
+            if (nb > 0) bulk_store(to, o, (uint32_t) (nb * sizeof(R)));
+            for (int k = nb; k < nz - 1; k++) to[k] = o[k];
+         }
+      }
+      bulk_commit();
+      bulk_wait_all();
+   }
 }
 
 // Pass 5: half spectrum rows -> phi rows (unnormalised inverse, Hermitian).
-template <class R, int PPT, int L>
+template <class R, int PPT, int L, bool FOLD>
 __device__ __forceinline__ void zinv_body(const cpx<R> *__restrict__ spec, R *__restrict__ phi, const Dims &d,
                                           const FftPlan &ph, const cpx<R> *__restrict__ twz, int LSo, uint32_t *err,
                                           long long r0) {
@@ -267,30 +437,27 @@ __device__ __forceinline__ void zinv_body(const cpx<R> *__restrict__ spec, R *__
    C *buf = in + ((in_elems + 7) & ~7);
    C *tw = buf + h * L;
    const int nr = (int) ((d.nxy - r0) < L ? (d.nxy - r0) : L);
+   // the roots do not depend on the previous kernel: their copies start
+   // before it has finished
    if (threadIdx.x == 0) {
       mbar_init(&bar, 1);
       fence_mbar_init();
+      mbar_arrive_expect_tx(&bar, (uint32_t) ((nr * nzp + ztab_len(h)) * sizeof(C)));
+      bulk_load(tw, twz, (uint32_t) (ztab_len(h) * sizeof(C)), &bar);
    }
-   __syncthreads();
+   pdl_wait();
    if (threadIdx.x == 0) {
-      mbar_arrive_expect_tx(&bar, (uint32_t) (nr * nzp * sizeof(C) + nz * sizeof(C)));
-      bulk_load(tw, twz, (uint32_t) (nz * sizeof(C)), &bar);
       bulk_load(in, spec + r0 * nzp, (uint32_t) (nr * nzp * sizeof(C)), &bar);
    }
+   __syncthreads();
    for (int e = threadIdx.x; e < (L - nr) * nzp; e += blockDim.x) in[nr * nzp + e] = mk<R>(0, 0);
    if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
    for (int e = threadIdx.x; e < h * L; e += blockDim.x) {
       const int l = e % L, k = e / L;
-      C a = in[l * nzp + k];
-      C b = in[l * nzp + h - k];
-      if (k == 0) { a.y = 0; b.y = 0; }  // DC and Nyquist bins are real
-      b = cconj(b);
-      const C E = cadd(a, b);
-      const C O = cmul(csub(a, b), cconj(tw[k]));
-      buf[e] = mk<R>(E.x - O.y, E.y + O.x);
+      buf[e] = zinv_merge<R>(in + l * nzp, tw + ztab_roots(h), h, k);
    }
    __syncthreads();
-   fft_lines_ip<L, C, true, PPT>(buf, ph, tw, 2);
+   fft_lines_ip<L, C, true, PPT>(buf, ph, tw);
    const C *z = buf;
    R *out = (R *) in;  // [L][LSo]
    for (int e = threadIdx.x; e < h * L; e += blockDim.x) {
@@ -300,34 +467,250 @@ __device__ __forceinline__ void zinv_body(const cpx<R> *__restrict__ spec, R *__
       out[l * LSo + 2 * m + 1] = v.y;
    }
    __syncthreads();
-   // boundary plane z = nz-1 <- z = 0 for x < nx-1, y < ny-1, inside the row
-   // (the z part of calcpsidd2_kernel2b, imag3d-mpicuda.cu:1605-1625)
-   if (threadIdx.x < nr) {
-      const long long row = r0 + threadIdx.x;
-      const long long x = row / d.ny, y = row - x * d.ny;
-      if (x < d.nx - 1 && y < d.ny - 1) out[threadIdx.x * LSo + nz - 1] = out[threadIdx.x * LSo];
-   }
-   fence_proxy_async();
-   __syncthreads();
-   if (threadIdx.x == 0) {
-      for (int r = 0; r < nr; r++) bulk_store(phi + (r0 + r) * nz, out + r * LSo, (uint32_t) (nz * sizeof(R)));
-      bulk_commit();
-      bulk_wait_all();
-   }
+   zinv_finish<R, FOLD>(phi, out, LSo, d, r0, nr);
 }
 
 template <class R, int PPT, int L>
 __global__ void __launch_bounds__(256, L >= 16 ? 3 : 4) k_zinv(const cpx<R> *__restrict__ spec, R *__restrict__ phi, Dims d,
                                                  FftPlan ph, const cpx<R> *__restrict__ twz, int LSo, uint32_t *err) {
    pdl_trigger();
-   pdl_wait();
-   zinv_body<R, PPT, L>(spec, phi, d, ph, twz, LSo, err, (long long) blockIdx.x * L);
+   zinv_body<R, PPT, L, true>(spec, phi, d, ph, twz, LSo, err, (long long) blockIdx.x * L);
 }
 
-// Boundary planes of phi at one rank (calcpsidd2_kernel2a/2b with last = 1,
-// imag3d-mpicuda.cu:1591-1625): x = nx-1 <- x = 0 and y = ny-1 <- y = 0 here,
-// each excluding the other two last indices; z = nz-1 <- z = 0 is done inside
-// the rows by k_zinv.  The read and write sets are disjoint, so both copies
+// ---------------------------------------------------------------------------
+// The passes on lines of a compile-time length (fftn.cuh): one CTA of
+// len_threads(N, L) threads per tile (the batched kernels may launch more),
+// the roots from the stage-ordered tables (make_roots in solver.cu).  The z
+// passes take the first stage's points straight from the staged rows (|psi|^2
+// or the merged half spectrum) and the inverse one ends in the phi rows.
+// 256^3 on B200, before (run-time lengths) and after: see each kernel.
+
+// Bytes of the shared region of a z pass (psi or half-spectrum rows, lines,
+// output rows).
+template <class R, bool CPLX> __host__ __device__ constexpr int zfwd_region(int H, int L) {
+   constexpr int sp = (int) sizeof(R) * (CPLX ? 2 : 1), sc = 2 * (int) sizeof(R);
+   const int rows = L * (2 * H + 16 / sp) * sp, lines = L * (sizeof(R) == 4 ? (H + 2) & ~1 : H + 1) * sc;
+   return ((rows > lines ? rows : lines) + 127) & ~127;
+}
+template <class R> __host__ __device__ constexpr int zinv_region(int H, int L) {
+   constexpr int sc = 2 * (int) sizeof(R);
+   const int rows = L * (2 * H + 16 / (int) sizeof(R)) * (int) sizeof(R),
+             lines = L * (sizeof(R) == 4 ? (H + 2) & ~1 : H + 1) * sc;
+   return ((rows > lines ? rows : lines) + 127) & ~127;
+}
+
+// z forward: H = nz / 2; twz: H stage roots, then W^k, k <= H.
+template <class R, bool CPLX, int L, int H>
+__device__ __forceinline__ void zfwd_body_n(const typename Tr<R, CPLX>::P *__restrict__ psi, cpx<R> *__restrict__ spec,
+                                            const Dims &d, const cpx<R> *__restrict__ twz, uint32_t *err,
+                                            long long r0) {
+   using C = cpx<R>;
+   using P = typename Tr<R, CPLX>::P;
+   constexpr int NT = len_threads<R>(H, L), nz = 2 * H, LSr = nz + 16 / (int) sizeof(P);
+   constexpr int nzp = sizeof(R) == 4 ? (H + 2) & ~1 : H + 1;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   __shared__ __align__(8) uint64_t bar;
+   // one region for the psi rows, the lines being transformed and the output
+   // rows in turn (each is read into registers before the next is written):
+   // 37 instead of 53 KB at nz = 256 complex FP64, six CTAs per SM for four
+   P *rows = (P *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
+   C *buf = (C *) rows;
+   C *tw = (C *) ((unsigned char *) rows + zfwd_region<R, CPLX>(H, L));
+   const int nr = (int) ((d.nxy - r0) < L ? (d.nxy - r0) : L);
+   constexpr uint32_t row_bytes = (uint32_t) (nz * sizeof(P)), tw_bytes = (uint32_t) (ztab_len(H) * sizeof(C));
+   // the roots do not depend on the previous kernel: their copies start
+   // before it has finished
+   if (threadIdx.x == 0) {
+      mbar_init(&bar, 1);
+      fence_mbar_init();
+      mbar_arrive_expect_tx(&bar, row_bytes * nr + tw_bytes);
+      bulk_load(tw, twz, tw_bytes, &bar);
+   }
+   pdl_wait();
+   if (threadIdx.x == 0) {
+      for (int r = 0; r < nr; r++) bulk_load(rows + r * LSr, psi + (r0 + r) * nz, row_bytes, &bar);
+   }
+   __syncthreads();
+   for (int e = threadIdx.x; e < (L - nr) * LSr; e += blockDim.x) rows[nr * LSr + e] = zero_of<P>();
+   if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
+   fft_lines<H, L, NT, C, false>(
+       buf, tw,
+       [&](int l, int m) {
+          P a, b;
+          ld2(rows + l * LSr + 2 * m, a, b);
+          return mk<R>(dens2(a), dens2(b));
+       },
+       [&](int l, int i, C v) { buf[i * L + l] = v; });
+   __syncthreads();
+   C *out = buf;  // [L][nzp]
+   zfwd_split_n<R, L, H, NT>(buf, tw + ztab_roots(H), nzp, out);
+   fence_proxy_async();
+   __syncthreads();
+   if (threadIdx.x == 0) {
+      bulk_store(spec + r0 * nzp, out, (uint32_t) (nr * nzp * sizeof(C)));
+      bulk_commit();
+      bulk_wait_all();
+   }
+}
+
+template <class R, bool CPLX, int L, int H>
+__global__ void __launch_bounds__(len_threads<R>(H, L), len_ctas<R>(H, L))
+k_zfwd_n(const typename Tr<R, CPLX>::P *__restrict__ psi, cpx<R> *__restrict__ spec, Dims d,
+         const cpx<R> *__restrict__ twz, uint32_t *err) {
+   pdl_trigger();
+   zfwd_body_n<R, CPLX, L, H>(psi, spec, d, twz, err, (long long) blockIdx.x * L);
+}
+
+// z inverse; twz as above.
+template <class R, int L, int H, bool FOLD>
+__device__ __forceinline__ void zinv_body_n(const cpx<R> *__restrict__ spec, R *__restrict__ phi, const Dims &d,
+                                            const cpx<R> *__restrict__ twz, uint32_t *err, long long r0) {
+   using C = cpx<R>;
+   constexpr int NT = len_threads<R>(H, L), nz = 2 * H, LSo = nz + 16 / (int) sizeof(R);
+   constexpr int nzp = sizeof(R) == 4 ? (H + 2) & ~1 : H + 1;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   __shared__ __align__(8) uint64_t bar;
+   // one region for the half-spectrum rows, the lines and the phi rows in turn
+   C *in = (C *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
+   C *buf = in;
+   C *tw = (C *) ((unsigned char *) in + zinv_region<R>(H, L));
+   const int nr = (int) ((d.nxy - r0) < L ? (d.nxy - r0) : L);
+   constexpr uint32_t tw_bytes = (uint32_t) (ztab_len(H) * sizeof(C));
+   // the roots do not depend on the previous kernel: their copies start
+   // before it has finished
+   if (threadIdx.x == 0) {
+      mbar_init(&bar, 1);
+      fence_mbar_init();
+      mbar_arrive_expect_tx(&bar, (uint32_t) (nr * nzp * sizeof(C)) + tw_bytes);
+      bulk_load(tw, twz, tw_bytes, &bar);
+   }
+   pdl_wait();
+   if (threadIdx.x == 0) {
+      bulk_load(in, spec + r0 * nzp, (uint32_t) (nr * nzp * sizeof(C)), &bar);
+   }
+   __syncthreads();
+   for (int e = threadIdx.x; e < (L - nr) * nzp; e += blockDim.x) in[nr * nzp + e] = mk<R>(0, 0);
+   if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
+   R *out = (R *) in;  // [L][LSo], written by the last stage
+   fft_lines<H, L, NT, C, true>(
+       buf, tw, [&](int l, int k) { return zinv_merge<R>(in + l * nzp, tw + ztab_roots(H), H, k); },
+       [&](int l, int m, C v) { st2(out + l * LSo + 2 * m, v.x, v.y); });
+   __syncthreads();
+   zinv_finish<R, FOLD>(phi, out, LSo, d, r0, nr);
+}
+
+template <class R, int L, int H>
+__global__ void __launch_bounds__(len_threads<R>(H, L), len_ctas<R>(H, L))
+k_zinv_n(const cpx<R> *__restrict__ spec, R *__restrict__ phi, Dims d, const cpx<R> *__restrict__ twz, uint32_t *err) {
+   pdl_trigger();
+   zinv_body_n<R, L, H, true>(spec, phi, d, twz, err, (long long) blockIdx.x * L);
+}
+
+// y passes, forward and inverse; twy: N stage roots.
+template <class R, bool INV, int L, int N>
+__device__ __forceinline__ void yfft_body_n(const CUtensorMap *tm, const cpx<R> *__restrict__ twy, uint32_t *err, int x,
+                                            int k0) {
+   using C = cpx<R>;
+   constexpr int NT = len_threads<R>(N, L), boxn = N < 256 ? N : 256;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   __shared__ __align__(8) uint64_t bar;
+   C *buf = (C *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
+   C *tw = buf + N * L;
+   // the roots do not depend on the previous kernel: their copies start
+   // before it has finished
+   if (threadIdx.x == 0) {
+      mbar_init(&bar, 1);
+      fence_mbar_init();
+      mbar_arrive_expect_tx(&bar, (uint32_t) (N * L * sizeof(C) + N * sizeof(C)));
+      bulk_load(tw, twy, (uint32_t) (N * sizeof(C)), &bar);
+   }
+   pdl_wait();
+   if (threadIdx.x == 0) {
+      for (int b = 0; b < N; b += boxn) tma_load_3d(buf + b * L, tm, 2 * k0, b, x, &bar);
+   }
+   __syncthreads();
+   if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
+   fft_lines<N, L, NT, C, INV>(
+       buf, tw, [&](int l, int i) { return buf[i * L + l]; }, [&](int l, int i, C v) { buf[i * L + l] = v; });
+   fence_proxy_async();
+   __syncthreads();
+   if (threadIdx.x == 0) {
+      for (int b = 0; b < N; b += boxn) tma_store_3d(tm, 2 * k0, b, x, buf + b * L);
+      bulk_commit();
+      bulk_wait_all();
+   }
+}
+
+template <class R, bool INV, int L, int N>
+__global__ void __launch_bounds__(len_threads<R>(N, L), len_ctas<R>(N, L))
+k_yfft_n(const __grid_constant__ CUtensorMap tm, Dims d, const cpx<R> *__restrict__ twy, uint32_t *err) {
+   pdl_trigger();
+   const int nkb = (d.nzh + L - 1) / L;
+   const int x = blockIdx.x / nkb, k0 = (blockIdx.x - x * nkb) * L;
+   yfft_body_n<R, INV, L, N>(&tm, twy, err, x, k0);
+}
+
+// x convolution; twx: N forward and N inverse stage roots.  The multiply by
+// Udd happens on the last forward stage's registers.
+template <class R, int L, int N>
+__device__ __forceinline__ void xconv_body_n(const CUtensorMap *tm, const CUtensorMap *tm_udd, const double *udd, const Dims &d,
+                                             const cpx<R> *__restrict__ twx, const State *__restrict__ st,
+                                             uint32_t *err, int y, int k0) {
+   using C = cpx<R>;
+   constexpr int NT = len_threads<R>(N, L), boxn = N < 256 ? N : 256;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   __shared__ __align__(8) uint64_t bar;
+   const int ny = d.ny;
+   constexpr UddBox ub = udd_box(N, L);
+   C *buf = (C *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
+   double *ud = (double *) ((unsigned char *) buf + fft_tile_bytes<R>(N, L));  // [|kx|][L]
+   C *tw = (C *) ((unsigned char *) ud + ub.bytes);
+   constexpr int NTW = palin_plan<N>() ? N : 2 * N;  // stage roots
+   const int ay = (y <= ny / 2) ? y : ny - y;
+   // the roots and Udd do not depend on the previous kernel: their copies start
+   // before it has finished
+   if (threadIdx.x == 0) {
+      mbar_init(&bar, 1);
+      fence_mbar_init();
+      mbar_arrive_expect_tx(&bar, (uint32_t) ((N * L + NTW) * sizeof(C)) + (tm_udd ? (uint32_t) (ub.nb * ub.rows * L * 8) : 0u));
+      bulk_load(tw, twx, (uint32_t) (NTW * sizeof(C)), &bar);
+      if (tm_udd)
+         for (int b = 0; b < ub.nb; b++) tma_load_3d(ud + b * ub.rows * L, tm_udd, k0, ay, b * ub.rows, &bar);
+   }
+   if (!tm_udd) udd_copy(ud, udd, d, N, L, ay, k0);
+   pdl_wait();
+   if (threadIdx.x == 0) {
+      for (int b = 0; b < N; b += boxn) tma_load_3d(buf + b * L, tm, 2 * k0, y, b, &bar);
+   }
+   __syncthreads();
+   const double s2 = st->scale2;
+   if (!tm_udd) cp_async_wait_all();
+   if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
+   conv_lines<N, L, NT, C>(buf, tw, palin_plan<N>() ? tw : tw + N, [&](int l, int i) {
+      const int ax = i <= N / 2 ? i : N - i;
+      return (R) (ud[ax * L + l] * s2);
+   });
+   fence_proxy_async();
+   __syncthreads();
+   if (threadIdx.x == 0) {
+      for (int b = 0; b < N; b += boxn) tma_store_3d(tm, 2 * k0, y, b, buf + b * L);
+      bulk_commit();
+      bulk_wait_all();
+   }
+}
+
+template <class R, int L, int N>
+__global__ void __launch_bounds__(len_threads<R>(N, L), len_ctas<R>(N, L))
+k_xconv_n(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_udd, Dims d,
+          const cpx<R> *__restrict__ twx, const State *__restrict__ st, uint32_t *err) {
+   pdl_trigger();
+   const int nkb = (d.nzh + L - 1) / L;
+   const int y = blockIdx.x / nkb, k0 = (blockIdx.x - y * nkb) * L;
+   xconv_body_n<R, L, N>(&tm, &tm_udd, nullptr, d, twx, st, err, y, k0);
+}
+
+// Boundary planes x = nx-1 and y = ny-1 of phi as a pass of their own (batched
+// FP64 steps, whose inverse z pass does not fold them).  The read and write sets are disjoint, so both copies
 // run concurrently.  One CTA per copied row: blocks [0, ny-1) the rows (nx-1,
 // j) <- (0, j), blocks [ny-1, ny-1 + nx-1) the rows (i, ny-1) <- (i, 0), the
 // first nz-1 points of each (the grid has at least one block).
@@ -345,13 +728,6 @@ __device__ __forceinline__ void phifix_body(R *__restrict__ phi, const Dims &d, 
       return;
    }
    for (int k = threadIdx.x; k < d.nz - 1; k += blockDim.x) phi[dst + k] = phi[src + k];
-}
-
-template <class R>
-__global__ void k_phifix(R *__restrict__ phi, Dims d) {
-   pdl_trigger();
-   pdl_wait();
-   phifix_body<R>(phi, d, blockIdx.x);
 }
 
 // Self-test of the bounded waits: one CTA waits on an mbarrier that expects
@@ -424,8 +800,9 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_dens(const typename Tr<
 }
 
 // Sum of n tile partials in an order that depends on n only: 256 strided
-// partial sums, then a tree over them.  Every thread of the CTA calls it; the
-// result is valid in thread 0.  red: 256 doubles.
+// partial sums, a shuffle tree over each 32 of them, then the eight in turn.
+// Every thread of the CTA (whole warps) calls it; the result is valid in
+// thread 0.  red: 8 doubles.
 __device__ __forceinline__ double sum_tiles(const double *__restrict__ part, int n, double *red) {
    constexpr int U = 8;  // loads in flight per lane
    for (int v = threadIdx.x; v < 256; v += blockDim.x) {
@@ -437,14 +814,13 @@ __device__ __forceinline__ double sum_tiles(const double *__restrict__ part, int
 #pragma unroll
          for (int u = 0; u < U; u++) acc += x[u];
       }
-      red[v] = acc;
+      for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (v % 32 == 0) red[v / 32] = acc;
    }
    __syncthreads();
-   for (int h = 128; h; h >>= 1) {
-      for (int v = threadIdx.x; v < h; v += blockDim.x) red[v] += red[v + h];
-      __syncthreads();
-   }
-   return red[0];
+   double s = 0.;
+   for (int q = 0; q < 8; q++) s += red[q];
+   return s;
 }
 
 // The step's norm from S = sum w_x w_y S_z |psi|^2 into the state.
@@ -622,7 +998,7 @@ __device__ __forceinline__ double fd4(double m2, double m1, double p1, double p2
 // roots a point) took 2.5 ms at 256^3 complex FP64.
 constexpr int kMuY = 8, kMuZ = 32, kMuRing = 6;
 template <class R, bool CPLX>
-__global__ void __launch_bounds__(kMuY *kMuZ) k_muen(const typename Tr<R, CPLX>::P *__restrict__ psi,
+__global__ void __launch_bounds__(kMuY *kMuZ, 4) k_muen(const typename Tr<R, CPLX>::P *__restrict__ psi,
                                                      const R *__restrict__ phi, Dims d, Trap trap, double g, double gd,
                                                      double dx, double dy, double dz, double par, int xchunk,
                                                      double *__restrict__ part) {
@@ -634,17 +1010,30 @@ __global__ void __launch_bounds__(kMuY *kMuZ) k_muen(const typename Tr<R, CPLX>:
    const int tz = threadIdx.x % kMuZ, ty = threadIdx.x / kMuZ;
    const int j = y0 + ty, k = z0 + tz;
    const bool in = j < d.ny && k < d.nz;
-   auto plane = [&](int x) {  // |psi| of plane x with the halo, zero outside the grid
-      double *r = ring[(x + kMuRing) % kMuRing];
-      for (int e = threadIdx.x; e < PY * PZ; e += NT) {
+   // plane x with the halo, zero outside the grid: loaded into registers one
+   // plane ahead of the amplitudes' square roots and stores
+   using P = typename Tr<R, CPLX>::P;
+   constexpr int NE = (PY * PZ + NT - 1) / NT;
+   P raw[NE];
+   auto load = [&](int x) {
+#pragma unroll
+      for (int u = 0; u < NE; u++) {
+         const int e = threadIdx.x + u * NT;
          const int jj = y0 - 2 + e / PZ, kk = z0 - 2 + e % PZ;
-         double v = 0.;
-         if (x >= 0 && x < d.nx && jj >= 0 && jj < d.ny && kk >= 0 && kk < d.nz) {
-            const auto p = psi[((long long) x * d.ny + jj) * d.nz + kk];
-            if constexpr (CPLX) v = sqrt((double) dens2(p));
-            else v = (double) p;
+         raw[u] = zero_of<P>();
+         if (e < PY * PZ && x >= 0 && x < d.nx && jj >= 0 && jj < d.ny && kk >= 0 && kk < d.nz)
+            raw[u] = psi[((long long) x * d.ny + jj) * d.nz + kk];
+      }
+   };
+   auto keep = [&](int x) {
+      double *r = ring[(x + kMuRing) % kMuRing];
+#pragma unroll
+      for (int u = 0; u < NE; u++) {
+         const int e = threadIdx.x + u * NT;
+         if (e < PY * PZ) {
+            if constexpr (CPLX) r[e] = sqrt((double) dens2(raw[u]));
+            else r[e] = (double) raw[u];
          }
-         r[e] = v;
       }
    };
    const double invN = 1.0 / (double) d.npts, ipar = 1. / (3. - par);
@@ -653,10 +1042,20 @@ __global__ void __launch_bounds__(kMuY *kMuZ) k_muen(const typename Tr<R, CPLX>:
    const double wyz = in ? simp_w(j, d.ny) * simp_w(k, d.nz) : 0.;
    double mu = 0., en = 0.;
    const int c = (ty + 2) * PZ + tz + 2;
-   for (int x = x0 - 2; x < x0 + 2; x++) plane(x);
+   const long long sx = (long long) d.ny * d.nz;
+   const R *ph = phi + (long long) x0 * sx + (long long) (in ? j : 0) * d.nz + (in ? k : 0);
+   for (int x = x0 - 2; x < x0 + 2; x++) {
+      load(x);
+      keep(x);
+   }
+   load(x0 + 2);
+   R f = *ph;
    for (int x = x0; x < x1; x++) {
-      plane(x + 2);
+      keep(x + 2);
       __syncthreads();  // the slot this fills was last read two iterations ago (six planes, five in use)
+      load(x + 3);
+      const double fx = (double) f;
+      if (x + 1 < x1) f = ph[(x + 1 - x0) * sx];
       if (in) {
          const double *r = ring[x % kMuRing];
          auto rx = [&](int q) { return ring[(x + q + kMuRing) % kMuRing][c]; };
@@ -664,9 +1063,8 @@ __global__ void __launch_bounds__(kMuY *kMuZ) k_muen(const typename Tr<R, CPLX>:
          const double ddy = fd4(r[c - 2 * PZ], r[c - PZ], r[c + PZ], r[c + 2 * PZ], j, d.ny, hy2, hy12);
          const double ddz = fd4(r[c - 2], r[c - 1], r[c + 1], r[c + 2], k, d.nz, hz2, hz12);
          const double dpsi = (ddx * ddx + ddy * ddy + ddz * ddz) * ipar;
-         const long long q = ((long long) x * d.ny + j) * d.nz + k;
-         const double psi2 = (double) dens2(psi[q]);
-         const double lin = psi2 * g + ((double) phi[q] * invN) * gd;
+         const double psi2 = r[c] * r[c];
+         const double lin = psi2 * g + (fx * invN) * gd;
          const double v = trap.v(x, j, k), w = simp_w(x, d.nx) * wyz;
          mu = fma(w, fma(v + lin, psi2, dpsi), mu);
          en = fma(w, fma(v + 0.5 * lin, psi2, dpsi), en);

@@ -592,7 +592,6 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
                                                      const State *__restrict__ st, int tw_arg, int boxn, int nbox,
                                                      uint32_t *err) {
    pdl_trigger();
-   pdl_wait();
    using P = typename Tr<R, CPLX>::P;
    const int TW = TWC > 0 ? TWC : tw_arg;
    extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -634,8 +633,9 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
       for (int q = 0; q < S; q++) mbar_init(&full[q], 1);
       fence_mbar_init();
    }
-   __syncthreads();
+   pdl_wait();  // the tables above do not depend on the previous kernel
    if (threadIdx.x == 0 && (int) blockIdx.x < ntiles) copy_tile(blockIdx.x, 0, true);
+   __syncthreads();
    const double scale = NU ? st->scale : 1.;
    const int lg = __ffs(TW) - 1;  // TW is a power of two
    const int c = threadIdx.x & (TW - 1), p = threadIdx.x >> lg;
@@ -741,7 +741,7 @@ __device__ __forceinline__ void zsweep_tile(typename Tr<R, CPLX>::P *rows, int n
                const P *row = rows + rr * LS;
                sum += (double) dens2(row[n - 2]) - 0.25 * (double) dens2(row[n - 3]);
             }
-            const int i = (int) ((row0 + rr) / d.ny), j = (int) (row0 + rr) - i * d.ny;
+            const int row = (int) row0 + rr, i = row / d.ny, j = row - i * d.ny;
             sum *= o.hz3 * simp_w(i, d.nx) * simp_w(j, d.ny);
          } else {
             sum = 0.;
@@ -781,7 +781,6 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
                                                     int tr_arg, int LS, ZOut out, double hx, double hy,
                                                     State *st, double *out_norm, uint32_t *err) {
    pdl_trigger();
-   pdl_wait();
    const int TR = TWC > 0 ? TWC : tr_arg;
    using P = typename Tr<R, CPLX>::P;
    extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -825,6 +824,7 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
       fence_mbar_init();
    }
    __syncthreads();
+   pdl_wait();  // the tables above do not depend on the previous kernel
    if (threadIdx.x < 32 && (int) blockIdx.x < ntiles) copy_tile(blockIdx.x, 0, true);
    const int c = threadIdx.x % TR, p = threadIdx.x / TR;
    int i = 0;
@@ -843,7 +843,7 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
    if (threadIdx.x < 32) bulk_wait_all();
    if constexpr (MOM == 1) {
       __shared__ bool last;
-      __shared__ double red[256];
+      __shared__ double red[8];
       // the tile partials were written by this warp's lane 0
       if (threadIdx.x == blockDim.x - 32) {
          __threadfence();

@@ -20,9 +20,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t) 
 // Programmatic dependent launch.  pdl_trigger lets the next kernel of the
 // stream be scheduled once every CTA of this grid has started; pdl_wait
 // returns once the previous kernel has completed and its memory is visible.
-// Every step kernel calls both before its first global-memory access, so a
-// kernel launched with the attribute can occupy SMs freed by the tail of its
-// predecessor without reading or writing anything early.
+// Every step kernel calls both before it touches anything another kernel of a
+// step writes or reads; what it does earlier (barriers, copies of constant
+// tables) overlaps its predecessor's tail.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

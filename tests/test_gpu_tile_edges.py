@@ -85,6 +85,20 @@ def test_calcnu_exponent_ranges(gpe_lib, oracle_mod, mode, prec, g):
     o.close()
 
 
+# lengths with compile-time passes (24 ... 512 and half lengths) and without,
+# odd half lengths, partial row tiles, the longest lines
+@pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("n", [(24, 32, 48), (48, 64, 96), (96, 24, 64), (128, 8, 128), (8, 256, 192), (512, 10, 16),
+                               (10, 512, 512), (1024, 8, 20), (8, 1024, 24), (10, 8, 1024), (30, 50, 60), (90, 18, 36)])
+def test_convolution_lengths(gpe_lib, oracle_mod, mode, prec, n):
+    s, o, _ = pair(gpe_lib, oracle_mod, mode, prec, n)
+    s.calcpsidd2()
+    o.calcpsidd2()
+    assert rel(s.get_phi(), o.get_phi()) <= TOL[prec]  # boundary planes included
+    s.close()
+    o.close()
+
+
 @pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
 @pytest.mark.parametrize("n", [(8, 8, 8), (20, 18, 36), (10, 36, 100), (48, 50, 32)])
 def test_observables_at_tile_edges(gpe_lib, oracle_mod, mode, prec, n):
