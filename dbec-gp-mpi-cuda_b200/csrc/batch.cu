@@ -57,6 +57,8 @@ void drop_tables(gpe_batch *b) {
    for (Group &G : b->groups) {
       if (G.dtab) cudaFree(G.dtab);
       if (G.dwork) cudaFree(G.dwork);
+      for (SweepTile *t : G.dtile)
+         if (t) cudaFree(t);
    }
    b->groups.clear();
    b->tables = false;
@@ -76,6 +78,7 @@ void refresh(gpe_batch *b) {
 }
 
 constexpr size_t kSmemCap = 227 * 1024;
+constexpr size_t kSweepStatic = 2048;  // views, tile records and barriers of a sweep kernel, rounded up
 
 // Descriptors of a group (host copy), in member order.
 gpe_status group_descs(gpe_batch *b, const Group &G, std::vector<BatchDesc> &h) {
@@ -133,7 +136,7 @@ gpe_status build_tables(gpe_batch *b) {
             A.mseg[a] = std::max(A.mseg[a], g.mseg[a]);
             A.stage[a] = std::max(A.stage[a], g.stage[a]);
             A.xch[a] = std::max(A.xch[a], g.xch[a]);
-            A.extra[a] = std::max(A.extra[a], g.extra[a]);
+            A.tabs[a] = std::max(A.tabs[a], g.tabs[a]);
          }
          A.part = std::max(A.part, g.part);
       }
@@ -142,9 +145,11 @@ gpe_status build_tables(gpe_batch *b) {
       // sweeps: 2-stage pipelines; as many CTAs per SM as shared memory and
       // the kernels' register budget allow
       for (int a = 0; a < 3; a++) {
-         size_t sm = 128 + 2 * (size_t) A.stage[a] + A.xch[a] + A.extra[a];
+         size_t sm = 128 + 2 * (size_t) A.stage[a] + A.xch[a];
          if (a == 2) sm += 2 * (size_t) A.part;
-         if (sm > kSmemCap) return bfail(GPE_ERR_PARAM, "batch: sweep tiles exceed shared memory");
+         G.nbuf[a] = sm + 2 * (size_t) A.tabs[a] <= kSmemCap - kSweepStatic ? 2 : 1;
+         sm += (size_t) G.nbuf[a] * A.tabs[a];
+         if (sm > kSmemCap - kSweepStatic) return bfail(GPE_ERR_PARAM, "batch: sweep tiles exceed shared memory");
          // the kernels' register budget holds cap0 CTAs of 256 threads,
          // so more of fewer threads
          const int cap0 = kb_sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32));
@@ -153,14 +158,40 @@ gpe_status build_tables(gpe_batch *b) {
          G.sweep_smem[a] = sm;
          G.sweep_grid[a] = (int) std::min<long long>(A.tiles[kPXsweep + a], (long long) ctas * b->nsm);
       }
-      // work lists: every pass's tiles, instance by instance
+      // work lists: every pass's tiles, instance by instance; the sweeps' as
+      // whole records
+      auto sweep = [](int q) { return q >= kPXsweep && q <= kPZsweep; };
       G.off[0] = 0;
-      for (int q = 0; q < kNPass; q++) G.off[q + 1] = G.off[q] + A.tiles[q];
+      for (int q = 0; q < kNPass; q++) G.off[q + 1] = G.off[q] + (sweep(q) ? 0 : A.tiles[q]);
       std::vector<unsigned> work((size_t) G.off[kNPass]);
       for (int q = 0; q < kNPass; q++) {
+         if (sweep(q)) continue;
          size_t e = (size_t) G.off[q];
          for (int k = 0; k < n; k++)
             for (long long t = 0; t < geo[k].tiles[q]; t++) work[e++] = ((unsigned) k << kLocalBits) | (unsigned) t;
+      }
+      std::vector<SweepTile> rec[3];
+      for (int a = 0; a < 3; a++) {
+         rec[a].reserve((size_t) A.tiles[kPXsweep + a]);
+         for (int k = 0; k < n; k++) {
+            const BatchGeom &g = geo[k];
+            for (long long t = 0; t < g.tiles[kPXsweep + a]; t++) {
+               SweepTile r = g.tile[a];
+               r.inst = k;
+               if (a < 2) {
+                  r.a = (int) (t / g.across[a]);
+                  r.b = (int) (t % g.across[a]) * g.tw[a];
+               } else {
+                  r.a = (int) t * g.tw[a];
+                  r.b = (int) std::min<long long>(g.tw[a], g.nxy - r.a);
+                  r.psi = (unsigned char *) r.psi + (size_t) r.a * g.row_bytes;
+               }
+               rec[a].push_back(r);
+            }
+         }
+         BCK(cudaMalloc(&G.dtile[a], sizeof(SweepTile) * rec[a].size()));
+         BCK(cudaMemcpyAsync(G.dtile[a], rec[a].data(), sizeof(SweepTile) * rec[a].size(), cudaMemcpyHostToDevice,
+                             b->master));
       }
       std::vector<BatchDesc> h;
       BCKS(group_descs(b, G, h));

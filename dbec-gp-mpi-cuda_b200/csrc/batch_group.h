@@ -24,9 +24,11 @@ struct Group {
    BatchGeom geo{};           // maxima over the members (tiles: sums)
    long long off[kNPass + 1] = {};  // start of each pass's work list in dwork
    BatchDesc *dtab = nullptr;        // device descriptor table
-   unsigned *dwork = nullptr;        // device work lists (TileRef packed per tile)
+   unsigned *dwork = nullptr;        // device work lists (TileRef packed per tile; the sweeps' are in dtile)
+   SweepTile *dtile[3] = {nullptr, nullptr, nullptr};  // device tile records of the sweeps
    int sweep_grid[3] = {0, 0, 0};
    size_t sweep_smem[3] = {0, 0, 0};
+   int nbuf[3] = {2, 2, 2};  // table buffers of the sweeps (one where two do not fit: long complex lines)
 };
 
 inline gpe_status bfail(gpe_status st, const std::string &m) {

@@ -25,8 +25,9 @@
 
 namespace gpe {
 
-// Everything one sweep tile of one instance needs.
-struct SweepView {
+// Everything one sweep tile of one instance needs, next to its tables (a
+// 16-byte multiple: it travels to shared memory as one bulk copy).
+struct alignas(16) SweepView {
    SegTab tb;
    Trap trap;
    LinPhase lin;
@@ -62,6 +63,41 @@ struct alignas(64) BatchDesc {
    int LSr, LSo, boxy, nboxy, boxx, nboxx, Ly, Lx;
 };
 
+// One tile of a sweep.
+struct alignas(16) SweepTile {
+   int inst;
+   int a, b;          // x / y sweep: plane, first z column; z sweep: first row, rows
+   int geo;           // sweep_geo
+   const void *tabs;  // the instance's coefficient tables (and calcnu's x table)
+   union {
+      const State *st;   // x sweep: the pending renormalisation
+      void *psi;         // z sweep: the tile's first row
+   };
+};
+static_assert(sizeof(SweepTile) == 32, "tile record");
+// Lines of n points, TW per tile; x / y: rows staged, z: row stride in `ext`.
+__host__ __device__ __forceinline__ int sweep_geo(int n, int ext, int TW, int skip) {
+   int lg = 0;
+   while ((1 << lg) < TW) lg++;
+   return n | ext << 11 | lg << 23 | skip << 26;
+}
+struct SweepGeo {
+   int n, ext, TW, skip;
+};
+__device__ __forceinline__ SweepGeo sweep_geo(int g) {
+   return SweepGeo{g & 2047, g >> 11 & 4095, 1 << (g >> 23 & 7), (int) ((unsigned) g >> 26)};
+}
+// Bytes of an instance's table block: gamma | (M, alpha) | N and, for the x
+// sweep, calcnu's table along the line (xe bytes per entry) behind its zero
+// entries.
+__host__ __device__ __forceinline__ uint32_t sweep_tab_bytes(int n, int skip, int esz, int xe) {
+   return (uint32_t) (4 * (n - 2 + skip) * esz + (((n + skip) * xe + 15) & ~15));
+}
+// Bytes of an entry of calcnu's x table (NuXf::T).
+template <class R, bool CPLX> __host__ __device__ constexpr int nu_tab_esz() {
+   return (int) sizeof(R) * (CPLX && sizeof(R) == 8 ? 2 : 1);
+}
+
 // Launch geometry of one instance under the batch's fixed tile choices (z
 // passes: 8-row tiles; y / x passes: Ly / Lx kz columns; sweeps: the
 // instance's own lines per CTA and segments, 2-stage pipelines).
@@ -73,7 +109,11 @@ struct BatchGeom {
    int mseg[3];              // compile-time segment bound of each sweep
    uint32_t stage[3];        // sweeps: bytes of one pipeline stage
    uint32_t xch[3];          // sweeps: bytes of the exchange buffer
-   uint32_t extra[3];        // sweeps: FP64 tables (x: calcnu table; z: coefficient tables)
+   uint32_t tabs[3];         // sweeps: bytes of the table block
+   SweepTile tile[3];        // sweeps: the tiles' geo, tabs and state or psi
+   int across[3], tw[3];     // sweeps: x / y tiles per plane, lines per tile
+   long long nxy;            // z sweep: rows, bytes of a row
+   size_t row_bytes;
    uint32_t part;            // z sweep: bytes of one Simpson partial array
    int Ly, Lx;               // the instance's own FFT tile widths
 };
@@ -220,65 +260,85 @@ static __global__ void __launch_bounds__(256) kb_norm_final(const BatchDesc *__r
 // ------------------------------------------------------------------- sweeps
 // Persistent pipelined CTAs over the tiles of all instances (the pipeline of
 // k_sweep_xy / k_sweep_z): while a CTA sweeps tile t, tile t + gridDim.x
-// (possibly of another instance) is loading.  Every stage has room for the
-// largest tile of the group (stage_bytes); the view of the tile's instance
-// is copied into shared memory when the instance changes from one tile of
-// the CTA to the next, and so are the FP64 tables the single-solve kernels
-// stage once per CTA.
-
-// Words of a view copied by the CTA (every thread calls it).
-__device__ __forceinline__ void copy_view(SweepView &dst, const SweepView &src) {
-   constexpr int W = (int) (sizeof(SweepView) / sizeof(int));
-   static_assert(sizeof(SweepView) % sizeof(int) == 0, "view size");
-   for (int e = threadIdx.x; e < W; e += blockDim.x) ((int *) &dst)[e] = ((const int *) &src)[e];
-}
+// (usually of another instance) is loading.  Every stage has room for the
+// largest tile of the group (stage_bytes).  Nothing a tile needs is fetched
+// when it is due: its record comes three tiles ahead into a ring, and where the
+// instance changes its view and tables come with the tile, as bulk copies on
+// the same mbarrier, into the other of two buffers (looked up in global
+// memory by every tile, the records, views and tables cost a chain of L2
+// latencies per tile that every warp waited for at the next barrier: 64
+// mixed-precision grids, x / y / z sweep 286 / 155 / 154 us).
+template <class R, bool CPLX> struct BatchTabs {
+   using P = typename Tr<R, CPLX>::P;
+   // the view's tables in shared memory: gamma | (M, alpha) | N | calcnu's x table
+   __device__ __forceinline__ static SegTab at(const SegTab &tb, unsigned char *tabs) {
+      SegTab o = tb;
+      const int ne = tb.P * tb.m;
+      o.ga = tabs;
+      o.ma = (P *) tabs + ne;
+      o.nn = (P *) tabs + 3 * ne;
+      return o;
+   }
+   __device__ __forceinline__ static const void *xt(const SegTab &tb, unsigned char *tabs) {
+      return (P *) tabs + 4 * tb.P * tb.m;
+   }
+};
 
 template <class R, bool CPLX, int AXIS, bool NU, int MSEG, int S>
-__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_xy(const BatchDesc *__restrict__ tab,
-                                                                           const unsigned *__restrict__ work,
-                                                                           int ntiles, uint32_t stage_bytes,
-                                                                           uint32_t xch_bytes) {
+__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_xy(
+    const BatchDesc *__restrict__ tab, const SweepTile *__restrict__ tiles, int ntiles, uint32_t stage_bytes,
+    uint32_t xch_bytes, uint32_t tab_bytes, int nbuf) {
    using P = typename Tr<R, CPLX>::P;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t full[S];
-   __shared__ __align__(16) SweepView sv;
+   __shared__ SweepView views[2];
+   __shared__ SweepTile ring[8];
+   __shared__ __align__(16) State states[2];
+   static_assert(sizeof(State) % 16 == 0, "state size");
    constexpr int E = CPLX ? 2 : 1;
-   // layout: S stages | exchange buffer | FP64 calcnu table
+   // layout: S stages | exchange buffer | nbuf table buffers
    unsigned char *base = (unsigned char *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
    P *xch = (P *) (base + S * stage_bytes);
-   double *xtab = (double *) ((unsigned char *) xch + xch_bytes);
-   // tile t of the work list: its instance and its place in that instance
+   unsigned char *tabs = (unsigned char *) xch + xch_bytes;
+   const int g = gridDim.x;
    int acq = -1;  // thread 0: the instance whose tensor maps it last acquired
-   auto copy_tile = [&](int t, int q, bool load) {
-      const TileRef r = tile_ref(work, t);
-      const BatchDesc &D = tab[r.inst];
-      const SweepView &v = D.sv[AXIS];
-      const int TW = v.TW, rows = v.boxn * v.nbox, nzb = (v.d.nz + TW - 1) / TW;
-      const int other = r.local / nzb, z0 = (r.local - other * nzb) * TW;
-      const XyStage lay = xy_stage<R, CPLX, NU>(rows, TW, v.tb.skip);
+   // thread 0: the view and tables of tile T into buffer vb; their bytes are
+   // expected with the tile's
+   auto copy_tabs = [&](const SweepTile &T, int q, int vb) {
+      const SweepGeo o = sweep_geo(T.geo);
+      bulk_load(&views[vb], &tab[T.inst].sv[AXIS], (uint32_t) sizeof(SweepView), &full[q]);
+      bulk_load(tabs + vb * tab_bytes, T.tabs,
+                sweep_tab_bytes(o.n, o.skip, (int) sizeof(P), NU ? nu_tab_esz<R, CPLX>() : 0), &full[q]);
+      if (NU) bulk_load(&states[vb], T.st, (uint32_t) sizeof(State), &full[q]);
+   };
+   // thread 0: copies of tile T in stage q; expects view and tables too if `with`
+   auto copy_tile = [&](const SweepTile &T, int q, bool load, bool with) {
+      const SweepGeo o = sweep_geo(T.geo);
+      const BatchDesc &D = tab[T.inst];
+      const int TW = o.TW, rows = o.ext, boxn = rows <= 256 ? rows : 256;
+      const XyStage lay = xy_stage<R, CPLX, NU>(rows, TW, o.skip);
       P *tile = (P *) (base + q * stage_bytes + lay.psi);
       R *ptile = (R *) (base + q * stage_bytes + lay.phi);
       const CUtensorMap *tm_psi = &D.tm_psi[AXIS];
-      if (r.inst != acq) {
+      if (T.inst != acq) {
          tmap_acquire(tm_psi);
          if (NU) tmap_acquire(&D.tm_phi);
-         acq = r.inst;
+         acq = T.inst;
       }
       if (load) {
-         mbar_arrive_expect_tx(&full[q], (uint32_t) (rows * TW * sizeof(P)) + (NU ? (uint32_t) (rows * TW * sizeof(R)) : 0u));
+         uint32_t tx = (uint32_t) (rows * TW * sizeof(P)) + (NU ? (uint32_t) (rows * TW * sizeof(R)) : 0u);
+         const uint32_t tb = sweep_tab_bytes(o.n, o.skip, (int) sizeof(P), NU ? nu_tab_esz<R, CPLX>() : 0);
+         if (with) tx += (uint32_t) sizeof(SweepView) + tb + (NU ? (uint32_t) sizeof(State) : 0u);
+         mbar_arrive_expect_tx(&full[q], tx);
       }
-      for (int b = 0; b < v.nbox; b++) {
-         const int a0 = b * v.boxn;
+      for (int a0 = 0; a0 < rows; a0 += boxn) {
          if (load) {
-            if (AXIS == 0) tma_load_3d(tile + a0 * TW, tm_psi, E * z0, other, a0, &full[q]);
-            else tma_load_3d(tile + a0 * TW, tm_psi, E * z0, a0, other, &full[q]);
-            if (NU) {
-               if (AXIS == 0) tma_load_3d(ptile + a0 * TW, &D.tm_phi, z0, other, a0, &full[q]);
-               else tma_load_3d(ptile + a0 * TW, &D.tm_phi, z0, a0, other, &full[q]);
-            }
+            if (AXIS == 0) tma_load_3d(tile + a0 * TW, tm_psi, E * T.b, T.a, a0, &full[q]);
+            else tma_load_3d(tile + a0 * TW, tm_psi, E * T.b, a0, T.a, &full[q]);
+            if (NU) tma_load_3d(ptile + a0 * TW, &D.tm_phi, T.b, T.a, a0, &full[q]);
          } else {
-            if (AXIS == 0) tma_store_3d(tm_psi, E * z0, other, a0, tile + a0 * TW);
-            else tma_store_3d(tm_psi, E * z0, a0, other, tile + a0 * TW);
+            if (AXIS == 0) tma_store_3d(tm_psi, E * T.b, T.a, a0, tile + a0 * TW);
+            else tma_store_3d(tm_psi, E * T.b, a0, T.a, tile + a0 * TW);
          }
       }
       if (!load) bulk_commit();
@@ -286,128 +346,163 @@ __global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)
    if (threadIdx.x == 0) {
       for (int q = 0; q < S; q++) mbar_init(&full[q], 1);
       fence_mbar_init();
+      if ((int) blockIdx.x < ntiles) ring[0] = tiles[blockIdx.x];
+      for (int k = 1; k < 3; k++)
+         if ((int) blockIdx.x + k * g < ntiles) ring[k] = tiles[blockIdx.x + k * g];
+      if ((int) blockIdx.x < ntiles) {
+         copy_tile(ring[0], 0, true, true);
+         copy_tabs(ring[0], 0, 0);
+      }
    }
    __syncthreads();
-   if (threadIdx.x == 0 && (int) blockIdx.x < ntiles) copy_tile(blockIdx.x, 0, true);
-   int cur = -1;  // instance whose view is in sv
-   int it = 0;
-   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, it++) {
+   int vb = 0, it = 0;
+   for (int t = blockIdx.x; t < ntiles; t += g, it++) {
       const int q = it % S;
-      if (threadIdx.x == 0 && t + (int) gridDim.x < ntiles) {
+      const SweepTile &T = ring[it & 7], &N = ring[(it + 1) & 7];
+      const bool change = t + g < ntiles && N.inst != T.inst;
+      const int vn = change && nbuf == 2 ? vb ^ 1 : vb;
+      if (threadIdx.x == 0 && t + g < ntiles) {
          wait_stage_free<S>();
-         copy_tile(t + gridDim.x, (it + 1) % S, true);
+         copy_tile(N, (it + 1) % S, true, change);
+         if (change && nbuf == 2) copy_tabs(N, (it + 1) % S, vn);
       }
-      // the view and table of this tile's instance (the barrier after the
-      // copy wait publishes them)
-      const TileRef r = tile_ref(work, t);
-      const int i = r.inst;
-      if (i != cur) {
-         // every thread has finished with the previous view and table
-         __syncthreads();
-         const BatchDesc &D = tab[i];
-         copy_view(sv, D.sv[AXIS]);
-         if constexpr (NU && AXIS == 0 && std::is_same<R, double>::value) {
-            const SweepView &v = D.sv[AXIS];
-            stage_xtab<CPLX>(xtab, v.lin.ex, v.tb.n, v.tb.skip);
+      if (threadIdx.x == blockDim.x - 1) {
+         // the record asked for one tile ago is complete before the barrier
+         // below; the next one replaces a record no thread reads any more
+         cp_async_wait_all();
+         if (t + 3 * g < ntiles) {
+            unsigned char *to = (unsigned char *) &ring[(it + 3) & 7];
+            const unsigned char *from = (const unsigned char *) (tiles + t + 3 * g);
+            cp_async16(to, from);
+            cp_async16(to + 16, from + 16);
          }
-         cur = i;
       }
-      if (__syncthreads_or(!mbar_wait(&full[q], (it / S) & 1, tab[i].err))) break;
-      const int TW = sv.TW, rows = sv.boxn * sv.nbox, nzb = (sv.d.nz + TW - 1) / TW;
-      const int lg = __ffs(TW) - 1;
-      const int c = threadIdx.x & (TW - 1), p = threadIdx.x >> lg;
-      const XyStage lay = xy_stage<R, CPLX, NU>(rows, TW, sv.tb.skip);
+      const bool late = !mbar_wait(&full[q], (it / S) & 1, nullptr);
+      if (late) atomicOr(tab[T.inst].err, kErrTmaTimeout);
+      if (__syncthreads_or(late)) break;
+      const SweepView &sv = views[vb];
+      const SweepGeo o = sweep_geo(T.geo);
+      const int TW = o.TW, c = threadIdx.x & (TW - 1), p = threadIdx.x / TW;
+      const XyStage lay = xy_stage<R, CPLX, NU>(o.ext, TW, o.skip);
       P *col = (P *) (base + q * stage_bytes + lay.psi) + c;
+      const SegTab tbs = BatchTabs<R, CPLX>::at(sv.tb, tabs + vb * tab_bytes);
       if constexpr (NU) {
          static_assert(AXIS == 0, "calcnu is fused into the x sweep only");
-         const int other = r.local / nzb, z0 = (r.local - other * nzb) * TW;
-         seg_sweep_any<R, CPLX, MSEG, false, false, 0>(
-             col, TW, p, sv.tb, xch + c, TW,
-             nu_xf<R, CPLX>((R *) (base + q * stage_bytes + lay.phi) + c, TW, other, z0, c, sv.d, sv.trap, sv.lin,
-                            xtab + E * sv.tb.skip, sv.g, sv.gd, sv.dt, sv.st->scale));
+         seg_sweep_any<R, CPLX, MSEG, false, true, 0>(
+             col, TW, p, tbs, xch + c, TW,
+             nu_xf<R, CPLX, true>((R *) (base + q * stage_bytes + lay.phi) + c, TW, T.a, T.b, c, sv.d, sv.trap, sv.lin,
+                                  BatchTabs<R, CPLX>::xt(sv.tb, tabs + vb * tab_bytes), sv.tb.skip, sv.g, sv.gd, sv.dt,
+                                  states[vb].scale));
       } else {
-         seg_sweep_any<R, CPLX, MSEG, false, false, 0>(col, TW, p, sv.tb, xch + c, TW, NoXf());
+         seg_sweep_any<R, CPLX, MSEG, false, true, 0>(col, TW, p, tbs, xch + c, TW, NoXf());
       }
       fence_proxy_async();
       __syncthreads();
-      if (threadIdx.x == 0) copy_tile(t, q, false);
+      if (threadIdx.x == 0) {
+         copy_tile(T, q, false, false);
+         if (change && nbuf == 1) copy_tabs(N, (it + 1) % S, 0);
+      }
+      vb = vn;
    }
    if (threadIdx.x == 0) bulk_wait_all();
 }
 
 template <class R, bool CPLX, int MOM, int MSEG, int S>
-__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_z(const BatchDesc *__restrict__ tab,
-                                                                 const unsigned *__restrict__ work, int ntiles,
-                                                                 uint32_t stage_bytes, uint32_t xch_bytes,
-                                                                 uint32_t part_bytes) {
+__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_z(
+    const BatchDesc *__restrict__ tab, const SweepTile *__restrict__ tiles, int ntiles, uint32_t stage_bytes,
+    uint32_t xch_bytes, uint32_t tab_bytes, int nbuf, uint32_t part_bytes) {
    using P = typename Tr<R, CPLX>::P;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t full[S];
-   __shared__ __align__(16) SweepView sv;
-   // layout: S stages of rows | exchange buffer | Simpson partials (2 arrays) | FP64 tables
+   __shared__ SweepView views[2];
+   __shared__ SweepTile ring[8];
+   // layout: S stages of rows | exchange buffer | Simpson partials (2 arrays) | nbuf table buffers
    unsigned char *base = (unsigned char *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
    P *xch = (P *) (base + S * stage_bytes);
    double *part = (double *) ((unsigned char *) xch + xch_bytes);
    double *part2 = (double *) ((unsigned char *) part + part_bytes);
-   double *tabs = (double *) ((unsigned char *) part2 + part_bytes);
-   // FP64: the coefficient tables staged in shared memory, as k_sweep_z does
-   constexpr bool STAB = std::is_same<R, double>::value;
+   unsigned char *tabs = (unsigned char *) part2 + part_bytes;
+   const int g = gridDim.x;
    // one bulk copy per row, issued by the 32 lanes of warp 0 (the short rows
    // of small grids make many small copies); every lane commits and waits
    // for its own store groups
    const int lane = threadIdx.x & 31;
-   auto copy_tile = [&](int t, int q, bool load) {
-      const TileRef r = tile_ref(work, t);
-      const SweepView &v = tab[r.inst].sv[2];
-      const int TR = v.TW, nz = v.d.nz;
-      const long long r0 = (long long) r.local * TR;
-      const int nr = (int) ((v.d.nxy - r0) < TR ? (v.d.nxy - r0) : TR);
+   auto copy_tabs = [&](const SweepTile &T, int q, int vb) {
+      if (lane != 0) return;
+      const SweepGeo o = sweep_geo(T.geo);
+      bulk_load(&views[vb], &tab[T.inst].sv[2], (uint32_t) sizeof(SweepView), &full[q]);
+      bulk_load(tabs + vb * tab_bytes, T.tabs, sweep_tab_bytes(o.n, o.skip, (int) sizeof(P), 0), &full[q]);
+   };
+   auto copy_tile = [&](const SweepTile &T, int q, bool load, bool with) {
+      const SweepGeo o = sweep_geo(T.geo);
+      const int nz = o.n, nr = T.b;
       const uint32_t row_bytes = (uint32_t) (nz * sizeof(P));
-      P *tile = (P *) (base + q * stage_bytes) + zrow_pad(v.tb.skip, (int) sizeof(P));
-      if (load && lane == 0) mbar_arrive_expect_tx(&full[q], row_bytes * nr);
+      P *tile = (P *) (base + q * stage_bytes) + zrow_pad(o.skip, (int) sizeof(P));
+      if (load && lane == 0) {
+         const uint32_t more = with ? (uint32_t) sizeof(SweepView) + sweep_tab_bytes(nz, o.skip, (int) sizeof(P), 0) : 0u;
+         mbar_arrive_expect_tx(&full[q], row_bytes * nr + more);
+      }
       __syncwarp();
       for (int rr = lane; rr < nr; rr += 32) {
-         P *g = (P *) v.psi + (r0 + rr) * nz;
-         if (load) bulk_load(tile + rr * v.LS, g, row_bytes, &full[q]);
-         else bulk_store(g, tile + rr * v.LS, row_bytes);
+         P *gp = (P *) T.psi + (long long) rr * nz;
+         if (load) bulk_load(tile + rr * o.ext, gp, row_bytes, &full[q]);
+         else bulk_store(gp, tile + rr * o.ext, row_bytes);
       }
       if (!load) bulk_commit();
    };
    if (threadIdx.x == 0) {
       for (int q = 0; q < S; q++) mbar_init(&full[q], 1);
       fence_mbar_init();
+      if ((int) blockIdx.x < ntiles) ring[0] = tiles[blockIdx.x];
+      for (int k = 1; k < 3; k++)
+         if ((int) blockIdx.x + k * g < ntiles) ring[k] = tiles[blockIdx.x + k * g];
    }
    __syncthreads();
-   if (threadIdx.x < 32 && (int) blockIdx.x < ntiles) copy_tile(blockIdx.x, 0, true);
-   int cur = -1;
-   int it = 0;
-   SegTab tbs{};
-   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, it++) {
+   if (threadIdx.x < 32 && (int) blockIdx.x < ntiles) {
+      copy_tile(ring[0], 0, true, true);
+      copy_tabs(ring[0], 0, 0);
+   }
+   int vb = 0, it = 0;
+   for (int t = blockIdx.x; t < ntiles; t += g, it++) {
       const int q = it % S;
-      if (threadIdx.x < 32 && t + (int) gridDim.x < ntiles) {
+      const SweepTile &T = ring[it & 7], &N = ring[(it + 1) & 7];
+      const bool change = t + g < ntiles && N.inst != T.inst;
+      const int vn = change && nbuf == 2 ? vb ^ 1 : vb;
+      if (threadIdx.x < 32 && t + g < ntiles) {
          wait_stage_free<S>();
-         copy_tile(t + gridDim.x, (it + 1) % S, true);
+         copy_tile(N, (it + 1) % S, true, change);
+         if (change && nbuf == 2) copy_tabs(N, (it + 1) % S, vn);
       }
-      const TileRef r = tile_ref(work, t);
-      const int i = r.inst;
-      if (i != cur) {
-         // every thread has finished with the previous view and tables
-         __syncthreads();
-         const SweepView &v = tab[i].sv[2];
-         copy_view(sv, v);
-         tbs = v.tb;
-         if constexpr (STAB) tbs = stage_segtab<CPLX>(tabs, v.tb);
-         cur = i;
+      if (threadIdx.x == blockDim.x - 1) {
+         // the record asked for one tile ago is complete before the barrier
+         // below; the next one replaces a record no thread reads any more
+         cp_async_wait_all();
+         if (t + 3 * g < ntiles) {
+            unsigned char *to = (unsigned char *) &ring[(it + 3) & 7];
+            const unsigned char *from = (const unsigned char *) (tiles + t + 3 * g);
+            cp_async16(to, from);
+            cp_async16(to + 16, from + 16);
+         }
       }
-      if (__syncthreads_or(!mbar_wait(&full[q], (it / S) & 1, tab[i].err))) break;
-      const int TR = sv.TW;
-      const int c = threadIdx.x % TR, p = threadIdx.x / TR;
-      const long long r0 = (long long) r.local * TR;
-      const int nr = (int) ((sv.d.nxy - r0) < TR ? (sv.d.nxy - r0) : TR);
-      P *rows = (P *) (base + q * stage_bytes) + zrow_pad(sv.tb.skip, (int) sizeof(P));
-      zsweep_tile<R, CPLX, MOM, MSEG, STAB, true>(rows, nr, TR, sv.LS, c, p, tbs, xch, part, part2, sv.d,
-                                                        sv.zo, r0, r.local);
-      if (threadIdx.x < 32) copy_tile(t, q, false);
+      const bool late = !mbar_wait(&full[q], (it / S) & 1, nullptr);
+      if (late) atomicOr(tab[T.inst].err, kErrTmaTimeout);
+      if (__syncthreads_or(late)) break;
+      const SweepView &sv = views[vb];
+      const SweepGeo o = sweep_geo(T.geo);
+      const int TR = o.TW, c = threadIdx.x % TR, p = threadIdx.x / TR;
+      P *rows = (P *) (base + q * stage_bytes) + zrow_pad(o.skip, (int) sizeof(P));
+      // the row sums run beyond the tile's last barrier: what they need of the
+      // view, whose buffer the next copies may replace, is taken before
+      const Dims d = sv.d;
+      const ZOut zo = sv.zo;
+      zsweep_tile<R, CPLX, MOM, MSEG, true, true>(rows, T.b, TR, o.ext, c, p,
+                                                  BatchTabs<R, CPLX>::at(sv.tb, tabs + vb * tab_bytes), xch, part, part2,
+                                                  d, zo, T.a, T.a / TR);
+      if (threadIdx.x < 32) {
+         copy_tile(T, q, false, false);
+         if (change && nbuf == 1) copy_tabs(N, (it + 1) % S, 0);
+      }
+      vb = vn;
    }
    if (threadIdx.x < 32) bulk_wait_all();
 }

@@ -99,20 +99,20 @@ template <class R, bool CPLX> struct BatchStep {
       BCKS(with_mseg(A.mseg[0], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
          return launch(kb_sweep_xy<R, CPLX, 0, true, M, 2>, (unsigned) G.sweep_grid[0], A.threads[kPXsweep],
-                       G.sweep_smem[0], st, tab, S(kPXsweep), (int) A.tiles[kPXsweep], A.stage[0], A.xch[0]);
+                       G.sweep_smem[0], st, tab, (const SweepTile *) G.dtile[0], (int) A.tiles[kPXsweep], A.stage[0], A.xch[0], A.tabs[0], G.nbuf[0]);
       }));
       BCKS(mark(kPXsweep));
       BCKS(with_mseg(A.mseg[1], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
          return launch(kb_sweep_xy<R, CPLX, 1, false, M, 2>, (unsigned) G.sweep_grid[1], A.threads[kPYsweep],
-                       G.sweep_smem[1], st, tab, S(kPYsweep), (int) A.tiles[kPYsweep], A.stage[1], A.xch[1]);
+                       G.sweep_smem[1], st, tab, (const SweepTile *) G.dtile[1], (int) A.tiles[kPYsweep], A.stage[1], A.xch[1], A.tabs[1], G.nbuf[1]);
       }));
       BCKS(mark(kPYsweep));
       BCKS(with_mseg(A.mseg[2], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
          constexpr int MOM = CPLX ? 0 : 1;
          return launch(kb_sweep_z<R, CPLX, MOM, M, 2>, (unsigned) G.sweep_grid[2], A.threads[kPZsweep],
-                       G.sweep_smem[2], st, tab, S(kPZsweep), (int) A.tiles[kPZsweep], A.stage[2], A.xch[2],
+                       G.sweep_smem[2], st, tab, (const SweepTile *) G.dtile[2], (int) A.tiles[kPZsweep], A.stage[2], A.xch[2], A.tabs[2], G.nbuf[2],
                        A.part);
       }));
       BCKS(mark(kPZsweep));

@@ -505,6 +505,8 @@ template <class R, bool CPLX> struct Impl {
       g->threads[kPPhifix] = (unsigned) std::min<long>(256, std::max<long>(32, (d.nz - 1 + 31) / 32 * 32));
       // sweeps
       const size_t esz = s->esz_psi;
+      g->nxy = d.nxy;
+      g->row_bytes = (size_t) d.nz * esz;
       for (int ax = 0; ax < 3; ax++) {
          const auto &w = s->sw[ax];
          const int TW = w.TW, P = w.tab.P;
@@ -516,10 +518,15 @@ template <class R, bool CPLX> struct Impl {
          const size_t stage = ax < 2 ? sweep_stage(s, ax, w.boxn * w.nbox, TW, w.tab.skip) : (size_t) TW * w.LS * esz;
          g->stage[ax] = (uint32_t) ((stage + 127) & ~(size_t) 127);
          g->xch[ax] = (uint32_t) ((2 * (size_t) P * TW * esz + 15) & ~(size_t) 15);
-         if (!s->fp32) {
-            if (ax == 0) g->extra[ax] = (uint32_t) ((d.nx + w.tab.skip) * (s->cplx ? 16 : 8));
-            if (ax == 2) g->extra[ax] = (uint32_t) (4 * (size_t) P * w.MSEG * esz);
-         }
+         g->tabs[ax] = sweep_tab_bytes(w.tab.n, w.tab.skip, (int) esz, ax == 0 ? nu_tab_esz<R, CPLX>() : 0);
+         g->tw[ax] = TW;
+         g->across[ax] = nzb;
+         SweepTile &r = g->tile[ax];
+         r = SweepTile{};
+         r.geo = sweep_geo(w.tab.n, ax < 2 ? w.boxn * w.nbox : w.LS, TW, w.tab.skip);
+         r.tabs = w.tabs;
+         if (ax < 2) r.st = s->state;
+         else r.psi = s->psi;
          if (ax == 2) g->part = (uint32_t) (((size_t) P * TW * sizeof(double) + 15) & ~(size_t) 15);
       }
       // norm (imaginary time)

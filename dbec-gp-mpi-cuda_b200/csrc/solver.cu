@@ -248,33 +248,38 @@ static gpe_status make_segtab(gpe_solver *s, int ax, long n, int m, int P) {
    int D = 1;
    for (long double r = dec; D < P && r > drop; r *= dec) D++;
    auto &w = s->sw[ax];
-   std::vector<Z> *src[3] = {&tg, &tma, &tn};
-   for (int q = 0; q < 3; q++) {
-      if (w.tabs[q]) cudaFree(w.tabs[q]);
-      w.tabs[q] = nullptr;
-      const std::vector<Z> &z = *src[q];
-      std::vector<double> h(z.size() * E);
-      for (size_t e = 0; e < z.size(); e++) {
-         h[E * e] = (double) z[e].real();
-         if (s->cplx) h[E * e + 1] = (double) z[e].imag();
+   // gamma | (M, alpha) | N, and for the x sweep calcnu's table behind `skip`
+   // zero entries, in one block (the batched sweeps copy it whole)
+   const size_t r = s->esz_r;
+   const int xe = ax == 0 ? (int) (s->nu_x.size() / (size_t) n) : 0;
+   std::vector<unsigned char> blk(sweep_tab_bytes((int) n, (int) skip, (int) s->esz_psi, xe), 0);
+   const std::vector<Z> *src[3] = {&tg, &tma, &tn};
+   size_t at = 0;
+   for (int q = 0; q < 3; q++)
+      for (const Z &z : *src[q]) {
+         double h[2] = {(double) z.real(), (double) z.imag()};
+         for (int c = 0; c < E; c++, at += r) {
+            if (s->fp32) {
+               // FP32 copies of the FP64 values (alpha and gamma stay FP64 in
+               // HBM as computed; the FP32 kernels read these once-rounded
+               // copies).  In real time the gamma copy holds gamma + 1
+               // (SegOps::back_step): gamma is -1 plus a small number, which
+               // FP32 keeps to its own relative precision.
+               const float f = (float) (q == 0 && s->cplx && c == 0 ? h[c] + 1. : h[c]);
+               std::memcpy(&blk[at], &f, 4);
+            } else {
+               std::memcpy(&blk[at], &h[c], 8);
+            }
+         }
       }
-      if (s->fp32) {
-         // FP32 copies of the FP64 values (alpha and gamma stay FP64 in HBM
-         // as computed; the FP32 kernels read these once-rounded copies).  In
-         // real time the gamma copy holds gamma + 1 (SegOps::back_step):
-         // gamma is -1 plus a small number, which FP32 keeps to its own
-         // relative precision.
-         std::vector<float> f(h.size());
-         for (size_t e = 0; e < h.size(); e++) f[e] = (float) (q == 0 && s->cplx && e % 2 == 0 ? h[e] + 1. : h[e]);
-         CKS(upload(&w.tabs[q], f.data(), f.size()));
-      } else {
-         CKS(upload(&w.tabs[q], h.data(), h.size()));
-      }
-   }
+   if (ax == 0) std::memcpy(&blk[at + (size_t) skip * xe], s->nu_x.data(), s->nu_x.size());
+   if (w.tabs) cudaFree(w.tabs);
+   w.tabs = nullptr;
+   CKS(upload(&w.tabs, blk.data(), blk.size()));
    SegTab &t = w.tab;
-   t.ga = w.tabs[0];
-   t.ma = w.tabs[1];
-   t.nn = w.tabs[2];
+   t.ga = w.tabs;
+   t.ma = (unsigned char *) w.tabs + (size_t) ne * s->esz_psi;
+   t.nn = (unsigned char *) w.tabs + 3 * (size_t) ne * s->esz_psi;
    t.A = s->A[ax];
    t.n = (int) n;
    t.m = m;
@@ -579,8 +584,7 @@ static void free_all(gpe_solver *s) {
    for (int a = 0; a < 3; a++) {
       if (s->alpha[a]) cudaFree(s->alpha[a]);
       if (s->gamma[a]) cudaFree(s->gamma[a]);
-      for (void *q : s->sw[a].tabs)
-         if (q) cudaFree(q);
+      if (s->sw[a].tabs) cudaFree(s->sw[a].tabs);
    }
    if (s->wz) cudaFree(s->wz - kTabPad);
    for (float *q : {s->x2f, s->y2f, s->z2f})
@@ -638,9 +642,6 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    CKS(make_coef(s, 1, d.ny, p->dy * p->dy));
    CKS(make_coef(s, 2, d.nz, p->dz * p->dz));
    CKS(make_udd(s));
-   CKS(plan_tiles(s));
-   CKS(setup_static(s));
-
    // space mesh (initpsi, imag3d-mpicuda.cu:842-855)
    const long nx2 = d.nx / 2, ny2 = d.ny / 2, nz2 = d.nz / 2;
    s->hx.resize(d.nx); s->hy.resize(d.ny); s->hz.resize(d.nz);
@@ -649,6 +650,7 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    for (long j = 0; j < d.ny; j++) { s->hy[j] = (j - ny2) * p->dy; s->hy2[j] = s->hy[j] * s->hy[j]; }
    for (long k = 0; k < d.nz; k++) { s->hz[k] = (k - nz2) * p->dz; s->hz2[k] = s->hz[k] * s->hz[k]; }
    void *t = nullptr;
+   auto keep_x = [&](const void *p, size_t n) { s->nu_x.assign((const unsigned char *) p, (const unsigned char *) p + n); };
    CKS(upload(&t, s->hx2.data(), d.nx)); s->x2 = (double *) t;
    CKS(upload(&t, s->hy2.data(), d.ny)); s->y2 = (double *) t;
    CKS(upload(&t, s->hz2.data(), d.nz)); s->z2 = (double *) t;
@@ -660,6 +662,7 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
          f.insert(f.end(), sq[a]->begin(), sq[a]->end());
          CKS(upload(&t, f.data(), f.size()));
          *dst[a] = (float *) t + kTabPad;
+         if (a == 0 && s->cplx) keep_x(f.data() + kTabPad, sizeof(float) * sq[a]->size());
       }
    }
    // trap factors per axis for calcnu: exp(-dt 0.5 par c x^2) in imaginary
@@ -678,6 +681,7 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
             tab[i] = make_double2((double) cosl(th), (double) sinl(th));
          }
          CKS(upload(&s->lin[a], tab.data(), tab.size()));
+         if (a == 0) keep_x(tab.data(), sizeof(double2) * tab.size());
       }
    }
    if (!s->cplx) {
@@ -694,11 +698,16 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
             f.insert(f.end(), tab.begin(), tab.end());
             CKS(upload(&t, f.data(), f.size()));
             s->lin[a] = (float *) t + kTabPad;
+            if (a == 0) keep_x(f.data() + kTabPad, sizeof(float) * n);
          } else {
             CKS(upload(&s->lin[a], tab.data(), tab.size()));
+            if (a == 0) keep_x(tab.data(), sizeof(double) * n);
          }
       }
    }
+   CKS(plan_tiles(s));
+   CKS(setup_static(s));
+
    CK(cudaDeviceSynchronize());
    return GPE_OK;
 }

@@ -79,6 +79,7 @@ struct gpe_solver {
    long long row_cap = 0;  // doubles in rowA / rowB: the largest of nx*ny, nx*nz, ny*nz
    State *state = nullptr;
    std::vector<double> hx, hy, hz, hx2, hy2, hz2;
+   std::vector<unsigned char> nu_x;  // calcnu's table along x as the sweeps hold it
    long long launches = 0;
    size_t obs_cap = 0;
    // sweep configuration per axis (x, y: TMA tensor tiles; z: bulk rows)
@@ -87,8 +88,9 @@ struct gpe_solver {
       size_t smem = 0;
       CUtensorMap tm_psi{}, tm_phi{};
       SegTab tab{};
-      // coefficient tables (FP64, or rounded once to FP32 in mixed precision)
-      void *tabs[3] = {nullptr, nullptr, nullptr};
+      // block of coefficient tables (FP64, or rounded once to FP32 in mixed
+      // precision): sweep_tab_bytes
+      void *tabs = nullptr;
    } sw[3];
    double *wz = nullptr;      // Simpson weights along z (norm partials)
    double *wz2 = nullptr;     // wz[k] * z[k]^2 (rms partials)

@@ -154,8 +154,8 @@ struct NoXf {
 // transforms the two points above the last segment itself.
 //
 // SIMP 1: *simp receives this thread's share of sum_i |psi'_i|^2 with the
-// interior Simpson weights, 4 at odd i and 2 at even i, by parity (lo is
-// even); the caller adds the end correction of an even-length line.  SIMP 2:
+// Simpson weights, 4 at odd i and 2 at even i inside the line by parity (lo is
+// even).  SIMP 2:
 // with the weights w1[i] into *simp and w2[i] into *simp2 (both arrays have
 // skip entries before index 0).
 template <class R, bool CPLX, int M, bool ROW, bool STAB, int SIMP, class XF>
@@ -300,7 +300,12 @@ __device__ __forceinline__ void seg_sweep(typename Tr<R, CPLX>::P *line, int es_
       if (p == 0) line[0] = zero_of<P>();
       if (top) line[(tb.n - 1) * es] = zero_of<P>();
    }
-   if constexpr (SIMP == 1) *simp = fma(4., acc_o, 2. * acc_e);
+   if constexpr (SIMP == 1) {
+      *simp = fma(4., acc_o, 2. * acc_e);
+      // the end correction of an even line: the weights of points n-2 and n-3
+      // are 3 and 3.75 where the interior weights give 2 and 4
+      if (top && !(tb.n & 1)) *simp += (double) dens2(bt[M - 1]) - 0.25 * (double) dens2(bt[M - 2]);
+   }
    if constexpr (SIMP == 2) {
       *simp = acc;
       *simp2 = acc2;
@@ -430,7 +435,8 @@ __device__ __forceinline__ float2 expi_f32(float t) {
    return make_float2((q + 1) & 2 ? -c : c, q & 2 ? s : -s);
 }
 
-template <class R, bool CPLX> struct NuXf {
+// XS: the table along the line is in shared memory (always in FP64).
+template <class R, bool CPLX, bool XS> struct NuXf {
    using P = typename Tr<R, CPLX>::P;
    using T = typename std::conditional<CPLX && std::is_same<R, double>::value, double2, R>::type;
    static constexpr bool kNu = true;
@@ -443,6 +449,10 @@ template <class R, bool CPLX> struct NuXf {
    R scale, dtg, dtgd;      // 1/norm, dt g, dt gd / N
    R ca, to, tz, hp, dt;    // FP32 real time: V = hp ((ca x^2 + to) + tz)
 
+   __device__ __forceinline__ static T ldx(const T *p) {
+      if constexpr (XS) return *p;
+      else return __ldg(p);
+   }
    __device__ __forceinline__ void zero_row(int i) const { ph[i * es] = (R) 0; }
 
    __device__ __forceinline__ R expo(P p, R f) const {  // nonlinear exponent
@@ -489,10 +499,10 @@ template <class R, bool CPLX> struct NuXf {
             w[q] = cmul(p, cmul(cmul(x[q], fix), expi_series7(t)));
          } else if constexpr (!CPLX) {
             const float p = lp[q * es] * scale;
-            w[q] = p * ((__ldg(x + q) * fix) * expf(-expo(p, f[q * es])));
+            w[q] = p * ((ldx(x + q) * fix) * expf(-expo(p, f[q * es])));
          } else {
             const float2 p = lp[q * es];
-            const float t = expo32(p, f[q * es], __ldg(x + q));
+            const float t = expo32(p, f[q * es], ldx(x + q));
             big |= !(fabsf(t) <= 256.f);
             w[q] = cmul(p, expi_f32(t));
          }
@@ -508,21 +518,22 @@ template <class R, bool CPLX> struct NuXf {
 
 // The functor of tile column c of an x sweep tile covering z columns
 // [z0, z0 + TW) of plane y = other; pcol is phi's column in the tile, xtab the
-// staged table (FP64; the FP32 sweeps read theirs through L1).
-template <class R, bool CPLX>
-__device__ __forceinline__ NuXf<R, CPLX> nu_xf(R *pcol, int TW, int other, int z0, int c, const Dims &d,
-                                               const Trap &trap, const LinPhase &lin, const double *xtab, double g,
-                                               double gd, double dt, double scale) {
+// table along the line staged in shared memory, `skip` zero entries before
+// index 0 (XS; else the FP32 tables are read through L1).
+template <class R, bool CPLX, bool XS>
+__device__ __forceinline__ NuXf<R, CPLX, XS> nu_xf(R *pcol, int TW, int other, int z0, int c, const Dims &d,
+                                                   const Trap &trap, const LinPhase &lin, const void *xtab, int skip,
+                                                   double g, double gd, double dt, double scale) {
    const int k = min(z0 + c, d.nz - 1);  // columns past nz are zero fill, never stored
-   NuXf<R, CPLX> f;
-   using T = typename NuXf<R, CPLX>::T;
+   NuXf<R, CPLX, XS> f;
+   using T = typename NuXf<R, CPLX, XS>::T;
    f.ph = pcol;
    f.es = TW;
    f.scale = (R) scale;
    f.dtg = (R) (dt * g);
    f.dtgd = (R) (dt * gd / (double) d.npts);
    if constexpr (std::is_same<R, float>::value && CPLX) {
-      f.xt = trap.x2f;
+      f.xt = XS ? (const T *) xtab + skip : trap.x2f;
       f.fix = 0.f;
       f.ca = (float) trap.vg2;
       f.to = __fmul_rn((float) trap.vn2, trap.y2f[other]);
@@ -533,8 +544,7 @@ __device__ __forceinline__ NuXf<R, CPLX> nu_xf(R *pcol, int TW, int other, int z
       const T ey = __ldg((const T *) lin.ey + other), ez = __ldg((const T *) lin.ez + k);
       if constexpr (CPLX) f.fix = cmul(ey, ez);
       else f.fix = ey * ez;
-      if constexpr (std::is_same<R, double>::value) f.xt = (const T *) xtab;
-      else f.xt = (const T *) lin.ex;
+      f.xt = XS ? (const T *) xtab + skip : (const T *) lin.ex;
       f.ca = f.to = f.tz = f.hp = f.dt = (R) 0;
    }
    return f;
@@ -654,8 +664,8 @@ __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k
          const int other = t / nzb, z0 = (t - other * nzb) * TW;
          seg_sweep<R, CPLX, MSEG, false, false, 0>(
              col, TW, p, tb, xch + c, TW,
-             nu_xf<R, CPLX>((R *) (base + q * lay.bytes + lay.phi) + c, TW, other, z0, c, d, trap, lin,
-                            xtab + E * tb.skip, g, gd, dt, scale));
+             nu_xf<R, CPLX, std::is_same<R, double>::value>((R *) (base + q * lay.bytes + lay.phi) + c, TW, other, z0, c,
+                                                            d, trap, lin, xtab, tb.skip, g, gd, dt, scale));
       } else {
          seg_sweep<R, CPLX, MSEG, false, false, 0>(col, TW, p, tb, xch + c, TW, NoXf());
       }
@@ -733,14 +743,6 @@ __device__ __forceinline__ void zsweep_tile(typename Tr<R, CPLX>::P *rows, int n
       }
       if (MOM == 1) {
          if (ln < nr) {
-            if (!(tbs.n & 1)) {
-               // the end correction of an even nz: the weights of points nz-2
-               // and nz-3 are 3 and 3.75 where the interior weights give 2
-               // and 4
-               const int n = tbs.n;
-               const P *row = rows + rr * LS;
-               sum += (double) dens2(row[n - 2]) - 0.25 * (double) dens2(row[n - 3]);
-            }
             const int row = (int) row0 + rr, i = row / d.ny, j = row - i * d.ny;
             sum *= o.hz3 * simp_w(i, d.nx) * simp_w(j, d.ny);
          } else {
