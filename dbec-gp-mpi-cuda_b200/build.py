@@ -28,7 +28,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
                   "-Xcompiler", "-fPIC", "-I" + INCLUDE, "-I" + CSRC]
 
-LIB_SOURCES = ["conv_f64.cu", "conv_f32.cu", "impl_f64i.cu", "impl_f64r.cu", "impl_f32i.cu", "impl_f32r.cu",
+LIB_SOURCES = ["conv_f64_zf_lens.cu", "conv_f32_zf_lens.cu", "conv_f64_y_lens.cu", "conv_f32_y_lens.cu",
+               "conv_f64_x_lens.cu", "conv_f32_x_lens.cu", "conv_f64_z_lens.cu", "conv_f32_z_lens.cu",
+               "conv_f64.cu", "conv_f32.cu", "impl_f64i.cu", "impl_f64r.cu", "impl_f32i.cu", "impl_f32r.cu",
                "batch_f64i.cu", "batch_f64r.cu", "batch_f32i.cu", "batch_f32r.cu", "solver.cu", "noalloc.cu", "batch.cu",
                "server.cpp"]
 LIB_DEPS = LIB_SOURCES + ["common.cuh", "fft.cuh", "fftn.cuh", "kernels.cuh", "step_kernels.cuh", "sweep_kernels.cuh", "tma.cuh",

@@ -127,6 +127,16 @@ __device__ __forceinline__ double dens2(double2 v) { return v.x * v.x + v.y * v.
 __device__ __forceinline__ float dens2(float v) { return v * v; }
 __device__ __forceinline__ float dens2(float2 v) { return v.x * v.x + v.y * v.y; }
 
+// The same, rounded as written: where the result feeds further sums in
+// registers the compiler may not fuse its products into them, so that a pass
+// that keeps it in registers gives the values of one that stores it first.
+__device__ __forceinline__ double dens_rn(double v) { return __dmul_rn(v, v); }
+__device__ __forceinline__ double dens_rn(double2 v) { return __fma_rn(v.x, v.x, __dmul_rn(v.y, v.y)); }
+__device__ __forceinline__ float dens_rn(float v) { return __fmul_rn(v, v); }
+__device__ __forceinline__ float dens_rn(float2 v) { return __fmaf_rn(v.x, v.x, __fmul_rn(v.y, v.y)); }
+__device__ __forceinline__ double2 scale_rn(double2 a, double s) { return make_double2(__dmul_rn(a.x, s), __dmul_rn(a.y, s)); }
+__device__ __forceinline__ float2 scale_rn(float2 a, float s) { return make_float2(__fmul_rn(a.x, s), __fmul_rn(a.y, s)); }
+
 __device__ __forceinline__ double scl(double v, double s) { return v * s; }
 __device__ __forceinline__ double2 scl(double2 v, double s) { return make_double2(v.x * s, v.y * s); }
 __device__ __forceinline__ float scl(float v, double s) { return (float) (v * s); }

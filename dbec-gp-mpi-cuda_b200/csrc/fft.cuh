@@ -45,11 +45,11 @@ struct FftPlan {
 // x 8), so that a transform and the inverse that runs its stages backwards
 // share one table of roots; then the threes and fives.  Returns their number (0 when n has
 // another factor).
-inline int make_radices(int n, int log2max, int *rad) {
+__host__ __device__ constexpr int make_radices(int n, int log2max, int *rad) {
    int a = 0, k = 0;
    while (n % 2 == 0) { n /= 2; a++; }
    const int st2 = (a + log2max - 1) / log2max;
-   int e[32];
+   int e[32] = {};
    for (int q = 0, r = a; q < st2; q++) {
       e[q] = (r + st2 - q - 1) / (st2 - q);
       r -= e[q];

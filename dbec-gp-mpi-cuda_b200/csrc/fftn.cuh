@@ -1,5 +1,5 @@
-// fftn.cuh -- FFTs of compile-time length on lines in shared memory, for the
-// lengths most grids have; fft.cuh transforms any other length.
+// fftn.cuh -- FFTs of compile-time length on lines in shared memory; fft.cuh
+// transforms any other length.
 //
 // The transform is the one of fft.cuh (Stockham stages in the order of the
 // same radix plan, the same roots of unity, L lines interleaved [j][L]), so
@@ -19,6 +19,7 @@
 #pragma once
 
 #include <type_traits>
+#include <utility>
 
 #include "fft.cuh"
 
@@ -26,33 +27,89 @@ namespace gpe {
 
 template <int... RS> struct Rads {};
 
-// Radix plan of a compile-time length: RadixPlan<N, LOG> with radices up to
-// 2^LOG, as make_radices (fft.cuh) lists them, and its reverse.
-template <int N, int LOG> struct RadixPlan;
-#define GPE_RADIX_PLAN(N, LOG, FWD, REV)          \
-   template <> struct RadixPlan<N, LOG> {         \
-      using fwd = Rads<GPE_UNPAREN FWD>;          \
-      using rev = Rads<GPE_UNPAREN REV>;          \
-   };
-#define GPE_UNPAREN(...) __VA_ARGS__
-GPE_RADIX_PLAN(24, 4, (8, 3), (3, 8))
-GPE_RADIX_PLAN(32, 4, (8, 4), (4, 8))
-GPE_RADIX_PLAN(48, 4, (16, 3), (3, 16))
-GPE_RADIX_PLAN(64, 4, (8, 8), (8, 8))
-GPE_RADIX_PLAN(96, 4, (8, 4, 3), (3, 4, 8))
-GPE_RADIX_PLAN(128, 4, (16, 8), (8, 16))
-GPE_RADIX_PLAN(256, 4, (16, 16), (16, 16))
-GPE_RADIX_PLAN(512, 4, (8, 8, 8), (8, 8, 8))
+// Points per thread of these passes, in both precisions.  FP64 threads hold 16
+// points in 64 of their 128 registers; twice as many threads with 8 points and
+// radices up to 8 measured slower at 256^3 (us: x 92 -> 78, z inverse 55.5 ->
+// 50.6, z forward 60 -> 57).
+constexpr int kLenPpt = 16;
 
-// Points per thread, in both precisions, and log2 of the largest radix.  FP64
-// threads hold 16 points in 64 of their 128 registers; half as many threads
-// with 8 points, three stages of radix 8 and 4 for two of radix 16, measured
-// slower at 256^3 (us: x 92 -> 78, z inverse 55.5 -> 50.6, z forward 60 -> 57).
-constexpr int kLenPpt = 16, kLenLog = 4;
+// The lengths: a common set, compiled for one solve and for batches, with
+// radices up to 16 in both precisions, and most other even lengths up to
+// 400 that factor into 2, 3 and 5, with half lengths for z, compiled for one
+// solve only (above 256 a line is two boxes of 64-byte rows, so a multiple of 4).  The latter keep the radices of the run-time passes (16 in FP32,
+// 8 in FP64), so a batch, which transforms them at run time, gives the same
+// values bit for bit.
+#define GPE_LENS(X) X(24) X(32) X(48) X(64) X(96) X(128) X(256) X(512)
+#define GPE_LENS_XY(X)                                                                                             \
+   X(16) X(18) X(20) X(30) X(36) X(40) X(50) X(54) X(60) X(72) X(80) X(90) X(100) X(108) X(120) X(144) X(150) X(160) \
+       X(162) X(180) X(192) X(200) X(216) X(240) X(250) X(288) X(300) X(320) X(324) X(360) X(384) X(400)
+#define GPE_LENS_Z(X)                                                                                            \
+   X(8) X(9) X(10) X(12) X(15) X(16) X(18) X(20) X(25) X(27) X(30) X(36) X(40) X(45) X(50) X(54) X(60) X(72) X(75) \
+       X(80) X(81) X(90) X(100) X(108) X(120) X(125) X(135) X(144) X(150) X(160) X(162) X(180) X(192) X(200)
+#define GPE_LEN_CASE(n) case n:
+__host__ __device__ constexpr bool has_len(int n) {
+   switch (n) {
+      GPE_LENS(GPE_LEN_CASE) return true;
+   default: return false;
+   }
+}
+__host__ __device__ constexpr bool has_len_xy(int n) {
+   switch (n) {
+      GPE_LENS_XY(GPE_LEN_CASE) return true;
+   default: return false;
+   }
+}
+__host__ __device__ constexpr bool has_len_z(int h) {
+   switch (h) {
+      GPE_LENS_Z(GPE_LEN_CASE) return true;
+   default: return false;
+   }
+}
+#define GPE_LEN_CALL(n) \
+   case n: return f(std::integral_constant<int, n>());
+// runs f(std::integral_constant<int, n>) for a length of a set, with 0 for any
+// other
+template <class F> __host__ __device__ __forceinline__ auto with_len(int n, F f) {
+   switch (n) {
+      GPE_LENS(GPE_LEN_CALL)
+   default: return f(std::integral_constant<int, 0>());
+   }
+}
+template <class F> auto with_len_xy(int n, F f) {
+   switch (n) {
+      GPE_LENS_XY(GPE_LEN_CALL)
+   default: return f(std::integral_constant<int, 0>());
+   }
+}
+template <class F> auto with_len_z(int h, F f) {
+   switch (h) {
+      GPE_LENS_Z(GPE_LEN_CALL)
+   default: return f(std::integral_constant<int, 0>());
+   }
+}
+
+// Radix plan of a length, as make_radices lists it, and its reverse.
+template <class R> __host__ __device__ constexpr int len_log(int n) { return has_len(n) || sizeof(R) == 4 ? 4 : 3; }
+struct RadixList {
+   int k;
+   int r[kMaxStages];
+};
+constexpr RadixList radix_list(int n, int log2max) {
+   RadixList l{};
+   l.k = make_radices(n, log2max, l.r);
+   return l;
+}
+template <int N, int LOG> struct RadixPlan {
+   static constexpr RadixList l = radix_list(N, LOG);
+   template <size_t... I> static Rads<l.r[I]...> up(std::index_sequence<I...>);
+   template <size_t... I> static Rads<l.r[l.k - 1 - (int) I]...> down(std::index_sequence<I...>);
+   using fwd = decltype(up(std::make_index_sequence<(size_t) l.k>()));
+   using rev = decltype(down(std::make_index_sequence<(size_t) l.k>()));
+};
 
 // whether a convolution's inverse reads the same table of roots as its forward
-template <int N> __host__ __device__ constexpr bool palin_plan() {
-   using PL = RadixPlan<N, kLenLog>;
+template <class R, int N> __host__ __device__ constexpr bool palin_plan() {
+   using PL = RadixPlan<N, len_log<R>(N)>;
    return std::is_same<typename PL::fwd, typename PL::rev>::value;
 }
 
@@ -128,7 +185,7 @@ __device__ __forceinline__ void stages(Rads<R0, RS...>, C *buf, const C *tw, con
 // goes to st(l, i, value).
 template <int N, int L, int NT, class C, bool INV, class LD, class ST>
 __device__ __forceinline__ void fft_lines(C *buf, const C *tw, const LD &ld, const ST &st) {
-   using PL = RadixPlan<N, kLenLog>;
+   using PL = RadixPlan<N, len_log<decltype(C::x)>(N)>;
    stages<N, L, NT, C, INV, 1>(typename PL::fwd(), buf, tw, ld, st);
 }
 
@@ -152,7 +209,7 @@ __device__ __forceinline__ void conv_stages(Rads<R0, RS...>, Rads<I0, IS...> inv
       __syncthreads();
       conv_stages<N, L, NT, C, NS * R0>(Rads<RS...>(), inv, buf, NS == 1 ? tw : tw + (R0 - 1) * NS, twi, mul);
    } else {
-      static_assert(R0 == I0 && sizeof...(IS) > 0, "the inverse plan starts with the forward plan's last radix");
+      static_assert(R0 == I0, "the inverse plan starts with the forward plan's last radix");
       {
          C v[U][R0];
          stage_read<N, L, NT, R0, NS, C, false>(v, tw, ld);
@@ -162,20 +219,22 @@ __device__ __forceinline__ void conv_stages(Rads<R0, RS...>, Rads<I0, IS...> inv
             if ((int) threadIdx.x < NT && ((N / R0 * L) % NT == 0 || b < N / R0 * L)) {
                const int l = b % L, j = b / L;
 #pragma unroll
-               for (int t = 0; t < R0; t++) v[u][t] = cscale(v[u][t], mul(l, j + t * (N / R0)));
+               for (int t = 0; t < R0; t++) v[u][t] = scale_rn(v[u][t], mul(l, j + t * (N / R0)));
                dftr<R0, C, true>(v[u]);
             }
          }
          __syncthreads();
          stage_write<N, L, NT, R0, 1, C>(v, st);
       }
-      __syncthreads();
-      stages<N, L, NT, C, true, R0>(Rads<IS...>(), buf, twi, ld, st);
+      if constexpr (sizeof...(IS) > 0) {
+         __syncthreads();
+         stages<N, L, NT, C, true, R0>(Rads<IS...>(), buf, twi, ld, st);
+      }
    }
 }
 template <int N, int L, int NT, class C, class MUL>
 __device__ __forceinline__ void conv_lines(C *buf, const C *tw, const C *twi, const MUL &mul) {
-   using PL = RadixPlan<N, kLenLog>;
+   using PL = RadixPlan<N, len_log<decltype(C::x)>(N)>;
    conv_stages<N, L, NT, C, 1>(typename PL::fwd(), typename PL::rev(), buf, tw, twi, mul);
 }
 

@@ -46,6 +46,12 @@ inline gpe_status smem_attr(const void *f, size_t bytes) {
    return GPE_OK;
 }
 
+// The passes on the lengths compiled for one solve only (conv_*_lens.cu).
+template <class R> gpe_status yfft_lens(gpe_solver *s, bool inv, unsigned grid, size_t sm);
+template <class R> gpe_status xconv_lens(gpe_solver *s, unsigned grid, size_t sm);
+template <class R> gpe_status zinv_lens(gpe_solver *s, size_t sm);
+template <class R, bool CPLX> gpe_status zfwd_lens(gpe_solver *s, size_t sm);
+
 // The passes of the dipolar convolution that do not see psi: y, x and inverse
 // z FFTs, for one real type.
 template <class R> struct Conv {
@@ -89,23 +95,29 @@ template <class R> struct Conv {
    // Whether a pass runs its compile-time kernel (plan_tiles: the length has
    // one and the tile and radix choices are the defaults it is compiled for).
    static constexpr int kCols = LenCols<R>::L;
-   static bool len_x(const gpe_solver *s) { return s->fastx; }
-   static bool len_y(const gpe_solver *s) { return s->fasty; }
-   static bool len_z(const gpe_solver *s) { return s->fastz; }
+   // (the common set: the batched passes know no other)
+   static bool len_x(const gpe_solver *s) { return s->fastx == 1; }
+   static bool len_y(const gpe_solver *s) { return s->fasty == 1; }
+   static bool len_z(const gpe_solver *s) { return s->fastz == 1; }
 
-   // dynamic shared memory of the y and x passes
-   static size_t yfft_smem(const gpe_solver *s, int L) {
-      return 128 + ((size_t) s->boxy * s->nboxy * L + s->d.ny) * sizeof(C);
+   // dynamic shared memory of the y and x passes on tiles of so many rows
+   static size_t yfft_smem(const gpe_solver *s, int L, int rows) {
+      return 128 + ((size_t) rows * L + s->d.ny) * sizeof(C);
    }
-   static size_t xconv_smem(const gpe_solver *s, int L) {
-      return 128 + (size_t) fft_tile_bytes<R>(s->boxx * s->nboxx, L) + udd_box(s->d.nx, L).bytes +
+   static size_t xconv_smem(const gpe_solver *s, int L, int rows) {
+      return 128 + (size_t) fft_tile_bytes<R>(rows, L) + udd_box(s->d.nx, L).bytes +
              (size_t) conv_roots(s->px) * sizeof(C);
    }
 
    template <bool INV, int L> static gpe_status yfft(gpe_solver *s) {
       const Dims &d = s->d;
       const unsigned grid = (unsigned) (d.nx * ((d.nzh + L - 1) / L));
-      const size_t sm = yfft_smem(s, L);
+      const size_t sm = yfft_smem(s, L, s->fasty ? d.ny : s->boxy * s->nboxy);
+      if (s->fasty == 2) {
+         CKS(yfft_lens<R>(s, INV, grid, sm));
+         mark(s);
+         return GPE_OK;
+      }
       CKS(with_len(len_y(s) ? d.ny : 0, [&](auto nc) -> gpe_status {
          constexpr int N = decltype(nc)::value;
          if constexpr (N > 0 && L == kCols) {
@@ -125,7 +137,12 @@ template <class R> struct Conv {
    template <int L> static gpe_status xconv(gpe_solver *s) {
       const Dims &d = s->d;
       const unsigned grid = (unsigned) (d.ny * ((d.nzh + L - 1) / L));
-      const size_t sm = xconv_smem(s, L);
+      const size_t sm = xconv_smem(s, L, s->fastx ? d.nx : s->boxx * s->nboxx);
+      if (s->fastx == 2) {
+         CKS(xconv_lens<R>(s, grid, sm));
+         mark(s);
+         return GPE_OK;
+      }
       CKS(with_len(len_x(s) ? d.nx : 0, [&](auto nc) -> gpe_status {
          constexpr int N = decltype(nc)::value;
          if constexpr (N > 0 && L == kCols) {
@@ -202,6 +219,9 @@ template <class R> gpe_status Conv<R>::rest(gpe_solver *s) {
    CKS(with_L(s->Ly, [&](auto Lc) { return yfft<true, decltype(Lc)::value>(s); }));
    if (len_z(s)) {
       CKS(zinv_n(s));
+   } else if (s->fastz == 2) {
+      CKS(zinv_lens<R>(s, zinv_n_smem(s)));
+      mark(s);
    } else {
       const int L = zrows(s, 8, zinv_smem);
       const size_t sm = zinv_smem(s, L);
@@ -262,6 +282,9 @@ template <class R, bool CPLX> struct Impl {
       const Dims &d = s->d;
       if (CV::len_z(s)) {
          CKS(zfwd_n(s));
+      } else if (s->fastz == 2) {
+         CKS((zfwd_lens<R, CPLX>(s, zfwd_n_smem(s))));
+         mark(s);
       } else {
          // real rows: 8-row tiles on CTAs sized to them, except FP64 rows
          // shorter than 128 points, which keep 16 rows on 256 threads (sized
@@ -498,8 +521,8 @@ template <class R, bool CPLX> struct Impl {
       g->tiles[kPXconv] = (long long) d.ny * ((d.nzh + Lx - 1) / Lx);
       g->threads[kPYfft] = g->threads[kPYinv] = CV::len_y(s) ? (unsigned) len_threads<R>(d.ny, Ly) : CV::fft_threads(ry, Ly);
       g->threads[kPXconv] = CV::len_x(s) ? (unsigned) len_threads<R>(d.nx, Lx) : CV::fft_threads(rx, Lx);
-      g->smem[kPYfft] = g->smem[kPYinv] = CV::yfft_smem(s, Ly);
-      g->smem[kPXconv] = CV::xconv_smem(s, Lx);
+      g->smem[kPYfft] = g->smem[kPYinv] = CV::yfft_smem(s, Ly, (int) ry);
+      g->smem[kPXconv] = CV::xconv_smem(s, Lx, (int) rx);
       // boundary planes of phi
       g->tiles[kPPhifix] = std::max<long>(1, (d.ny - 1) + (d.nx - 1));
       g->threads[kPPhifix] = (unsigned) std::min<long>(256, std::max<long>(32, (d.nz - 1 + 31) / 32 * 32));

@@ -500,22 +500,25 @@ static gpe_status plan_tiles(gpe_solver *s) {
       if (mr != 16 && mr != 8 && mr != 4 && mr != 2)
          return fail(GPE_ERR_PARAM, "tuning: fft_max_radix must be 16, 8, 4 or 2");
       if (mr == 16 && !s->fp32) return fail(GPE_ERR_PARAM, "tuning: radix 16 is for mixed precision only");
-      // lengths with a compile-time pass: radices up to 16 in both precisions
-      // (their threads hold 16 points)
+      // compile-time passes (fftn.cuh) where the tile and radix choices are the
+      // defaults; the common set takes radices up to 16 in both precisions
       const bool plain = s->tune.fft_max_radix <= 0 || s->tune.fft_max_radix == (s->fp32 ? 16 : 8);
-      const int rx = plain && has_len(d.nx) && s->Lx == len_cols(s->fp32) ? 16 : mr;
-      const int ry = plain && has_len(d.ny) && s->Ly == len_cols(s->fp32) ? 16 : mr;
-      const int rz = plain && has_len(d.nz / 2) && d.nz / 2 <= kLenMaxH ? 16 : mr;
-      s->fastx = rx == 16 && has_len(d.nx) && s->Lx == len_cols(s->fp32);
-      s->fasty = ry == 16 && has_len(d.ny) && s->Ly == len_cols(s->fp32);
-      s->fastz = rz == 16 && has_len(d.nz / 2) && d.nz / 2 <= kLenMaxH;
+      auto level = [&](bool common, bool own) { return !plain ? 0 : (common ? 1 : (own ? 2 : 0)); };
+      const int h = d.nz / 2;
+      s->fastx = s->Lx == len_cols(s->fp32) ? level(has_len(d.nx), has_len_xy(d.nx)) : 0;
+      s->fasty = s->Ly == len_cols(s->fp32) ? level(has_len(d.ny), has_len_xy(d.ny)) : 0;
+      s->fastz = level(has_len(h) && h <= kLenMaxH, has_len_z(h));
+      const int rx = s->fastx == 1 ? 16 : mr, ry = s->fasty == 1 ? 16 : mr, rz = s->fastz == 1 ? 16 : mr;
       make_plan(d.nx, s->px, rx);
       s->pxi = reverse_plan(s->px);
       make_plan(d.ny, s->py, ry);
       make_plan(d.nz / 2, s->ph, rz);
       CKS(make_roots(s));
-      CKS(make_tmap(&s->tm_spec_y, s->spec, rsz, 2 * d.nzh, d.ny, d.nx, 2 * s->Ly, s->boxy, 1, 2 * d.nzp));
-      CKS(make_tmap(&s->tm_spec_x, s->spec, rsz, 2 * d.nzh, d.ny, d.nx, 2 * s->Lx, 1, s->boxx, 2 * d.nzp));
+      // a line over 256 points compiled for one solve arrives in two halves,
+      // without padded rows (a batch's run-time pass has boxes of its own)
+      const int by = s->fasty == 2 && d.ny > 256 ? d.ny / 2 : s->boxy, bx = s->fastx == 2 && d.nx > 256 ? d.nx / 2 : s->boxx;
+      CKS(make_tmap(&s->tm_spec_y, s->spec, rsz, 2 * d.nzh, d.ny, d.nx, 2 * s->Ly, by, 1, 2 * d.nzp));
+      CKS(make_tmap(&s->tm_spec_x, s->spec, rsz, 2 * d.nzh, d.ny, d.nx, 2 * s->Lx, 1, bx, 2 * d.nzp));
       CKS(make_udd_tmap(s, &s->tm_udd, s->Lx));
    }
    return GPE_OK;

@@ -54,7 +54,9 @@ struct gpe_solver {
    Dims d{};
    double par = 1.;
    FftPlan px{}, pxi{}, py{}, ph{};  // x lines forward and inverse, y lines and half-length z lines
-   bool fastx = false, fasty = false, fastz = false;  // x, y, z passes on compile-time lengths
+   // x, y, z passes: 1 a compile-time length of the common set, 2 one of the
+   // sets for one solve, 0 the run-time pass
+   int fastx = 0, fasty = 0, fastz = 0;
    int LSr = 0, LSo = 0;                  // shared row strides of the z passes
    CUtensorMap tm_spec_y{}, tm_spec_x{};  // spectrum tiles of the y and x passes
    CUtensorMap tm_udd{};                  // Udd columns of the x pass's tiles

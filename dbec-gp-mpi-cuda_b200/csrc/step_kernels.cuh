@@ -81,7 +81,7 @@ __device__ __forceinline__ void zfwd_pack(const typename Tr<R, CPLX>::P *rows, i
    for (int e = threadIdx.x; e < h * L; e += blockDim.x) {
       const int l = e % L, m = e / L;
       const typename Tr<R, CPLX>::P *rw = rows + l * LS + 2 * m;
-      buf[e] = mk<R>(dens2(rw[0]), dens2(rw[1]));
+      buf[e] = mk<R>(dens_rn(rw[0]), dens_rn(rw[1]));
    }
 }
 
@@ -156,29 +156,11 @@ __device__ __forceinline__ cpx<R> zinv_merge(const cpx<R> *row, const cpx<R> *W,
    return mk<R>(E.x - O.y, E.y + O.x);
 }
 
-// Lengths with compile-time transforms (RadixPlan in fftn.cuh): runs
-// f(std::integral_constant<int, n>), with 0 for any other length.
-template <class F> __host__ __device__ __forceinline__ auto with_len(int n, F f) {
-   switch (n) {
-   case 24: return f(std::integral_constant<int, 24>());
-   case 32: return f(std::integral_constant<int, 32>());
-   case 48: return f(std::integral_constant<int, 48>());
-   case 64: return f(std::integral_constant<int, 64>());
-   case 96: return f(std::integral_constant<int, 96>());
-   case 128: return f(std::integral_constant<int, 128>());
-   case 256: return f(std::integral_constant<int, 256>());
-   case 512: return f(std::integral_constant<int, 512>());
-   default: return f(std::integral_constant<int, 0>());
-   }
-}
 // kz columns of the y and x tiles these are compiled for, rows of the z tiles
 // and the longest half-length z line.
 __host__ __device__ constexpr int len_cols(bool fp32) { return fp32 ? 8 : 4; }
 template <class R> struct LenCols { static constexpr int L = len_cols(sizeof(R) == 4); };
 constexpr int kLenRows = 8, kLenMaxH = 256;
-__host__ __device__ __forceinline__ bool has_len(int n) {
-   return n == 24 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 256 || n == 512;
-}
 // Threads of a CTA that transforms L lines of N points, and the resident CTAs
 // its kernels are compiled for: 64 registers per FP32 thread, 128 per FP64 one.
 template <class R> __host__ __device__ constexpr int len_threads(int N, int L) {
@@ -352,7 +334,7 @@ __device__ __forceinline__ void xconv_body(const CUtensorMap *tm, const CUtensor
       const int xx = e / L, c = e - xx * L;
       const int ax = (xx <= nx / 2) ? xx : nx - xx;
       const R u = (R) (ud[ax * L + c] * s2);
-      res[e] = cscale(res[e], u);
+      res[e] = scale_rn(res[e], u);
    }
    __syncthreads();
    fft_lines_ip<L, C, true, PPT, true>(buf, pxi, ntw > nx ? tw + nx : tw);
@@ -506,7 +488,8 @@ __device__ __forceinline__ void zfwd_body_n(const typename Tr<R, CPLX>::P *__res
                                             long long r0) {
    using C = cpx<R>;
    using P = typename Tr<R, CPLX>::P;
-   constexpr int NT = len_threads<R>(H, L), nz = 2 * H, LSr = nz + 16 / (int) sizeof(P);
+   constexpr int NT = len_threads<R>(H, L), nz = 2 * H;
+   constexpr int U16 = 16 / (int) sizeof(P), LSr = (nz / U16 | 1) * U16;  // an odd number of 16-byte units
    constexpr int nzp = sizeof(R) == 4 ? (H + 2) & ~1 : H + 1;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
@@ -538,7 +521,7 @@ __device__ __forceinline__ void zfwd_body_n(const typename Tr<R, CPLX>::P *__res
        [&](int l, int m) {
           P a, b;
           ld2(rows + l * LSr + 2 * m, a, b);
-          return mk<R>(dens2(a), dens2(b));
+          return mk<R>(dens_rn(a), dens_rn(b));
        },
        [&](int l, int i, C v) { buf[i * L + l] = v; });
    __syncthreads();
@@ -566,7 +549,8 @@ template <class R, int L, int H, bool FOLD>
 __device__ __forceinline__ void zinv_body_n(const cpx<R> *__restrict__ spec, R *__restrict__ phi, const Dims &d,
                                             const cpx<R> *__restrict__ twz, uint32_t *err, long long r0) {
    using C = cpx<R>;
-   constexpr int NT = len_threads<R>(H, L), nz = 2 * H, LSo = nz + 16 / (int) sizeof(R);
+   constexpr int NT = len_threads<R>(H, L), nz = 2 * H;
+   constexpr int U16 = 16 / (int) sizeof(R), LSo = (nz / U16 | 1) * U16;  // an odd number of 16-byte units
    constexpr int nzp = sizeof(R) == 4 ? (H + 2) & ~1 : H + 1;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
@@ -611,7 +595,8 @@ template <class R, bool INV, int L, int N>
 __device__ __forceinline__ void yfft_body_n(const CUtensorMap *tm, const cpx<R> *__restrict__ twy, uint32_t *err, int x,
                                             int k0) {
    using C = cpx<R>;
-   constexpr int NT = len_threads<R>(N, L), boxn = N < 256 ? N : 256;
+   constexpr int NT = len_threads<R>(N, L), boxn = N <= 256 ? N : N / 2;
+   static_assert(N <= 256 || boxn * L * 2 * (int) sizeof(R) % 128 == 0, "TMA boxes start on 128 bytes");
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
    C *buf = (C *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
@@ -657,7 +642,8 @@ __device__ __forceinline__ void xconv_body_n(const CUtensorMap *tm, const CUtens
                                              const cpx<R> *__restrict__ twx, const State *__restrict__ st,
                                              uint32_t *err, int y, int k0) {
    using C = cpx<R>;
-   constexpr int NT = len_threads<R>(N, L), boxn = N < 256 ? N : 256;
+   constexpr int NT = len_threads<R>(N, L), boxn = N <= 256 ? N : N / 2;
+   static_assert(N <= 256 || boxn * L * 2 * (int) sizeof(R) % 128 == 0, "TMA boxes start on 128 bytes");
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
    const int ny = d.ny;
@@ -665,7 +651,7 @@ __device__ __forceinline__ void xconv_body_n(const CUtensorMap *tm, const CUtens
    C *buf = (C *) (((uintptr_t) smem_raw + 127) & ~(uintptr_t) 127);
    double *ud = (double *) ((unsigned char *) buf + fft_tile_bytes<R>(N, L));  // [|kx|][L]
    C *tw = (C *) ((unsigned char *) ud + ub.bytes);
-   constexpr int NTW = palin_plan<N>() ? N : 2 * N;  // stage roots
+   constexpr int NTW = palin_plan<R, N>() ? N : 2 * N;  // stage roots
    const int ay = (y <= ny / 2) ? y : ny - y;
    // the roots and Udd do not depend on the previous kernel: their copies start
    // before it has finished
@@ -686,7 +672,7 @@ __device__ __forceinline__ void xconv_body_n(const CUtensorMap *tm, const CUtens
    const double s2 = st->scale2;
    if (!tm_udd) cp_async_wait_all();
    if (__syncthreads_or(!mbar_wait(&bar, 0, err))) return;
-   conv_lines<N, L, NT, C>(buf, tw, palin_plan<N>() ? tw : tw + N, [&](int l, int i) {
+   conv_lines<N, L, NT, C>(buf, tw, palin_plan<R, N>() ? tw : tw + N, [&](int l, int i) {
       const int ax = i <= N / 2 ? i : N - i;
       return (R) (ud[ax * L + l] * s2);
    });

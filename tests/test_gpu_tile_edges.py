@@ -123,3 +123,35 @@ def test_mixed_psi_round_trip_is_exact(gpe_lib, mode, n):
     s.set_psi(psi)
     assert np.array_equal(s.get_psi(), psi.astype(np.complex64 if mode else np.float32))
     s.close()
+
+
+# Lengths that have a compiled pass for one solve only: each of them along x, y
+# and z (as a half length), against the oracle and against the run-time passes,
+# which a largest radix of its own selects.
+XY_LENGTHS = (16, 18, 20, 30, 36, 40, 50, 54, 60, 72, 80, 90, 100, 108, 120, 144, 150, 160, 162, 180, 192, 200, 216,
+              240, 250, 288, 300, 320, 324, 360, 384, 400)
+Z_HALVES = (8, 9, 10, 12, 15, 16, 18, 20, 25, 27, 30, 36, 40, 45, 50, 54, 60, 72, 75, 80, 81, 90, 100, 108, 120, 125,
+            135, 144, 150, 160, 162, 180, 192, 200)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("axis,n", [(0, n) for n in XY_LENGTHS] + [(1, n) for n in XY_LENGTHS] +
+                         [(2, 2 * h) for h in Z_HALVES])
+def test_convolution_compiled_lengths(gpe_lib, oracle_mod, prec, axis, n):
+    if prec and axis == 2 and n % 4:
+        pytest.skip("mixed precision takes rows of a multiple of 4 points")
+    shape = [10, 12, 8]
+    shape[axis] = n
+    s, o, psi = pair(gpe_lib, oracle_mod, 0, prec, tuple(shape))
+    s.calcpsidd2()
+    o.calcpsidd2()
+    phi = s.get_phi()
+    assert rel(phi, o.get_phi()) <= TOL[prec]
+    t = gpe_lib.Tuning()
+    t.fft_max_radix = 4
+    s.set_tuning(t)
+    s.set_psi(psi)
+    s.calcpsidd2()
+    assert rel(phi, s.get_phi()) <= TOL[prec]
+    s.close()
+    o.close()
