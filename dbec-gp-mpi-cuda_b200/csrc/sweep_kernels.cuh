@@ -100,8 +100,11 @@ template <class R, bool CPLX> struct SegOps {
    // mixed path; rounding alpha, A, psi, phi or the calcnu phase factor to
    // FP32 instead changes mu by at most 2e-8 there, measured with the FP64
    // oracle).  So the FP32 table holds gamma + 1, whose rounding error is
-   // that of the small part, and gamma u = (gamma + 1) u - u costs the same
-   // two multiply-adds per component.
+   // that of the small part.  The small products are summed before u (and, in
+   // fma_, before c): one rounding at psi's magnitude per component where a
+   // chain of two multiply-adds has two.  After 100 mixed real-time steps, over
+   // 48 draws of spacing, time step and g, rms against FP64: psi 2.2e-6 ->
+   // 1.6e-6, mu 6.8e-7 -> 5.0e-7, for 352 -> 358 us a step at 256^3.
    __device__ static P back_step(P b, P w2, P w1, P w0, P g, R a) {
       if constexpr (CPLX) {
          const R tx = fma((R) 2, w1.x, -w2.x) - w0.x, ty = fma((R) 2, w1.y, -w2.y) - w0.y;
@@ -109,8 +112,8 @@ template <class R, bool CPLX> struct SegOps {
          const R ux = fma(-a, dy, -w1.x), uy = fma(a, dx, -w1.y);
          P r;
          if constexpr (std::is_same<R, float>::value) {  // g = gamma + 1
-            r.x = fma(g.x, ux, fma(-g.y, uy, -ux));
-            r.y = fma(g.x, uy, fma(g.y, ux, -uy));
+            r.x = fma(g.x, ux, -g.y * uy) - ux;
+            r.y = fma(g.x, uy, g.y * ux) - uy;
          } else {
             r.x = fma(g.x, ux, -g.y * uy);
             r.y = fma(g.x, uy, g.y * ux);
@@ -124,10 +127,15 @@ template <class R, bool CPLX> struct SegOps {
    __device__ static P fma_(P a, P b, P c) {  // a * b + c
       if constexpr (CPLX) {
          P r;
-         r.x = fma(a.x, b.x, c.x);
-         r.x = fma(-a.y, b.y, r.x);
-         r.y = fma(a.x, b.y, c.y);
-         r.y = fma(a.y, b.x, r.y);
+         if constexpr (std::is_same<R, float>::value) {
+            r.x = c.x + fma(a.x, b.x, -a.y * b.y);
+            r.y = c.y + fma(a.x, b.y, a.y * b.x);
+         } else {
+            r.x = fma(a.x, b.x, c.x);
+            r.x = fma(-a.y, b.y, r.x);
+            r.y = fma(a.x, b.y, c.y);
+            r.y = fma(a.y, b.x, r.y);
+         }
          return r;
       } else {
          return fma(a, b, c);
