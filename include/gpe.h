@@ -143,7 +143,9 @@ gpe_status gpe_time_calcpsidd2(gpe_solver *s, long nrep, double *ms);
 /* Per-kernel timing: runs nsteps plain steps with a CUDA event around every
  * kernel of the step and returns, per kernel of one step, the mean duration in
  * milliseconds (ms[i], i < *count <= cap).  gpe_step_kernel_name(i) names
- * kernel i, gpe_step_kernel_bytes(s, i) its algorithmic bytes per launch. */
+ * kernel i, gpe_step_kernel_bytes(s, i) its algorithmic bytes per launch.
+ * What runs inside another kernel (the boundary planes, the norm) keeps its
+ * entry: the time between two events. */
 gpe_status gpe_profile_step(gpe_solver *s, long nsteps, double g, double gd, double *ms, int cap, int *count);
 const char *gpe_step_kernel_name(gpe_solver *s, int i);
 double gpe_step_kernel_bytes(gpe_solver *s, int i);
@@ -155,7 +157,9 @@ typedef struct gpe_tuning {
    int sweep_tw[3];     /* lines per CTA of the x, y, z sweeps (a power of two) */
    int sweep_stages[3]; /* TMA pipeline depth of the x, y, z sweeps: 2 or 3 */
    int fft_tile[2];     /* kz columns per tile of the y and x FFT passes */
-   int fft_max_radix;   /* largest radix of the FFT plans: 16 (mixed precision only), 8, 4 or 2 */
+   int fft_max_radix;   /* largest radix of the FFT plans: 16 (mixed precision only), 8, 4 or 2;
+                           at the default (16 mixed, 8 FP64) lines of 24, 32, 48, 64, 96,
+                           128, 256 or 512 points take radix 16 in FP64 too */
    int sweep_seg[3];    /* points per recurrence segment of the x, y, z sweeps: 8, 16 or
                            32 (32: mixed-precision imaginary time only; complex FP64
                            lines: 8) at most 256 threads per CTA */
@@ -193,9 +197,9 @@ gpe_status gpe_snapshot_load(gpe_solver *s, const char *path, double *g, double 
  * Many independent solves with their own grids and parameters (no reference
  * counterpart: the reference runs one solve per MPI job).  Each instance is a
  * full handle (its own stream and device memory); one batch step runs one
- * split step of every instance: the instances' kernels, captured once into a
- * CUDA graph with one branch per instance, are relaunched as one graph per
- * step, so small instances run concurrently on the GPU. */
+ * split step of every instance: per (mode, precision) one launch per pass over
+ * the tiles of all its instances, captured once into a CUDA graph that is
+ * relaunched for every step. */
 typedef struct gpe_batch gpe_batch;
 /* params[i] and couplings g[i], gd[i] of instance i (n >= 1).  Instances in
  * mixed-precision imaginary time start with 32-point segments in their y and z
@@ -222,7 +226,8 @@ gpe_status gpe_batch_time_steps(gpe_batch *b, long nsteps, double *ms);
  * CUDA event after every pass; ms[q] (q < *count = 10, cap >= 10) receives the
  * mean milliseconds of pass q per step, summed over the groups, in the order
  * z forward FFT, y FFT, x convolution, inverse y FFT, z inverse FFT, phi
- * boundary planes, x sweep with calcnu, y sweep, z sweep, norm. */
+ * boundary planes (mixed precision: stored by the inverse z pass), x sweep
+ * with calcnu, y sweep, z sweep, norm. */
 gpe_status gpe_batch_profile_step(gpe_batch *b, long nsteps, double *ms, int cap, int *count);
 /* Kernel launches executed by batch steps so far. */
 gpe_status gpe_batch_launch_count(gpe_batch *b, long long *count);
