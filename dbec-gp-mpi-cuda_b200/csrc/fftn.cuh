@@ -34,11 +34,13 @@ template <int... RS> struct Rads {};
 constexpr int kLenPpt = 16;
 
 // The lengths: a common set, compiled for one solve and for batches, with
-// radices up to 16 in both precisions, and most other even lengths up to
-// 400 that factor into 2, 3 and 5, with half lengths for z, compiled for one
-// solve only (above 256 a line is two boxes of 64-byte rows, so a multiple of 4).  The latter keep the radices of the run-time passes (16 in FP32,
-// 8 in FP64), so a batch, which transforms them at run time, gives the same
-// values bit for bit.
+// radices up to 16 in both precisions, and most other even lengths up to 400
+// that factor into 2, 3 and 5, with half lengths for z, compiled for one solve
+// only (above 256 a line is two boxes of 64-byte rows, so a multiple of 4).  The
+// latter keep the radices of the run-time passes (16 in FP32, 8 in FP64), so a
+// batch, which transforms them at run time, gives the same values bit for bit.
+// A whole step, their lengths at run time -> compiled, us: 128x96x80 FP64 70 ->
+// 64, 90x100x72 FP64 complex 80 -> 72, 160x144x120 FP32 complex 120 -> 93.
 #define GPE_LENS(X) X(24) X(32) X(48) X(64) X(96) X(128) X(256) X(512)
 #define GPE_LENS_XY(X)                                                                                             \
    X(16) X(18) X(20) X(30) X(36) X(40) X(50) X(54) X(60) X(72) X(80) X(90) X(100) X(108) X(120) X(144) X(150) X(160) \

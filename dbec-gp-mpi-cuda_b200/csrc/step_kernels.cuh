@@ -464,8 +464,12 @@ __global__ void __launch_bounds__(256, L >= 16 ? 3 : 4) k_zinv(const cpx<R> *__r
 // len_threads(N, L) threads per tile (the batched kernels may launch more),
 // the roots from the stage-ordered tables (make_roots in solver.cu).  The z
 // passes take the first stage's points straight from the staged rows (|psi|^2
-// or the merged half spectrum) and the inverse one ends in the phi rows.
-// 256^3 on B200, before (run-time lengths) and after: see each kernel.
+// or the merged half spectrum) and the inverse one ends in the phi rows.  With
+// run-time lengths these passes were bound by issue, most of it index
+// arithmetic (z inverse 180 instructions a complex point, now 56); they are now
+// bound by the series load, stages, store of the five to eight CTAs that fit an
+// SM.  256^3 on B200, run-time lengths -> these: at each kernel, with the time
+// of its bytes at 6.65 TB/s.
 
 // Bytes of the shared region of a z pass (psi or half-spectrum rows, lines,
 // output rows).
@@ -481,7 +485,8 @@ template <class R> __host__ __device__ constexpr int zinv_region(int H, int L) {
    return ((rows > lines ? rows : lines) + 127) & ~127;
 }
 
-// z forward: H = nz / 2; twz: H stage roots, then W^k, k <= H.
+// z forward: H = nz / 2; twz: H stage roots, then W^k, k <= H.  us: FP64 complex
+// 103 -> 73 (bytes 61), real 89 -> 57 (40), FP32 real 56 -> 29 (20).
 template <class R, bool CPLX, int L, int H>
 __device__ __forceinline__ void zfwd_body_n(const typename Tr<R, CPLX>::P *__restrict__ psi, cpx<R> *__restrict__ spec,
                                             const Dims &d, const cpx<R> *__restrict__ twz, uint32_t *err,
@@ -544,7 +549,8 @@ k_zfwd_n(const typename Tr<R, CPLX>::P *__restrict__ psi, cpx<R> *__restrict__ s
    zfwd_body_n<R, CPLX, L, H>(psi, spec, d, twz, err, (long long) blockIdx.x * L);
 }
 
-// z inverse; twz as above.
+// z inverse; twz as above.  us, with the boundary planes: FP64 78 + 7 -> 53
+// (bytes 41), FP32 49 + 7 -> 28 (20).
 template <class R, int L, int H, bool FOLD>
 __device__ __forceinline__ void zinv_body_n(const cpx<R> *__restrict__ spec, R *__restrict__ phi, const Dims &d,
                                             const cpx<R> *__restrict__ twz, uint32_t *err, long long r0) {
@@ -590,7 +596,8 @@ k_zinv_n(const cpx<R> *__restrict__ spec, R *__restrict__ phi, Dims d, const cpx
    zinv_body_n<R, L, H, true>(spec, phi, d, twz, err, (long long) blockIdx.x * L);
 }
 
-// y passes, forward and inverse; twy: N stage roots.
+// y passes, forward and inverse; twy: N stage roots.  us: FP64 57 -> 54 (bytes
+// 41), FP32 30 -> 28 (20); they were nearest to their bytes before.
 template <class R, bool INV, int L, int N>
 __device__ __forceinline__ void yfft_body_n(const CUtensorMap *tm, const cpx<R> *__restrict__ twy, uint32_t *err, int x,
                                             int k0) {
@@ -636,7 +643,9 @@ k_yfft_n(const __grid_constant__ CUtensorMap tm, Dims d, const cpx<R> *__restric
 }
 
 // x convolution; twx: N forward and N inverse stage roots.  The multiply by
-// Udd happens on the last forward stage's registers.
+// Udd happens on the last forward stage's registers.  us: FP64 111 -> 68 (bytes
+// 42), FP32 61 -> 37 (21), 512x512x256 FP32 (three stages) 166 (92); 41 % of
+// its cycles are FP64 arithmetic.
 template <class R, int L, int N>
 __device__ __forceinline__ void xconv_body_n(const CUtensorMap *tm, const CUtensorMap *tm_udd, const double *udd, const Dims &d,
                                              const cpx<R> *__restrict__ twx, const State *__restrict__ st,
@@ -757,7 +766,7 @@ __global__ void k_calcnu(typename Tr<R, CPLX>::P *__restrict__ psi, const R *__r
 // |psi|^2, by a warp per row with the weights wz, wz2 (in units of h / 3): the
 // loads of a warp are consecutive and four rounds of them are in flight.  One
 // thread per row left the loads of a warp a row apart (96 us at 256^3 FP64,
-// whose 134 MB take 20 us).
+// whose 134 MB take 20 us; a whole calcnorm call 97 -> 54 us).
 constexpr int kRowWarps = 8;
 template <class R, bool CPLX>
 __global__ void __launch_bounds__(32 * kRowWarps) k_rows_dens(const typename Tr<R, CPLX>::P *__restrict__ psi, Dims d,
@@ -981,7 +990,8 @@ __device__ __forceinline__ double fd4(double m2, double m1, double p1, double p2
 // of the Simpson weights of the three axes (the nested rule of simpint is
 // that product); part[2 CTA] receives the CTA's sums, k_sum2 adds them.  One
 // thread per (x, y) row walking z (32 rows apart in a warp's loads, 13 square
-// roots a point) took 2.5 ms at 256^3 complex FP64.
+// roots a point) took 2.5 ms at 256^3 complex FP64; a whole calcmuen call at
+// 256^3 real FP64, with its convolution, 1615 -> 680 us.
 constexpr int kMuY = 8, kMuZ = 32, kMuRing = 6;
 template <class R, bool CPLX>
 __global__ void __launch_bounds__(kMuY *kMuZ, 4) k_muen(const typename Tr<R, CPLX>::P *__restrict__ psi,

@@ -602,7 +602,12 @@ template <bool CPLX> __device__ __forceinline__ void stage_xtab(double *xtab, co
 // x or y sweep.  Tile: TW consecutive z columns of one y (x sweep) or one x
 // (y sweep) plane, the whole line along the swept axis, brought in by TMA.
 // With NU the x sweep first applies the pending 1/norm and calcnu to the tile
-// (needs phi).
+// (needs phi).  Bound by issue, not bytes: two CTAs of 128 registers (four of 64
+// in FP32) issue on a third (FP32 half) of the cycles.  256^3 on B200, with a
+// scan over the segments -> with carries from D segments, us (bytes at 6.65
+// TB/s): x FP64 complex 209 -> 167 (101), real 144 -> 90 (60), FP32 real 88
+// -> 54 (30), complex 98 now (50); y FP64 complex 127 -> 106 (81), real 70 -> 52 (40),
+// FP32 real 51 -> 30 (20).
 template <class R, bool CPLX, int AXIS, bool NU, int MSEG, int S, int TWC>
 __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k_sweep_xy(const __grid_constant__ CUtensorMap tm_psi,
                                                      const __grid_constant__ CUtensorMap tm_phi, Dims d, SegTab tb,
@@ -785,7 +790,10 @@ template <bool CPLX> __device__ __forceinline__ SegTab stage_segtab(double *tabs
 // norm of the step (simpint, diffint.cu:106): the last CTA to finish adds the
 // tile partials and sets the state (hx, hy; out_norm may be null), which was a
 // launch of its own.  MOM 2 yields the row partials of calcrms, so an rms
-// sample after the step needs no extra pass over psi.
+// sample after the step needs no extra pass over psi.  Bound as the y sweep,
+// with the Simpson sums on top; 256^3 on B200, us (bytes at 6.65 TB/s): FP64
+// complex 131 -> 113 (81), real with the norm 89 + 10 -> 63 (40), FP32 real 62 +
+// 10 -> 39 (20).
 template <class R, bool CPLX, int MOM, int MSEG, int S, int TWC>
 __global__ void __launch_bounds__(256, sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) k_sweep_z(typename Tr<R, CPLX>::P *__restrict__ psi, Dims d, SegTab tb,
                                                     int tr_arg, int LS, ZOut out, double hx, double hy,
