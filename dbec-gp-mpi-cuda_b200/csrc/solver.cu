@@ -105,9 +105,12 @@ extern "C" gpe_status gpe_device_bytes(const gpe_params *p, long long *bytes) {
 }
 
 // ------------------------------------------------------------------ tables
-template <class T> static gpe_status upload(void **dst, const T *src, size_t n) {
+// On the handle's stream: a copy on the legacy stream from pageable memory may
+// return before its data has arrived, and nothing would order it before the
+// kernels of the handle's own non-blocking stream.
+template <class T> static gpe_status upload(const gpe_solver *s, void **dst, const T *src, size_t n) {
    CK(cudaMalloc(dst, sizeof(T) * n));
-   CK(cudaMemcpy(*dst, src, sizeof(T) * n, cudaMemcpyHostToDevice));
+   CK(cudaMemcpyAsync(*dst, src, sizeof(T) * n, cudaMemcpyHostToDevice, s->st));
    return GPE_OK;
 }
 
@@ -132,10 +135,10 @@ static gpe_status make_roots(gpe_solver *s) {
    auto put = [&](const std::vector<double2> &t, void **dst) -> gpe_status {
       if (*dst) cudaFree(*dst);
       *dst = nullptr;
-      if (!s->fp32) return upload(dst, t.data(), t.size());
+      if (!s->fp32) return upload(s, dst, t.data(), t.size());
       std::vector<float2> f(t.size());
       for (size_t e = 0; e < t.size(); e++) f[e] = make_float2((float) t[e].x, (float) t[e].y);
-      return upload(dst, f.data(), f.size());
+      return upload(s, dst, f.data(), f.size());
    };
    std::vector<double2> t;
    stage_roots(s->px, t);
@@ -157,15 +160,10 @@ static gpe_status make_roots(gpe_solver *s) {
 }
 
 // gencoef (imag3d-mpicuda.cu:894-931, real3d-mpicuda.cu:991-1035).
-static gpe_status make_coef(gpe_solver *s, int ax, long n, double d2) {
+static void make_coef(gpe_solver *s, int ax, long n, double d2) {
    const double c = s->p.dt / d2 / (3. - s->par);
    typedef std::complex<double> Z;
-   Z A0, A0r, A, mA;
-   if (!s->cplx) {
-      A0 = 1. + c; A0r = 1. - c; A = -0.5 * c; mA = -A;
-   } else {
-      A0 = Z(1., c); A0r = std::conj(A0); A = Z(0., -0.5 * c); mA = Z(0., -A.imag());
-   }
+   const Z A0 = s->cplx ? Z(1., c) : Z(1. + c), A = s->cplx ? Z(0., -0.5 * c) : Z(-0.5 * c);
    std::vector<Z> al(n - 1), ga(n - 1);
    al[n - 2] = 0.;
    ga[n - 2] = Z(-1.) / A0;
@@ -174,25 +172,11 @@ static gpe_status make_coef(gpe_solver *s, int ax, long n, double d2) {
       ga[i - 1] = Z(-1.) / (A0 + A * al[i - 1]);
    }
    s->A[ax] = make_double2(A.real(), A.imag());
-   s->A0r[ax] = make_double2(A0r.real(), A0r.imag());
-   s->mA[ax] = make_double2(mA.real(), mA.imag());
-   // uploaded padded to n entries (the last is 0 and never used) so that the
-   // sweep kernels can bulk-copy them in 16-byte multiples
-   if (!s->cplx) {
-      std::vector<double> a(n, 0.), g(n, 0.);
-      for (long i = 0; i < n - 1; i++) { a[i] = al[i].real(); g[i] = ga[i].real(); }
-      CKS(upload(&s->alpha[ax], a.data(), n));
-      CKS(upload(&s->gamma[ax], g.data(), n));
-   } else {
-      std::vector<double2> a(n, make_double2(0., 0.)), g(n, make_double2(0., 0.));
-      for (long i = 0; i < n - 1; i++) {
-         a[i] = make_double2(al[i].real(), al[i].imag());
-         g[i] = make_double2(ga[i].real(), ga[i].imag());
-      }
-      CKS(upload(&s->alpha[ax], a.data(), n));
-      CKS(upload(&s->gamma[ax], g.data(), n));
-   }
-   return GPE_OK;
+   if (!s->cplx)
+      for (auto *v : {&al, &ga})
+         for (Z &z : *v) z = z.real();
+   s->alpha[ax] = std::move(al);
+   s->gamma[ax] = std::move(ga);
 }
 
 // Segment tables of the parallel Thomas sweep of axis ax (line length n, P
@@ -207,17 +191,7 @@ static gpe_status make_segtab(gpe_solver *s, int ax, long n, int m, int P) {
    if (m % 2 || n % 2) return fail(GPE_ERR_PARAM, "segment and line lengths must be even");
    typedef std::complex<long double> Z;
    const int E = s->cplx ? 2 : 1;
-   // coefficients as uploaded (double), promoted: the tables multiply exactly those
-   std::vector<Z> al(n - 1), ga(n - 1);
-   {
-      std::vector<double> ad((size_t) E * (n - 1)), gd((size_t) E * (n - 1));
-      CK(cudaMemcpy(ad.data(), s->alpha[ax], sizeof(double) * ad.size(), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(gd.data(), s->gamma[ax], sizeof(double) * gd.size(), cudaMemcpyDeviceToHost));
-      for (long i = 0; i < n - 1; i++) {
-         al[i] = s->cplx ? Z(ad[2 * i], ad[2 * i + 1]) : Z(ad[i], 0.L);
-         ga[i] = s->cplx ? Z(gd[2 * i], gd[2 * i + 1]) : Z(gd[i], 0.L);
-      }
-   }
+   std::vector<Z> al(s->alpha[ax].begin(), s->alpha[ax].end()), ga(s->gamma[ax].begin(), s->gamma[ax].end());
    const Z A(s->A[ax].x, s->A[ax].y);
    const long skip = (long) P * m - (n - 2), ne = (long) P * m;
    std::vector<Z> tg(ne, Z(0)), tma(2 * ne, Z(0)), tn(ne, Z(0));
@@ -260,9 +234,7 @@ static gpe_status make_segtab(gpe_solver *s, int ax, long n, int m, int P) {
          double h[2] = {(double) z.real(), (double) z.imag()};
          for (int c = 0; c < E; c++, at += r) {
             if (s->fp32) {
-               // FP32 copies of the FP64 values (alpha and gamma stay FP64 in
-               // HBM as computed; the FP32 kernels read these once-rounded
-               // copies).  In real time the gamma copy holds gamma + 1
+               // FP32 copies of the FP64 values, rounded once.  In real time the gamma copy holds gamma + 1
                // (SegOps::back_step): gamma is -1 plus a small number, which
                // FP32 keeps to its own relative precision.
                const float f = (float) (q == 0 && s->cplx && c == 0 ? h[c] + 1. : h[c]);
@@ -275,7 +247,7 @@ static gpe_status make_segtab(gpe_solver *s, int ax, long n, int m, int P) {
    if (ax == 0) std::memcpy(&blk[at + (size_t) skip * xe], s->nu_x.data(), s->nu_x.size());
    if (w.tabs) cudaFree(w.tabs);
    w.tabs = nullptr;
-   CKS(upload(&w.tabs, blk.data(), blk.size()));
+   CKS(upload(s, &w.tabs, blk.data(), blk.size()));
    SegTab &t = w.tab;
    t.ga = w.tabs;
    t.ma = (unsigned char *) w.tabs + (size_t) ne * s->esz_psi;
@@ -355,7 +327,8 @@ static int sweep_candidates(int n, int tw_base, int esz, int *TW, int *MSEG, int
 
 // Tile configuration of the sweeps and of the y / x FFT passes, and the FFT
 // plans: the heuristics below, or the values of s->tune where set.  May be
-// called again (gpe_set_tuning); it reuploads only the segment tables.
+// called again (gpe_set_tuning); it uploads the segment tables, calcnu's x table
+// and the roots of unity anew, in the order of the handle's stream.
 static gpe_status plan_tiles(gpe_solver *s) {
    s->plan_gen++;
    const Dims &d = s->d;
@@ -535,17 +508,17 @@ static gpe_status setup_static(gpe_solver *s) {
    void *t = nullptr;
    // (kTabPad zero entries before index 0, for the sweeps' rows below the line)
    wz.insert(wz.begin(), kTabPad, 0.);
-   CKS(upload(&t, wz.data(), wz.size()));
+   CKS(upload(s, &t, wz.data(), wz.size()));
    s->wz = (double *) t + kTabPad;
    std::vector<double> wz2(kTabPad + d.nz, 0.);
    for (int k = 0; k < N; k++) {
       const double z = (k - d.nz / 2) * s->p.dz;  // the mesh of initpsi
       wz2[kTabPad + k] = wz[kTabPad + k] * (z * z);
    }
-   CKS(upload(&t, wz2.data(), wz2.size()));
+   CKS(upload(s, &t, wz2.data(), wz2.size()));
    s->wz2 = (double *) t + kTabPad;
    CK(cudaMalloc(&s->err, sizeof(uint32_t)));
-   CK(cudaMemset(s->err, 0, sizeof(uint32_t)));
+   CK(cudaMemsetAsync(s->err, 0, sizeof(uint32_t), s->st));
    return GPE_OK;
 }
 
@@ -574,7 +547,7 @@ static gpe_status make_udd(gpe_solver *s) {
          }
    u[0] = 0.;  // imag3d-mpicuda.cu:975-977
    void *dp = nullptr;
-   CKS(upload(&dp, u.data(), u.size()));
+   CKS(upload(s, &dp, u.data(), u.size()));
    s->udd = (double *) dp;
    return GPE_OK;
 }
@@ -585,8 +558,6 @@ static void free_all(gpe_solver *s) {
    for (void *q : ptrs)
       if (q) cudaFree(q);
    for (int a = 0; a < 3; a++) {
-      if (s->alpha[a]) cudaFree(s->alpha[a]);
-      if (s->gamma[a]) cudaFree(s->gamma[a]);
       if (s->sw[a].tabs) cudaFree(s->sw[a].tabs);
    }
    if (s->wz) cudaFree(s->wz - kTabPad);
@@ -628,7 +599,7 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    CK(cudaMalloc(&s->psi, s->esz_psi * d.npts));
    CK(cudaMalloc(&s->spec, s->esz_c * (size_t) d.nzp * d.nxy));
    CK(cudaMalloc(&s->phi, r * d.npts));
-   CK(cudaMemset(s->psi, 0, s->esz_psi * d.npts));
+   CK(cudaMemsetAsync(s->psi, 0, s->esz_psi * d.npts, s->st));
    s->row_cap = std::max(d.nxy, std::max((long long) d.nx * d.nz, (long long) d.ny * d.nz));
    CK(cudaMalloc(&s->rowA, sizeof(double) * s->row_cap));
    CK(cudaMalloc(&s->rowB, sizeof(double) * s->row_cap));
@@ -639,11 +610,11 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    CK(cudaMalloc(&s->state, sizeof(State)));
    State st0{};
    st0.norm = 1.; st0.scale = 1.; st0.scale2 = 1.;
-   CK(cudaMemcpy(s->state, &st0, sizeof(State), cudaMemcpyHostToDevice));
+   CK(cudaMemcpyAsync(s->state, &st0, sizeof(State), cudaMemcpyHostToDevice, s->st));
 
-   CKS(make_coef(s, 0, d.nx, p->dx * p->dx));
-   CKS(make_coef(s, 1, d.ny, p->dy * p->dy));
-   CKS(make_coef(s, 2, d.nz, p->dz * p->dz));
+   make_coef(s, 0, d.nx, p->dx * p->dx);
+   make_coef(s, 1, d.ny, p->dy * p->dy);
+   make_coef(s, 2, d.nz, p->dz * p->dz);
    CKS(make_udd(s));
    // space mesh (initpsi, imag3d-mpicuda.cu:842-855)
    const long nx2 = d.nx / 2, ny2 = d.ny / 2, nz2 = d.nz / 2;
@@ -654,16 +625,16 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    for (long k = 0; k < d.nz; k++) { s->hz[k] = (k - nz2) * p->dz; s->hz2[k] = s->hz[k] * s->hz[k]; }
    void *t = nullptr;
    auto keep_x = [&](const void *p, size_t n) { s->nu_x.assign((const unsigned char *) p, (const unsigned char *) p + n); };
-   CKS(upload(&t, s->hx2.data(), d.nx)); s->x2 = (double *) t;
-   CKS(upload(&t, s->hy2.data(), d.ny)); s->y2 = (double *) t;
-   CKS(upload(&t, s->hz2.data(), d.nz)); s->z2 = (double *) t;
+   CKS(upload(s, &t, s->hx2.data(), d.nx)); s->x2 = (double *) t;
+   CKS(upload(s, &t, s->hy2.data(), d.ny)); s->y2 = (double *) t;
+   CKS(upload(s, &t, s->hz2.data(), d.nz)); s->z2 = (double *) t;
    if (s->fp32) {
       const std::vector<double> *sq[3] = {&s->hx2, &s->hy2, &s->hz2};
       float **dst[3] = {&s->x2f, &s->y2f, &s->z2f};
       for (int a = 0; a < 3; a++) {
          std::vector<float> f(kTabPad, 0.f);
          f.insert(f.end(), sq[a]->begin(), sq[a]->end());
-         CKS(upload(&t, f.data(), f.size()));
+         CKS(upload(s, &t, f.data(), f.size()));
          *dst[a] = (float *) t + kTabPad;
          if (a == 0 && s->cplx) keep_x(f.data() + kTabPad, sizeof(float) * sq[a]->size());
       }
@@ -683,7 +654,7 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
             const long double th = -dt * hp * cf[a] * (long double) (*sq[a])[i];
             tab[i] = make_double2((double) cosl(th), (double) sinl(th));
          }
-         CKS(upload(&s->lin[a], tab.data(), tab.size()));
+         CKS(upload(s, &s->lin[a], tab.data(), tab.size()));
          if (a == 0) keep_x(tab.data(), sizeof(double2) * tab.size());
       }
    }
@@ -699,11 +670,11 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
          if (s->fp32) {
             std::vector<float> f(kTabPad, 0.f);
             f.insert(f.end(), tab.begin(), tab.end());
-            CKS(upload(&t, f.data(), f.size()));
+            CKS(upload(s, &t, f.data(), f.size()));
             s->lin[a] = (float *) t + kTabPad;
             if (a == 0) keep_x(f.data() + kTabPad, sizeof(float) * n);
          } else {
-            CKS(upload(&s->lin[a], tab.data(), tab.size()));
+            CKS(upload(s, &s->lin[a], tab.data(), tab.size()));
             if (a == 0) keep_x(tab.data(), sizeof(double) * n);
          }
       }

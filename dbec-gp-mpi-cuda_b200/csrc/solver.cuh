@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <complex>
 #include <cstring>
 #include <string>
 #include <type_traits>
@@ -70,8 +71,8 @@ struct gpe_solver {
    void *psi = nullptr, *spec = nullptr, *phi = nullptr;
    void *twx = nullptr, *twy = nullptr, *twz = nullptr;
    double *udd = nullptr;
-   void *alpha[3] = {nullptr, nullptr, nullptr}, *gamma[3] = {nullptr, nullptr, nullptr};
-   double2 A[3], A0r[3], mA[3];
+   std::vector<std::complex<double>> alpha[3], gamma[3];  // the Thomas coefficients (gencoef)
+   double2 A[3];
    double *x2 = nullptr, *y2 = nullptr, *z2 = nullptr;
    float *x2f = nullptr, *y2f = nullptr, *z2f = nullptr;  // FP32 copies (mixed precision)
    void *lin[3] = {nullptr, nullptr, nullptr};  // per-axis trap factors of calcnu, imag (LinPhase)
