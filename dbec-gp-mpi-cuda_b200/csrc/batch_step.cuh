@@ -4,10 +4,9 @@
 #include "batch_group.h"
 
 template <class K, class... A>
-gpe_status launch(K kern, unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+gpe_status launch(const Group &G, K kern, unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
    if (grid == 0) return GPE_OK;
-   if (smem > 48 * 1024)
-      BCK(cudaFuncSetAttribute((const void *) kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+   if (smem > 0) BCK(G.roomy.allow((const void *) kern));
    kern<<<grid, block, smem, st>>>(args...);
    BCK(cudaGetLastError());
    return GPE_OK;
@@ -45,25 +44,25 @@ template <class R> gpe_status BatchConv<R>::run(const Group &G, cudaStream_t st,
    };
    BCKS(with_L(G.Ly, [&](auto lc) {
       constexpr int L = decltype(lc)::value;
-      return launch(kb_yfft<R, false, L>, T(kPYfft), A.threads[kPYfft], A.smem[kPYfft], st, tab, S(kPYfft));
+      return launch(G, kb_yfft<R, false, L>, T(kPYfft), A.threads[kPYfft], A.smem[kPYfft], st, tab, S(kPYfft));
    }));
    BCKS(mark(kPYfft));
    BCKS(with_L(G.Lx, [&](auto lc) {
       constexpr int L = decltype(lc)::value;
-      return launch(kb_xconv<R, L>, T(kPXconv), A.threads[kPXconv], A.smem[kPXconv], st, tab, S(kPXconv));
+      return launch(G, kb_xconv<R, L>, T(kPXconv), A.threads[kPXconv], A.smem[kPXconv], st, tab, S(kPXconv));
    }));
    BCKS(mark(kPXconv));
    BCKS(with_L(G.Ly, [&](auto lc) {
       constexpr int L = decltype(lc)::value;
-      return launch(kb_yfft<R, true, L>, T(kPYinv), A.threads[kPYinv], A.smem[kPYinv], st, tab, S(kPYinv));
+      return launch(G, kb_yfft<R, true, L>, T(kPYinv), A.threads[kPYinv], A.smem[kPYinv], st, tab, S(kPYinv));
    }));
    BCKS(mark(kPYinv));
    BCKS(with_ppt(A.zppt, [&](auto pc) {
       constexpr int PPT = decltype(pc)::value;
-      return launch(kb_zinv<R, PPT, ZL, kFold>, T(kPZinv), A.threads[kPZinv], A.smem[kPZinv], st, tab, S(kPZinv));
+      return launch(G, kb_zinv<R, PPT, ZL, kFold>, T(kPZinv), A.threads[kPZinv], A.smem[kPZinv], st, tab, S(kPZinv));
    }));
    BCKS(mark(kPZinv));
-   if (!kFold) BCKS(launch(kb_phifix<R>, T(kPPhifix), A.threads[kPPhifix], 0, st, tab, S(kPPhifix)));
+   if (!kFold) BCKS(launch(G, kb_phifix<R>, T(kPPhifix), A.threads[kPPhifix], 0, st, tab, S(kPPhifix)));
    BCKS(mark(kPPhifix));
    return GPE_OK;
 }
@@ -92,31 +91,31 @@ template <class R, bool CPLX> struct BatchStep {
       };
       BCKS(BatchConv<R>::with_ppt(A.zppt, [&](auto pc) {
          constexpr int PPT = decltype(pc)::value;
-         return launch(kb_zfwd<R, CPLX, PPT, ZL>, T(kPZfwd), A.threads[kPZfwd], A.smem[kPZfwd], st, tab, S(kPZfwd));
+         return launch(G, kb_zfwd<R, CPLX, PPT, ZL>, T(kPZfwd), A.threads[kPZfwd], A.smem[kPZfwd], st, tab, S(kPZfwd));
       }));
       BCKS(mark(kPZfwd));
       BCKS(BatchConv<R>::run(G, st, ev));
       BCKS(with_mseg(A.mseg[0], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
-         return launch(kb_sweep_xy<R, CPLX, 0, true, M, 2>, (unsigned) G.sweep_grid[0], A.threads[kPXsweep],
+         return launch(G, kb_sweep_xy<R, CPLX, 0, true, M, 2>, (unsigned) G.sweep_grid[0], A.threads[kPXsweep],
                        G.sweep_smem[0], st, tab, (const SweepTile *) G.dtile[0], (int) A.tiles[kPXsweep], A.stage[0], A.xch[0], A.tabs[0], G.nbuf[0]);
       }));
       BCKS(mark(kPXsweep));
       BCKS(with_mseg(A.mseg[1], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
-         return launch(kb_sweep_xy<R, CPLX, 1, false, M, 2>, (unsigned) G.sweep_grid[1], A.threads[kPYsweep],
+         return launch(G, kb_sweep_xy<R, CPLX, 1, false, M, 2>, (unsigned) G.sweep_grid[1], A.threads[kPYsweep],
                        G.sweep_smem[1], st, tab, (const SweepTile *) G.dtile[1], (int) A.tiles[kPYsweep], A.stage[1], A.xch[1], A.tabs[1], G.nbuf[1]);
       }));
       BCKS(mark(kPYsweep));
       BCKS(with_mseg(A.mseg[2], [&](auto mc) {
          constexpr int M = decltype(mc)::value;
          constexpr int MOM = CPLX ? 0 : 1;
-         return launch(kb_sweep_z<R, CPLX, MOM, M, 2>, (unsigned) G.sweep_grid[2], A.threads[kPZsweep],
+         return launch(G, kb_sweep_z<R, CPLX, MOM, M, 2>, (unsigned) G.sweep_grid[2], A.threads[kPZsweep],
                        G.sweep_smem[2], st, tab, (const SweepTile *) G.dtile[2], (int) A.tiles[kPZsweep], A.stage[2], A.xch[2], A.tabs[2], G.nbuf[2],
                        A.part);
       }));
       BCKS(mark(kPZsweep));
-      if (!CPLX) BCKS(launch(kb_norm_final, T(kPNorm), A.threads[kPNorm], 0, st, tab, S(kPNorm)));
+      if (!CPLX) BCKS(launch(G, kb_norm_final, T(kPNorm), A.threads[kPNorm], 0, st, tab, S(kPNorm)));
       BCKS(mark(kPNorm));
       *kernels += (CPLX ? 9 : 10) - (kFold ? 1 : 0);
       return GPE_OK;

@@ -6,7 +6,6 @@ template <class R> gpe_status xconv_lens(gpe_solver *s, unsigned grid, size_t sm
    return with_len_xy(s->d.nx, [&](auto nc) -> gpe_status {
       constexpr int N = decltype(nc)::value;
       if constexpr (N > 0) {
-         CKS(smem_attr((const void *) k_xconv_n<R, L, N>, sm));
          return launch_pdl(k_xconv_n<R, L, N>, grid, len_threads<R>(N, L), sm, s, s->tm_spec_x, s->tm_udd, s->d,
                            (const cpx<R> *) s->twx, s->state, s->err);
       } else {

@@ -7,7 +7,6 @@ template <class R> gpe_status yfft_lens(gpe_solver *s, bool inv, unsigned grid, 
       constexpr int N = decltype(nc)::value;
       if constexpr (N > 0) {
          auto go = [&](auto k) -> gpe_status {
-            CKS(smem_attr((const void *) k, sm));
             return launch_pdl(k, grid, len_threads<R>(N, L), sm, s, s->tm_spec_y, s->d, (const cpx<R> *) s->twy, s->err);
          };
          return inv ? go(k_yfft_n<R, true, L, N>) : go(k_yfft_n<R, false, L, N>);

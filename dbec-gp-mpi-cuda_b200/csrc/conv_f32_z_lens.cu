@@ -5,7 +5,6 @@ template <class R> gpe_status zinv_lens(gpe_solver *s, size_t sm) {
    return with_len_z(s->d.nz / 2, [&](auto nc) -> gpe_status {
       constexpr int H = decltype(nc)::value;
       if constexpr (H > 0 && (sizeof(R) == 8 || H % 2 == 0)) {  // mixed precision: nz divisible by 4
-         CKS(smem_attr((const void *) k_zinv_n<R, kLenRows, H>, sm));
          return launch_pdl(k_zinv_n<R, kLenRows, H>, blocks_for(s->d.nxy, kLenRows), len_threads<R>(H, kLenRows), sm, s,
                            (const cpx<R> *) s->spec, (R *) s->phi, s->d, (const cpx<R> *) s->twz, s->err);
       } else {

@@ -6,7 +6,6 @@ template <class R, bool CPLX> gpe_status zfwd_lens(gpe_solver *s, size_t sm) {
       constexpr int H = decltype(nc)::value;
       if constexpr (H > 0 && (sizeof(R) == 8 || H % 2 == 0)) {  // mixed precision: nz divisible by 4
          using P = typename Tr<R, CPLX>::P;
-         CKS(smem_attr((const void *) k_zfwd_n<R, CPLX, kLenRows, H>, sm));
          return launch_pdl(k_zfwd_n<R, CPLX, kLenRows, H>, blocks_for(s->d.nxy, kLenRows), len_threads<R>(H, kLenRows), sm,
                            s, (const P *) s->psi, (cpx<R> *) s->spec, s->d, (const cpx<R> *) s->twz, s->err);
       } else {

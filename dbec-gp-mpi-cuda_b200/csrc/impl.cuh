@@ -26,6 +26,7 @@ inline unsigned blocks_for(long long n, int bs) { return (unsigned) ((n + bs - 1
 // 0.107 -> 0.103 ms at 128^3, 512x512x256 unchanged at 1.69 ms, on B200).
 template <class... KP, class... A>
 gpe_status launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, const gpe_solver *s, A... args) {
+   if (smem > 0) CK(s->roomy.allow((const void *) k));
    cudaLaunchAttribute at[1];
    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
    at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -37,12 +38,6 @@ gpe_status launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, cons
    cfg.attrs = at;
    cfg.numAttrs = 1;
    CK(cudaLaunchKernelEx(&cfg, k, ((KP) args)...));
-   return GPE_OK;
-}
-
-// dynamic shared memory beyond the default limit
-inline gpe_status smem_attr(const void *f, size_t bytes) {
-   if (bytes > 48 * 1024) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes));
    return GPE_OK;
 }
 
@@ -121,11 +116,9 @@ template <class R> struct Conv {
       CKS(with_len(len_y(s) ? d.ny : 0, [&](auto nc) -> gpe_status {
          constexpr int N = decltype(nc)::value;
          if constexpr (N > 0 && L == kCols) {
-            CKS(smem_attr((const void *) k_yfft_n<R, INV, L, N>, sm));
             return launch_pdl(k_yfft_n<R, INV, L, N>, grid, len_threads<R>(N, L), sm, s, s->tm_spec_y, d,
                               (const C *) s->twy, s->err);
          } else {
-            CKS(smem_attr((const void *) k_yfft<R, INV, L>, sm));
             return launch_pdl(k_yfft<R, INV, L>, grid, fft_threads(s->boxy * s->nboxy, L), sm, s, s->tm_spec_y, d,
                               s->py, (const C *) s->twy, s->boxy, s->nboxy, s->err);
          }
@@ -146,11 +139,9 @@ template <class R> struct Conv {
       CKS(with_len(len_x(s) ? d.nx : 0, [&](auto nc) -> gpe_status {
          constexpr int N = decltype(nc)::value;
          if constexpr (N > 0 && L == kCols) {
-            CKS(smem_attr((const void *) k_xconv_n<R, L, N>, sm));
             return launch_pdl(k_xconv_n<R, L, N>, grid, len_threads<R>(N, L), sm, s, s->tm_spec_x,
                               s->tm_udd, d, (const C *) s->twx, s->state, s->err);
          } else {
-            CKS(smem_attr((const void *) k_xconv<R, L>, sm));
             return launch_pdl(k_xconv<R, L>, grid, fft_threads(s->boxx * s->nboxx, L), sm, s, s->tm_spec_x,
                               s->tm_udd, d, s->px, s->pxi, (const C *) s->twx, s->state, s->boxx, s->nboxx, s->err);
          }
@@ -163,7 +154,6 @@ template <class R> struct Conv {
       const Dims &d = s->d;
       return with_ppt(zppt(s, L), [&](auto pc) {
          constexpr int PPT = decltype(pc)::value;
-         CKS(smem_attr((const void *) k_zinv<R, PPT, L>, sm));
          CKS(launch_pdl(k_zinv<R, PPT, L>, blocks_for(d.nxy, L), z_threads(s, L, PPT), sm, s, (const C *) s->spec, (R *) s->phi, d, s->ph,
                         (const C *) s->twz, s->LSo, s->err));
          CKL();
@@ -198,7 +188,6 @@ template <class R> struct Conv {
       CKS(with_len(d.nz / 2, [&](auto nc) -> gpe_status {
          constexpr int H = decltype(nc)::value;
          if constexpr (H > 0 && H <= kLenMaxH) {
-            CKS(smem_attr((const void *) k_zinv_n<R, kLenRows, H>, sm));
             return launch_pdl(k_zinv_n<R, kLenRows, H>, blocks_for(d.nxy, kLenRows), len_threads<R>(H, kLenRows), sm, s,
                               (const C *) s->spec, (R *) s->phi, d, (const C *) s->twz, s->err);
          } else {
@@ -242,7 +231,6 @@ template <class R, bool CPLX> struct Impl {
       const Dims &d = s->d;
       return CV::with_ppt(CV::zppt(s, L), [&](auto pc) {
          constexpr int PPT = decltype(pc)::value;
-         CKS(smem_attr((const void *) k_zfwd<R, CPLX, PPT, L>, sm));
          const unsigned nt = sized ? CV::z_threads(s, L, PPT) : 256u;
          CKS(launch_pdl(k_zfwd<R, CPLX, PPT, L>, blocks_for(d.nxy, L), nt, sm, s, (const P *) s->psi, (C *) s->spec, d,
                         s->ph, (const C *) s->twz, s->LSr, s->err));
@@ -268,7 +256,6 @@ template <class R, bool CPLX> struct Impl {
       CKS(with_len(d.nz / 2, [&](auto nc) -> gpe_status {
          constexpr int H = decltype(nc)::value;
          if constexpr (H > 0 && H <= kLenMaxH) {
-            CKS(smem_attr((const void *) k_zfwd_n<R, CPLX, kLenRows, H>, sm));
             return launch_pdl(k_zfwd_n<R, CPLX, kLenRows, H>, blocks_for(d.nxy, kLenRows), len_threads<R>(H, kLenRows),
                               sm, s, (const P *) s->psi, (C *) s->spec, d, (const C *) s->twz, s->err);
          } else {
@@ -302,8 +289,6 @@ template <class R, bool CPLX> struct Impl {
    template <int AXIS, bool NU, int MSEG, int S, int TWC> static gpe_status sweep_xy_launch_t(gpe_solver *s, double g, double gd) {
       auto &w = s->sw[AXIS];
       const Dims &d = s->d;
-      const void *f = (const void *) k_sweep_xy<R, CPLX, AXIS, NU, MSEG, S, TWC>;
-      CKS(smem_attr(f, w.smem));
       const int nzb = (d.nz + w.TW - 1) / w.TW;
       const int ntiles = (AXIS == 0 ? d.ny : d.nx) * nzb;
       const unsigned grid = (unsigned) std::min(ntiles, w.ctas * s->nsm);
@@ -348,8 +333,6 @@ template <class R, bool CPLX> struct Impl {
    template <int MOM, int MSEG, int S, int TWC> static gpe_status sweep_z_launch_t(gpe_solver *s, double *dev_norm) {
       auto &w = s->sw[2];
       const Dims &d = s->d;
-      const void *f = (const void *) k_sweep_z<R, CPLX, MOM, MSEG, S, TWC>;
-      CKS(smem_attr(f, w.smem));
       const long long ntiles = (d.nxy + w.TW - 1) / w.TW;
       const unsigned grid = (unsigned) std::min<long long>(ntiles, (long long) w.ctas * s->nsm);
       CKS(launch_pdl(k_sweep_z<R, CPLX, MOM, MSEG, S, TWC>, grid, ((w.TW * w.tab.P + 31) & ~31), w.smem, s,

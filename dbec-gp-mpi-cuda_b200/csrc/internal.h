@@ -12,6 +12,22 @@
 namespace gpe {
 
 void set_last_error(const std::string &msg);
+
+// Kernels allowed the device's whole shared memory (less what they hold
+// statically) as dynamic shared memory.  The limit belongs to the kernel, not to
+// a handle: handles of other sizes on other threads share it, so it is always
+// set to that maximum and never to the bytes of one launch, which would take
+// room away from another thread between its own call and its launch.  Each
+// handle and batch group remembers the kernels it has passed (a few dozen) and
+// belongs to one thread at a time.
+class RoomyKernels {
+ public:
+   cudaError_t allow(const void *kernel);
+
+ private:
+   std::vector<const void *> done_;
+};
+
 // Queues nsteps split steps at fixed couplings on the handle's stream, with no
 // synchronisation; in imaginary time the last renormalisation stays pending.
 gpe_status queue_steps(gpe_solver *s, long nsteps, double g, double gd);

@@ -28,6 +28,20 @@ static thread_local std::string g_err;
 
 namespace gpe {
 void set_last_error(const std::string &msg) { g_err = msg; }
+
+cudaError_t RoomyKernels::allow(const void *kernel) {
+   for (const void *k : done_)
+      if (k == kernel) return cudaSuccess;
+   int dev = 0, most = 0;
+   cudaFuncAttributes a{};
+   cudaError_t e = cudaGetDevice(&dev);
+   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+   if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int) a.sharedSizeBytes);
+   if (e == cudaSuccess) done_.push_back(kernel);
+   return e;
+}
 }  // namespace gpe
 
 gpe_status fail(gpe_status st, const std::string &msg) {

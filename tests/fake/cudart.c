@@ -24,6 +24,7 @@ typedef struct { int flags; } stream;
 
 static long long live, launches, unordered, lowered;
 static int failing, pending;
+static __thread err_t last;
 
 long long fake_live_bytes(void) { return live; }
 long long fake_launches(void) { return launches; }
@@ -31,18 +32,15 @@ long long fake_unordered(void) { return unordered; }
 long long fake_lowered(void) { return lowered; }
 void fake_fail_mallocs(int on) { failing = on; }
 
-/* ---- kernels */
-#define STATIC_SMEM 64
+/* ---- kernels: dynamic shared memory up to 48 KB less the static bytes unless
+ * raised, to the opt-in maximum less them (static: a bound on what the batched
+ * kernels, whose names start with kb_, and the others hold) */
 #define OPTIN_SMEM 232448
-static struct { const void *f; int dyn; } attr[1 << 16];
-static int *dyn_of(const void *f) {
+static struct { const void *f; int dyn, fixed; } attr[1 << 16];
+static unsigned at(const void *f) {
    unsigned h = (unsigned) (((uintptr_t) f >> 4) * 2654435761u) & 0xffff;
    while (attr[h].f && attr[h].f != f) h = (h + 1) & 0xffff;
-   if (!attr[h].f) {
-      attr[h].f = f;
-      attr[h].dyn = 48 * 1024 - STATIC_SMEM;
-   }
-   return &attr[h].dyn;
+   return h;
 }
 void **__cudaRegisterFatBinary(void *f) { static void *h; (void) f; return &h; }
 void __cudaRegisterFatBinaryEnd(void **h) { (void) h; }
@@ -51,23 +49,26 @@ void __cudaRegisterVar(void **h, char *v, char *a, const char *n, int e, size_t 
    (void) h; (void) v; (void) a; (void) n; (void) e; (void) s; (void) c; (void) g;
 }
 void __cudaRegisterFunction(void **h, const char *f, char *d, const char *n, int l, void *t, void *b, void *bd, void *gd, int *w) {
-   (void) h; (void) f; (void) d; (void) n; (void) l; (void) t; (void) b; (void) bd; (void) gd; (void) w;
+   const unsigned k = at(f);
+   (void) h; (void) d; (void) l; (void) t; (void) b; (void) bd; (void) gd; (void) w;
+   attr[k].f = f;
+   attr[k].fixed = strstr(n, "kb_") ? 1152 : 128;
+   attr[k].dyn = 48 * 1024 - attr[k].fixed;
 }
 err_t cudaFuncSetAttribute(const void *f, int a, int v) {
-   int *d = dyn_of(f);
-   if (a != 8 || v < 0 || v > OPTIN_SMEM - STATIC_SMEM) return INVALID;
-   if (v < *d) lowered++;
-   *d = v;
+   const unsigned k = at(f);
+   if (!attr[k].f || a != 8 || v < 0 || v > OPTIN_SMEM - attr[k].fixed) return INVALID;
+   if (v < attr[k].dyn) lowered++;
+   attr[k].dyn = v;
    return OK;
 }
 err_t cudaFuncGetAttributes(void *out, const void *f) { /* sharedSizeBytes comes first */
-   (void) f;
    memset(out, 0, 64);
-   *(size_t *) out = STATIC_SMEM;
+   *(size_t *) out = (size_t) attr[at(f)].fixed;
    return OK;
 }
 static err_t launch(const void *f, dim g, dim b, size_t smem, stream *s) {
-   if (!g.x || !g.y || !g.z || !b.x || b.x * b.y * b.z > 1024 || smem > (size_t) *dyn_of(f)) return INVALID;
+   if (!g.x || !g.y || !g.z || !b.x || b.x * b.y * b.z > 1024 || smem > (size_t) attr[at(f)].dyn) return last = INVALID;
    if (pending && s && (s->flags & 1)) unordered++;
    launches++;
    return OK;
@@ -151,7 +152,7 @@ err_t cudaDeviceGetAttribute(int *v, int a, int d) {
    return OK;
 }
 err_t cudaDeviceGetStreamPriorityRange(int *least, int *greatest) { *least = 0; *greatest = -5; return OK; }
-err_t cudaGetLastError(void) { return OK; }
+err_t cudaGetLastError(void) { const err_t e = last; last = OK; return e; }
 const char *cudaGetErrorString(err_t e) { return e == OOM ? "out of memory" : "invalid value"; }
 
 /* the tensor map encoder: the checks the driver makes of a 3D map */

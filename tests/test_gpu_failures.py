@@ -6,6 +6,8 @@
   GPE_ERR_TIMEOUT and the handle keeps working.
 * The real-time program given a truncated imag3d-den.bin (the reference
   reads stale data there) exits with an error and says why.
+* Handles of different sizes on threads of their own share kernels: no thread's
+  launch fails for what another one asked of them.
 * A cancelled request: a queued one finishes at once, an admitted one stops
   at its next chunk boundary, both with GPE_ERR_CANCELLED; the server then
   serves the next request normally.
@@ -77,3 +79,35 @@ def test_server_cancel(gpe_lib):
     rc = sv.wait(c, timeout=120)
     assert rc.status == 0 and rc.steps > 0 and np.isfinite(rc.mu)
     sv.close()
+
+
+def test_handles_of_two_threads_share_kernels(gpe_lib):
+    """Lines of 1000 and 640 points along z: the same sweep and run-time FFT
+    kernels, other bytes of shared memory; each thread's psi is that of a run
+    alone."""
+    import threading
+
+    gpe = gpe_lib
+    ps = [gpe.make_params(1, 8, 8, nz, .25, .25, .25, 6e-4, .5, 1., 1.5, 1.) for nz in (1000, 640)]
+
+    def go(p, out):
+        try:
+            with gpe.Solver(p) as s:
+                s.init_gaussian()
+                for _ in range(200):
+                    s.run(1, 20., 5.)
+                out.append(s.get_psi())
+        except gpe.GpeError as e:
+            out.append(e)
+
+    alone, both = [[], []], [[], []]
+    for p, o in zip(ps, alone):
+        go(p, o)
+    threads = [threading.Thread(target=go, args=a) for a in zip(ps, both)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, both):
+        assert not isinstance(b[0], gpe.GpeError), b[0]
+        assert np.array_equal(a[0], b[0])

@@ -20,6 +20,7 @@ import gpe
 fake = ctypes.CDLL(%r)
 for f in ("live_bytes", "launches", "unordered", "lowered"):
     getattr(fake, "fake_" + f).restype = ctypes.c_longlong
+lengths = [n for n in range(8, 1025, 2) if 2 ** 10 * 3 ** 6 * 5 ** 4 %% n == 0]  # the sides a handle takes
 def params(mode, n, prec=0):
     return gpe.make_params(mode, *n, .25, .25, .25, .1 * .25 ** 2, .5, 1., 1.5, .125 * min(n), precision=prec)
 """
@@ -55,3 +56,42 @@ s.run(2, 50., 10.)
 assert fake.fake_launches() > 100
 assert fake.fake_unordered() == 0, fake.fake_unordered()
 """ % (mode, prec))
+
+
+def test_a_launch_takes_no_shared_memory_from_another_handle(fake):
+    """Handles of different sizes share kernels, and each may belong to a thread
+    of its own: a kernel's dynamic shared memory limit is never set below what
+    another handle was allowed, by steps, batch steps or operators."""
+    fake("""
+ok = [params(m, n, p) for n in ((8, 8, 1000), (8, 8, 64), (720, 8, 8), (40, 8, 8), (8, 1000, 8), (8, 540, 8))
+      for m in (0, 1) for p in (0, 1)]
+solvers = [gpe.Solver(p) for p in ok]
+for s in solvers + solvers[::-1]:
+    s.run(1, 50., 10.)
+    s.calcluz()
+for group in (ok[4:], ok[8:], ok[4:8]):
+    b = gpe.Batch(group, [50.] * len(group), [10.] * len(group))
+    b.run(1)
+    b.close()
+assert fake.fake_launches() > 100
+assert fake.fake_lowered() == 0, fake.fake_lowered()
+""")
+
+
+def test_tiles_near_the_default_shared_memory_limit(fake):
+    """A launch whose dynamic bytes fit 48 KB only without the kernel's static
+    ones (the batched y sweep of 144-point FP64 lines: 48512 and 944) is let
+    through as any other."""
+    fake("""
+for n in lengths:
+    for m in (0, 1):
+        for shape in ((n, 8, 8), (8, n, 8), (8, 8, n)):
+            for p in (0, 1) if shape[2] % 4 == 0 and not (m == 0 and shape[2] > 512) else (0,):
+                q = params(m, shape, p)
+                s = gpe.Solver(q)
+                s.run(1, 50., 10., rms_every=1)
+                s.close()
+                b = gpe.Batch([q], [50.], [10.])
+                b.run(1)
+                b.close()
+""")
