@@ -203,7 +203,8 @@ gpe_status gpe_snapshot_load(gpe_solver *s, const char *path, double *g, double 
 typedef struct gpe_batch gpe_batch;
 /* params[i] and couplings g[i], gd[i] of instance i (n >= 1).  Instances in
  * mixed-precision imaginary time start with 32-point segments in their y and z
- * sweeps (gpe_tuning.sweep_seg), the batched launches' faster choice; any
+ * sweeps (gpe_tuning.sweep_seg; z lines of more than 514 points keep
+ * gpe_create's choice), the batched launches' faster choice; any
  * instance's tiles can be changed with gpe_set_tuning on its handle. */
 gpe_status gpe_batch_create(const gpe_params *params, const double *g, const double *gd, int n, gpe_batch **out);
 void gpe_batch_destroy(gpe_batch *b);

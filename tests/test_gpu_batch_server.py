@@ -172,6 +172,27 @@ def test_batch_groups_and_new_couplings_bitwise(gpe_lib):
     b.close()
 
 
+@pytest.mark.parametrize("nz", [512, 540, 1024])
+def test_batch_of_long_z_lines(gpe_lib, nz):
+    """Mixed-precision imaginary time on z lines up to and beyond those the
+    batch's 16-row tiles of 32-point segments hold (514 points)."""
+    gpe = gpe_lib
+    ps = [params(gpe, 0, (8, 10, nz), prec=1), params(gpe, 0, (16, 8, 32), prec=1)]
+    b = gpe.Batch(ps, [20., 30.], [5., 2.])
+    for i in range(2):
+        b.solver(i).init_gaussian()
+        b.solver(i).calcnorm(True)
+    b.run(5)
+    for i, p in enumerate(ps):
+        with gpe.Solver(p) as s:
+            s.set_tuning(b.solver(i).get_tuning())
+            s.init_gaussian()
+            s.calcnorm(True)
+            s.run(5, [20., 30.][i], [5., 2.][i])
+            assert np.array_equal(s.get_psi(), b.solver(i).get_psi()), i
+    b.close()
+
+
 def test_batch_follows_a_retuned_instance(gpe_lib):
     """An instance re-planned through its own handle after the batch has
     stepped (gpe_set_tuning) makes the batch rebuild its descriptors and
