@@ -111,7 +111,7 @@ extern "C" gpe_status gpe_device_bytes(const gpe_params *p, long long *bytes) {
    const long long nzp = (p->precision == GPE_PREC_MIXED) ? (nzh + 1) & ~1LL : nzh;
    b += nzp * p->nx * p->ny * (long long) (2 * r);       // spectrum (rows padded to 16 bytes)
    b += npts * (long long) r;                            // phi
-   b += nzh * (p->nx / 2 + 1) * (p->ny / 2 + 1) * 8;     // Udd octant
+   b += udd_pitch((int) nzh) * (p->nx / 2 + 1) * (p->ny / 2 + 1) * 8;  // Udd octant
    b += 4 * std::max(p->nx * p->ny, std::max(p->nx * p->nz, p->ny * p->nz)) * 8;  // row sums
    b += 1 << 20;                                         // tables, state
    if (bytes) *bytes = b;

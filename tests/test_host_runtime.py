@@ -97,3 +97,20 @@ for n in lengths:
                 b.run(1)
                 b.close()
 """)
+
+
+def test_device_bytes_covers_a_handles_allocations(fake):
+    """gpe_device_bytes, by which the server admits, is at least what gpe_create
+    allocates, and at most 1.5 MB (its allowance for tables) and two planes of row
+    sums more."""
+    fake("""
+for n in ((1024, 1024, 8), (1024, 512, 12), (8, 8, 1024), (8, 1024, 8), (48, 40, 32), (90, 100, 72), (8, 8, 8)):
+    for m in (0, 1):
+        for p in (0, 1):
+            before = fake.fake_live_bytes()
+            s = gpe.Solver(params(m, n, p))
+            held, said = fake.fake_live_bytes() - before, gpe.device_bytes(s.params)
+            assert held <= said <= held + 1.5 * 2 ** 20 + 2 * 8 * max(n[0] * n[1], n[0] * n[2], n[1] * n[2]), (n, m, p, held, said)
+            s.close()
+            assert fake.fake_live_bytes() == before
+""")
