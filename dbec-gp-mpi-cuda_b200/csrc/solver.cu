@@ -128,6 +128,15 @@ template <class T> static gpe_status upload(const gpe_solver *s, void **dst, con
    return GPE_OK;
 }
 
+// The same into a table that a later plan fills again (at most `cap` bytes): it
+// is allocated once, by gpe_create, so that no plan after that can fail halfway
+// and leave a handle without tables.
+template <class T> static gpe_status replace(const gpe_solver *s, void **dst, const T *src, size_t n, size_t cap) {
+   if (!*dst) CK(cudaMalloc(dst, cap));
+   CK(cudaMemcpyAsync(*dst, src, sizeof(T) * n, cudaMemcpyHostToDevice, s->st));
+   return GPE_OK;
+}
+
 // Roots of unity of the stages of pl in the order fft_lines / conv_lines read
 // them: per stage after the first, exp(-2 pi i t k / (Ns r)) at [t - 1][k].
 static void stage_roots(const FftPlan &pl, std::vector<double2> &out) {
@@ -147,12 +156,10 @@ static void stage_roots(const FftPlan &pl, std::vector<double2> &out) {
 static gpe_status make_roots(gpe_solver *s) {
    const Dims &d = s->d;
    auto put = [&](const std::vector<double2> &t, void **dst) -> gpe_status {
-      if (*dst) cudaFree(*dst);
-      *dst = nullptr;
-      if (!s->fp32) return upload(s, dst, t.data(), t.size());
+      if (!s->fp32) return replace(s, dst, t.data(), t.size(), t.size() * sizeof(double2));
       std::vector<float2> f(t.size());
       for (size_t e = 0; e < t.size(); e++) f[e] = make_float2((float) t[e].x, (float) t[e].y);
-      return upload(s, dst, f.data(), f.size());
+      return replace(s, dst, f.data(), f.size(), f.size() * sizeof(float2));
    };
    std::vector<double2> t;
    stage_roots(s->px, t);
@@ -259,9 +266,8 @@ static gpe_status make_segtab(gpe_solver *s, int ax, long n, int m, int P) {
          }
       }
    if (ax == 0) std::memcpy(&blk[at + (size_t) skip * xe], s->nu_x.data(), s->nu_x.size());
-   if (w.tabs) cudaFree(w.tabs);
-   w.tabs = nullptr;
-   CKS(upload(s, &w.tabs, blk.data(), blk.size()));
+   // (skip < m <= 32)
+   CKS(replace(s, &w.tabs, blk.data(), blk.size(), sweep_tab_bytes((int) n, 31, (int) s->esz_psi, xe)));
    SegTab &t = w.tab;
    t.ga = w.tabs;
    t.ma = (unsigned char *) w.tabs + (size_t) ne * s->esz_psi;
@@ -342,7 +348,8 @@ static int sweep_candidates(int n, int tw_base, int esz, int *TW, int *MSEG, int
 // Tile configuration of the sweeps and of the y / x FFT passes, and the FFT
 // plans: the heuristics below, or the values of s->tune where set.  May be
 // called again (gpe_set_tuning); it uploads the segment tables, calcnu's x table
-// and the roots of unity anew, in the order of the handle's stream.
+// and the roots of unity anew, in the order of the handle's stream and without
+// an allocation.
 static gpe_status plan_tiles(gpe_solver *s) {
    s->plan_gen++;
    const Dims &d = s->d;

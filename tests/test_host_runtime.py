@@ -114,3 +114,21 @@ for n in ((1024, 1024, 8), (1024, 512, 12), (8, 8, 1024), (8, 1024, 8), (48, 40,
             s.close()
             assert fake.fake_live_bytes() == before
 """)
+
+
+@pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_planning_again_allocates_nothing(fake, mode, prec):
+    """gpe_set_tuning with no device memory left: the handle keeps its tables
+    (it lost them where an allocation of the new plan failed)."""
+    fake("""
+s = gpe.Solver(params(%d, (48, 40, 32), %d))
+held = fake.fake_live_bytes()
+fake.fake_fail_mallocs(1)
+for radix, seg in ((4, 8), (2, 0), (0, 0)):
+    t = gpe.Tuning()
+    t.fft_max_radix = radix
+    t.sweep_seg[0] = seg
+    s.set_tuning(t)
+    s.run(1, 50., 10.)
+assert fake.fake_live_bytes() == held
+""" % (mode, prec))
