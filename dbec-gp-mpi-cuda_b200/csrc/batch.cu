@@ -78,7 +78,8 @@ void refresh(gpe_batch *b) {
 }
 
 constexpr size_t kSmemCap = 227 * 1024;
-constexpr size_t kSweepStatic = 2048;  // views, tile records and barriers of a sweep kernel, rounded up
+constexpr size_t kSweepStatic = 1152;  // views, tile records and barriers of a sweep kernel, rounded up
+static_assert(2 * sizeof(SweepView) + 8 * sizeof(SweepTile) + 2 * sizeof(State) + 64 <= kSweepStatic, "static bytes of a sweep");
 
 // Descriptors of a group (host copy), in member order.
 gpe_status group_descs(gpe_batch *b, const Group &G, std::vector<BatchDesc> &h) {
@@ -154,7 +155,7 @@ gpe_status build_tables(gpe_batch *b) {
          // so more of fewer threads
          const int cap0 = kb_sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32));
          const int cap = std::max(1, std::min(32, 256 * cap0 / std::max(32, (int) A.threads[kPXsweep + a])));
-         const int ctas = std::max(1, std::min(cap, (int) (kSmemCap / sm)));
+         const int ctas = std::max(1, std::min(cap, smem_ctas(sm, kSweepStatic)));
          G.sweep_smem[a] = sm;
          G.sweep_grid[a] = (int) std::min<long long>(A.tiles[kPXsweep + a], (long long) ctas * b->nsm);
       }

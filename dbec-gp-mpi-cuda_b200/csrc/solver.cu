@@ -448,10 +448,23 @@ static gpe_status plan_tiles(gpe_solver *s) {
       // of fewer threads
       const int thr = (w.TW * P + 31) & ~31;
       const int ct_max = std::min(32, 256 * ctas_of(pick) / thr);
+      // a third stage only where it leaves the tables that are read through L1
+      // (all but the FP64 z sweep's) their room there: us with three -> two,
+      // FP32 complex x of 720 points 43 -> 37, FP64 complex y of 1024 points 74 ->
+      // 66 and of 512 points 30 -> 28, FP64 real x of 1024 points 80 -> 70
+      const size_t l1 = ax == 2 && !s->fp32 ? 0 : 4 * (size_t) P * w.MSEG * esz;
+      auto stages_fit = [&](int ct, int S) {
+         const size_t b = fixed + S * stage;
+         if (b + kSweepFixed > sm_cap || smem_ctas(b, kSweepFixed) < ct) return false;
+         return S == s_lo || ct * (b + kSweepFixed + kCtaReserved) + l1 <= kSmSmem;
+      };
       w.ctas = 0;
       for (int ct = ct_max; ct >= 1 && !w.ctas; ct--)
          for (int S = s_hi; S >= s_lo && !w.ctas; S--)
-            if ((fixed + S * stage) * ct <= sm_cap) { w.ctas = ct; w.S = S; }
+            if (stages_fit(ct, S)) {
+               w.ctas = ct;
+               w.S = S;
+            }
       if (!w.ctas) return fail(GPE_ERR_PARAM, "grid too large for the sweep tiles (shared memory)");
       w.smem = fixed + w.S * stage;
    }

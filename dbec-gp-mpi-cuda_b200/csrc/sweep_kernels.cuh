@@ -573,6 +573,16 @@ __host__ __device__ constexpr int sweep_ctas(bool fp32, bool cplx, int m) {
    return !cplx && m == 8 ? 3 : 2;
 }
 
+// CTAs of `bytes` of dynamic shared memory that an SM holds: each also takes the
+// kernel's static bytes (`fixed`: at most 128 for these kernels) and the 1 KB the
+// system reserves.  A persistent grid of more CTAs than that runs the surplus
+// after the others have finished: 16 complex FP64 64^3 solves in a batch, six
+// CTAs launched where five fit, x sweep 111 us, z 48; as many as fit 86 and 35.
+constexpr size_t kSmSmem = 228 * 1024, kCtaReserved = 1024, kSweepFixed = 128;
+inline int smem_ctas(size_t bytes, size_t fixed) {
+   return (int) (kSmSmem / ((bytes + fixed + kCtaReserved + 127) & ~(size_t) 127));
+}
+
 // Shared-memory layout of one pipeline stage of an x or y sweep tile: zero
 // rows below the tile, the tile, and with calcnu the same for phi.
 struct XyStage {

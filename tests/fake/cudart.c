@@ -10,6 +10,8 @@
  *                          its data has arrived)
  *   fake_lowered           cudaFuncSetAttribute calls that took dynamic shared
  *                          memory away from a kernel
+ *   fake_surplus           launches of a sweep, whose CTAs walk over the tiles,
+ *                          with more CTAs than the device holds at once
  *   fake_fail_mallocs(1)   lets every allocation fail
  */
 #include <stdint.h>
@@ -22,7 +24,7 @@ enum { OK = 0, INVALID = 1, OOM = 2 };
 typedef struct { unsigned x, y, z; } dim;
 typedef struct { int flags; } stream;
 
-static long long live, launches, unordered, lowered;
+static long long live, launches, unordered, lowered, surplus;
 static int failing, pending;
 static __thread err_t last;
 
@@ -30,13 +32,15 @@ long long fake_live_bytes(void) { return live; }
 long long fake_launches(void) { return launches; }
 long long fake_unordered(void) { return unordered; }
 long long fake_lowered(void) { return lowered; }
+long long fake_surplus(void) { return surplus; }
 void fake_fail_mallocs(int on) { failing = on; }
 
 /* ---- kernels: dynamic shared memory up to 48 KB less the static bytes unless
  * raised, to the opt-in maximum less them (static: a bound on what the batched
  * kernels, whose names start with kb_, and the others hold) */
 #define OPTIN_SMEM 232448
-static struct { const void *f; int dyn, fixed; } attr[1 << 16];
+#define SM_SMEM (228 * 1024)
+static struct { const void *f; int dyn, fixed, sweep; } attr[1 << 16];
 static unsigned at(const void *f) {
    unsigned h = (unsigned) (((uintptr_t) f >> 4) * 2654435761u) & 0xffff;
    while (attr[h].f && attr[h].f != f) h = (h + 1) & 0xffff;
@@ -54,6 +58,7 @@ void __cudaRegisterFunction(void **h, const char *f, char *d, const char *n, int
    attr[k].f = f;
    attr[k].fixed = strstr(n, "kb_") ? 1152 : 128;
    attr[k].dyn = 48 * 1024 - attr[k].fixed;
+   attr[k].sweep = strstr(n, "k_sweep") || strstr(n, "kb_sweep");
 }
 err_t cudaFuncSetAttribute(const void *f, int a, int v) {
    const unsigned k = at(f);
@@ -70,6 +75,7 @@ err_t cudaFuncGetAttributes(void *out, const void *f) { /* sharedSizeBytes comes
 static err_t launch(const void *f, dim g, dim b, size_t smem, stream *s) {
    if (!g.x || !g.y || !g.z || !b.x || b.x * b.y * b.z > 1024 || smem > (size_t) attr[at(f)].dyn) return last = INVALID;
    if (pending && s && (s->flags & 1)) unordered++;
+   if (attr[at(f)].sweep && g.x > 148 * (SM_SMEM / (smem + (size_t) attr[at(f)].fixed + 1024))) surplus++;
    launches++;
    return OK;
 }

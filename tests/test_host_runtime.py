@@ -18,7 +18,7 @@ import ctypes, sys
 sys.path.insert(0, %r)
 import gpe
 fake = ctypes.CDLL(%r)
-for f in ("live_bytes", "launches", "unordered", "lowered"):
+for f in ("live_bytes", "launches", "unordered", "lowered", "surplus"):
     getattr(fake, "fake_" + f).restype = ctypes.c_longlong
 lengths = [n for n in range(8, 1025, 2) if 2 ** 10 * 3 ** 6 * 5 ** 4 %% n == 0]  # the sides a handle takes
 def params(mode, n, prec=0):
@@ -132,3 +132,22 @@ for radix, seg in ((4, 8), (2, 0), (0, 0)):
     s.run(1, 50., 10.)
 assert fake.fake_live_bytes() == held
 """ % (mode, prec))
+
+
+@pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_sweeps_launch_no_more_ctas_than_fit(fake, mode, prec):
+    """A sweep's CTAs walk over the tiles: more of them than the SMs hold (shared
+    memory, static bytes and the system's 1 KB included) would run a second
+    wave behind the first."""
+    fake("""
+for n in (30, 60, 64, 72, 80, 96, 120, 128, 144, 180, 256, 320, 400, 500, 512, 540, 640, 750):
+    for shape in ((n, 64, 64), (64, n, 64), (64, 64, n)):
+        if %(p)d and shape[2] %% 4:
+            continue
+        q = params(%(m)d, shape, %(p)d)
+        b = gpe.Batch([q] * 4, [50.] * 4, [10.] * 4)
+        b.solver(0).run(1, 50., 10.)
+        b.run(1)
+        b.close()
+        assert fake.fake_surplus() == 0, shape
+""" % dict(m=mode, p=prec))
