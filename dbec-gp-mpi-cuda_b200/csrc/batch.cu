@@ -153,7 +153,7 @@ gpe_status build_tables(gpe_batch *b) {
          if (sm > kSmemCap - kSweepStatic) return bfail(GPE_ERR_PARAM, "batch: sweep tiles exceed shared memory");
          // the kernels' register budget holds cap0 CTAs of 256 threads,
          // so more of fewer threads
-         const int cap0 = kb_sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32));
+         const int cap0 = kb_sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32), a == 0);
          const int cap = std::max(1, std::min(32, 256 * cap0 / std::max(32, (int) A.threads[kPXsweep + a])));
          const int ctas = std::max(1, std::min(cap, smem_ctas(sm, kSweepStatic)));
          G.sweep_smem[a] = sm;

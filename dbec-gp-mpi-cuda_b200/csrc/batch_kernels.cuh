@@ -147,9 +147,14 @@ __device__ __forceinline__ void stage_plan(FftPlan &dst, const FftPlan &src) {
 // Resident CTAs of 256 threads per SM (register budgets): 128 registers for
 // the FP64 FFT passes, whose compile-time transforms hold 16 points per
 // thread, 64 for FP32; the sweeps as sweep_ctas, with 80 for the FP32 ones of
-// up to 16-point segments, which hold the code of two segment lengths.
+// up to 16-point segments, which hold the code of two segment lengths, and one
+// CTA fewer for FP32 x sweeps in real time (`nu`), whose calcnu takes the whole
+// view's constants into registers: at 64 registers it spilled 244 bytes a thread
+// (batches of 160x144x120, 80^3, 48^3: 231, 162, 61 us; at 80 registers 138, 117,
+// 48).
 template <class R> constexpr int kb_fft_ctas() { return sizeof(R) == 8 ? 2 : 4; }
-__host__ __device__ constexpr int kb_sweep_ctas(bool fp32, bool cplx, int m) {
+__host__ __device__ constexpr int kb_sweep_ctas(bool fp32, bool cplx, int m, bool nu) {
+   if (fp32 && cplx && nu) return m == 16 ? 2 : 3;
    return fp32 && m == 16 ? 3 : sweep_ctas(fp32, cplx, m);
 }
 
@@ -286,7 +291,7 @@ template <class R, bool CPLX> struct BatchTabs {
 };
 
 template <class R, bool CPLX, int AXIS, bool NU, int MSEG, int S>
-__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_xy(
+__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG, NU)) kb_sweep_xy(
     const BatchDesc *__restrict__ tab, const SweepTile *__restrict__ tiles, int ntiles, uint32_t stage_bytes,
     uint32_t xch_bytes, uint32_t tab_bytes, int nbuf) {
    using P = typename Tr<R, CPLX>::P;
@@ -409,7 +414,7 @@ __global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)
 }
 
 template <class R, bool CPLX, int MOM, int MSEG, int S>
-__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG)) kb_sweep_z(
+__global__ void __launch_bounds__(256, kb_sweep_ctas(sizeof(R) == 4, CPLX, MSEG, false)) kb_sweep_z(
     const BatchDesc *__restrict__ tab, const SweepTile *__restrict__ tiles, int ntiles, uint32_t stage_bytes,
     uint32_t xch_bytes, uint32_t tab_bytes, int nbuf, uint32_t part_bytes) {
    using P = typename Tr<R, CPLX>::P;
