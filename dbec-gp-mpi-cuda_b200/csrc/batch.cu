@@ -131,8 +131,9 @@ gpe_status build_tables(gpe_batch *b) {
             A.tiles[q] += g.tiles[q];
             A.threads[q] = std::max(A.threads[q], g.threads[q]);
             A.smem[q] = std::max(A.smem[q], g.smem[q]);
+            A.lens[q] = A.lens[q] || g.lens[q];
+            A.pts[q] = std::max(A.pts[q], g.pts[q]);
          }
-         A.zppt = std::max(A.zppt, g.zppt);
          for (int a = 0; a < 3; a++) {
             A.mseg[a] = std::max(A.mseg[a], g.mseg[a]);
             A.stage[a] = std::max(A.stage[a], g.stage[a]);
@@ -140,6 +141,11 @@ gpe_status build_tables(gpe_batch *b) {
             A.tabs[a] = std::max(A.tabs[a], g.tabs[a]);
          }
          A.part = std::max(A.part, g.part);
+      }
+      for (int q : {kPZfwd, kPYfft, kPXconv, kPYinv, kPZinv}) {
+         A.ppt[q] = G.fp32 ? batch_ppt<float>(A.lens[q], A.pts[q]) : batch_ppt<double>(A.lens[q], A.pts[q]);
+         const long t = (A.pts[q] + A.ppt[q] - 1) / A.ppt[q];
+         A.threads[q] = std::max(A.threads[q], (unsigned) std::min<long>(256, std::max<long>(32, (t + 31) / 32 * 32)));
       }
       for (long long t : A.tiles)
          if (t > (1LL << 31) - 1) return bfail(GPE_ERR_PARAM, "batch: too many tiles in one pass");

@@ -103,9 +103,11 @@ template <class R, bool CPLX> __host__ __device__ constexpr int nu_tab_esz() {
 // instance's own lines per CTA and segments, 2-stage pipelines).
 struct BatchGeom {
    long long tiles[kNPass];  // CTAs (FFT passes, norm, planes) or tiles (sweeps)
-   unsigned threads[kNPass];
+   unsigned threads[kNPass]; // (0: an FFT pass of run-time length, whose group decides)
+   long pts[kNPass];         // FFT passes: points of a tile of run-time length, else 0
    size_t smem[kNPass];      // dynamic shared memory of one CTA (FFT passes)
-   int zppt;                 // points per thread of the z passes
+   bool lens[kNPass];        // FFT passes: a compile-time length
+   int ppt[kNPass];          // FFT passes (group): points per thread at run-time lengths
    int mseg[3];              // compile-time segment bound of each sweep
    uint32_t stage[3];        // sweeps: bytes of one pipeline stage
    uint32_t xch[3];          // sweeps: bytes of the exchange buffer
@@ -145,14 +147,14 @@ __device__ __forceinline__ void stage_plan(FftPlan &dst, const FftPlan &src) {
 }
 
 // Resident CTAs of 256 threads per SM (register budgets): 128 registers for
-// the FP64 FFT passes, whose compile-time transforms hold 16 points per
-// thread, 64 for FP32; the sweeps as sweep_ctas, with 80 for the FP32 ones of
+// the FP64 FFT passes with compile-time transforms, which hold 16 points per
+// thread, 64 for the others; the sweeps as sweep_ctas, with 80 for the FP32 ones of
 // up to 16-point segments, which hold the code of two segment lengths, and one
 // CTA fewer for FP32 x sweeps in real time (`nu`), whose calcnu takes the whole
 // view's constants into registers: at 64 registers it spilled 244 bytes a thread
 // (batches of 160x144x120, 80^3, 48^3: 231, 162, 61 us; at 80 registers 138, 117,
 // 48).
-template <class R> constexpr int kb_fft_ctas() { return sizeof(R) == 8 ? 2 : 4; }
+template <class R, bool LENS> constexpr int kb_fft_ctas() { return sizeof(R) == 8 && LENS ? 2 : 4; }
 __host__ __device__ constexpr int kb_sweep_ctas(bool fp32, bool cplx, int m, bool nu) {
    if (fp32 && cplx && nu) return m == 16 ? 2 : 3;
    return fp32 && m == 16 ? 3 : sweep_ctas(fp32, cplx, m);
@@ -160,9 +162,25 @@ __host__ __device__ constexpr int kb_sweep_ctas(bool fp32, bool cplx, int m, boo
 
 // ---------------------------------------------------------------- FFT passes
 // One CTA per tile; tile numbering of each instance as its single-solve grid.
+// LENS: some instance of the group has a compile-time length in this pass.  A
+// group without one runs kernels that hold the run-time pass alone, on half the
+// registers in FP64 (us of the FFT passes of a step: FP64 imaginary time, 16 grids
+// of 72^3 355 -> 246, 24 of 40^3 124 -> 100; FP32 real time, 6 of 160x144x120 407
+// -> 357).
+// PPT: points per thread at run-time lengths.  Beside compile-time transforms,
+// whose registers they then have, FP64 tiles of more than a warp's 256 points take
+// 16 (us, 8 -> 16: y pass of 80^3 78 -> 63, x pass of 72^3 102 -> 86; tiles of one
+// warp are slower with 16, z pass of 100x90x60 56 -> 63); FP32 always does.
+template <class R> constexpr int batch_ppt(bool lens, long pts) {
+   return sizeof(R) == 4 || pts > (lens ? 256 : 2048) ? 16 : 8;
+}
+template <bool LENS, class F> __device__ __forceinline__ void batch_len(int n, F f) {
+   if constexpr (LENS) with_len(n, f);
+   else f(std::integral_constant<int, 0>());
+}
 
-template <class R, bool CPLX, int PPT, int L>
-__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_zfwd(const BatchDesc *__restrict__ tab,
+template <class R, bool CPLX, int PPT, int L, bool LENS>
+__global__ void __launch_bounds__(256, kb_fft_ctas<R, LENS>()) kb_zfwd(const BatchDesc *__restrict__ tab,
                                                                 const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
@@ -170,7 +188,7 @@ __global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_zfwd(const BatchDesc
    __shared__ FftPlan pl;
    const Dims d = D.d;
    const long long r0 = (long long) r.local * L;
-   with_len(D.fastz ? d.nz / 2 : 0, [&](auto nc) {
+   batch_len<LENS>(D.fastz ? d.nz / 2 : 0, [&](auto nc) {
       constexpr int H = decltype(nc)::value;
       if constexpr (H > 0 && H <= kLenMaxH && L == kLenRows) {
          zfwd_body_n<R, CPLX, L, H>((const P *) D.psi, (cpx<R> *) D.spec, d, (const cpx<R> *) D.twz, D.err, r0);
@@ -181,15 +199,15 @@ __global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_zfwd(const BatchDesc
    });
 }
 
-template <class R, bool INV, int L>
-__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_yfft(const BatchDesc *__restrict__ tab,
+template <class R, bool INV, int PPT, int L, bool LENS>
+__global__ void __launch_bounds__(256, kb_fft_ctas<R, LENS>()) kb_yfft(const BatchDesc *__restrict__ tab,
                                                   const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
    __shared__ FftPlan pl;
    if (threadIdx.x == 0) tmap_acquire(&D.tm_spec_y);
    const Dims d = D.d;
-   with_len(D.fasty ? d.ny : 0, [&](auto nc) {
+   batch_len<LENS>(D.fasty ? d.ny : 0, [&](auto nc) {
       constexpr int N = decltype(nc)::value, LT = N > 0 ? LenCols<R>::L : L;
       const int nkb = (d.nzh + LT - 1) / LT;
       const int x = r.local / nkb, k0 = (r.local - x * nkb) * LT;
@@ -197,20 +215,20 @@ __global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_yfft(const BatchDesc
          yfft_body_n<R, INV, LT, N>(&D.tm_spec_y, (const cpx<R> *) D.twy, D.err, x, k0);
       } else {
          stage_plan(pl, D.py);
-         yfft_body<R, INV, L>(&D.tm_spec_y, d, pl, (const cpx<R> *) D.twy, D.boxy, D.nboxy, D.err, x, k0);
+         yfft_body<R, INV, L, PPT>(&D.tm_spec_y, d, pl, (const cpx<R> *) D.twy, D.boxy, D.nboxy, D.err, x, k0);
       }
    });
 }
 
-template <class R, int L>
-__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_xconv(const BatchDesc *__restrict__ tab,
+template <class R, int PPT, int L, bool LENS>
+__global__ void __launch_bounds__(256, kb_fft_ctas<R, LENS>()) kb_xconv(const BatchDesc *__restrict__ tab,
                                                    const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
    __shared__ FftPlan pl, pli;
    if (threadIdx.x == 0) tmap_acquire(&D.tm_spec_x);
    const Dims d = D.d;
-   with_len(D.fastx ? d.nx : 0, [&](auto nc) {
+   batch_len<LENS>(D.fastx ? d.nx : 0, [&](auto nc) {
       constexpr int N = decltype(nc)::value, LT = N > 0 ? LenCols<R>::L : L;
       const int nkb = (d.nzh + LT - 1) / LT;
       const int y = r.local / nkb, k0 = (r.local - y * nkb) * LT;
@@ -219,21 +237,21 @@ __global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_xconv(const BatchDes
       } else {
          stage_plan(pl, D.px);
          stage_plan(pli, D.pxi);
-         xconv_body<R, L>(&D.tm_spec_x, nullptr, D.udd, d, pl, pli, (const cpx<R> *) D.twx, D.state, D.boxx,
+         xconv_body<R, L, PPT>(&D.tm_spec_x, nullptr, D.udd, d, pl, pli, (const cpx<R> *) D.twx, D.state, D.boxx,
                           D.nboxx, D.err, y, k0);
       }
    });
 }
 
-template <class R, int PPT, int L, bool FOLD>
-__global__ void __launch_bounds__(256, kb_fft_ctas<R>()) kb_zinv(const BatchDesc *__restrict__ tab,
+template <class R, int PPT, int L, bool FOLD, bool LENS>
+__global__ void __launch_bounds__(256, kb_fft_ctas<R, LENS>()) kb_zinv(const BatchDesc *__restrict__ tab,
                                                                 const unsigned *__restrict__ work) {
    const TileRef r = tile_ref(work, blockIdx.x);
    const BatchDesc &D = tab[r.inst];
    __shared__ FftPlan pl;
    const Dims d = D.d;
    const long long r0 = (long long) r.local * L;
-   with_len(D.fastz ? d.nz / 2 : 0, [&](auto nc) {
+   batch_len<LENS>(D.fastz ? d.nz / 2 : 0, [&](auto nc) {
       constexpr int H = decltype(nc)::value;
       if constexpr (H > 0 && H <= kLenMaxH && L == kLenRows) {
          zinv_body_n<R, L, H, FOLD>((const cpx<R> *) D.spec, (R *) D.phi, d, (const cpx<R> *) D.twz, D.err, r0);

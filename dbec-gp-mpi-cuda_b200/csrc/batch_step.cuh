@@ -18,10 +18,14 @@ template <class R> struct BatchConv {
    // (batch of 64: a pass of 13 us less); an FP64 batch step keeps its
    // documented launch per pass
    static constexpr bool kFold = std::is_same<R, float>::value;
-   template <class F> static gpe_status with_ppt(int ppt, F f) {
-      if (ppt <= 8) return f(std::integral_constant<int, 8>());
-      if (ppt <= 16) return f(std::integral_constant<int, 16>());
-      return f(std::integral_constant<int, 32>());
+   // runs f(lens, points per thread) as compile-time constants
+   template <class F> static gpe_status with_fft(const BatchGeom &A, int q, F f) {
+      auto go = [&](auto lens) -> gpe_status {
+         if constexpr (std::is_same<R, double>::value)
+            if (A.ppt[q] == 8) return f(lens, std::integral_constant<int, 8>());
+         return f(lens, std::integral_constant<int, 16>());
+      };
+      return A.lens[q] ? go(std::true_type()) : go(std::false_type());
    }
    template <class F> static gpe_status with_L(int L, F f) {
       if (L >= 16) return f(std::integral_constant<int, 16>());
@@ -43,23 +47,29 @@ template <class R> gpe_status BatchConv<R>::run(const Group &G, cudaStream_t st,
       return GPE_OK;
    };
    BCKS(with_L(G.Ly, [&](auto lc) {
-      constexpr int L = decltype(lc)::value;
-      return launch(G, kb_yfft<R, false, L>, T(kPYfft), A.threads[kPYfft], A.smem[kPYfft], st, tab, S(kPYfft));
+      return with_fft(A, kPYfft, [&](auto nc, auto pc) {
+         return launch(G, kb_yfft<R, false, decltype(pc)::value, decltype(lc)::value, decltype(nc)::value>, T(kPYfft), A.threads[kPYfft],
+                       A.smem[kPYfft], st, tab, S(kPYfft));
+      });
    }));
    BCKS(mark(kPYfft));
    BCKS(with_L(G.Lx, [&](auto lc) {
-      constexpr int L = decltype(lc)::value;
-      return launch(G, kb_xconv<R, L>, T(kPXconv), A.threads[kPXconv], A.smem[kPXconv], st, tab, S(kPXconv));
+      return with_fft(A, kPXconv, [&](auto nc, auto pc) {
+         return launch(G, kb_xconv<R, decltype(pc)::value, decltype(lc)::value, decltype(nc)::value>, T(kPXconv), A.threads[kPXconv],
+                       A.smem[kPXconv], st, tab, S(kPXconv));
+      });
    }));
    BCKS(mark(kPXconv));
    BCKS(with_L(G.Ly, [&](auto lc) {
-      constexpr int L = decltype(lc)::value;
-      return launch(G, kb_yfft<R, true, L>, T(kPYinv), A.threads[kPYinv], A.smem[kPYinv], st, tab, S(kPYinv));
+      return with_fft(A, kPYinv, [&](auto nc, auto pc) {
+         return launch(G, kb_yfft<R, true, decltype(pc)::value, decltype(lc)::value, decltype(nc)::value>, T(kPYinv), A.threads[kPYinv],
+                       A.smem[kPYinv], st, tab, S(kPYinv));
+      });
    }));
    BCKS(mark(kPYinv));
-   BCKS(with_ppt(A.zppt, [&](auto pc) {
-      constexpr int PPT = decltype(pc)::value;
-      return launch(G, kb_zinv<R, PPT, ZL, kFold>, T(kPZinv), A.threads[kPZinv], A.smem[kPZinv], st, tab, S(kPZinv));
+   BCKS(with_fft(A, kPZinv, [&](auto nc, auto pc) {
+      return launch(G, kb_zinv<R, decltype(pc)::value, ZL, kFold, decltype(nc)::value>, T(kPZinv), A.threads[kPZinv],
+                    A.smem[kPZinv], st, tab, S(kPZinv));
    }));
    BCKS(mark(kPZinv));
    if (!kFold) BCKS(launch(G, kb_phifix<R>, T(kPPhifix), A.threads[kPPhifix], 0, st, tab, S(kPPhifix)));
@@ -89,9 +99,9 @@ template <class R, bool CPLX> struct BatchStep {
          if (ev) BCK(cudaEventRecord(ev[q], st));
          return GPE_OK;
       };
-      BCKS(BatchConv<R>::with_ppt(A.zppt, [&](auto pc) {
-         constexpr int PPT = decltype(pc)::value;
-         return launch(G, kb_zfwd<R, CPLX, PPT, ZL>, T(kPZfwd), A.threads[kPZfwd], A.smem[kPZfwd], st, tab, S(kPZfwd));
+      BCKS(BatchConv<R>::with_fft(A, kPZfwd, [&](auto nc, auto pc) {
+         return launch(G, kb_zfwd<R, CPLX, decltype(pc)::value, ZL, decltype(nc)::value>, T(kPZfwd), A.threads[kPZfwd],
+                       A.smem[kPZfwd], st, tab, S(kPZfwd));
       }));
       BCKS(mark(kPZfwd));
       BCKS(BatchConv<R>::run(G, st, ev));

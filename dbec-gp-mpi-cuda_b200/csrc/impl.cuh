@@ -481,14 +481,16 @@ template <class R, bool CPLX> struct Impl {
       g->Ly = s->Ly;
       g->Lx = s->Lx;
       if (Ly <= 0 || Lx <= 0) return GPE_OK;
-      // z passes: 8-row tiles on CTAs sized to them
+      // z passes: 8-row tiles
       constexpr int L = 8;
-      const int zp = CV::zppt(s, L);
-      const int ppt = zp <= 8 ? 8 : (zp <= 16 ? 16 : 32);
-      g->zppt = ppt;
-      g->tiles[kPZfwd] = g->tiles[kPZinv] = (d.nxy + L - 1) / L;
-      g->threads[kPZfwd] = g->threads[kPZinv] =
-          CV::len_z(s) ? (unsigned) len_threads<R>(d.nz / 2, L) : CV::z_threads(s, L, ppt);
+      auto fft = [&](int q, long long tiles, bool len, long pts, int lt) {
+         g->tiles[q] = tiles;
+         g->lens[q] = len;
+         g->pts[q] = len ? 0 : pts;
+         g->threads[q] = len ? (unsigned) lt : 0u;
+      };
+      for (int q : {kPZfwd, kPZinv})
+         fft(q, (d.nxy + L - 1) / L, CV::len_z(s), (long) (d.nz / 2) * L, len_threads<R>(d.nz / 2, L));
       // y / x passes
       const long ry = (long) s->boxy * s->nboxy, rx = (long) s->boxx * s->nboxx;
       g->smem[kPZfwd] = CV::len_z(s) ? zfwd_n_smem(s) : zfwd_smem(s, L);
@@ -500,10 +502,9 @@ template <class R, bool CPLX> struct Impl {
       Lx = CV::len_x(s) ? CV::kCols : Lx;
       if (ry * Ly > 256L * FftL<R>::PPT || rx * Lx > 256L * FftL<R>::PPT)
          return fail(GPE_ERR_PARAM, "batch: FFT tile too wide for this grid");
-      g->tiles[kPYfft] = g->tiles[kPYinv] = (long long) d.nx * ((d.nzh + Ly - 1) / Ly);
-      g->tiles[kPXconv] = (long long) d.ny * ((d.nzh + Lx - 1) / Lx);
-      g->threads[kPYfft] = g->threads[kPYinv] = CV::len_y(s) ? (unsigned) len_threads<R>(d.ny, Ly) : CV::fft_threads(ry, Ly);
-      g->threads[kPXconv] = CV::len_x(s) ? (unsigned) len_threads<R>(d.nx, Lx) : CV::fft_threads(rx, Lx);
+      for (int q : {kPYfft, kPYinv})
+         fft(q, (long long) d.nx * ((d.nzh + Ly - 1) / Ly), CV::len_y(s), ry * Ly, len_threads<R>(d.ny, Ly));
+      fft(kPXconv, (long long) d.ny * ((d.nzh + Lx - 1) / Lx), CV::len_x(s), rx * Lx, len_threads<R>(d.nx, Lx));
       g->smem[kPYfft] = g->smem[kPYinv] = CV::yfft_smem(s, Ly, (int) ry);
       g->smem[kPXconv] = CV::xconv_smem(s, Lx, (int) rx);
       // boundary planes of phi

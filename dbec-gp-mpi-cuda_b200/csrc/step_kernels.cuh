@@ -234,12 +234,11 @@ __global__ void __launch_bounds__(256, L >= 16 ? 3 : 4) k_zfwd(const typename Tr
 // the CTA at one thread per PPT points of the tile (128 threads for the
 // 4-column FP64 tiles, so that eight fit on an SM); the register budget
 // (launch bounds 256 x 4) allows any of these sizes.
-template <class R, bool INV, int L>
+template <class R, bool INV, int L, int PPT = FftL<R>::PPT>
 __device__ __forceinline__ void yfft_body(const CUtensorMap *tm, const Dims &d, const FftPlan &py,
                                           const cpx<R> *__restrict__ twy, int boxn, int nbox, uint32_t *err, int x,
                                           int k0) {
    using C = cpx<R>;
-   constexpr int PPT = FftL<R>::PPT;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
    const int ny = d.ny, rows = boxn * nbox;
@@ -293,13 +292,12 @@ __device__ __forceinline__ void udd_copy(double *ud, const double *udd, const Di
 // Pass 3: FFT along x, multiply by Udd(k) * scale^2, inverse FFT along x, for
 // L kz columns of one y plane.  Udd octant layout [|kx|][|ky|][kz].  CTA size
 // as for the y passes.
-template <class R, int L>
+template <class R, int L, int PPT = FftL<R>::PPT>
 __device__ __forceinline__ void xconv_body(const CUtensorMap *tm, const CUtensorMap *tm_udd, const double *udd, const Dims &d,
                                            const FftPlan &px, const FftPlan &pxi, const cpx<R> *__restrict__ twx,
                                            const State *__restrict__ st, int boxn, int nbox, uint32_t *err, int y,
                                            int k0) {
    using C = cpx<R>;
-   constexpr int PPT = FftL<R>::PPT;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    __shared__ __align__(8) uint64_t bar;
    const int nx = d.nx, ny = d.ny, rows = boxn * nbox;

@@ -155,3 +155,40 @@ def test_convolution_compiled_lengths(gpe_lib, oracle_mod, prec, axis, n):
     assert rel(phi, s.get_phi()) <= TOL[prec]
     s.close()
     o.close()
+
+
+# A batch runs its own kernels on every length: the common ones compiled, the
+# others at run time, on registers and points per thread that depend on which of
+# the two its other members have.  Each instance is its solo run bit for bit.
+@pytest.mark.parametrize("mode,prec", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("others", [(), ((64, 64, 64),), ((128, 48, 96), (24, 256, 32))])
+def test_batch_lengths_bitwise(gpe_lib, mode, prec, others):
+    gpe = gpe_lib
+    shapes = list(others)
+    for axis, lengths in enumerate((XY_LENGTHS + (270, 432, 640), XY_LENGTHS + (270, 486, 720),
+                                    tuple(2 * h for h in Z_HALVES) + (432, 640))):
+        for n in lengths:
+            shape = [10, 12, 8]
+            shape[axis] = n
+            if not (prec and shape[2] % 4):
+                shapes.append(tuple(shape))
+    dx = 0.25
+    ps = [gpe.make_params(mode, *n, dx, 1.1 * dx, 0.9 * dx, 0.1 * dx * dx, 0.5, 1.0, 1.5, 0.5 * min(n) * dx, precision=prec)
+          for n in shapes]
+    r = np.random.default_rng(7)
+    psi = [r.standard_normal(n) * (0.3 + (0.2j if mode else 0.)) for n in shapes]
+    g = [float(v) for v in r.uniform(1., 20., len(ps))]
+    b = gpe.Batch(ps, g, [0.2 * v for v in g])
+    for i, f in enumerate(psi):
+        b.solver(i).set_psi(f)
+    b.run(2)
+    bad = []
+    for i, p in enumerate(ps):
+        with gpe.Solver(p) as s:
+            s.set_tuning(b.solver(i).get_tuning())
+            s.set_psi(psi[i])
+            s.run(2, g[i], 0.2 * g[i])
+            if not np.array_equal(s.get_psi(), b.solver(i).get_psi()):
+                bad.append(shapes[i])
+    b.close()
+    assert not bad, bad
