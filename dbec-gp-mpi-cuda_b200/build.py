@@ -34,7 +34,7 @@ LIB_SOURCES = ["conv_f64_zf_lens.cu", "conv_f32_zf_lens.cu", "conv_f64_y_lens.cu
                "batch_f64i.cu", "batch_f64r.cu", "batch_f32i.cu", "batch_f32r.cu", "solver.cu", "noalloc.cu", "batch.cu",
                "server.cpp"]
 LIB_DEPS = LIB_SOURCES + ["common.cuh", "fft.cuh", "fftn.cuh", "kernels.cuh", "step_kernels.cuh", "sweep_kernels.cuh", "tma.cuh",
-                          "batch_kernels.cuh", "batch_group.h", "batch_step.cuh", "impl.cuh", "solver.cuh",
+                          "batch_kernels.cuh", "batch_group.h", "batch_step.cuh", "conv_lens.cuh", "impl.cuh", "solver.cuh",
                           "internal.h"]
 OBJ_DIR = os.path.join(PKG, "_build")
 HOST_COMMON = ["cfg.cpp", "cli.cpp"]

@@ -28,8 +28,9 @@ template <class R> struct BatchConv {
       return A.lens[q] ? go(std::true_type()) : go(std::false_type());
    }
    template <class F> static gpe_status with_L(int L, F f) {
-      if (L >= 16) return f(std::integral_constant<int, 16>());
-      if (L == 8) return f(std::integral_constant<int, 8>());
+      if constexpr (std::is_same<R, float>::value)  // a tile row is 128 bytes at most
+         if (L >= 16) return f(std::integral_constant<int, 16>());
+      if (L >= 8) return f(std::integral_constant<int, 8>());
       if (L == 4) return f(std::integral_constant<int, 4>());
       return f(std::integral_constant<int, 2>());
    }
@@ -84,7 +85,8 @@ template <class R, bool CPLX> struct BatchStep {
    template <class F> static gpe_status with_mseg(int m, F f) {
       if constexpr (std::is_same<R, float>::value && !CPLX)
          if (m > 16) return f(std::integral_constant<int, 32>());
-      if (m > 8) return f(std::integral_constant<int, 16>());
+      if constexpr (!(std::is_same<R, double>::value && CPLX))  // 16-byte elements: 8-point segments
+         if (m > 8) return f(std::integral_constant<int, 16>());
       return f(std::integral_constant<int, 8>());
    }
 

@@ -4,11 +4,11 @@
 // transform, not cuFFT's).
 //
 // A CTA transforms L lines of length n held in shared memory in the
-// interleaved layout [j][L]: element j of line l at base[j * L + l].  L is
-// 128 bytes of elements (8 complex doubles, 16 complex floats), so the L
-// threads that handle one butterfly position of the L lines touch one
-// 128-byte row: bank-conflict free.  This is also the layout a TMA box of L
-// columns by the whole line lands in.
+// interleaved layout [j][L]: element j of line l at base[j * L + l], so the L
+// threads that handle one butterfly position of the L lines touch consecutive
+// elements (L: 2 to 16 kz columns of a y or x tile, 64 bytes of them by default,
+// at most 128; 8 rows, or 16, of a z tile).  This is also the layout a TMA box of
+// L columns by the whole line lands in.
 //
 // Radices 2, 3, 4, 5, 8 and (FP32, 16 points per thread) 16.  Each radix-r
 // stage (autosort Stockham, decimation in time) computes

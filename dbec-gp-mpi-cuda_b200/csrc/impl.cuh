@@ -41,7 +41,7 @@ gpe_status launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, cons
    return GPE_OK;
 }
 
-// The passes on the lengths compiled for one solve only (conv_*_lens.cu).
+// The passes on the lengths compiled for one solve only (conv_lens.cuh).
 template <class R> gpe_status yfft_lens(gpe_solver *s, bool inv, unsigned grid, size_t sm);
 template <class R> gpe_status xconv_lens(gpe_solver *s, unsigned grid, size_t sm);
 template <class R> gpe_status zinv_lens(gpe_solver *s, size_t sm);
@@ -55,7 +55,8 @@ template <class R> struct Conv {
    // runs f(std::integral_constant<int, v>) for v in {2, 4, 8, 16} (tile
    // widths) or {8, 16, 32} (points per thread)
    template <class F> static gpe_status with_L(int L, F f) {
-      if (L == 16) return f(std::integral_constant<int, 16>());
+      if constexpr (std::is_same<R, float>::value)  // a tile row is 128 bytes at most
+         if (L == 16) return f(std::integral_constant<int, 16>());
       if (L == 8) return f(std::integral_constant<int, 8>());
       if (L == 4) return f(std::integral_constant<int, 4>());
       return f(std::integral_constant<int, 2>());
@@ -277,7 +278,7 @@ template <class R, bool CPLX> struct Impl {
          // shorter than 128 points, which keep 16 rows on 256 threads (sized
          // CTAs of 32 threads measured slower at 64^3: 8.8 -> 10.8 us)
          const bool sized = !CPLX && (sizeof(R) == 4 || d.nz >= 128);
-         const int L = CV::zrows(s, (!CPLX && !sized) ? 16 : ZRows<R, CPLX>::fwd, zfwd_smem);
+         const int L = CV::zrows(s, (!CPLX && !sized) ? 16 : zfwd_rows<R, CPLX>(), zfwd_smem);
          const size_t sm = zfwd_smem(s, L);
          CKS(CV::with_zrows(L, [&](auto lc) { return zfwd_L<decltype(lc)::value>(s, sm, sized); }));
       }
@@ -305,21 +306,26 @@ template <class R, bool CPLX> struct Impl {
    template <int AXIS, bool NU, int MSEG, int S> static gpe_status sweep_xy_launch(gpe_solver *s, double g, double gd) {
       if constexpr (std::is_same<R, double>::value) {
          if (s->sw[AXIS].TW == 8) return sweep_xy_launch_t<AXIS, NU, MSEG, S, 8>(s, g, gd);
-         if (s->sw[AXIS].TW == 16) return sweep_xy_launch_t<AXIS, NU, MSEG, S, 16>(s, g, gd);
+         if constexpr (!kWide)
+            if (s->sw[AXIS].TW == 16) return sweep_xy_launch_t<AXIS, NU, MSEG, S, 16>(s, g, gd);
       }
       return sweep_xy_launch_t<AXIS, NU, MSEG, S, 0>(s, g, gd);
    }
 
-   // 32-point segments exist for FP32 real lines only (register budget)
+   // 32-point segments exist for FP32 real lines only, 16-point ones not for FP64
+   // complex lines, whose tiles are 8 of them at most (sweep_candidates)
    static constexpr bool kSeg32 = std::is_same<R, float>::value && !CPLX;
+   static constexpr bool kWide = std::is_same<R, double>::value && CPLX;
 
    template <int AXIS, bool NU> static gpe_status sweep_xy(gpe_solver *s, double g, double gd) {
       const auto &w = s->sw[AXIS];
       if constexpr (kSeg32)
          if (w.MSEG == 32)
             return w.S == 3 ? sweep_xy_launch<AXIS, NU, 32, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 32, 2>(s, g, gd);
-      if (w.MSEG == 8) return w.S == 3 ? sweep_xy_launch<AXIS, NU, 8, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 8, 2>(s, g, gd);
-      return w.S == 3 ? sweep_xy_launch<AXIS, NU, 16, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 16, 2>(s, g, gd);
+      if (kWide || w.MSEG == 8)
+         return w.S == 3 ? sweep_xy_launch<AXIS, NU, 8, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 8, 2>(s, g, gd);
+      if constexpr (!kWide)
+         return w.S == 3 ? sweep_xy_launch<AXIS, NU, 16, 3>(s, g, gd) : sweep_xy_launch<AXIS, NU, 16, 2>(s, g, gd);
    }
 
    // x sweep; with nu the pending 1/norm and calcnu are applied on load
@@ -346,7 +352,8 @@ template <class R, bool CPLX> struct Impl {
    template <int MOM, int MSEG, int S> static gpe_status sweep_z_launch(gpe_solver *s, double *nrm) {
       if constexpr (std::is_same<R, double>::value) {
          if (s->sw[2].TW == 8) return sweep_z_launch_t<MOM, MSEG, S, 8>(s, nrm);
-         if (s->sw[2].TW == 16) return sweep_z_launch_t<MOM, MSEG, S, 16>(s, nrm);
+         if constexpr (!kWide)
+            if (s->sw[2].TW == 16) return sweep_z_launch_t<MOM, MSEG, S, 16>(s, nrm);
       }
       return sweep_z_launch_t<MOM, MSEG, S, 0>(s, nrm);
    }
@@ -355,8 +362,9 @@ template <class R, bool CPLX> struct Impl {
       const auto &w = s->sw[2];
       if constexpr (kSeg32)
          if (w.MSEG == 32) return w.S == 3 ? sweep_z_launch<MOM, 32, 3>(s, nrm) : sweep_z_launch<MOM, 32, 2>(s, nrm);
-      if (w.MSEG == 8) return w.S == 3 ? sweep_z_launch<MOM, 8, 3>(s, nrm) : sweep_z_launch<MOM, 8, 2>(s, nrm);
-      return w.S == 3 ? sweep_z_launch<MOM, 16, 3>(s, nrm) : sweep_z_launch<MOM, 16, 2>(s, nrm);
+      if (kWide || w.MSEG == 8) return w.S == 3 ? sweep_z_launch<MOM, 8, 3>(s, nrm) : sweep_z_launch<MOM, 8, 2>(s, nrm);
+      if constexpr (!kWide)
+         return w.S == 3 ? sweep_z_launch<MOM, 16, 3>(s, nrm) : sweep_z_launch<MOM, 16, 2>(s, nrm);
    }
 
    // z sweep; mom 1: also the norm of the step (dev_norm may be null) and the

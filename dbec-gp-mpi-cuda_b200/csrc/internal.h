@@ -40,7 +40,6 @@ gpe_status read_muen(gpe_solver *s, double *mu, double *en);
 cudaStream_t stream_of(gpe_solver *s);
 gpe_status params_of(gpe_solver *s, gpe_params *p);
 int device_of(gpe_solver *s);
-long long kernels_per_step(gpe_solver *s);
 // Counts the handle's tile plannings (gpe_set_tuning, gpe_autotune): a batch
 // compares it with the value its descriptors were built for.
 unsigned long long plan_generation(gpe_solver *s);

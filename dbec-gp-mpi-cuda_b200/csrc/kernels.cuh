@@ -1,10 +1,12 @@
 // kernels.cuh -- device kernels of one split step and of the observables.
 //
-// Layouts in HBM (dense, no pitch):
+// Layouts in HBM (z contiguous):
 //   psi   [nx][ny][nz]        R (imaginary time) or complex R (real time)
-//   spec  [nzh][nx][ny]       complex R, nzh = nz/2+1  (plane-major half spectrum)
+//   spec  [nx][ny][nzp]       complex R half spectrum, nzh = nz/2+1 points a row
+//                             (nzp: nzh, padded to even in FP32)
 //   phi   [nx][ny][nz]        R, unnormalised inverse FFT (the reference's psidd2)
-//   udd   [nzh][nx/2+1][ny/2+1] FP64 octant of Udd(k) (depends on kx^2, ky^2, kz^2)
+//   udd   [nx/2+1][ny/2+1][nzh padded to even]  FP64 octant of Udd(k) (depends
+//                             on kx^2, ky^2, kz^2)
 #pragma once
 
 #include "common.cuh"
@@ -26,7 +28,8 @@ struct State {
    double scale2;  // scale * scale, applied to |psi|^2 spectra
    double g, gd;   // couplings of the current step
    double pad[2];
-   unsigned int ticket;  // CTAs of k_norm_final done (back to 0 after each launch)
+   unsigned int ticket;  // CTAs done of the reduction under way: the z sweep's norm,
+                         // k_norm_final or k_rms_final (back to 0 after each launch)
    unsigned int pad_u;
 };
 
@@ -63,6 +66,24 @@ struct LinPhase {
    const void *ex, *ey, *ez;
 };
 
+// Maclaurin series of exp on |t| <= 1/8 through t^10 (first omitted term
+// below 3e-18).
+__device__ __forceinline__ double exp_series10(double t) {
+   constexpr double f2 = 1. / 2, f3 = f2 / 3, f4 = f3 / 4, f5 = f4 / 5, f6 = f5 / 6, f7 = f6 / 7, f8 = f7 / 8,
+                    f9 = f8 / 9, f10 = f9 / 10;
+   double e = f10;
+   e = fma(e, t, f9);
+   e = fma(e, t, f8);
+   e = fma(e, t, f7);
+   e = fma(e, t, f6);
+   e = fma(e, t, f5);
+   e = fma(e, t, f4);
+   e = fma(e, t, f3);
+   e = fma(e, t, f2);
+   e = fma(e, t, 1.);
+   return fma(e, t, 1.);
+}
+
 // exp(t) for the nonlinear part of the step's exponent, which is small in
 // practice: Taylor series on |t| <= 1/8 (through t^10; the first omitted
 // term is below 3e-18) and on |t| <= 0.5 (through t^16; below 2.2e-20
@@ -71,22 +92,10 @@ struct LinPhase {
 // measured 0.667 -> 0.663 ms on B200.
 __device__ __forceinline__ double exp_small(double t) {
    if (fabs(t) > 0.5) return exp(t);
+   if (fabs(t) <= 0.125) return exp_series10(t);
    constexpr double f2 = 1. / 2, f3 = f2 / 3, f4 = f3 / 4, f5 = f4 / 5, f6 = f5 / 6, f7 = f6 / 7, f8 = f7 / 8,
                     f9 = f8 / 9, f10 = f9 / 10, f11 = f10 / 11, f12 = f11 / 12, f13 = f12 / 13, f14 = f13 / 14,
                     f15 = f14 / 15, f16 = f15 / 16;
-   if (fabs(t) <= 0.125) {
-      double e = f10;
-      e = fma(e, t, f9);
-      e = fma(e, t, f8);
-      e = fma(e, t, f7);
-      e = fma(e, t, f6);
-      e = fma(e, t, f5);
-      e = fma(e, t, f4);
-      e = fma(e, t, f3);
-      e = fma(e, t, f2);
-      e = fma(e, t, 1.);
-      return fma(e, t, 1.);
-   }
    double e = f16;
    e = fma(e, t, f15);
    e = fma(e, t, f14);
@@ -106,13 +115,6 @@ __device__ __forceinline__ double exp_small(double t) {
    return fma(e, t, 1.);
 }
 
-// calcnu of one FP64 element with the trap factor lin = exp(-dt V) from the
-// axis tables: the same step as nu_op up to rounding.
-__device__ __forceinline__ double nu_split(double p, double phi, double lin, double g, double gd, double dt,
-                                           double invN) {
-   const double thn = dt * fma(p * p, g, (phi * invN) * gd);
-   return p * (lin * exp_small(-thn));
-}
 // calcnu on one element (imag3d-mpicuda.cu:1759-1783, real3d:1856-1883).
 template <class R>
 __device__ __forceinline__ R nu_op(R p, R phi, R V, R g, R gd, R dt, R invN) {

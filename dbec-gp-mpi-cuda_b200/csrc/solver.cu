@@ -638,8 +638,7 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    CK(cudaMalloc(&s->rowA, sizeof(double) * s->row_cap));
    CK(cudaMalloc(&s->rowB, sizeof(double) * s->row_cap));
    CK(cudaMalloc(&s->tmp, sizeof(double) * std::max<long long>(d.nxy, std::max(d.nx, std::max(d.ny, d.nz))) * 2));
-   s->obs_cap = 64;
-   CK(cudaMalloc(&s->obs, sizeof(double) * s->obs_cap));
+   CK(cudaMalloc(&s->obs, sizeof(double) * 64));
    CK(cudaMalloc(&s->rms_buf, sizeof(double) * 4 * kRmsSlots));
    CK(cudaMalloc(&s->state, sizeof(State)));
    State st0{};
@@ -1328,7 +1327,6 @@ gpe_status params_of(gpe_solver *s, gpe_params *p) {
    return GPE_OK;
 }
 int device_of(gpe_solver *s) { return s->dev; }
-long long kernels_per_step(gpe_solver *) { return 8; }
 unsigned long long plan_generation(gpe_solver *s) { return s->plan_gen; }
 gpe_status tuning_as_set(gpe_solver *s, gpe_tuning *t) {
    CHECK_HANDLE(s);

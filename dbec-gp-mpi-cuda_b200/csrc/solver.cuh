@@ -84,7 +84,6 @@ struct gpe_solver {
    std::vector<double> hx, hy, hz, hx2, hy2, hz2;
    std::vector<unsigned char> nu_x;  // calcnu's table along x as the sweeps hold it
    long long launches = 0;
-   size_t obs_cap = 0;
    // sweep configuration per axis (x, y: TMA tensor tiles; z: bulk rows)
    struct Sweep {
       int TW = 8, MSEG = 8, boxn = 0, nbox = 1, LS = 0, S = 2, ctas = 1;

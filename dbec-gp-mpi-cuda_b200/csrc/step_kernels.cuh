@@ -22,28 +22,22 @@ namespace gpe {
 // interleaved layout the FFT engine works in.
 // ===========================================================================
 
-// L: lines per tile of the z passes (128-byte rows); PPT: points per thread
-// of the y and x passes, whose tile width the host picks so that a tile of a
-// whole line holds at most 256 PPT points (32 KB).
+// Points per thread of the y and x passes, whose tile width (kz columns) the host
+// picks so that a tile of a whole line holds at most 256 PPT points (32 KB).
 template <class R> struct FftL {
-   static constexpr int L = 128 / (2 * (int) sizeof(R));
    static constexpr int PPT = sizeof(R) == 8 ? 8 : 16;
 };
 
-// Preferred rows per CTA of the z passes.  Forward: 16 over complex FP32
-// rows, so that the radix-8 stages (nz/2-point lines) keep all 256 threads
-// busy; 8 over complex FP64 rows (4 KB each), which measured faster with four
-// CTAs per SM; 8 over real rows on a CTA sized to them (128 threads at nz =
-// 256; 512x512x256 FP32 280 -> 238 us, 256^3 FP64 93 -> 87 us), where the
-// host keeps 16 rows on 256 threads for FP64 rows shorter than 128 points.
-// Inverse: 8 rows on a CTA sized to them (128 threads at nz = 256), six
-// per SM, measured faster than 16 rows on 256 threads (256^3 FP64 82 -> 78
-// us, 512x512x256 FP32 238 -> 210 us).  The host halves the rows while the
-// tile does not fit shared memory.
-template <class R, bool CPLX> struct ZRows {
-   static constexpr int fwd = (sizeof(R) == 4 && CPLX) ? 16 : 8;
-   static constexpr int inv = 8;
-};
+// Preferred rows per CTA of the forward z pass: 16 over complex FP32 rows, so
+// that the radix-8 stages (nz/2-point lines) keep all 256 threads busy; 8 over
+// complex FP64 rows (4 KB each), which measured faster with four CTAs per SM; 8
+// over real rows on a CTA sized to them (128 threads at nz = 256; 512x512x256
+// FP32 280 -> 238 us, 256^3 FP64 93 -> 87 us), where the host keeps 16 rows on
+// 256 threads for FP64 rows shorter than 128 points.  The inverse pass takes 8
+// rows on a CTA sized to them, six per SM (256^3 FP64 82 -> 78 us, 512x512x256
+// FP32 238 -> 210 us).  The host halves the rows while the tile does not fit
+// shared memory.
+template <class R, bool CPLX> constexpr int zfwd_rows() { return sizeof(R) == 4 && CPLX ? 16 : 8; }
 
 // Tables of roots: a y line has n stage roots (padded to n entries), an x line
 // n forward and n inverse ones (one set where the plan reads the same both

@@ -334,6 +334,18 @@ __device__ __forceinline__ void seg_sweep_any(typename Tr<R, CPLX>::P *line, int
    seg_sweep<R, CPLX, 8, ROW, STAB, SIMP>(line, es, p, tb, xch, xs, xf, w1t, w2t, simp, simp2);
 }
 
+// (cos t, -sin t) on |t| <= 1/32: sin through t^7, cos through t^6 (omitted
+// terms below 3e-18 relative to sin and 3e-17 to cos).
+__device__ __forceinline__ double2 expi_series7(double t) {
+   constexpr double s3 = 1. / 6, s5 = s3 / 20, s7 = s5 / 42, c2 = 1. / 2, c4 = c2 / 12, c6 = c4 / 30;
+   const double t2 = t * t;
+   double sq = fma(-s7, t2, s5);
+   sq = fma(sq, t2, -s3);
+   double cq = fma(-c6, t2, c4);
+   cq = fma(cq, t2, -c2);
+   return make_double2(fma(cq, t2, 1.), -fma(sq * t2, t, t));
+}
+
 // exp(-i t) = (cos t, -sin t) for the nonlinear part of the real-time phase,
 // which is small in practice: Maclaurin series on |t| <= 1/32 (through t^7
 // for sin and t^6 for cos; the first omitted terms are below 3e-18 relative
@@ -347,18 +359,10 @@ __device__ __forceinline__ double2 expi_small(double t) {
       sincos(-t, &sn, &cs);
       return make_double2(cs, sn);
    }
+   if (fabs(t) <= 0.03125) return expi_series7(t);
    constexpr double s3 = 1. / 6, s5 = s3 / 20, s7 = s5 / 42, s9 = s7 / 72, s11 = s9 / 110;
    constexpr double c2 = 1. / 2, c4 = c2 / 12, c6 = c4 / 30, c8 = c6 / 56, c10 = c8 / 90, c12 = c10 / 132;
    const double t2 = t * t;
-   if (fabs(t) <= 0.03125) {
-      double sq = fma(-s7, t2, s5);
-      sq = fma(sq, t2, -s3);
-      const double sn = fma(sq * t2, t, t);
-      double cq = fma(-c6, t2, c4);
-      cq = fma(cq, t2, -c2);
-      const double cs = fma(cq, t2, 1.);
-      return make_double2(cs, -sn);
-   }
    double sp = fma(-s11, t2, s9);
    sp = fma(sp, t2, -s7);
    sp = fma(sp, t2, s5);
@@ -386,36 +390,6 @@ __device__ __forceinline__ double2 expi_small(double t) {
 // point) and reloads them.  Transforming the tile in a pass of its own took
 // 82 instructions per FP64 point in imaginary time, mostly indexing and the
 // second trip through shared memory.
-
-// Maclaurin series of exp on |t| <= 1/8 through t^10 (first omitted term
-// below 3e-18).
-__device__ __forceinline__ double exp_series10(double t) {
-   constexpr double f2 = 1. / 2, f3 = f2 / 3, f4 = f3 / 4, f5 = f4 / 5, f6 = f5 / 6, f7 = f6 / 7, f8 = f7 / 8,
-                    f9 = f8 / 9, f10 = f9 / 10;
-   double e = f10;
-   e = fma(e, t, f9);
-   e = fma(e, t, f8);
-   e = fma(e, t, f7);
-   e = fma(e, t, f6);
-   e = fma(e, t, f5);
-   e = fma(e, t, f4);
-   e = fma(e, t, f3);
-   e = fma(e, t, f2);
-   e = fma(e, t, 1.);
-   return fma(e, t, 1.);
-}
-
-// (cos t, -sin t) on |t| <= 1/32: sin through t^7, cos through t^6 (omitted
-// terms below 3e-18 relative to sin and 3e-17 to cos).
-__device__ __forceinline__ double2 expi_series7(double t) {
-   constexpr double s3 = 1. / 6, s5 = s3 / 20, s7 = s5 / 42, c2 = 1. / 2, c4 = c2 / 12, c6 = c4 / 30;
-   const double t2 = t * t;
-   double sq = fma(-s7, t2, s5);
-   sq = fma(sq, t2, -s3);
-   double cq = fma(-c6, t2, c4);
-   cq = fma(cq, t2, -c2);
-   return make_double2(fma(cq, t2, 1.), -fma(sq * t2, t, t));
-}
 
 // (cos t, -sin t) in FP32 on |t| <= 256: t is reduced by the nearest multiple
 // of pi / 2 in two steps (Cody and Waite), then Maclaurin series on |r| <= pi/4

@@ -49,6 +49,25 @@ def test_sweeps_at_segment_edges(gpe_lib, oracle_mod, mode, prec, n, dtf):
     o.close()
 
 
+# Time steps whose carries reach all segments of a line (D = P): c = dt / (2 dx^2)
+# is 100.  The FP64 bar stands.  In FP32 the right-hand side psi + A t has terms of
+# 4c times psi, each rounded at 2^-24.  In imaginary time the inverse that follows
+# is bounded by 1; in real time each of the two recurrences passes such a rounding
+# on over about sqrt(c) points before it has decayed.
+@pytest.mark.parametrize("mode,prec,tol", [(0, 0, 1e-12), (1, 0, 1e-12), (0, 1, 2 ** -24 * 400), (1, 1, 2 ** -24 * 400 * 2 * 10)])
+@pytest.mark.parametrize("n", [(96, 128, 80), (250, 36, 64), (18, 300, 24)])
+def test_sweeps_at_large_time_steps(gpe_lib, oracle_mod, mode, prec, tol, n):
+    s, o, psi = pair(gpe_lib, oracle_mod, mode, prec, n, 200.)
+    for name in ("calclux", "calcluy", "calcluz"):
+        s.set_psi(psi)
+        o.set_psi(psi)
+        getattr(s, name)()
+        getattr(o, name)()
+        assert rel(s.get_psi(), o.get_psi()) <= tol, name
+    s.close()
+    o.close()
+
+
 @pytest.mark.parametrize("prec,tw,n", [(0, 4, (18, 10, 48)), (1, 4, (18, 10, 48)), (0, 2, (10, 18, 12)),
                                        (1, 8, (20, 12, 20))])
 def test_narrow_tiles_keep_copies_aligned(gpe_lib, oracle_mod, prec, tw, n):
@@ -138,11 +157,22 @@ Z_HALVES = (8, 9, 10, 12, 15, 16, 18, 20, 25, 27, 30, 36, 40, 45, 50, 54, 60, 72
 @pytest.mark.parametrize("axis,n", [(0, n) for n in XY_LENGTHS] + [(1, n) for n in XY_LENGTHS] +
                          [(2, 2 * h) for h in Z_HALVES])
 def test_convolution_compiled_lengths(gpe_lib, oracle_mod, prec, axis, n):
+    check_compiled_length(gpe_lib, oracle_mod, 0, prec, axis, n)
+
+
+# the forward z pass over complex rows: kernels of its own, other row strides
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("n", [2 * h for h in Z_HALVES])
+def test_convolution_compiled_lengths_of_complex_rows(gpe_lib, oracle_mod, prec, n):
+    check_compiled_length(gpe_lib, oracle_mod, 1, prec, 2, n)
+
+
+def check_compiled_length(gpe_lib, oracle_mod, mode, prec, axis, n):
     if prec and axis == 2 and n % 4:
         pytest.skip("mixed precision takes rows of a multiple of 4 points")
     shape = [10, 12, 8]
     shape[axis] = n
-    s, o, psi = pair(gpe_lib, oracle_mod, 0, prec, tuple(shape))
+    s, o, psi = pair(gpe_lib, oracle_mod, mode, prec, tuple(shape))
     s.calcpsidd2()
     o.calcpsidd2()
     phi = s.get_phi()
