@@ -77,7 +77,6 @@ void refresh(gpe_batch *b) {
       }
 }
 
-constexpr size_t kSmemCap = 227 * 1024;
 constexpr size_t kSweepStatic = 1152;  // views, tile records and barriers of a sweep kernel, rounded up
 static_assert(2 * sizeof(SweepView) + 8 * sizeof(SweepTile) + 2 * sizeof(State) + 64 <= kSweepStatic, "static bytes of a sweep");
 
@@ -154,9 +153,9 @@ gpe_status build_tables(gpe_batch *b) {
       for (int a = 0; a < 3; a++) {
          size_t sm = 128 + 2 * (size_t) A.stage[a] + A.xch[a];
          if (a == 2) sm += 2 * (size_t) A.part;
-         G.nbuf[a] = sm + 2 * (size_t) A.tabs[a] <= kSmemCap - kSweepStatic ? 2 : 1;
+         G.nbuf[a] = sm + 2 * (size_t) A.tabs[a] <= kMaxSmem ? 2 : 1;
          sm += (size_t) G.nbuf[a] * A.tabs[a];
-         if (sm > kSmemCap - kSweepStatic) return bfail(GPE_ERR_PARAM, "batch: sweep tiles exceed shared memory");
+         if (sm > kMaxSmem) return bfail(GPE_ERR_PARAM, "batch: sweep tiles exceed shared memory");
          // the kernels' register budget holds cap0 CTAs of 256 threads,
          // so more of fewer threads
          const int cap0 = kb_sweep_ctas(G.fp32, G.cplx, A.mseg[a] <= 8 ? 8 : (A.mseg[a] <= 16 ? 16 : 32), a == 0);

@@ -28,7 +28,7 @@ struct Group {
    SweepTile *dtile[3] = {nullptr, nullptr, nullptr};  // device tile records of the sweeps
    int sweep_grid[3] = {0, 0, 0};
    size_t sweep_smem[3] = {0, 0, 0};
-   mutable RoomyKernels roomy;  // launched with dynamic shared memory
+   mutable RoomyKernels roomy;  // launched with more dynamic shared memory than the default
    int nbuf[3] = {2, 2, 2};  // table buffers of the sweeps (one where two do not fit: long complex lines)
 };
 

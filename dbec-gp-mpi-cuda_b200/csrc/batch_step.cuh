@@ -6,7 +6,7 @@
 template <class K, class... A>
 gpe_status launch(const Group &G, K kern, unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
    if (grid == 0) return GPE_OK;
-   if (smem > 0) BCK(G.roomy.allow((const void *) kern));
+   BCK(G.roomy.allow((const void *) kern, smem));
    kern<<<grid, block, smem, st>>>(args...);
    BCK(cudaGetLastError());
    return GPE_OK;

@@ -26,7 +26,7 @@ inline unsigned blocks_for(long long n, int bs) { return (unsigned) ((n + bs - 1
 // 0.107 -> 0.103 ms at 128^3, 512x512x256 unchanged at 1.69 ms, on B200).
 template <class... KP, class... A>
 gpe_status launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, const gpe_solver *s, A... args) {
-   if (smem > 0) CK(s->roomy.allow((const void *) k));
+   CK(s->roomy.allow((const void *) k, smem));
    cudaLaunchAttribute at[1];
    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
    at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -170,7 +170,7 @@ template <class R> struct Conv {
    }
    template <class SM> static int zrows(const gpe_solver *s, int pref, SM smem) {
       int L = pref;
-      while (L > 4 && smem(s, L) > 227 * 1024) L /= 2;
+      while (L > 4 && smem(s, L) > kMaxSmem) L /= 2;
       return L;
    }
    template <class F> static gpe_status with_zrows(int L, F f) {
@@ -503,7 +503,7 @@ template <class R, bool CPLX> struct Impl {
       const long ry = (long) s->boxy * s->nboxy, rx = (long) s->boxx * s->nboxx;
       g->smem[kPZfwd] = CV::len_z(s) ? zfwd_n_smem(s) : zfwd_smem(s, L);
       g->smem[kPZinv] = CV::len_z(s) ? CV::zinv_n_smem(s) : CV::zinv_smem(s, L);
-      if (g->smem[kPZfwd] > 227 * 1024 || g->smem[kPZinv] > 227 * 1024)
+      if (g->smem[kPZfwd] > kMaxSmem || g->smem[kPZinv] > kMaxSmem)
          return fail(GPE_ERR_PARAM, "batch: z rows too long for 8-row tiles");
       // an instance with a compile-time pass keeps that pass's tile width
       Ly = CV::len_y(s) ? CV::kCols : Ly;

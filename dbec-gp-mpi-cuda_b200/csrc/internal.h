@@ -13,16 +13,20 @@ namespace gpe {
 
 void set_last_error(const std::string &msg);
 
-// Kernels allowed the device's whole shared memory (less what they hold
-// statically) as dynamic shared memory.  The limit belongs to the kernel, not to
-// a handle: handles of other sizes on other threads share it, so it is always
-// set to that maximum and never to the bytes of one launch, which would take
-// room away from another thread between its own call and its launch.  Each
-// handle and batch group remembers the kernels it has passed (a few dozen) and
-// belongs to one thread at a time.
+// Dynamic shared memory of a launch at most: the 227 KB a CTA can have less 2 for
+// the kernels' static bytes (at most 1152).
+constexpr size_t kMaxSmem = 225 * 1024;
+
+// Kernels allowed as much dynamic shared memory as the device has for a CTA.  The
+// limit belongs to the kernel, not to a handle: handles of other sizes on other
+// threads share it, so it is always set to kMaxSmem (the largest launch takes 213 KB) and
+// never to the bytes of one launch, which would take room away from another thread
+// between its own call and its launch.  A launch of up to 46 KB fits the default
+// limit and needs nothing.  Each handle and batch group remembers the kernels it
+// has passed (a few dozen) and belongs to one thread at a time.
 class RoomyKernels {
  public:
-   cudaError_t allow(const void *kernel);
+   cudaError_t allow(const void *kernel, size_t bytes);
 
  private:
    std::vector<const void *> done_;

@@ -29,16 +29,12 @@ static thread_local std::string g_err;
 namespace gpe {
 void set_last_error(const std::string &msg) { g_err = msg; }
 
-cudaError_t RoomyKernels::allow(const void *kernel) {
+cudaError_t RoomyKernels::allow(const void *kernel, size_t bytes) {
+   if (bytes <= 46 * 1024) return cudaSuccess;
+   if (bytes > kMaxSmem) return cudaErrorInvalidValue;
    for (const void *k : done_)
       if (k == kernel) return cudaSuccess;
-   int dev = 0, most = 0;
-   cudaFuncAttributes a{};
-   cudaError_t e = cudaGetDevice(&dev);
-   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
-   if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int) a.sharedSizeBytes);
+   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kMaxSmem);
    if (e == cudaSuccess) done_.push_back(kernel);
    return e;
 }
@@ -455,7 +451,7 @@ static gpe_status plan_tiles(gpe_solver *s) {
       const size_t l1 = ax == 2 && !s->fp32 ? 0 : 4 * (size_t) P * w.MSEG * esz;
       auto stages_fit = [&](int ct, int S) {
          const size_t b = fixed + S * stage;
-         if (b + kSweepFixed > sm_cap || smem_ctas(b, kSweepFixed) < ct) return false;
+         if (b > kMaxSmem || smem_ctas(b, kSweepFixed) < ct) return false;
          return S == s_lo || ct * (b + kSweepFixed + kCtaReserved) + l1 <= kSmSmem;
       };
       w.ctas = 0;

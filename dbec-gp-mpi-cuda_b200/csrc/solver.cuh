@@ -98,7 +98,7 @@ struct gpe_solver {
    double *wz2 = nullptr;     // wz[k] * z[k]^2 (rms partials)
    int nsm = 148;             // streaming multiprocessors of the device
    uint32_t *err = nullptr;   // device status word (bounded waits)
-   mutable RoomyKernels roomy;  // launched with dynamic shared memory
+   mutable RoomyKernels roomy;  // launched with more dynamic shared memory than the default
    // per-kernel profiling: when prof_ev is set, mark() records an event
    // after every kernel of a step
    cudaEvent_t *prof_ev = nullptr;

@@ -67,11 +67,6 @@ err_t cudaFuncSetAttribute(const void *f, int a, int v) {
    attr[k].dyn = v;
    return OK;
 }
-err_t cudaFuncGetAttributes(void *out, const void *f) { /* sharedSizeBytes comes first */
-   memset(out, 0, 64);
-   *(size_t *) out = (size_t) attr[at(f)].fixed;
-   return OK;
-}
 static err_t launch(const void *f, dim g, dim b, size_t smem, stream *s) {
    if (!g.x || !g.y || !g.z || !b.x || b.x * b.y * b.z > 1024 || smem > (size_t) attr[at(f)].dyn) return last = INVALID;
    if (pending && s && (s->flags & 1)) unordered++;
