@@ -39,6 +39,10 @@ constexpr int kLenPpt = 16;
 // only (above 256 a line is two boxes of 64-byte rows, so a multiple of 4).  The
 // latter keep the radices of the run-time passes (16 in FP32, 8 in FP64), so a
 // batch, which transforms them at run time, gives the same values bit for bit.
+// The common set is the lines and half rows of sides of 48, 64, 96, 128, 256 and
+// 512 points.  A batched kernel holds the code of all its lengths (a tile's
+// instance is known at run time only), and in FP64 their 16 points a thread cost
+// the run-time pass beside them half its warps (kb_fft_ctas), so the set is short.
 // A whole step, their lengths at run time -> compiled, us: 128x96x80 FP64 70 ->
 // 64, 90x100x72 FP64 complex 80 -> 72, 160x144x120 FP32 complex 120 -> 93.
 #define GPE_LENS(X) X(24) X(32) X(48) X(64) X(96) X(128) X(256) X(512)

@@ -210,7 +210,7 @@ gpe_status gpe_batch_create(const gpe_params *params, const double *g, const dou
 void gpe_batch_destroy(gpe_batch *b);
 /* The handle of instance i (owned by the batch): initial state, observables. */
 gpe_status gpe_batch_solver(gpe_batch *b, int i, gpe_solver **s);
-/* New couplings for every instance (the step graph is captured again). */
+/* New couplings for every instance (the captured step stays valid). */
 gpe_status gpe_batch_set_couplings(gpe_batch *b, const double *g, const double *gd);
 /* Autotunes one instance per distinct (grid, mode, precision) with
  * gpe_autotune (nsteps per trial) and applies its choice to the others, then
@@ -237,9 +237,9 @@ gpe_status gpe_batch_launch_count(gpe_batch *b, long long *count);
  * Request server with continuous batching (no reference counterpart).  A
  * worker thread admits queued requests while the summed gpe_device_bytes of
  * the active solves stays within the HBM budget and fewer than max_active are
- * running, keeps each psi resident on the device, runs all active solves
- * concurrently in chunks (each on its own stream), and retires a solve when it
- * has converged (ground state) or done its steps (evolution); requests that
+ * running, keeps each psi resident on the device, steps the active solves in
+ * chunks (those of one size class, mode and precision together, as a batch, on a
+ * stream of their own), and retires a solve when it has converged (ground state) or done its steps (evolution); requests that
  * arrive meanwhile are admitted at the next chunk boundary. */
 typedef struct gpe_server gpe_server;
 enum { GPE_REQ_GROUND = 0, GPE_REQ_EVOLVE = 1 };
