@@ -711,7 +711,8 @@ static gpe_status create_impl(const gpe_params *p, void *stream, gpe_solver *s) 
    CKS(plan_tiles(s));
    CKS(setup_static(s));
 
-   CK(cudaDeviceSynchronize());
+   // (the stream, not the device: another thread may be capturing a batch step)
+   CK(cudaStreamSynchronize(s->st));
    return GPE_OK;
 }
 

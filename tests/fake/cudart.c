@@ -8,6 +8,8 @@
  *                          fill on the legacy stream that nothing waited for
  *                          (such a copy from pageable memory may return before
  *                          its data has arrived)
+ *   fake_device_syncs      waits for the whole device, which fail, and spoil the
+ *                          capture, while another thread captures a stream
  *   fake_lowered           cudaFuncSetAttribute calls that took dynamic shared
  *                          memory away from a kernel
  *   fake_surplus           launches of a sweep, whose CTAs walk over the tiles,
@@ -24,7 +26,7 @@ enum { OK = 0, INVALID = 1, OOM = 2 };
 typedef struct { unsigned x, y, z; } dim;
 typedef struct { int flags; } stream;
 
-static long long live, launches, unordered, lowered, surplus;
+static long long live, launches, unordered, lowered, surplus, device_syncs;
 static int failing, pending;
 static __thread err_t last;
 
@@ -33,6 +35,7 @@ long long fake_launches(void) { return launches; }
 long long fake_unordered(void) { return unordered; }
 long long fake_lowered(void) { return lowered; }
 long long fake_surplus(void) { return surplus; }
+long long fake_device_syncs(void) { return device_syncs; }
 void fake_fail_mallocs(int on) { failing = on; }
 
 /* ---- kernels: dynamic shared memory up to 48 KB less the static bytes unless
@@ -144,7 +147,7 @@ err_t cudaEventRecord(void *e, stream *s) { (void) e; (void) s; return OK; }
 err_t cudaEventSynchronize(void *e) { (void) e; return OK; }
 err_t cudaEventQuery(void *e) { (void) e; return OK; }
 err_t cudaEventElapsedTime(float *ms, void *a, void *b) { (void) a; (void) b; *ms = 1.f; return OK; }
-err_t cudaDeviceSynchronize(void) { pending = 0; return OK; }
+err_t cudaDeviceSynchronize(void) { pending = 0; device_syncs++; return OK; }
 err_t cudaSetDevice(int d) { return d == 0 ? OK : 101; }
 err_t cudaGetDevice(int *d) { *d = 0; return OK; }
 err_t cudaDeviceGetAttribute(int *v, int a, int d) {

@@ -8,6 +8,7 @@
   reads stale data there) exits with an error and says why.
 * Handles of different sizes on threads of their own share kernels: no thread's
   launch fails for what another one asked of them.
+* Handles come and go on one thread while another captures batch steps.
 * A cancelled request: a queued one finishes at once, an admitted one stops
   at its next chunk boundary, both with GPE_ERR_CANCELLED; the server then
   serves the next request normally.
@@ -111,3 +112,37 @@ def test_handles_of_two_threads_share_kernels(gpe_lib):
     for a, b in zip(alone, both):
         assert not isinstance(b[0], gpe.GpeError), b[0]
         assert np.array_equal(a[0], b[0])
+
+
+def test_handles_come_and_go_while_a_batch_is_captured(gpe_lib):
+    import threading
+
+    gpe = gpe_lib
+    p = gpe.make_params(0, 16, 16, 16, .25, .25, .25, .00625, .5, 1., 1.5, 2.)
+    done, errors, psi = threading.Event(), [], []
+
+    def handles():
+        try:
+            while not done.is_set():
+                with gpe.Solver(p) as s:
+                    s.init_gaussian()
+                    s.run(2, 20., 5.)
+                    psi.append(s.get_psi())
+        except gpe.GpeError as e:
+            errors.append(e)
+
+    t = threading.Thread(target=handles)
+    t.start()
+    try:
+        for _ in range(30):  # a capture each
+            b = gpe.Batch([p] * 3, [20.] * 3, [5.] * 3)
+            for i in range(3):
+                b.solver(i).init_gaussian()
+            b.run(2)
+            psi.append(b.solver(2).get_psi())
+            b.close()
+    finally:
+        done.set()
+        t.join()
+    assert not errors, errors
+    assert all(np.array_equal(f, psi[0]) for f in psi)

@@ -18,7 +18,7 @@ import ctypes, sys
 sys.path.insert(0, %r)
 import gpe
 fake = ctypes.CDLL(%r)
-for f in ("live_bytes", "launches", "unordered", "lowered", "surplus"):
+for f in ("live_bytes", "launches", "unordered", "lowered", "surplus", "device_syncs"):
     getattr(fake, "fake_" + f).restype = ctypes.c_longlong
 lengths = [n for n in range(8, 1025, 2) if 2 ** 10 * 3 ** 6 * 5 ** 4 %% n == 0]  # the sides a handle takes
 def params(mode, n, prec=0):
@@ -151,3 +151,21 @@ for n in (30, 60, 64, 72, 80, 96, 120, 128, 144, 180, 256, 320, 400, 500, 512, 5
         b.close()
         assert fake.fake_surplus() == 0, shape
 """ % dict(m=mode, p=prec))
+
+
+def test_no_call_waits_for_the_whole_device(fake):
+    """Another thread may be capturing a batch step (the server's does): a wait for
+    the device fails then and spoils the capture."""
+    fake("""
+for m in (0, 1):
+    for p in (0, 1):
+        s = gpe.Solver(params(m, (16, 12, 8), p))
+        s.init_gaussian()
+        s.run(2, 50., 10., rms_every=1)
+        s.set_tuning(None)
+        s.close()
+b = gpe.Batch([params(0, (16, 12, 8))] * 2, [1., 2.], [0., 0.])
+b.run(2)
+b.close()
+assert fake.fake_device_syncs() == 0
+""")
