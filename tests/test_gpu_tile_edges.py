@@ -157,22 +157,29 @@ Z_HALVES = (8, 9, 10, 12, 15, 16, 18, 20, 25, 27, 30, 36, 40, 45, 50, 54, 60, 72
 @pytest.mark.parametrize("axis,n", [(0, n) for n in XY_LENGTHS] + [(1, n) for n in XY_LENGTHS] +
                          [(2, 2 * h) for h in Z_HALVES])
 def test_convolution_compiled_lengths(gpe_lib, oracle_mod, prec, axis, n):
-    check_compiled_length(gpe_lib, oracle_mod, 0, prec, axis, n)
-
-
-# the forward z pass over complex rows: kernels of its own, other row strides
-@pytest.mark.parametrize("prec", [0, 1])
-@pytest.mark.parametrize("n", [2 * h for h in Z_HALVES])
-def test_convolution_compiled_lengths_of_complex_rows(gpe_lib, oracle_mod, prec, n):
-    check_compiled_length(gpe_lib, oracle_mod, 1, prec, 2, n)
-
-
-def check_compiled_length(gpe_lib, oracle_mod, mode, prec, axis, n):
     if prec and axis == 2 and n % 4:
         pytest.skip("mixed precision takes rows of a multiple of 4 points")
     shape = [10, 12, 8]
     shape[axis] = n
-    s, o, psi = pair(gpe_lib, oracle_mod, mode, prec, tuple(shape))
+    s, o, psi = pair(gpe_lib, oracle_mod, 0, prec, tuple(shape))
+    s.calcpsidd2()
+    o.calcpsidd2()
+    phi = s.get_phi()
+    assert rel(phi, o.get_phi()) <= TOL[prec]
+    t = gpe_lib.Tuning()
+    t.fft_max_radix = 4
+    s.set_tuning(t)
+    s.set_psi(psi)
+    s.calcpsidd2()
+    assert rel(phi, s.get_phi()) <= TOL[prec]
+    s.close()
+    o.close()
+
+
+# The forward z pass over complex rows: kernels of its own, with other row strides.
+@pytest.mark.parametrize("prec,n", [(p, 2 * h) for p in (0, 1) for h in Z_HALVES if not (p and h % 2)])
+def test_convolution_compiled_lengths_of_complex_rows(gpe_lib, oracle_mod, prec, n):
+    s, o, psi = pair(gpe_lib, oracle_mod, 1, prec, (10, 12, n))
     s.calcpsidd2()
     o.calcpsidd2()
     phi = s.get_phi()
